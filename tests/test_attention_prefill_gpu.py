@@ -1,0 +1,95 @@
+"""The tcgen05 prompt kernel over every way its query tiles are paired and every option, against float64: runs around the
+tiles' edges (64, 128, 256 rows), sequences that hold earlier positions, grouped and ungrouped heads, windows with kept
+positions, cells, caps (scores on both sides of a quarter of the cap), distance biases, sinks."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def attend(q, k, v, first, scale, window, keep, cell, cap, bias, sink):
+    """float64: (output, sum of weight * |value|) for queries q [n, H, dk] at positions first, …"""
+    n, H, m = q.shape[0], q.shape[1], k.shape[0]
+    i, j = torch.arange(first, first + n, device=q.device)[:, None], torch.arange(m, device=q.device)[None]
+    see = j <= i
+    if cell:
+        see = see & (i // cell == j // cell)
+    elif window:
+        see = see & ((i - j < window) | (j < keep))
+    o, mag = (torch.empty((n, H, v.shape[2]), dtype=torch.float64, device=q.device) for _ in range(2))
+    for h in range(H):
+        g = h * k.shape[1] // H
+        s = q[:, h] @ k[:, g].t() * scale
+        if cap:
+            s = cap * torch.tanh(s / cap)
+        if bias is not None:
+            s = s + bias[h][torch.clamp(i - j, 0, bias.shape[1] - 1)]
+        s = s.masked_fill(~see, -float("inf"))
+        if sink is not None:
+            p = torch.softmax(torch.cat([s, sink[h].expand(n, 1)], 1), 1)[:, :-1]
+        else:
+            p = torch.softmax(s, 1)
+        o[:, h], mag[:, h] = p @ v[:, g], p @ v[:, g].abs()
+    return o, mag
+
+
+CASES = [  # H, G, dk, dv, planes, runs, held, window, keep, cell, cap, bias rows, sink
+    (16, 16, 128, 128, 2, [1, 128, 129, 300], [0, 0, 0, 0], 0, 0, 0, 0.0, 0, False),
+    (4, 4, 64, 64, 2, [257], [100], 0, 0, 0, 0.0, 0, False),
+    (4, 2, 64, 64, 2, [65, 640], [0, 63], 200, 0, 0, 0.0, 0, False),
+    (16, 2, 128, 128, 1, [700, 900, 512, 2, 640, 700], [0, 0, 0, 0, 0, 40], 0, 0, 0, 0.0, 0, True),      # head pairs
+    (16, 2, 128, 128, 1, [1100, 900, 512, 60, 640, 700], [0, 7, 0, 0, 0, 40], 0, 0, 0, 30.0, 0, False),  # head pairs, capped
+    (6, 2, 128, 64, 1, [200, 17], [500, 0], 0, 0, 0, 0.0, 0, True),
+    (8, 2, 128, 128, 1, [500, 33], [0, 700], 256, 4, 0, 0.0, 700, True),
+    (3, 1, 64, 128, 1, [383, 64], [0, 300], 100, 70, 0, 0.0, 90, False),
+    (4, 2, 64, 128, 1, [400, 129], [11, 0], 0, 0, 96, 0.0, 0, False),
+    (4, 2, 64, 128, 1, [300], [190], 0, 0, 64, 20.0, 50, True),
+    (2, 1, 128, 128, 1, [640], [0], 128, 0, 0, 4.0, 0, True),
+]
+
+
+@pytest.mark.parametrize("case", range(len(CASES)))
+@pytest.mark.parametrize("spread", [1.0, 6.0])       # 6: maxima grow by more than the rescaling threshold, scores pass the cap
+def test_prompt_kernel(case, spread):
+    from turboquant_cpp_b200.kernels import attention as KA
+    from turboquant_cpp_b200.kernels.gemm_tc import check_status
+    H, G, dk, dv, planes, runs, held, window, keep, cell, cap, rows, with_sink = CASES[case]
+    g = torch.Generator(device=DEV).manual_seed(case * 31 + int(spread))
+    rand = lambda *shape: torch.randn(shape, generator=g, device=DEV)
+    bias = rand(H, rows) if rows else None
+    sink = 2.0 * rand(H) if with_sink else None
+    total = [n + h for n, h in zip(runs, held)]
+    counts = [-(-t // 64) for t in total]
+    order = torch.randperm(sum(counts), generator=torch.Generator().manual_seed(case)).split(counts)
+    cache = torch.zeros((sum(counts), planes, G, 64, dk if planes == 2 else dk + dv), dtype=torch.bfloat16, device=DEV)
+    table = torch.full((len(runs), max(counts)), -1, dtype=torch.int32)
+    q = (spread * rand(sum(runs), H, dk)).to(torch.bfloat16)
+    kv = []
+    for i, t in enumerate(total):
+        k, v = rand(t, G, dk).to(torch.bfloat16), rand(t, G, dv).to(torch.bfloat16)
+        kv.append((k, v))
+        table[i, :counts[i]] = order[i].to(torch.int32)
+        at = torch.arange(t, device=DEV)
+        page = order[i].to(DEV)[at // 64]
+        if planes == 2:
+            cache[page, 0, :, at % 64], cache[page, 1, :, at % 64] = k, v
+        else:
+            cache[page, 0, :, at % 64] = torch.cat([k, v], -1)
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device=DEV)
+    out = torch.empty((sum(runs), H * dv), dtype=torch.bfloat16, device=DEV)
+    scale = dk ** -0.5
+    KA.prefill_rows(q, cache, planes, i32(np.concatenate([[0], np.cumsum(runs)])), i32(held), table.to(DEV), 64, window, scale, out,
+                    len(runs), max(runs), H, G, dk, dv, keep_first=keep, cell=cell, softcap=cap, bias_t=bias, sink=sink)
+    check_status()
+    at = 0
+    for (k, v), n, first in zip(kv, runs, held):
+        got = out[at:at + n].view(n, H, dv).double()
+        want, mag = attend(q[at:at + n].double(), k.double(), v.double(), first, scale, window, keep, cell, cap,
+                           None if bias is None else bias.double(), None if sink is None else sink.double())
+        at += n
+        # weights rounded to bfloat16 (eight significant bits: at most 2^-8 of each; their sum is taken before), the output
+        # too (2^-8 of it); the float32 scores, |s| up to about 40, add 2^-16 of relative weight
+        bound = (2.0 ** -8 + 2.0 ** -16) * mag + 2.0 ** -8 * want.abs() + 1e-6
+        assert bool(((got - want).abs() <= bound).all()), float(((got - want).abs() / bound).max())

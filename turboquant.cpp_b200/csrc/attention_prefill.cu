@@ -1,28 +1,30 @@
 // Causal attention for prompts on the 5th-generation tensor cores: S = Q K^T and O = P V as
 // tcgen05.mma with the accumulators in tensor memory, Q/K/V tiles brought in by TMA straight from
-// the query buffer and the paged key/value cache, online softmax in fp32 registers.
+// the query buffer and the paged cache, online softmax in fp32 registers.
 //
-// Same mathematics as the exact kernel (csrc/attention.cu) and as the reference's per-token loop
-// (src/engine/tq_transformer.c:1909-1936 scores with scale 1/sqrt(hd), :1960 softmax, :2183-2191
+// Same mathematics as the exact kernels (csrc/attention.cu, csrc/bias_attention.cu) and as the reference's
+// per-token loop (src/engine/tq_transformer.c:1909-1936 scores with scale 1/sqrt(hd), :1960 softmax, :2183-2191
 // weighted sum of V, head h reading KV head h/(nh/nkv) :1679, window start :1646-1654): scores,
 // running maximum, sum and the output accumulator are fp32; only P is rounded to bf16 to feed the
-// second product.
+// second product.  One kernel serves every softmax attention over rows: keys and values of 64 or 128 elements each
+// in planes of their own or side by side in a row, a window (with a sequence's first positions kept) or cells of
+// positions, a cap on the scores, a bias per distance, a sink in the denominator.  Keys may also be 192 long, and lie
+// in plain matrices instead of pages, the last 64 elements shared by all heads (latent attention's prompts).
 //
-// A unit of work = 128 consecutive query tokens of one sequence x one query head; persistent CTAs (one per SM)
-// each take several, heavy and light ones alternating, and walk a unit's keys in tiles of 128 (= two cache
-// pages; the last tile may hold one).  While one unit's result is divided and written out, the next unit's
-// Q is already loaded and its products run into the second O buffer:
-//   warp 0        TMA: Q once, then K and V pages through two-stage rings
-//   warp 1        owns tensor memory, issues  S = Q K^T  (M 128, N 128, K hd) one tile ahead into one
-//                 of two S buffers, and  O += P V  (M 128, N hd, K 128; V is the MN-major operand, read
-//                 as stored), accumulating in tensor memory over all key tiles
-//   warps 2..9    two threads per query row (each warp reads its quarter of the tensor-memory lanes;
-//                 the two threads of a row split the tile's 64 keys and the head's elements): read S,
-//                 mask, online softmax, write P (bf16, 128-byte swizzled) to one of two buffers in
-//                 shared memory.  O stays in tensor memory: it is rescaled there only when a row's
-//                 maximum grows by more than 2^8 over the one its exponentials are taken against
-//                 (until then P is simply larger, at most 256, and the row's sum carries the same
-//                 factor), so a tile's softmax never waits for the products before it.
+// A unit of work = two query tiles of 128 rows (slots A and B) that walk the same keys in tiles of 128 (= two cache
+// pages; the last tile may hold one): two heads of one key/value head, or two tiles of one head's run.  Persistent
+// CTAs, one per SM, take units until none is left:
+//   warps 0..3    softmax of slot A, a thread per row; warps 4..7 of slot B: read S, mask, online softmax, write P
+//                 (bf16) over S in tensor memory, where the second product takes it as its left operand.  O stays in
+//                 tensor memory: it is rescaled there only when a row's maximum grows by more than 2^8 over the one
+//                 its exponentials are taken against (until then P is simply larger, at most 256, and the row's sum
+//                 carries the same factor)
+//   warp 8        TMA: Q of both slots, then K and V pages through rings that both slots read
+//   warp 9        owns tensor memory, issues  O += P V  of a slot's tile and right behind it  S = Q K^T  of its next
+// The two slots take turns: while one's scores are exponentiated the other's products run, which is what bounds a
+// tile pair: 2 x 16,384 exponentials at 16 a cycle and SM (2,048 cycles) beside 32 products of 128 x 128 x 16.  With one
+// slot (the eight warps sharing one tile, P through shared memory) a 128 x 128 tile took 6,000 cycles, because
+// nothing ran beside its chain of product, maximum, exponentials, product.
 // Every wait on an mbarrier is bounded; a wait that runs out sets *status and the CTA
 // leaves cleanly.
 #include <cuda.h>
@@ -33,7 +35,9 @@ TQ_DEFINE_LAST_ERROR
 namespace {
 
 constexpr int BM = 128;      // query rows per CTA
-constexpr int THREADS = 320;   // TMA warp, MMA warp, eight softmax warps
+// eight softmax warps; TMA warp, MMA warp and two that only fill their warpgroup.  Registers: 384 threads start with 168 each,
+// the last warpgroup gives back all but 72 and the softmax warps take 216 (256 * 216 + 128 * 72 = 384 * 168)
+constexpr int THREADS = 384;
 constexpr uint32_t WAIT_LIMIT = 1u << 20;
 constexpr uint64_t WAIT_NS = 2000000000ull;
 
@@ -94,15 +98,36 @@ __device__ __forceinline__ uint64_t desc_mn_major(uint32_t addr, uint32_t lbo_by
 __device__ __forceinline__ uint32_t idesc(int n, int b_mn) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)b_mn << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
 }
-__device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t id, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(a), "l"(b), "r"(id), "r"(accumulate) : "memory");
+// One lane of the warp, the same each time.  The products and commits below are issued under its predicate by code the
+// whole warp runs, so that their operands stay in uniform registers: issued from a one-lane branch each product cost
+// some 140 cycles of moving its descriptors there, more than the product itself.
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+    return e;
 }
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+__device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t id, uint32_t accumulate, uint32_t elected) {
+    asm volatile(
+        "{\n\t.reg .pred p, e;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 e, %5, 0;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(a), "l"(b), "r"(id), "r"(accumulate), "r"(elected) : "memory");
+}
+// the same with the left operand in tensor memory: a lane per row, two K elements in each 32-bit column
+__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t b, uint32_t id, uint32_t accumulate, uint32_t elected) {
+    asm volatile(
+        "{\n\t.reg .pred p, e;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 e, %5, 0;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(b), "r"(id), "r"(accumulate), "r"(elected) : "memory");
+}
+__device__ __forceinline__ void umma_commit(uint32_t bar, uint32_t elected) {
+    asm volatile(
+        "{\n\t.reg .pred e;\n\t"
+        "setp.ne.b32 e, %1, 0;\n\t"
+        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar), "r"(elected) : "memory");
 }
 // 2^x, one MUFU instruction; 2^-inf = 0
 __device__ __forceinline__ float ex2(float x) {
@@ -133,102 +158,162 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32
 }
 
 constexpr int PAGE = 64;     // tokens per cache page
-constexpr int BN = 128;      // keys per tile = two cache pages (the last tile of a CTA may hold one)
+constexpr int BN = 128;      // keys per tile = two cache pages (a unit's last tile may hold one)
+constexpr float LOG2E = 1.4426950408889634f;
 
-template <int HD>
+template <int DK, int DV>
 struct Cfg {
-    static constexpr int HALVES = HD / 64;                 // 64-element (128-byte) column blocks of a head
-    static constexpr int Q_BYTES = BM * HD * 2;
-    static constexpr int PAGE_BYTES = PAGE * HD * 2;       // one page of K or of V for one KV head
-    static constexpr int KV_BYTES = BN * HD * 2;           // a tile of K or of V
-    static constexpr int P_BYTES = BM * BN * 2;
-    static constexpr int STAGES = 2;                       // K and V tiles in flight
-    static constexpr int TILE_BYTES = Q_BYTES + 2 * STAGES * KV_BYTES + 2 * P_BYTES;
-    static constexpr int SUMS_BYTES = 2 * BM * 4;          // the two threads of a row exchange their sums here
-    static constexpr int SMEM_BYTES = TILE_BYTES + 1024 /* alignment slack */ + 256 /* barriers */ + SUMS_BYTES;
-    static constexpr int TMEM_COLS = 512;                  // S twice (2 x 128 columns), O twice (2 x HD columns)
-    static_assert(HD == 64 || HD == 128, "head size 64 or 128");
+    static constexpr int KB = DK / 64, VB = DV / 64;       // 64-element (128-byte) column blocks of a key and of a value
+    static constexpr int Q_BYTES = BM * DK * 2;            // one slot's queries
+    static constexpr int K_BYTES = BN * DK * 2, V_BYTES = BN * DV * 2;
+    static constexpr int K_PAGE = PAGE * DK * 2, V_PAGE = PAGE * DV * 2;
+    static constexpr int KST = 2, VST = DK > 128 ? 1 : 2;  // tiles of K and of V in flight
+    static constexpr int TILE_BYTES = 2 * Q_BYTES + KST * K_BYTES + VST * V_BYTES;
+    static constexpr int SMEM_BYTES = TILE_BYTES + 1024 /* alignment slack */ + 256 /* barriers */;
+    static constexpr int TMEM_COLS = 512;                  // S (with P over it) and O of both slots: 2 x 128 + 2 x DV
+    static_assert((DK == 64 || DK == 128 || DK == 192) && (DV == 64 || DV == 128), "key and value sizes");
     static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
 };
 
-// A unit of work: 128 consecutive query tokens of one sequence x one query head.
-struct Item { int seq, h, t0, rows, p_first, pg_first, n_pages, n_tiles; bool valid; };
+// What a launch looks like.  A page's key row: page * kp + kv head * kg in map_k, its value row the same + v_plane in
+// map_v; the head's columns begin at kv head * kc in map_k and at v_col + kv head * vc in map_v.  table null: keys lie
+// densely, sequence s from page page_base[s] on.
+struct Shape {
+    int nh, nkv, n_seqs, n_qt, pairing;
+    int kp, kg, v_plane, kc, vc, v_col, k_blocks;          // k_blocks: 64-element blocks of a key that map_k holds; the rest come from map_r
+    int table_stride, n_pages, window, keep_first, cell, far;
+    float scale, softcap;
+};
+enum { PAIR_HEADS, PAIR_ROWS };
 
-// Units are numbered with the query tile slowest and last tiles first (they see the most keys), and dealt to the
-// CTAs in rounds that alternate direction (0..G-1, then G-1..0, ...), so every CTA gets a heavy and a light one.
-__device__ __forceinline__ int unit_of_round(int round, int cta, int n_ctas) {
-    return round * n_ctas + ((round & 1) ? n_ctas - 1 - cta : cta);
+// Two tiles of 128 consecutive query tokens of one sequence, each of one query head.
+struct Unit { int seq, g, p0, first, kept, n_pages, n_tiles, h[2], t0[2], rows[2], p_first[2], n[2]; bool valid; };
+
+// The query tile is the slowest index, last tiles (which see the most keys) first.
+__device__ __forceinline__ Unit unit_of(int unit, const Shape& S, const int* cu_seqlens, const int* seq_start) {
+    Unit u;
+    const int hs = S.pairing == PAIR_HEADS ? S.nh / 2 : S.nh;
+    const int per = S.n_seqs * hs, x = unit / per, rem = unit - x * per;
+    u.seq = rem / hs;
+    const int hx = rem - u.seq * hs;
+    const int t_begin = cu_seqlens[u.seq], run = cu_seqlens[u.seq + 1] - t_begin;
+    const int start = seq_start[u.seq], tiles = (run + BM - 1) / BM;
+    int qa, qb;                                            // the slots' query tiles (-1: none)
+    if (S.pairing == PAIR_HEADS) {
+        qa = qb = S.n_qt - 1 - x;
+        u.h[0] = 2 * hx; u.h[1] = 2 * hx + 1;
+        u.valid = qa < tiles;
+    } else {
+        u.h[0] = u.h[1] = hx;
+        qa = 2 * ((S.n_qt + 1) / 2 - 1 - x);
+        qb = qa + 1 < tiles ? qa + 1 : -1;
+        u.valid = qa < tiles;
+    }
+    u.g = u.h[0] / (S.nh / S.nkv);
+    u.p0 = start + qa * BM;
+    u.first = S.cell > 0 ? (u.p0 - u.p0 % S.cell) / PAGE : (S.window > 0 ? max(0, u.p0 + 1 - S.window) / PAGE : 0);
+    u.kept = S.window > 0 && S.cell == 0 ? min((S.keep_first + PAGE - 1) / PAGE, u.first) : 0;
+    u.n_pages = 0;
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+        const int q = s ? qb : qa;
+        u.t0[s] = t_begin + q * BM;
+        u.rows[s] = min(BM, run - q * BM);
+        u.p_first[s] = start + q * BM;
+        const int pages = u.kept + (u.p_first[s] + u.rows[s] - 1) / PAGE - u.first + 1;
+        u.n[s] = q < 0 || !u.valid ? 0 : (pages + 1) / 2;
+        if (u.n[s]) u.n_pages = max(u.n_pages, pages);
+    }
+    u.n_tiles = max(u.n[0], u.n[1]);
+    return u;
 }
-__device__ __forceinline__ Item item_of(int unit, int n_qt, int n_seqs, int nh, const int* cu_seqlens, const int* seq_start,
-                                        int window) {
-    Item it;
-    const int per_qt = n_seqs * nh;
-    const int x = unit / per_qt, rem = unit - x * per_qt;
-    it.seq = rem / nh;
-    it.h = rem - it.seq * nh;
-    const int qt = n_qt - 1 - x;
-    const int t_begin = cu_seqlens[it.seq], t_end = cu_seqlens[it.seq + 1];
-    it.t0 = t_begin + qt * BM;
-    it.valid = it.t0 < t_end;
-    it.rows = min(BM, t_end - it.t0);
-    it.p_first = seq_start[it.seq] + qt * BM;              // position of row 0
-    const int p_last = it.p_first + it.rows - 1;
-    const int lo = window > 0 ? max(0, it.p_first + 1 - window) : 0;
-    it.pg_first = lo / PAGE;                               // cache pages this unit reads
-    it.n_pages = it.valid ? p_last / PAGE - it.pg_first + 1 : 0;
-    it.n_tiles = (it.n_pages + 1) / 2;
-    return it;
+// the n-th page a unit walks
+__device__ __forceinline__ int page_at(const Unit& u, int n) { return n < u.kept ? n : u.first + n - u.kept; }
+
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return tq_unpack2(tq_fma2(tq_pack2(a.x, a.y), tq_pack2(b.x, b.y), tq_pack2(c.x, c.y))); }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return tq_unpack2(tq_mul2(tq_pack2(a.x, a.y), tq_pack2(b.x, b.y))); }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return tq_unpack2(tq_add2(tq_pack2(a.x, a.y), tq_pack2(b.x, b.y))); }
+
+// softcap * tanh(s / softcap) of 32 scores times `scale`: the odd series up to x^9 where every score of the warp's rows lies
+// below a quarter of the cap (the first term left out is 4e-9 of the result there), the exponential form beyond.
+__device__ __forceinline__ void cap_scores(uint32_t (&v)[32], float scale, float cap, float inv_cap) {
+    const float k = scale * inv_cap;
+    float top = 0.f, top2 = 0.f;
+#pragma unroll
+    for (int c = 0; c < 32; c += 2) { top = fmaxf(top, fabsf(__uint_as_float(v[c]))); top2 = fmaxf(top2, fabsf(__uint_as_float(v[c + 1]))); }
+    const bool beyond = __any_sync(0xffffffffu, !(fmaxf(top, top2) * fabsf(k) <= 0.25f));
+    const float2 kk = make_float2(k, k), cc = make_float2(cap, cap);
+    const float2 c9 = make_float2(62.0f / 2835.0f, 62.0f / 2835.0f), c7 = make_float2(-17.0f / 315.0f, -17.0f / 315.0f),
+                 c5 = make_float2(2.0f / 15.0f, 2.0f / 15.0f), c3 = make_float2(-1.0f / 3.0f, -1.0f / 3.0f), one = make_float2(1.f, 1.f);
+    if (!beyond) {
+#pragma unroll
+        for (int c = 0; c < 32; c += 2) {
+            const float2 x = mul2(make_float2(__uint_as_float(v[c]), __uint_as_float(v[c + 1])), kk), x2 = mul2(x, x);
+            const float2 t = mul2(mul2(cc, x), fma2(x2, fma2(x2, fma2(x2, fma2(x2, c9, c7), c5), c3), one));
+            v[c] = __float_as_uint(t.x);
+            v[c + 1] = __float_as_uint(t.y);
+        }
+    } else {
+#pragma unroll
+        for (int c = 0; c < 32; ++c) {
+            const float x = __uint_as_float(v[c]) * k, x2 = x * x;
+            const float near = x * fmaf(x2, fmaf(x2, fmaf(x2, fmaf(x2, c9.x, c7.x), c5.x), c3.x), 1.0f);
+            v[c] = __float_as_uint(cap * (fabsf(x) <= 0.25f ? near : 1.0f - __fdividef(2.0f, __expf(2.0f * x) + 1.0f)));
+        }
+    }
 }
 
-template <int HD>
+// SHAPED: scores pass through a cap and/or a bias per distance before the softmax.
+template <int DK, int DV, bool SHAPED>
 __global__ void __launch_bounds__(THREADS, 1)
-attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,
-                         const int* __restrict__ cu_seqlens, const int* __restrict__ seq_start,
-                         const int* __restrict__ page_table, int table_stride, int window, float scale_log2e,
-                         __nv_bfloat16* __restrict__ out, int nh, int nkv, int n_qt, int n_seqs,
-                         int* __restrict__ status) {
+attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+                         const __grid_constant__ CUtensorMap map_r, const __grid_constant__ CUtensorMap map_v,
+                         const __grid_constant__ Shape S, const int* __restrict__ cu_seqlens, const int* __restrict__ seq_start,
+                         const int* __restrict__ page_table, const int* __restrict__ page_base,
+                         const float* __restrict__ bias_t, const float* __restrict__ sink,
+                         __nv_bfloat16* __restrict__ out, int* __restrict__ status) {
     tq_grid_wait();                    // everything below may read what the previous kernel wrote
-    using C = Cfg<HD>;
+    using C = Cfg<DK, DV>;
     extern __shared__ uint8_t smem_raw[];
     __shared__ int s_abort;
     __shared__ uint32_t s_tmem_base;
+    __shared__ __align__(16) uint4 s_answer;               // the hardware's answer to a request for another block
+    __shared__ int s_unit[2];                              // the units this CTA takes, two in turn
+    __shared__ float s_bias[SHAPED ? 8 : 1][2][96];        // a warp's rows and a page's keys: the bias of their 95 distances
 
-    const int n_units = n_qt * n_seqs * nh;
-    const int cta = blockIdx.x, n_ctas = gridDim.x;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int kv_group = nh / nkv;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // the same for the whole warp, and known to be
 
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t q_smem = base;
-    auto k_smem = [&](int s) { return base + C::Q_BYTES + s * C::KV_BYTES; };
-    auto v_smem = [&](int s) { return base + C::Q_BYTES + (C::STAGES + s) * C::KV_BYTES; };
-    auto p_smem = [&](int b) { return base + C::Q_BYTES + 2 * C::STAGES * C::KV_BYTES + b * C::P_BYTES; };
+    auto q_smem = [&](int s) { return base + s * C::Q_BYTES; };
+    auto k_smem = [&](int s) { return base + 2 * C::Q_BYTES + s * C::K_BYTES; };
+    auto v_smem = [&](int s) { return base + 2 * C::Q_BYTES + C::KST * C::K_BYTES + s * C::V_BYTES; };
     const uint32_t bars = base + C::TILE_BYTES;
-    constexpr int NS = C::STAGES;
-    const uint32_t q_full = bars, q_free = bars + 8u;                     // Q of a unit is in / is no longer read
-    auto k_full = [&](int s) { return bars + 8u * (2 + s); };
-    auto k_empty = [&](int s) { return bars + 8u * (2 + NS + s); };
-    auto v_full = [&](int s) { return bars + 8u * (2 + 2 * NS + s); };
-    auto v_empty = [&](int s) { return bars + 8u * (2 + 3 * NS + s); };
-    auto s_ready = [&](int b) { return bars + 8u * (2 + 4 * NS + b); };
-    auto p_ready = [&](int b) { return bars + 8u * (4 + 4 * NS + b); };   // P of a tile is in its buffer (and S has been read)
-    auto pv_done = [&](int b) { return bars + 8u * (6 + 4 * NS + b); };   // the products that read P buffer b are done
-    const uint32_t sums_ready = bars + 8u * (8 + 4 * NS);                 // every softmax warp has written its rows' sums
-    const uint32_t sums_read = bars + 8u * (9 + 4 * NS);                  // ... and has read its partners'
-    static_assert((10 + 4 * NS) * 8 <= 256, "barriers");
-    float* s_sums = reinterpret_cast<float*>(smem_raw + (bars + 256u - smem_u32(smem_raw)));
+    auto q_full = [&](int s) { return bars + 8u * s; };                   // a slot's Q is in / is no longer read
+    auto q_free = [&](int s) { return bars + 8u * (2 + s); };
+    auto k_full = [&](int s) { return bars + 8u * (4 + s); };
+    auto k_empty = [&](int s) { return bars + 8u * (6 + s); };
+    auto v_full = [&](int s) { return bars + 8u * (8 + s); };
+    auto v_empty = [&](int s) { return bars + 8u * (10 + s); };
+    auto s_ready = [&](int s) { return bars + 8u * (12 + s); };           // S of a slot's tile is done, and all products before it
+    auto p_ready = [&](int s) { return bars + 8u * (14 + s); };           // P of a slot's tile is in place of its S
+    auto o_done = [&](int s) { return bars + 8u * (16 + s); };            // a slot's last product of a unit is done
+    auto o_free = [&](int s) { return bars + 8u * (18 + s); };            // ... and has been read
+    auto n_full = [&](int s) { return bars + 8u * (20 + s); };            // a unit's number is there / has been read
+    auto n_free = [&](int s) { return bars + 8u * (22 + s); };
+    const uint32_t answered = bars + 8u * 24;
 
     if (threadIdx.x == 0) {
         s_abort = 0;
-        mbar_init(q_full, 1);
-        mbar_init(q_free, 1);
-        mbar_init(sums_ready, 8);
-        mbar_init(sums_read, 8);
-        for (int s = 0; s < C::STAGES; ++s) { mbar_init(k_full(s), 1); mbar_init(k_empty(s), 1); mbar_init(v_full(s), 1); mbar_init(v_empty(s), 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(s_ready(b), 1); mbar_init(p_ready(b), 8); mbar_init(pv_done(b), 1); }   // 8: one arrival per softmax warp
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(q_full(s), 1); mbar_init(q_free(s), 1); mbar_init(k_full(s), 1); mbar_init(k_empty(s), 1);
+            mbar_init(v_full(s), 1); mbar_init(v_empty(s), 1); mbar_init(s_ready(s), 1); mbar_init(o_done(s), 1);
+            mbar_init(p_ready(s), 4); mbar_init(o_free(s), 4);            // 4: one arrival per softmax warp of the slot
+            mbar_init(n_full(s), 1); mbar_init(n_free(s), 9);             // 9: the softmax warps and the MMA warp
+        }
+        mbar_init(answered, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 1) {
+    if (warp == 9) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                      ::"r"(smem_u32(&s_tmem_base)), "r"((uint32_t)C::TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -239,286 +324,389 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     // only now: a dependent kernel that took tensor memory first could starve a CTA of this grid that
     // had not allocated yet, and then wait forever for this grid to finish
     tq_grid_launch_dependents();
-    auto tmem_s = [&](int b) { return s_tmem_base + (uint32_t)(b * BN); };              // S, twice: BN columns each
-    auto tmem_o = [&](int b) { return s_tmem_base + (uint32_t)(2 * BN + b * HD); };     // O, twice: HD columns each
+    auto tmem_s = [&](int s) { return s_tmem_base + (uint32_t)(s * BN); };              // S, and P over its first half
+    auto tmem_o = [&](int s) { return s_tmem_base + (uint32_t)(2 * BN + s * DV); };
 
-    // Every role walks the same units in the same order and counts tiles across units: tile number `ti` picks the
-    // K/V stage (ti % STAGES), the S and P buffers (ti & 1) and the barriers' phases; unit number `it` picks the O
-    // buffer (it & 1), so one unit's result is written out while the next unit's products accumulate.
-    if (warp == 0) {
+    // Every role walks the same units in the same order: the block's own first, then those of blocks that have not
+    // started yet, which the TMA warp asks the hardware for (a block whose place is taken over never starts) and hands
+    // on one unit ahead.  Heavy units come first in the grid, so the light ones fill the end.
+    auto take_unit = [&](int k) -> int {                       // the CTA's k-th unit, -1: there is none; called by whole warps
+        if (!__all_sync(0xffffffffu, mbar_wait(n_full(k & 1), (uint32_t)(k >> 1) & 1u, &s_abort))) return -1;
+        const int unit = *(volatile int*)&s_unit[k & 1];
+        __syncwarp();
+        if (lane == 0) mbar_arrive(n_free(k & 1));
+        return __shfl_sync(0xffffffffu, unit, 0);
+    };
+    // Tile number `ti`, counted across units, picks the K and V
+    // stages and their barriers' phases; a slot's tiles and units, counted for the slot, the phases of its own.
+    if (warp >= 8) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+    if (warp == 8) {
         // ------------------------------ TMA producer ------------------------------
-        if (lane == 0) {
-            int ti = 0, it = 0;
-            bool ok = true;
-            for (int round = 0; ok; ++round) {
-                const int unit = unit_of_round(round, cta, n_ctas);
-                if (unit >= n_units) break;
-                const Item u = item_of(unit, n_qt, n_seqs, nh, cu_seqlens, seq_start, window);
-                if (!u.valid) continue;
-                const int g = u.h / kv_group;
-                const int* table = page_table + (size_t)u.seq * table_stride;
-                // the products that read the previous unit's Q must be done
-                if (it > 0 && !mbar_wait(q_free, (uint32_t)(it - 1) & 1u, &s_abort)) break;
-                mbar_expect_tx(q_full, (uint32_t)C::Q_BYTES);
+            const uint32_t elected = elect_one();
+            int ti = 0, vi = 0, asked = 0, units[2] = {0, 0};
+            bool ok = true, pending = false;
+            auto wait = [&](uint32_t bar, uint32_t parity) { return (bool)__all_sync(0xffffffffu, mbar_wait(bar, parity, &s_abort)); };
+            auto ask = [&]() {
+                if (elected) {
+                    mbar_expect_tx(answered, 16);
+                    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+                                 ::"r"(smem_u32(&s_answer)), "r"(answered) : "memory");
+                }
+                pending = true;
+            };
+            auto answer = [&]() -> int {                       // the block taken over, -1: all have started (no request follows)
+                if (!wait(answered, (uint32_t)asked & 1u)) { ok = false; return -1; }
+                pending = false;
+                ++asked;
+                uint32_t x, got;
+                asm volatile(
+                    "{\n\t.reg .b128 h;\n\t.reg .pred p;\n\t"
+                    "ld.shared.b128 h, [%2];\n\t"
+                    "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\t"
+                    "selp.u32 %1, 1, 0, p;\n\t"
+                    "mov.u32 %0, 0;\n\t"
+                    "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, h;\n\t}"
+                    : "=r"(x), "=r"(got) : "r"(smem_u32(&s_answer)) : "memory");
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // this read before the next answer is written
+                __syncwarp();
+                return __shfl_sync(0xffffffffu, got ? (int)x : -1, 0);
+            };
+            // from a block on, the first whose unit exists (a short run has none at a late tile)
+            auto settle = [&](int unit) -> int {
+                while (ok && unit >= 0 && !unit_of(unit, S, cu_seqlens, seq_start).valid) { ask(); unit = answer(); }
+                return ok ? unit : -1;
+            };
+            auto hand_on = [&](int k, int unit) {
+                if (k >= 2 && !wait(n_free(k & 1), (uint32_t)((k >> 1) - 1) & 1u)) { ok = false; return; }
+                if (elected) {
+                    *(volatile int*)&s_unit[k & 1] = unit;
+                    mbar_arrive(n_full(k & 1));
+                }
+                __syncwarp();
+            };
+            int unit = settle(blockIdx.x);
+            hand_on(0, unit);
+            for (int k = 0; ok && unit >= 0; ++k) {
+                ask();
+                int following = -1;
+                const Unit u = unit_of(unit, S, cu_seqlens, seq_start);
+                auto load_q = [&](int s) {
+                    if (!u.n[s]) return true;
+                    // the products that read the slot's previous Q must be done
+                    if (units[s] > 0 && !wait(q_free(s), (uint32_t)(units[s] - 1) & 1u)) return false;
+                    if (elected) {
+                    mbar_expect_tx(q_full(s), (uint32_t)C::Q_BYTES);
 #pragma unroll
-                for (int c = 0; c < C::HALVES; ++c) tma_load_2d(q_smem + c * (BM * 128), &map_q, u.h * HD + c * 64, u.t0, q_full);
-                ++it;
+                    for (int c = 0; c < C::KB; ++c) tma_load_2d(q_smem(s) + c * (BM * 128), &map_q, u.h[s] * DK + c * 64, u.t0[s], q_full(s));
+                    }
+                    ++units[s];
+                    return true;
+                };
+                ok = load_q(0);
+                if (!ok) break;
                 for (int i = 0; i < u.n_tiles; ++i, ++ti) {
-                    const int s = ti % C::STAGES;
-                    const uint32_t ph = (uint32_t)(ti / C::STAGES) & 1u;
                     const int np = min(2, u.n_pages - 2 * i);
-                    const int page0 = table[u.pg_first + 2 * i], page1 = np > 1 ? table[u.pg_first + 2 * i + 1] : 0;
+                    int page[2] = {0, 0};
+                    for (int pg = 0; pg < np; ++pg) {
+                        const int n = page_at(u, 2 * i + pg);
+                        page[pg] = page_table != nullptr
+                            ? TQ_CHECKED(page_table[(size_t)u.seq * S.table_stride + TQ_CHECKED(n, S.table_stride, TQ_IDX_TABLE_COLUMN)], S.n_pages, TQ_IDX_PAGE)
+                            : page_base[u.seq] + n - u.first;
+                    }
                     // a tile in shared memory: [column block of 64 elements][128 keys][128 bytes]; a page is 64 keys of it
-                    if (!mbar_wait(k_empty(s), ph ^ 1u, &s_abort)) { ok = false; break; }
-                    mbar_expect_tx(k_full(s), (uint32_t)(np * C::PAGE_BYTES));
-                    for (int pg = 0; pg < np; ++pg) {
-                        const int krow = (((pg ? page1 : page0) * 2 + 0) * nkv + g) * PAGE;
+                    const int ks = ti % C::KST;
+                    if (!wait(k_empty(ks), ((uint32_t)(ti / C::KST) & 1u) ^ 1u)) { ok = false; break; }
+                    if (elected) {
+                    mbar_expect_tx(k_full(ks), (uint32_t)(np * C::K_PAGE));
+                    for (int pg = 0; pg < np; ++pg)
 #pragma unroll
-                        for (int c = 0; c < C::HALVES; ++c)
-                            tma_load_2d(k_smem(s) + c * (BN * 128) + pg * (PAGE * 128), &map_kv, c * 64, krow, k_full(s));
+                        for (int c = 0; c < C::KB; ++c) {
+                            const uint32_t dst = k_smem(ks) + c * (BN * 128) + pg * (PAGE * 128);
+                            if (c < S.k_blocks) tma_load_2d(dst, &map_k, u.g * S.kc + c * 64, page[pg] * S.kp + u.g * S.kg, k_full(ks));
+                            else tma_load_2d(dst, &map_r, (c - S.k_blocks) * 64, page[pg] * S.kp, k_full(ks));
+                        }
                     }
-                    if (!mbar_wait(v_empty(s), ph ^ 1u, &s_abort)) { ok = false; break; }
-                    mbar_expect_tx(v_full(s), (uint32_t)(np * C::PAGE_BYTES));
-                    for (int pg = 0; pg < np; ++pg) {
-                        const int vrow = (((pg ? page1 : page0) * 2 + 1) * nkv + g) * PAGE;
+                    if (i == 0 && !load_q(1)) { ok = false; ++ti; break; }
+                    const int vs = ti % C::VST;
+                    if (!wait(v_empty(vs), ((uint32_t)(ti / C::VST) & 1u) ^ 1u)) { ok = false; ++ti; break; }
+                    if (elected) {
+                    mbar_expect_tx(v_full(vs), (uint32_t)(np * C::V_PAGE));
+                    for (int pg = 0; pg < np; ++pg)
 #pragma unroll
-                        for (int c = 0; c < C::HALVES; ++c)
-                            tma_load_2d(v_smem(s) + c * (BN * 128) + pg * (PAGE * 128), &map_kv, c * 64, vrow, v_full(s));
+                        for (int c = 0; c < C::VB; ++c)
+                            tma_load_2d(v_smem(vs) + c * (BN * 128) + pg * (PAGE * 128), &map_v, S.v_col + u.g * S.vc + c * 64,
+                                        page[pg] * S.kp + u.g * S.kg + S.v_plane, v_full(vs));
+                    }
+                    vi = ti + 1;
+                    if (i == 0) {                              // the MMA warp looks one unit ahead: it must know before this one's last tile
+                        following = settle(answer());
+                        if (ok) hand_on(k + 1, following);
+                        if (!ok) { ++ti; break; }
                     }
                 }
+                unit = following;
             }
-            if (s_abort) {      // let the copies this thread started land before the CTA goes away (bounded)
-                if (it > 0) for (uint32_t i = 0; i < WAIT_LIMIT && !mbar_try_wait(q_full, (uint32_t)(it - 1) & 1u); ++i) {}
-                for (int i = ti > C::STAGES ? ti - C::STAGES : 0; i < ti; ++i) {
-                    const uint32_t ph = (uint32_t)(i / C::STAGES) & 1u;
-                    for (uint32_t j = 0; j < WAIT_LIMIT && !mbar_try_wait(k_full(i % C::STAGES), ph); ++j) {}
-                    for (uint32_t j = 0; j < WAIT_LIMIT && !mbar_try_wait(v_full(i % C::STAGES), ph); ++j) {}
-                }
+            if (s_abort) {      // let the answer and the copies this thread started land before the CTA goes away (bounded)
+                if (pending) for (uint32_t j = 0; j < WAIT_LIMIT && !mbar_try_wait(answered, (uint32_t)asked & 1u); ++j) {}
+                for (int s = 0; s < 2; ++s)
+                    if (units[s]) for (uint32_t j = 0; j < WAIT_LIMIT && !mbar_try_wait(q_full(s), (uint32_t)(units[s] - 1) & 1u); ++j) {}
+                for (int i = ti > C::KST ? ti - C::KST : 0; i < ti; ++i)
+                    for (uint32_t j = 0; j < WAIT_LIMIT && !mbar_try_wait(k_full(i % C::KST), (uint32_t)(i / C::KST) & 1u); ++j) {}
+                for (int i = vi > C::VST ? vi - C::VST : 0; i < vi; ++i)
+                    for (uint32_t j = 0; j < WAIT_LIMIT && !mbar_try_wait(v_full(i % C::VST), (uint32_t)(i / C::VST) & 1u); ++j) {}
             }
-        }
-    } else if (warp == 1) {
+    } else if (warp == 9) {
         // ------------------------------ MMA issuer ------------------------------
-        // A product of M = 128 costs some 130-145 cycles whatever its N up to 128: tiles of 128 keys make the
-        // most of each one (8 products for S, 8 for O per 128 keys).  S = Q K^T of a tile is issued one tile ahead
-        // of the P V product, across units too: two cursors walk the same sequence of tiles.
-        if (lane == 0) {
-            const uint32_t id_o = idesc(HD, 1);
-            struct Cursor { int round, it, ti, i; Item u; bool live; };
-            auto enter = [&](Cursor& c) {           // the next valid unit from c.round on
-                c.live = false;
-                for (;; ++c.round) {
-                    const int unit = unit_of_round(c.round, cta, n_ctas);
-                    if (unit >= n_units) return;
-                    c.u = item_of(unit, n_qt, n_seqs, nh, cu_seqlens, seq_start, window);
-                    if (c.u.valid) break;
-                }
-                c.i = 0;
-                c.live = true;
+        // Tile by tile, slot by slot: the slot's P V product of this tile as soon as its P is there, then its scores of
+        // the next tile (which may be the next unit's first): products are carried out in the order they are issued,
+        // so the scores overwrite a P that has been read.
+            const uint32_t elected = elect_one(), id_o = idesc(DV, 1);
+            const uint32_t tm = __shfl_sync(0xffffffffu, s_tmem_base, 0);
+            int ti = 0, taken = 0, tiles[2] = {0, 0}, units[2] = {0, 0};
+            auto wait = [&](uint32_t bar, uint32_t parity) { return (bool)__all_sync(0xffffffffu, mbar_wait(bar, parity, &s_abort)); };
+            auto next_unit = [&](Unit& u) {
+                const int unit = take_unit(taken++);
+                if (unit >= 0) u = unit_of(unit, S, cu_seqlens, seq_start);
+                return unit >= 0;
             };
-            auto advance = [&](Cursor& c) {
-                ++c.ti;
-                if (++c.i == c.u.n_tiles) { ++c.round; ++c.it; enter(c); }
-            };
-            Cursor qk{0, 0, 0, 0, Item{}, false}, pv{0, 0, 0, 0, Item{}, false};
-            enter(qk);
-            enter(pv);
-            bool ok = true;
-            auto issue_qk = [&]() -> bool {
-                const int s = qk.ti % C::STAGES, b = qk.ti & 1;
-                const int np = min(2, qk.u.n_pages - 2 * qk.i);
-                if (qk.i == 0 && !mbar_wait(q_full, (uint32_t)qk.it & 1u, &s_abort)) return false;
-                if (!mbar_wait(k_full(s), (uint32_t)(qk.ti / C::STAGES) & 1u, &s_abort)) return false;
+            const uint64_t q_desc = desc_k_major(q_smem(0)), k_desc = desc_k_major(k_smem(0)), v_desc = desc_mn_major(v_smem(0), BN * 128);
+            // the scores of slot s for tile i of unit u, which is tile number t of the CTA; first, last: whether the other slot reads
+            // the keys before or after it
+            auto issue_qk = [&](const Unit& u, int i, int t, int s, bool first, bool last) -> bool {
+                const int st = t % C::KST, np = min(2, u.n_pages - 2 * i);
+                if (i == 0 && !wait(q_full(s), (uint32_t)units[s] & 1u)) return false;
+                if (first && !wait(k_full(st), (uint32_t)(t / C::KST) & 1u)) return false;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t id_s = idesc(PAGE * np, 0);
+                const uint64_t qd = q_desc + (uint64_t)(s * (C::Q_BYTES / 16)), kd = k_desc + (uint64_t)(st * (C::K_BYTES / 16));
 #pragma unroll
-                for (int k = 0; k < HD / 16; ++k) {
-                    const uint32_t off = (k / 4) * (BM * 128) + (k % 4) * 32, koff = (k / 4) * (BN * 128) + (k % 4) * 32;
-                    umma(tmem_s(b), desc_k_major(q_smem + off), desc_k_major(k_smem(s) + koff), id_s, k > 0 ? 1u : 0u);
-                }
-                umma_commit(s_ready(b));
-                umma_commit(k_empty(s));
-                if (qk.i == qk.u.n_tiles - 1) umma_commit(q_free);       // the unit's last read of Q
-                advance(qk);
+                for (int k = 0; k < DK / 16; ++k)           // descriptors count in 16 bytes
+                    umma(tm + (uint32_t)(s * BN), qd + (k / 4) * (BM * 8) + (k % 4) * 2, kd + (k / 4) * (BN * 8) + (k % 4) * 2, id_s, k > 0 ? 1u : 0u, elected);
+                umma_commit(s_ready(s), elected);
+                if (last) umma_commit(k_empty(st), elected);
+                if (i == u.n[s] - 1) umma_commit(q_free(s), elected);           // the unit's last read of the slot's Q
                 return true;
             };
-            if (qk.live) ok = issue_qk();
-            while (pv.live && ok) {
-                // the other S buffer is free: its tile's P was complete before the P V product before this one was issued
-                if (qk.live) ok = issue_qk();
-                if (!ok) break;
-                const int s = pv.ti % C::STAGES, b = pv.ti & 1;
-                ok = mbar_wait(p_ready(b), (uint32_t)(pv.ti >> 1) & 1u, &s_abort) &&
-                     mbar_wait(v_full(s), (uint32_t)(pv.ti / C::STAGES) & 1u, &s_abort);
-                if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const int steps = (PAGE / 16) * min(2, pv.u.n_pages - 2 * pv.i);   // 16 keys per product; a missing second page is not read
-                const uint32_t acc = tmem_o(pv.it & 1);
-                for (int k = 0; k < steps; ++k)                  // O += P V (a unit's first tile starts the sum)
-                    umma(acc, desc_k_major(p_smem(b) + (k / 4) * (BM * 128) + (k % 4) * 32),
-                         desc_mn_major(v_smem(s) + k * 2048, BN * 128), id_o, (pv.i > 0 || k > 0) ? 1u : 0u);
-                umma_commit(pv_done(b));
-                umma_commit(v_empty(s));
-                advance(pv);
+            Unit u, v;
+            bool more = next_unit(u), ok = true;
+            if (more) {
+                for (int s = 0; s < 2 && ok; ++s)
+                    if (u.n[s]) ok = issue_qk(u, 0, 0, s, s == 0 || u.n[0] == 0, s == 1 || u.n[1] == 0);
             }
-        }
+            while (more && ok) {
+                const bool follows = next_unit(v);
+                for (int i = 0; i < u.n_tiles && ok; ++i, ++ti) {
+                    const bool crosses = i + 1 == u.n_tiles;             // the next tile is the next unit's first
+                    const int np = min(2, u.n_pages - 2 * i), st = ti % C::VST;
+                    const int n0 = crosses ? (follows ? v.n[0] : 0) : u.n[0], n1 = crosses ? (follows ? v.n[1] : 0) : u.n[1];
+                    const int j = crosses ? 0 : i + 1;                   // the next tile within its unit
+                    for (int s = 0; s < 2 && ok; ++s) {
+                        if (i < u.n[s]) {
+                            ok = wait(p_ready(s), (uint32_t)tiles[s] & 1u);
+                            if (ok && (s == 0 || i >= u.n[0])) ok = wait(v_full(st), (uint32_t)(ti / C::VST) & 1u);
+                            if (ok && i == 0 && units[s] > 0) ok = wait(o_free(s), (uint32_t)(units[s] - 1) & 1u);
+                            if (!ok) break;
+                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                            const uint64_t vd = v_desc + (uint64_t)(st * (C::V_BYTES / 16));
+                            const uint32_t o = tm + (uint32_t)(2 * BN + s * DV), p = tm + (uint32_t)(s * BN);
+#pragma unroll
+                            for (int k = 0; k < BN / 16; ++k)            // O += P V, 16 keys at a time (a unit's first tile starts the sum)
+                                if (k < PAGE / 16 || np > 1)             // a missing second page is not read
+                                    umma_ts(o, p + (uint32_t)(k * 8), vd + k * 128, id_o, (i > 0 || k > 0) ? 1u : 0u, elected);
+                            if (s == 1 || i >= u.n[1]) umma_commit(v_empty(st), elected);
+                            ++tiles[s];
+                            if (i == u.n[s] - 1) { umma_commit(o_done(s), elected); ++units[s]; }
+                        }
+                        if (j < (s ? n1 : n0)) ok = issue_qk(crosses ? v : u, j, ti + 1, s, s == 0 || j >= n0, s == 1 || j >= n1);
+                    }
+                }
+                more = follows;
+                u = v;
+            }
+    }
     } else {
-        // ------------------------------ softmax: two threads per query row ------------------------------
-        constexpr int HK = PAGE / 2, HDH = HD / 2;    // keys of a page and head elements of one thread
+        // ------------------------------ softmax: a thread per query row ------------------------------
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
         constexpr float RESCALE_LOG2 = 8.0f;          // O is rescaled when a row's maximum has grown by more than 2^8
-        const int quarter = warp & 3, part = (warp - 2) >> 2;
-        const int r = quarter * 32 + lane;
+        const int slot = warp >> 2, quarter = warp & 3, r = quarter * 32 + lane;
         const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
-        int ti = 0, it = 0;
+        const uint32_t s_addr = tmem_s(slot) + lane_addr, acc = tmem_o(slot) + lane_addr;
+        const float factor = SHAPED ? LOG2E : S.scale * LOG2E;            // from a score as it stands to an exponent of two
+        const float inv_cap = SHAPED && S.softcap > 0.f ? 1.0f / S.softcap : 0.f;
+        int tiles = 0, units = 0, taken = 0;
         bool ok = true;
-        for (int round = 0; ok; ++round) {
-            const int unit = unit_of_round(round, cta, n_ctas);
-            if (unit >= n_units) break;
-            const Item u = item_of(unit, n_qt, n_seqs, nh, cu_seqlens, seq_start, window);
-            if (!u.valid) continue;
-            const int qpos = u.p_first + r;
-            const int start = window > 0 ? max(0, qpos + 1 - window) : 0;
-            const uint32_t acc = tmem_o(it & 1);
-            // m: the maximum the row's exponentials are taken against (both threads of a row hold the same);
-            // l: the sum of this thread's keys' exponentials
+        for (int unit = take_unit(taken++); ok && unit >= 0; unit = ok ? take_unit(taken++) : -1) {
+            const Unit u = unit_of(unit, S, cu_seqlens, seq_start);
+            const int n = u.n[slot];
+            if (n == 0) continue;
+            const int h = u.h[slot], p_first = u.p_first[slot], qpos = p_first + r, p_last = p_first + BM - 1;
+            const int start = S.cell > 0 ? qpos - qpos % S.cell : (S.window > 0 ? max(0, qpos + 1 - S.window) : 0);
+            const int keep = S.cell > 0 || S.window == 0 ? 0 : S.keep_first;   // positions below it are seen besides those from `start` on
+            // a page from here on is seen whole by every row that lies behind it
+            const int open_from = S.cell > 0 ? p_last - p_last % S.cell : (S.window > 0 ? p_last + 1 - S.window : 0);
+            const float* bias = SHAPED && bias_t != nullptr ? bias_t + (size_t)h * (S.far + 1) : nullptr;
+            float nb[6];                               // the next tile's bias values on their way to shared memory
+            auto fetch_bias = [&](int i) {
+#pragma unroll
+                for (int j = 0; j < 6; ++j) {
+                    const int d = p_first + quarter * 32 - page_at(u, 2 * i + j / 3) * PAGE - (PAGE - 1) + (j % 3) * 32 + lane;
+                    nb[j] = __ldg(bias + min(max(d, 0), S.far));
+                }
+            };
+            if (SHAPED && bias != nullptr) fetch_bias(0);
+            // m: the maximum the row's exponentials are taken against; l: the sum of its exponentials
+            const float floor_m = sink != nullptr ? sink[h] * (LOG2E / factor) : -INFINITY;
             float m = -INFINITY, l = 0.f;
-            for (int i = 0; i < u.n_tiles && ok; ++i, ++ti) {
-                const int b = ti & 1;
+            for (int i = 0; i < n; ++i, ++tiles) {
                 const int np = min(2, u.n_pages - 2 * i);
-                const int k0 = (u.pg_first + 2 * i) * PAGE;
-                ok = __all_sync(0xffffffffu, mbar_wait(s_ready(b), (uint32_t)(ti >> 1) & 1u, &s_abort));   // warp-uniform
+                if (SHAPED && bias != nullptr) {
+                    __syncwarp();                      // the previous tile's values have been read
+#pragma unroll
+                    for (int j = 0; j < 6; ++j) s_bias[SHAPED ? warp : 0][j / 3][(j % 3) * 32 + lane] = nb[j];
+                    __syncwarp();
+                    if (i + 1 < n) fetch_bias(i + 1);
+                }
+                ok = __all_sync(0xffffffffu, mbar_wait(s_ready(slot), (uint32_t)tiles & 1u, &s_abort));   // warp-uniform
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                // this thread's 32 keys of each page of the tile, and (for the maximum only) the other thread's
-                uint32_t sv[2][32];
-                float mx = m;
+                // a page at a time, in one pass: shape and mask its scores, see whether they outgrow the maximum the row's
+                // exponentials are taken against, and write them, in bf16, over scores already read.  The loop is kept:
+                // unrolled, its code does not fit the instruction caches that ten warps share (1.6 times the time).
+                float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll 1
+                for (int hf = 0; hf < np; ++hf) {
+                    uint32_t sv[2][32];
+                    tmem_ld32(s_addr + hf * PAGE, sv[0]);
+                    tmem_ld32(s_addr + hf * PAGE + 32, sv[1]);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    const int kh = page_at(u, 2 * i + hf) * PAGE;
+                    if (SHAPED) {
 #pragma unroll
-                for (int hf = 0; hf < 2; ++hf) {
-                    if (hf < np) {                                 // uniform across the CTA
-                        uint32_t other[32];
-                        tmem_ld32(tmem_s(b) + lane_addr + hf * PAGE + part * HK, sv[hf]);
-                        tmem_ld32(tmem_s(b) + lane_addr + hf * PAGE + (1 - part) * HK, other);
-                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                        const int kh = k0 + hf * PAGE;
-                        const bool visible = (kh + PAGE - 1 <= u.p_first) && (window == 0 || kh >= u.p_first + BM - window);
-                        if (visible) {                             // every key of the page is seen by every row: no masking
+                        for (int q = 0; q < 2; ++q) {
+                            const bool capped = S.softcap > 0.f;
+                            if (capped) cap_scores(sv[q], S.scale, S.softcap, inv_cap);
+                            const float f = capped ? 1.f : S.scale;
+                            if (bias != nullptr) {
+                                const float* sb = &s_bias[SHAPED ? warp : 0][hf][lane + PAGE - 1 - q * 32];
 #pragma unroll
-                            for (int c = 0; c < HK; ++c)
-                                mx = fmaxf(mx, fmaxf(__uint_as_float(sv[hf][c]), __uint_as_float(other[c])));
-                        } else {
+                                for (int c = 0; c < 32; ++c) sv[q][c] = __float_as_uint(fmaf(__uint_as_float(sv[q][c]), f, sb[-c]));
+                            } else if (!capped) {
 #pragma unroll
-                            for (int c = 0; c < HK; ++c) {
-                                const int kp = kh + part * HK + c, kq = kh + (1 - part) * HK + c;
-                                float a = __uint_as_float(sv[hf][c]), bq = __uint_as_float(other[c]);
-                                if (kp > qpos || kp < start) a = -INFINITY;
-                                if (kq > qpos || kq < start) bq = -INFINITY;
-                                sv[hf][c] = __float_as_uint(a);
-                                mx = fmaxf(mx, fmaxf(a, bq));
+                                for (int c = 0; c < 32; ++c) sv[q][c] = __float_as_uint(__uint_as_float(sv[q][c]) * f);
                             }
                         }
                     }
-                }
-                // keep m unless the maximum grew by more than 2^8 (or nothing had been seen yet)
-                float corr = 1.0f;
-                if (m == -INFINITY) {
-                    m = mx;                                // l and O are still zero: nothing to rescale
-                } else if ((mx - m) * scale_log2e > RESCALE_LOG2) {
-                    corr = ex2((m - mx) * scale_log2e);
-                    l *= corr;
-                    m = mx;
-                }
-                // the P buffer must be free (the products of two tiles ago are done), and O can only be rescaled
-                // between the previous tile's products and this tile's
-                if (ti >= 2) ok = __all_sync(0xffffffffu, mbar_wait(pv_done(b), (uint32_t)((ti >> 1) - 1) & 1u, &s_abort));
-                if (!ok) break;
-                if (__any_sync(0xffffffffu, corr != 1.0f)) {           // only with i > 0: the previous tile is this unit's
-                    ok = __all_sync(0xffffffffu, mbar_wait(pv_done(b ^ 1), (uint32_t)((ti - 1) >> 1) & 1u, &s_abort));
-                    if (!ok) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    if (kh + PAGE - 1 > p_first || kh < open_from) {           // some row does not see some key of the page
 #pragma unroll
-                    for (int c0 = 0; c0 < HDH; c0 += 32) {
-                        uint32_t ov[32];
-                        tmem_ld32(acc + lane_addr + part * HDH + c0, ov);
-                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                        for (int q = 0; q < 2; ++q) {
+                            // bit c: the row sees key kh + 32 q + c, i.e. c <= last and (c >= lo or c < kp)
+                            const int last = qpos - kh - 32 * q, lo = start - kh - 32 * q, kp = keep - kh - 32 * q;
+                            const uint32_t behind = last < 0 ? 0u : 0xffffffffu >> (31 - min(last, 31));
+                            const uint32_t inside = lo >= 32 ? 0u : 0xffffffffu << max(lo, 0);
+                            const uint32_t kept = kp <= 0 ? 0u : 0xffffffffu >> (32 - min(kp, 32));
+                            const uint32_t seen = behind & (inside | kept);
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) ov[j] = __float_as_uint(__uint_as_float(ov[j]) * corr);
-                        tmem_st32(acc + lane_addr + part * HDH + c0, ov);
-                    }
-                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                }
-                const float mref = m == -INFINITY ? 0.f : m * scale_log2e;   // nothing visible yet: exponents of -inf
-                float lsum = 0.f;
-                // P in bf16: [page of the tile][128 rows][128 bytes = 64 keys], 16-byte chunks of 8 keys written with
-                // the 128-byte swizzle of a K-major operand
-#pragma unroll
-                for (int hf = 0; hf < 2; ++hf) {
-                    if (hf < np) {
-                        const uint32_t prow = p_smem(b) + (uint32_t)hf * (BM * 128) + (uint32_t)(r / 8) * 1024u + (uint32_t)(r % 8) * 128u;
-#pragma unroll
-                        for (int ch = 0; ch < HK / 8; ++ch) {
-                            uint32_t packed[4];
-#pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                const int c = ch * 8 + 2 * e;
-                                const float a = ex2(fmaf(__uint_as_float(sv[hf][c]), scale_log2e, -mref));
-                                const float bq = ex2(fmaf(__uint_as_float(sv[hf][c + 1]), scale_log2e, -mref));
-                                lsum += a + bq;
-                                const __nv_bfloat162 pk = __floats2bfloat162_rn(a, bq);
-                                packed[e] = *reinterpret_cast<const uint32_t*>(&pk);
-                            }
-                            const uint32_t dst = prow + (uint32_t)(((part * (HK / 8) + ch) ^ (r % 8)) * 16);
-                            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(packed[0]), "r"(packed[1]),
-                                         "r"(packed[2]), "r"(packed[3]) : "memory");
+                            for (int c = 0; c < 32; ++c)
+                                if (!(seen & (1u << c))) sv[q][c] = 0xff800000u;
                         }
                     }
+                    float top[4] = {fmaxf(m, floor_m), -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+                    for (int c = 0; c < PAGE; ++c) top[c % 4] = fmaxf(top[c % 4], __uint_as_float(sv[c / 32][c % 32]));
+                    const float mx = fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3]));
+                    // keep m unless the maximum grew by more than 2^8 (or nothing had been seen yet)
+                    float corr = 1.0f;
+                    if (m == -INFINITY) {
+                        m = mx;                            // l, P and O are still zero: nothing to rescale
+                    } else if ((mx - m) * factor > RESCALE_LOG2) {
+                        corr = ex2((m - mx) * factor);
+                        l *= corr;
+                        m = mx;
+                    }
+                    if (__any_sync(0xffffffffu, corr != 1.0f)) {
+                        const float2 cc = make_float2(corr, corr);
+                        sum[0] = mul2(sum[0], cc);
+                        sum[1] = mul2(sum[1], cc);
+                        if (i > 0) {                       // the products so far are done (s_ready)
+#pragma unroll 1
+                            for (int c0 = 0; c0 < DV; c0 += 32) {
+                                uint32_t ov[32];
+                                tmem_ld32(acc + c0, ov);
+                                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                                for (int j = 0; j < 32; ++j) ov[j] = __float_as_uint(__uint_as_float(ov[j]) * corr);
+                                tmem_st32(acc + c0, ov);
+                            }
+                        }
+                        if (hf > 0) {                      // the tile's first page as well
+                            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                            uint32_t pv[32];
+                            tmem_ld32(s_addr, pv);
+                            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                            for (int j = 0; j < 32; ++j) {
+                                const float2 w = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pv[j]));
+                                const __nv_bfloat162 two = __floats2bfloat162_rn(w.x * corr, w.y * corr);
+                                pv[j] = *reinterpret_cast<const uint32_t*>(&two);
+                            }
+                            tmem_st32(s_addr, pv);
+                        }
+                    }
+                    const float mref = m == -INFINITY ? 0.f : m * factor;    // nothing visible yet: exponents of -inf
+                    const float2 ff = make_float2(factor, factor), neg = make_float2(-mref, -mref);
+                    uint32_t pk[32];
+#pragma unroll
+                    for (int e = 0; e < 32; ++e) {
+                        float2 x = fma2(make_float2(__uint_as_float(sv[e / 16][2 * e % 32]), __uint_as_float(sv[e / 16][2 * e % 32 + 1])), ff, neg);
+                        x = make_float2(ex2(x.x), ex2(x.y));
+                        sum[e % 2] = add2(sum[e % 2], x);
+                        const __nv_bfloat162 two = __floats2bfloat162_rn(x.x, x.y);
+                        pk[e] = *reinterpret_cast<const uint32_t*>(&two);
+                    }
+                    tmem_st32(s_addr + hf * 32, pk);
                 }
-                l += lsum;
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy writes -> visible to the MMA
+                l += (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
-                if (lane == 0) mbar_arrive(p_ready(b));
+                if (lane == 0) mbar_arrive(p_ready(slot));
             }
-            // the unit's products done: O / (the row's sum = the sum of its two threads' sums, same maximum m in both)
-            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(pv_done((ti - 1) & 1), (uint32_t)((ti - 1) >> 1) & 1u, &s_abort));
+            if (!ok) break;
+            // the unit's products done: O / the row's sum
+            ok = __all_sync(0xffffffffu, mbar_wait(o_done(slot), (uint32_t)units & 1u, &s_abort));
+            if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            // (a warp may be here while another still reads the previous unit's sums: wait for those reads first)
-            if (ok && it > 0) ok = __all_sync(0xffffffffu, mbar_wait(sums_read, (uint32_t)(it - 1) & 1u, &s_abort));
-            s_sums[part * BM + r] = l;
+            if (sink != nullptr) l += ex2((floor_m - m) * factor);
+            const float inv = 1.0f / l;
+            __nv_bfloat16* dst = out + ((size_t)(u.t0[slot] + r) * S.nh + h) * DV;
+            uint32_t ov[DV / 32][32];
+#pragma unroll
+            for (int c = 0; c < DV / 32; ++c) tmem_ld32(acc + c * 32, ov[c]);  // every lane takes part: the load is warp-wide
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive(sums_ready);
-            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(sums_ready, (uint32_t)it & 1u, &s_abort));
-            const float lrow = s_sums[r] + s_sums[BM + r];
-            __syncwarp();
-            if (lane == 0) mbar_arrive(sums_read);
-            if (ok) {
-                const float inv = 1.0f / lrow;
-                __nv_bfloat16* dst = out + ((size_t)(u.t0 + r) * nh + u.h) * HD + part * HDH;
+            if (lane == 0) mbar_arrive(o_free(slot));
+            if (r < u.rows[slot]) {
 #pragma unroll
-                for (int c0 = 0; c0 < HDH; c0 += 32) {
-                    uint32_t ov[32];
-                    tmem_ld32(acc + lane_addr + part * HDH + c0, ov);      // every lane takes part: the load is warp-wide
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    if (r < u.rows) {
+                for (int d = 0; d < DV; d += 8) {
+                    uint32_t packed[4];
 #pragma unroll
-                        for (int d = 0; d < 32; d += 8) {
-                            uint32_t packed[4];
-#pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                const __nv_bfloat162 pk = __floats2bfloat162_rn(__uint_as_float(ov[d + 2 * e]) * inv,
-                                                                                __uint_as_float(ov[d + 2 * e + 1]) * inv);
-                                packed[e] = *reinterpret_cast<const uint32_t*>(&pk);
-                            }
-                            *reinterpret_cast<uint4*>(dst + c0 + d) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-                        }
+                    for (int e = 0; e < 4; ++e) {
+                        const int c = d + 2 * e;
+                        const __nv_bfloat162 two = __floats2bfloat162_rn(__uint_as_float(ov[c / 32][c % 32]) * inv,
+                                                                         __uint_as_float(ov[c / 32][c % 32 + 1]) * inv);
+                        packed[e] = *reinterpret_cast<const uint32_t*>(&two);
                     }
+                    *reinterpret_cast<uint4*>(dst + d) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
                 }
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");   // the reads of O are ordered before the next arrivals
             }
-            ++it;
+            ++units;
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 1) {
+    if (warp == 9) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(s_tmem_base), "r"((uint32_t)C::TMEM_COLS) : "memory");
     }
@@ -556,60 +744,79 @@ int make_map(CUtensorMap* map, const void* ptr, uint64_t rows, uint64_t cols, ui
     return 0;
 }
 
-template <int HD>
-int launch(const CUtensorMap& mq, const CUtensorMap& mkv, const int* cu, const int* starts, const int* table,
-           int table_stride, int window, float scale, void* out, int n_seqs, int max_q_len, int nh, int nkv, int* status,
-           cudaStream_t stream) {
-    using C = Cfg<HD>;
-    auto kern = attention_prefill_kernel<HD>;
+struct Maps { CUtensorMap q, k, r, v; };
+struct Args {
+    const int *cu, *starts, *table, *page_base;
+    const float *bias_t, *sink;
+    void* out;
+    int* status;
+};
+
+template <int DK, int DV, bool SHAPED>
+int launch(const Maps& m, const Shape& S, const Args& a, cudaStream_t stream) {
+    using C = Cfg<DK, DV>;
+    auto kern = attention_prefill_kernel<DK, DV, SHAPED>;
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
         if (e != cudaSuccess) TQ_FAIL(-1, "attention_prefill: cannot reserve %d bytes of shared memory: %s", C::SMEM_BYTES, cudaGetErrorString(e));
         configured = true;
     }
-    static int n_sm = 0;
-    if (n_sm == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n_sm <= 0) n_sm = 148;
-    }
-    // persistent CTAs, one per SM at most: each walks its units (query tile x sequence x head)
-    const int n_qt = (max_q_len + BM - 1) / BM;
-    const long long units = (long long)n_qt * n_seqs * nh;
-    const int grid = (int)(units < n_sm ? units : n_sm);
-    tq_launch(grid, THREADS, C::SMEM_BYTES, stream)(kern, mq, mkv, cu, starts, table, table_stride, window,
-                                                   scale * 1.4426950408889634f, (__nv_bfloat16*)out, nh, nkv, n_qt, n_seqs, status);
+    // a block per unit; those that run take over the ones that have not started
+    const int hs = S.pairing == PAIR_HEADS ? S.nh / 2 : S.nh, qs = S.pairing == PAIR_HEADS ? S.n_qt : (S.n_qt + 1) / 2;
+    const int grid = qs * S.n_seqs * hs;
+    tq_launch(grid, THREADS, C::SMEM_BYTES, stream)(kern, m.q, m.k, m.r, m.v, S, a.cu, a.starts, a.table, a.page_base, a.bias_t, a.sink,
+                                                   (__nv_bfloat16*)a.out, a.status);
     TQ_CHECK_LAUNCH("attention_prefill");
+    return 0;
+}
+
+int check_common(const Shape& S, int T_, int max_q_len, const void* q, const void* k, const void* v, const void* out, const int* status) {
+    TQ_REQUIRE(S.nkv >= 1 && S.nh % S.nkv == 0, "attention_prefill: %d heads are not a multiple of %d key/value heads", S.nh, S.nkv);
+    TQ_REQUIRE((long long)S.n_qt * S.n_seqs * S.nh < (1ll << 30), "attention_prefill: too many units of work");
+    TQ_REQUIRE(S.window >= 0 && S.keep_first >= 0 && S.cell >= 0 && S.far >= 0 && max_q_len >= 1 && T_ >= 1,
+               "attention_prefill: bad window %d, kept positions %d, cell %d or longest run %d", S.window, S.keep_first, S.cell, max_q_len);
+    TQ_REQUIRE(((uintptr_t)q % 16) == 0 && ((uintptr_t)k % 16) == 0 && ((uintptr_t)v % 16) == 0 && ((uintptr_t)out % 16) == 0,
+               "attention_prefill: q, cache and out must be 16-byte aligned");
+    TQ_REQUIRE(status != nullptr, "attention_prefill: a status word is required");
     return 0;
 }
 
 }  // namespace
 
-// q [T, nh, hd] bf16; cache [n_pages, 2, nkv, 64, hd] bf16 (keys and values of this step already written);
-// out [T, nh*hd] bf16.  cu_seqlens [n_seqs+1]: rows of each sequence in q; seq_start [n_seqs]: position of
-// each sequence's first row.  status: one int in device memory, set to 1 if a bounded wait ran out.
-TQ_EXPORT int tq_attention_prefill(const void* q, const void* cache, const int* cu_seqlens, const int* seq_start,
-                                   const int* page_table, int table_stride, int page_size, int n_pages, int window,
-                                   float scale, void* out, int T_, int n_seqs, int max_q_len, int nh, int nkv, int hd,
-                                   int* status, cudaStream_t stream) {
+// q [T, nh, dk] bf16; cache bf16 (keys and values of this step already written): planes 2: [n_pages, 2, nkv, 64, dk] with
+// dk == dv, planes 1: [n_pages, nkv, 64, dk + dv], a position's key followed by its value; out [T, nh*dv].
+// cu_seqlens [n_seqs+1]: rows of each sequence in q; seq_start [n_seqs]: position of each sequence's first row.
+// Position i sees j <= i with window == 0 or i - j < window or j < keep_first; with cell > 0 instead j <= i of its own
+// cell.  Scores times scale, capped (softcap > 0), plus bias_t [nh][far + 1] (or null) at distance min(i - j, far); sink
+// [nh] or null joins the denominator.  status: one int in device memory, set to 1 if a bounded wait ran out.
+TQ_EXPORT int tq_attention_prefill(const void* q, const void* cache, int planes, const int* cu_seqlens, const int* seq_start,
+                                   const int* page_table, int table_stride, int page_size, int n_pages, int window, int keep_first,
+                                   int cell, float scale, float softcap, const float* bias_t, int far, const float* sink, void* out,
+                                   int T_, int n_seqs, int max_q_len, int nh, int nkv, int dk, int dv, int* status, cudaStream_t stream) {
     if (T_ == 0 || n_seqs == 0) return 0;
-    TQ_REQUIRE(hd == 64 || hd == 128, "attention_prefill: head size %d is not 64 or 128", hd);
+    TQ_REQUIRE((dk == 64 || dk == 128) && (dv == 64 || dv == 128), "attention_prefill: key size %d or value size %d is not 64 or 128", dk, dv);
+    TQ_REQUIRE(planes == 1 || (planes == 2 && dk == dv), "attention_prefill: %d planes of keys of %d and values of %d", planes, dk, dv);
     TQ_REQUIRE(page_size == PAGE, "attention_prefill: page size %d must be %d", page_size, PAGE);
-    TQ_REQUIRE(nkv >= 1 && nh % nkv == 0, "attention_prefill: %d heads are not a multiple of %d key/value heads", nh, nkv);
-    TQ_REQUIRE((long long)((max_q_len + BM - 1) / BM) * n_seqs * nh < (1ll << 30), "attention_prefill: too many units of work");
-    TQ_REQUIRE(window >= 0 && max_q_len >= 1, "attention_prefill: bad window %d or longest run %d", window, max_q_len);
-    TQ_REQUIRE(((uintptr_t)q % 16) == 0 && ((uintptr_t)cache % 16) == 0 && ((uintptr_t)out % 16) == 0,
-               "attention_prefill: q, cache and out must be 16-byte aligned");
-    TQ_REQUIRE(status != nullptr, "attention_prefill: a status word is required");
-    CUtensorMap mq, mkv;
-    int rc = make_map(&mq, q, (uint64_t)T_, (uint64_t)nh * hd, BM);
+    Shape S{};
+    S.nh = nh; S.nkv = nkv; S.n_seqs = n_seqs; S.n_qt = (max_q_len + BM - 1) / BM;
+    S.kp = planes * nkv * PAGE; S.kg = PAGE; S.v_plane = (planes - 1) * nkv * PAGE; S.v_col = planes == 1 ? dk : 0; S.k_blocks = dk / 64;
+    S.table_stride = table_stride; S.n_pages = n_pages; S.window = window; S.keep_first = keep_first; S.cell = cell; S.far = far;
+    S.scale = scale; S.softcap = softcap;
+    int rc = check_common(S, T_, max_q_len, q, cache, cache, out, status);
     if (rc) return rc;
-    rc = make_map(&mkv, cache, (uint64_t)n_pages * 2 * nkv * PAGE, (uint64_t)hd, PAGE);
+    TQ_REQUIRE((long long)n_pages * S.kp < (1ll << 31), "attention_prefill: a cache of %d pages is too large for one tensor map", n_pages);
+    S.pairing = nh / nkv % 2 == 0 ? PAIR_HEADS : PAIR_ROWS;
+    Maps m;
+    rc = make_map(&m.q, q, (uint64_t)T_, (uint64_t)nh * dk, BM);
     if (rc) return rc;
-    if (hd == 64)
-        return launch<64>(mq, mkv, cu_seqlens, seq_start, page_table, table_stride, window, scale, out, n_seqs, max_q_len,
-                          nh, nkv, status, stream);
-    return launch<128>(mq, mkv, cu_seqlens, seq_start, page_table, table_stride, window, scale, out, n_seqs, max_q_len,
-                       nh, nkv, status, stream);
+    rc = make_map(&m.k, cache, (uint64_t)n_pages * S.kp, (uint64_t)(planes == 1 ? dk + dv : dk), PAGE);
+    if (rc) return rc;
+    m.r = m.v = m.k;
+    const Args a{cu_seqlens, seq_start, page_table, nullptr, bias_t, sink, out, status};
+    const bool shaped = softcap > 0.f || bias_t != nullptr || !(scale > 0.f);     // the other form compares unscaled scores
+#define AP_CASE(DK_, DV_) if (dk == DK_ && dv == DV_) return shaped ? launch<DK_, DV_, true>(m, S, a, stream) : launch<DK_, DV_, false>(m, S, a, stream);
+    AP_CASE(64, 64) AP_CASE(64, 128) AP_CASE(128, 64) AP_CASE(128, 128)
+#undef AP_CASE
+    return -2;
 }

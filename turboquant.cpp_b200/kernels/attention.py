@@ -204,17 +204,30 @@ def attention_prefill(q: torch.Tensor, cache_layer: torch.Tensor, cu_seqlens: to
     cores (csrc/attention_prefill.cu).  Row t of q belongs to the sequence whose [cu_seqlens[i],
     cu_seqlens[i+1]) holds t and sits at position seq_start[i] + (t - cu_seqlens[i]); the step's keys
     and values are already in the cache."""
+    if not prefill_usable(q.dtype, head_dim, page_size):
+        raise KernelError("attention_prefill: needs bfloat16, head size 64 or 128 and pages of 64 tokens")
+    return prefill_rows(q, cache_layer, 2, cu_seqlens, seq_start, page_table, page_size, window, scale, out, n_seqs, max_q_len,
+                        n_heads, n_kv_heads, head_dim, head_dim, status=status)
+
+
+def prefill_rows(q: torch.Tensor, cache_layer: torch.Tensor, planes: int, cu_seqlens: torch.Tensor, seq_start: torch.Tensor,
+                 page_table: torch.Tensor, page_size: int, window: int, scale: float, out: torch.Tensor, n_seqs: int, max_q_len: int,
+                 n_heads: int, n_kv_heads: int, dk: int, dv: int, keep_first: int = 0, cell: int = 0, softcap: float = 0.0,
+                 bias_t: Optional[torch.Tensor] = None, sink: Optional[torch.Tensor] = None,
+                 status: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """The tensor-core prompt kernel over a cache of two planes (keys, values) or one (rows [key | value]), with the
+    options of `kernels.bias_attention.attention_runs`."""
     from .gemm_tc import status_word
-    T = q.shape[0]
     want_int32(cu_seqlens, "cu_seqlens")
     want_int32(seq_start, "seq_start")
     want_int32(page_table, "page table")
-    if not prefill_usable(q.dtype, head_dim, page_size) or cache_layer.dtype != torch.bfloat16 or out.dtype != torch.bfloat16:
-        raise KernelError("attention_prefill: needs bfloat16, head size 64 or 128 and pages of 64 tokens")
+    if q.dtype != torch.bfloat16 or cache_layer.dtype != torch.bfloat16 or out.dtype != torch.bfloat16:
+        raise KernelError("attention_prefill: queries, cache and output must be bfloat16")
     lib = load_kernel("attention_prefill")
     check("attention_prefill", lib.tq_attention_prefill(
-        ptr(q), ptr(cache_layer), ptr(cu_seqlens), ptr(seq_start), ptr(page_table), c_int(page_table.shape[1]),
-        c_int(page_size), c_int(cache_layer.shape[0]), c_int(window), c_float(scale), ptr(out), c_int(T), c_int(n_seqs),
-        c_int(max_q_len), c_int(n_heads), c_int(n_kv_heads), c_int(head_dim),
+        ptr(q), ptr(cache_layer), c_int(planes), ptr(cu_seqlens), ptr(seq_start), ptr(page_table), c_int(page_table.shape[1]),
+        c_int(page_size), c_int(cache_layer.shape[0]), c_int(window), c_int(keep_first), c_int(cell), c_float(scale), c_float(softcap),
+        ptr(bias_t), c_int(0 if bias_t is None else bias_t.shape[1] - 1), ptr(sink), ptr(out), c_int(q.shape[0]), c_int(n_seqs),
+        c_int(max_q_len), c_int(n_heads), c_int(n_kv_heads), c_int(dk), c_int(dv),
         ptr(status if status is not None else status_word(q.device)), stream()))
     return out

@@ -9,6 +9,7 @@ import torch
 
 from ..csrc.build import load_kernel
 from ._call import KernelError, check, code, ptr, stream, want_f32, want_int32
+from .attention import prefill_rows
 
 _LIB = "bias_attention"
 MAX_DIM = 256        # csrc/bias_attention.cu BA_MAX_DIM: the most elements of a key or of a value
@@ -157,9 +158,11 @@ def runs_usable(dtype: torch.dtype, dk: int, dv: int, page_size: int) -> bool:
 def attention_runs(q: torch.Tensor, cache: torch.Tensor, bias_t: Optional[torch.Tensor], sink: Optional[torch.Tensor],
                    cu_seqlens: torch.Tensor, seq_start: torch.Tensor, page_table: torch.Tensor, page_size: int,
                    window: int, keep_first: int, scale: float, out: torch.Tensor, n_seqs: int, max_run: int,
-                   heads: int, kv_heads: int, dk: int, dv: int, softcap: float = 0.0, cell: int = 0) -> torch.Tensor:
-    """The same attention for steps with runs of new tokens (prompts), bfloat16 on tensor cores: blocks of 64
-    queries of a (sequence, head) walk the pages they can see.  bias_t float32 [heads, far + 1]: the bias per head
+                   heads: int, kv_heads: int, dk: int, dv: int, softcap: float = 0.0, cell: int = 0,
+                   status: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """The same attention for steps with runs of new tokens (prompts), bfloat16 on tensor cores: the tcgen05 kernel of
+    csrc/attention_prefill.cu for keys and values of 64 or 128 (`status`: the word its bounded waits report to), else
+    blocks of 64 queries of a (sequence, head) that walk the pages they can see.  bias_t float32 [heads, far + 1]: the bias per head
     and distance (the transpose of what `attention` takes).  softcap > 0: the scaled score s becomes
     softcap * tanh(s / softcap) before the bias.  cell > 0: instead of the window, position i sees
     j <= i of its own cell only (i // cell == j // cell)."""
@@ -171,6 +174,9 @@ def attention_runs(q: torch.Tensor, cache: torch.Tensor, bias_t: Optional[torch.
         far = bias_t.shape[1] - 1
     if sink is not None:
         want_f32(sink, "the sink")
+    if dk >= 64 and dv >= 64 and runs_usable(q.dtype, dk, dv, page_size):
+        return prefill_rows(q, cache, 1, cu_seqlens, seq_start, page_table, page_size, window, scale, out, n_seqs, max_run, heads,
+                            kv_heads, dk, dv, keep_first=keep_first, cell=cell, softcap=softcap, bias_t=bias_t, sink=sink, status=status)
     lib = load_kernel(_LIB)
     check(_LIB, lib.tq_bias_attention_runs(
         ptr(q), ptr(cache), c_int(code(q.dtype)), ptr(bias_t), c_int(far), ptr(sink), ptr(cu_seqlens), ptr(seq_start),

@@ -62,7 +62,7 @@ def paged_attention(q: torch.Tensor, cache: LayerCache, ctx: StepContext, heads:
     if ctx.max_q_len >= runs_min and KB.runs_usable(act, dim, vdim, cache.page_size):
         return KB.attention_runs(q, cache.kv, bias_t, sink, ctx.cu_seqlens, ctx.seq_start, cache.page_table, cache.page_size,
                                  window, keep_first, scale, o, ctx.n_seqs, ctx.max_q_len, heads, kv_heads, dim, vdim,
-                                 softcap=softcap, cell=cell)
+                                 softcap=softcap, cell=cell, status=ctx.status)
     if cell:
         longest = min(cell, ctx.max_kv_len)
     else:
@@ -153,7 +153,7 @@ class BiasedWindowAttentionMixer(Mixer):
             self.mix = float(store.get(p + "vmix").float().item())
 
     def kernels(self) -> List[str]:
-        return ["bias_attention"] + (["gemv"] if getattr(self, "run_dtype", None) == torch.bfloat16 else [])
+        return ["bias_attention"] + (["attention_prefill", "gemv"] if getattr(self, "run_dtype", None) == torch.bfloat16 else [])
 
     def cache_need(self) -> KVNeed:
         return KVNeed(self.kv_heads, self.dim + self.vdim, self.window, planes=1, keep_first=self.keep_first)
