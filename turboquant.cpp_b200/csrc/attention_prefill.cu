@@ -22,9 +22,12 @@
 //   warp 8        TMA: Q of both slots, then K and V pages through rings that both slots read
 //   warp 9        owns tensor memory, issues  O += P V  of a slot's tile and right behind it  S = Q K^T  of its next
 // The two slots take turns: while one's scores are exponentiated the other's products run, which is what bounds a
-// tile pair: 2 x 16,384 exponentials at 16 a cycle and SM (2,048 cycles) beside 32 products of 128 x 128 x 16.  With one
-// slot (the eight warps sharing one tile, P through shared memory) a 128 x 128 tile took 6,000 cycles, because
-// nothing ran beside its chain of product, maximum, exponentials, product.
+// tile pair: 2 x 16,384 exponentials at 16 a cycle and SM (2,048 cycles) beside 32 products of 128 x 128 x 16 (2,048).
+// Measured: 3,450 cycles a pair (softmax 1,950, then 1,400 until the slot's next scores are there), with a bias 5,250, with a
+// cap 6,400; with one slot (eight warps on one tile, P through shared memory, products issued by one lane) 6,000 a tile.
+// Prompts of 682 + 1,365 + 2,049 tokens, 16 heads of 128: 84.5 -> 57.5 us (16 kv heads, plain), 457 -> 80.8 us (4 kv
+// heads, cap 50) where the mma.sync kernel of csrc/bias_attention.cu served the second; 2,048 tokens, window 1,024 with a bias:
+// 97.3 -> 44.5 us.
 // Every wait on an mbarrier is bounded; a wait that runs out sets *status and the CTA
 // leaves cleanly.
 #include <cuda.h>
@@ -145,18 +148,20 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
           "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
         : "r"(taddr));
 }
-
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
     asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-        "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
-        ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
-          "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]),
-          "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]),
-          "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+        ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
+          "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
         : "memory");
 }
-
 constexpr int PAGE = 64;     // tokens per cache page
 constexpr int BN = 128;      // keys per tile = two cache pages (a unit's last tile may hold one)
 constexpr float LOG2E = 1.4426950408889634f;
@@ -234,31 +239,57 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return tq
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return tq_unpack2(tq_mul2(tq_pack2(a.x, a.y), tq_pack2(b.x, b.y))); }
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return tq_unpack2(tq_add2(tq_pack2(a.x, a.y), tq_pack2(b.x, b.y))); }
 
-// softcap * tanh(s / softcap) of 32 scores times `scale`: the odd series up to x^9 where every score of the warp's rows lies
-// below a quarter of the cap (the first term left out is 4e-9 of the result there), the exponential form beyond.
-__device__ __forceinline__ void cap_scores(uint32_t (&v)[32], float scale, float cap, float inv_cap) {
-    const float k = scale * inv_cap;
-    float top = 0.f, top2 = 0.f;
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+// the largest of 32 values and `from`
+__device__ __forceinline__ float max_of(const uint32_t (&v)[32], float from) {
+    float top[2] = {from, __uint_as_float(v[0])};
 #pragma unroll
-    for (int c = 0; c < 32; c += 2) { top = fmaxf(top, fabsf(__uint_as_float(v[c]))); top2 = fmaxf(top2, fabsf(__uint_as_float(v[c + 1]))); }
-    const bool beyond = __any_sync(0xffffffffu, !(fmaxf(top, top2) * fabsf(k) <= 0.25f));
-    const float2 kk = make_float2(k, k), cc = make_float2(cap, cap);
-    const float2 c9 = make_float2(62.0f / 2835.0f, 62.0f / 2835.0f), c7 = make_float2(-17.0f / 315.0f, -17.0f / 315.0f),
-                 c5 = make_float2(2.0f / 15.0f, 2.0f / 15.0f), c3 = make_float2(-1.0f / 3.0f, -1.0f / 3.0f), one = make_float2(1.f, 1.f);
-    if (!beyond) {
+    for (int c = 1; c < 31; c += 2) top[c / 2 % 2] = max3(top[c / 2 % 2], __uint_as_float(v[c]), __uint_as_float(v[c + 1]));
+    return max3(top[0], top[1], __uint_as_float(v[31]));
+}
+
+// softcap * tanh(s * scale / softcap) of 32 scores: the odd series up to x^9, x = s * scale / softcap, where every x of the
+// warp's rows lies below a quarter (the first term left out is 4e-9 of the result there), the exponential form beyond.
+// p: the series' coefficients in powers of s^2, times scale.
+struct CapSeries { float p[5], k, cap; };
+__device__ __forceinline__ CapSeries cap_series(float scale, float cap) {
+    CapSeries r;
+    r.cap = cap;
+    r.k = scale / cap;
+    const float k2 = r.k * r.k;
+    r.p[0] = scale;
+    r.p[1] = -1.0f / 3.0f * k2 * scale;
+    r.p[2] = 2.0f / 15.0f * k2 * k2 * scale;
+    r.p[3] = -17.0f / 315.0f * k2 * k2 * k2 * scale;
+    r.p[4] = 62.0f / 2835.0f * k2 * k2 * k2 * k2 * scale;
+    return r;
+}
+__device__ __forceinline__ void cap_scores(uint32_t (&v)[32], const CapSeries& s) {
+    float top = 0.f;
+#pragma unroll
+    for (int c = 0; c < 32; c += 2) top = max3(top, fabsf(__uint_as_float(v[c])), fabsf(__uint_as_float(v[c + 1])));
+    // (the maximum passes over NaN: such a score stays NaN in either form)
+    if (!__any_sync(0xffffffffu, !(top * fabsf(s.k) <= 0.25f))) {
 #pragma unroll
         for (int c = 0; c < 32; c += 2) {
-            const float2 x = mul2(make_float2(__uint_as_float(v[c]), __uint_as_float(v[c + 1])), kk), x2 = mul2(x, x);
-            const float2 t = mul2(mul2(cc, x), fma2(x2, fma2(x2, fma2(x2, fma2(x2, c9, c7), c5), c3), one));
+            const float2 x = make_float2(__uint_as_float(v[c]), __uint_as_float(v[c + 1])), x2 = mul2(x, x);
+            float2 t = make_float2(s.p[4], s.p[4]);
+#pragma unroll
+            for (int j = 3; j >= 0; --j) t = fma2(x2, t, make_float2(s.p[j], s.p[j]));
+            t = mul2(x, t);
             v[c] = __float_as_uint(t.x);
             v[c + 1] = __float_as_uint(t.y);
         }
     } else {
 #pragma unroll
         for (int c = 0; c < 32; ++c) {
-            const float x = __uint_as_float(v[c]) * k, x2 = x * x;
-            const float near = x * fmaf(x2, fmaf(x2, fmaf(x2, fmaf(x2, c9.x, c7.x), c5.x), c3.x), 1.0f);
-            v[c] = __float_as_uint(cap * (fabsf(x) <= 0.25f ? near : 1.0f - __fdividef(2.0f, __expf(2.0f * x) + 1.0f)));
+            const float f = __uint_as_float(v[c]), x = f * s.k, f2 = f * f;
+            const float near = f * fmaf(f2, fmaf(f2, fmaf(f2, fmaf(f2, s.p[4], s.p[3]), s.p[2]), s.p[1]), s.p[0]);
+            v[c] = __float_as_uint(fabsf(x) <= 0.25f ? near : s.cap * (1.0f - __fdividef(2.0f, __expf(2.0f * x) + 1.0f)));
         }
     }
 }
@@ -340,9 +371,9 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     // Tile number `ti`, counted across units, picks the K and V
     // stages and their barriers' phases; a slot's tiles and units, counted for the slot, the phases of its own.
     if (warp >= 8) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
-    if (warp == 8) {
-        // ------------------------------ TMA producer ------------------------------
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+        if (warp == 8) {
+            // ------------------------------ TMA producer ------------------------------
             const uint32_t elected = elect_one();
             int ti = 0, vi = 0, asked = 0, units[2] = {0, 0};
             bool ok = true, pending = false;
@@ -351,7 +382,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 if (elected) {
                     mbar_expect_tx(answered, 16);
                     asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
-                                 ::"r"(smem_u32(&s_answer)), "r"(answered) : "memory");
+                        ::"r"(smem_u32(&s_answer)), "r"(answered) : "memory");
                 }
                 pending = true;
             };
@@ -362,11 +393,11 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 uint32_t x, got;
                 asm volatile(
                     "{\n\t.reg .b128 h;\n\t.reg .pred p;\n\t"
-                    "ld.shared.b128 h, [%2];\n\t"
-                    "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\t"
-                    "selp.u32 %1, 1, 0, p;\n\t"
-                    "mov.u32 %0, 0;\n\t"
-                    "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, h;\n\t}"
+                        "ld.shared.b128 h, [%2];\n\t"
+                        "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\t"
+                        "selp.u32 %1, 1, 0, p;\n\t"
+                        "mov.u32 %0, 0;\n\t"
+                        "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, h;\n\t}"
                     : "=r"(x), "=r"(got) : "r"(smem_u32(&s_answer)) : "memory");
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // this read before the next answer is written
                 __syncwarp();
@@ -388,7 +419,6 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             int unit = settle(blockIdx.x);
             hand_on(0, unit);
             for (int k = 0; ok && unit >= 0; ++k) {
-                ask();
                 int following = -1;
                 const Unit u = unit_of(unit, S, cu_seqlens, seq_start);
                 auto load_q = [&](int s) {
@@ -396,9 +426,9 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                     // the products that read the slot's previous Q must be done
                     if (units[s] > 0 && !wait(q_free(s), (uint32_t)(units[s] - 1) & 1u)) return false;
                     if (elected) {
-                    mbar_expect_tx(q_full(s), (uint32_t)C::Q_BYTES);
+                        mbar_expect_tx(q_full(s), (uint32_t)C::Q_BYTES);
 #pragma unroll
-                    for (int c = 0; c < C::KB; ++c) tma_load_2d(q_smem(s) + c * (BM * 128), &map_q, u.h[s] * DK + c * 64, u.t0[s], q_full(s));
+                        for (int c = 0; c < C::KB; ++c) tma_load_2d(q_smem(s) + c * (BM * 128), &map_q, u.h[s] * DK + c * 64, u.t0[s], q_full(s));
                     }
                     ++units[s];
                     return true;
@@ -406,6 +436,9 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 ok = load_q(0);
                 if (!ok) break;
                 for (int i = 0; i < u.n_tiles; ++i, ++ti) {
+                    // asked for at the unit's last tile, not before: a CTA that took its next unit when it began a long
+                    // one held 24 tiles where others held 6
+                    if (i + 1 == u.n_tiles) ask();
                     const int np = min(2, u.n_pages - 2 * i);
                     int page[2] = {0, 0};
                     for (int pg = 0; pg < np; ++pg) {
@@ -418,10 +451,10 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                     const int ks = ti % C::KST;
                     if (!wait(k_empty(ks), ((uint32_t)(ti / C::KST) & 1u) ^ 1u)) { ok = false; break; }
                     if (elected) {
-                    mbar_expect_tx(k_full(ks), (uint32_t)(np * C::K_PAGE));
-                    for (int pg = 0; pg < np; ++pg)
+                        mbar_expect_tx(k_full(ks), (uint32_t)(np * C::K_PAGE));
+                        for (int pg = 0; pg < np; ++pg)
 #pragma unroll
-                        for (int c = 0; c < C::KB; ++c) {
+                            for (int c = 0; c < C::KB; ++c) {
                             const uint32_t dst = k_smem(ks) + c * (BN * 128) + pg * (PAGE * 128);
                             if (c < S.k_blocks) tma_load_2d(dst, &map_k, u.g * S.kc + c * 64, page[pg] * S.kp + u.g * S.kg, k_full(ks));
                             else tma_load_2d(dst, &map_r, (c - S.k_blocks) * 64, page[pg] * S.kp, k_full(ks));
@@ -431,15 +464,15 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                     const int vs = ti % C::VST;
                     if (!wait(v_empty(vs), ((uint32_t)(ti / C::VST) & 1u) ^ 1u)) { ok = false; ++ti; break; }
                     if (elected) {
-                    mbar_expect_tx(v_full(vs), (uint32_t)(np * C::V_PAGE));
-                    for (int pg = 0; pg < np; ++pg)
+                        mbar_expect_tx(v_full(vs), (uint32_t)(np * C::V_PAGE));
+                        for (int pg = 0; pg < np; ++pg)
 #pragma unroll
-                        for (int c = 0; c < C::VB; ++c)
+                            for (int c = 0; c < C::VB; ++c)
                             tma_load_2d(v_smem(vs) + c * (BN * 128) + pg * (PAGE * 128), &map_v, S.v_col + u.g * S.vc + c * 64,
-                                        page[pg] * S.kp + u.g * S.kg + S.v_plane, v_full(vs));
+                            page[pg] * S.kp + u.g * S.kg + S.v_plane, v_full(vs));
                     }
                     vi = ti + 1;
-                    if (i == 0) {                              // the MMA warp looks one unit ahead: it must know before this one's last tile
+                    if (i + 1 == u.n_tiles) {
                         following = settle(answer());
                         if (ok) hand_on(k + 1, following);
                         if (!ok) { ++ti; break; }
@@ -456,11 +489,11 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 for (int i = vi > C::VST ? vi - C::VST : 0; i < vi; ++i)
                     for (uint32_t j = 0; j < WAIT_LIMIT && !mbar_try_wait(v_full(i % C::VST), (uint32_t)(i / C::VST) & 1u); ++j) {}
             }
-    } else if (warp == 9) {
-        // ------------------------------ MMA issuer ------------------------------
-        // Tile by tile, slot by slot: the slot's P V product of this tile as soon as its P is there, then its scores of
-        // the next tile (which may be the next unit's first): products are carried out in the order they are issued,
-        // so the scores overwrite a P that has been read.
+        } else if (warp == 9) {
+            // ------------------------------ MMA issuer ------------------------------
+            // Tile by tile, slot by slot: the slot's P V product of this tile as soon as its P is there, then its scores of
+            // the next tile (which may be the next unit's first): products are carried out in the order they are issued,
+            // so the scores overwrite a P that has been read.
             const uint32_t elected = elect_one(), id_o = idesc(DV, 1);
             const uint32_t tm = __shfl_sync(0xffffffffu, s_tmem_base, 0);
             int ti = 0, taken = 0, tiles[2] = {0, 0}, units[2] = {0, 0};
@@ -495,9 +528,10 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                     if (u.n[s]) ok = issue_qk(u, 0, 0, s, s == 0 || u.n[0] == 0, s == 1 || u.n[1] == 0);
             }
             while (more && ok) {
-                const bool follows = next_unit(v);
+                bool follows = false;
                 for (int i = 0; i < u.n_tiles && ok; ++i, ++ti) {
                     const bool crosses = i + 1 == u.n_tiles;             // the next tile is the next unit's first
+                    if (crosses) follows = next_unit(v);
                     const int np = min(2, u.n_pages - 2 * i), st = ti % C::VST;
                     const int n0 = crosses ? (follows ? v.n[0] : 0) : u.n[0], n1 = crosses ? (follows ? v.n[1] : 0) : u.n[1];
                     const int j = crosses ? 0 : i + 1;                   // the next tile within its unit
@@ -513,7 +547,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
 #pragma unroll
                             for (int k = 0; k < BN / 16; ++k)            // O += P V, 16 keys at a time (a unit's first tile starts the sum)
                                 if (k < PAGE / 16 || np > 1)             // a missing second page is not read
-                                    umma_ts(o, p + (uint32_t)(k * 8), vd + k * 128, id_o, (i > 0 || k > 0) ? 1u : 0u, elected);
+                                umma_ts(o, p + (uint32_t)(k * 8), vd + k * 128, id_o, (i > 0 || k > 0) ? 1u : 0u, elected);
                             if (s == 1 || i >= u.n[1]) umma_commit(v_empty(st), elected);
                             ++tiles[s];
                             if (i == u.n[s] - 1) { umma_commit(o_done(s), elected); ++units[s]; }
@@ -524,16 +558,18 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 more = follows;
                 u = v;
             }
-    }
+        }
     } else {
         // ------------------------------ softmax: a thread per query row ------------------------------
         asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
+        constexpr int CW = SHAPED ? 1 : 2;            // 32-key pieces a thread takes at a time
         constexpr float RESCALE_LOG2 = 8.0f;          // O is rescaled when a row's maximum has grown by more than 2^8
         const int slot = warp >> 2, quarter = warp & 3, r = quarter * 32 + lane;
         const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
         const uint32_t s_addr = tmem_s(slot) + lane_addr, acc = tmem_o(slot) + lane_addr;
         const float factor = SHAPED ? LOG2E : S.scale * LOG2E;            // from a score as it stands to an exponent of two
-        const float inv_cap = SHAPED && S.softcap > 0.f ? 1.0f / S.softcap : 0.f;
+        const bool capped = SHAPED && S.softcap > 0.f;
+        const CapSeries series = cap_series(S.scale, capped ? S.softcap : 1.f);
         int tiles = 0, units = 0, taken = 0;
         bool ok = true;
         for (int unit = take_unit(taken++); ok && unit >= 0; unit = ok ? take_unit(taken++) : -1) {
@@ -555,8 +591,9 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 }
             };
             if (SHAPED && bias != nullptr) fetch_bias(0);
-            // m: the maximum the row's exponentials are taken against; l: the sum of its exponentials
-            const float floor_m = sink != nullptr ? sink[h] * (LOG2E / factor) : -INFINITY;
+            // m: what the row's exponents of two are counted from, its maximum or up to RESCALE_LOG2 below it; l: the sum of
+            // its exponentials
+            const float floor_m = sink != nullptr ? sink[h] * LOG2E : -INFINITY;
             float m = -INFINITY, l = 0.f;
             for (int i = 0; i < n; ++i, ++tiles) {
                 const int np = min(2, u.n_pages - 2 * i);
@@ -570,101 +607,111 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 ok = __all_sync(0xffffffffu, mbar_wait(s_ready(slot), (uint32_t)tiles & 1u, &s_abort));   // warp-uniform
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                // a page at a time, in one pass: shape and mask its scores, see whether they outgrow the maximum the row's
-                // exponentials are taken against, and write them, in bf16, over scores already read.  The loop is kept:
-                // unrolled, its code does not fit the instruction caches that ten warps share (1.6 times the time).
+                // half a page (plain scores: a page) at a time, in one pass: shape and mask its scores, see whether they outgrow the maximum the row's
+                // exponentials are taken against, and write them, in bf16, over scores already read.  The loop is kept
+                // small: instructions come in at some 250 cycles per 128 bytes the first time and fall out of the caches
+                // that ten warps share (the tile unrolled in two passes: 1.6 times the kernel's time).
                 float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll 1
-                for (int hf = 0; hf < np; ++hf) {
-                    uint32_t sv[2][32];
-                    tmem_ld32(s_addr + hf * PAGE, sv[0]);
-                    tmem_ld32(s_addr + hf * PAGE + 32, sv[1]);
+                for (int x = i == 0 ? -2 * np : 0; x < 2 * np; x += CW) {
+                    const int q = x < 0 ? x + 2 * np : x;  // a unit's first tile is walked once ahead for its maximum alone
+                    uint32_t sv[CW][32];
+#pragma unroll
+                    for (int w = 0; w < CW; ++w) tmem_ld32(s_addr + (q + w) * 32, sv[w]);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    const int kh = page_at(u, 2 * i + hf) * PAGE;
+                    const int kq = page_at(u, 2 * i + (q >> 1)) * PAGE + (q & 1) * 32;   // position of the first of these keys
                     if (SHAPED) {
+                        if (capped) cap_scores(sv[0], series);
+                        if (bias != nullptr) {
+                            const float2 f = capped ? make_float2(1.f, 1.f) : make_float2(S.scale, S.scale);
+                            const float* sb = &s_bias[SHAPED ? warp : 0][q >> 1][lane + PAGE - 1 - (q & 1) * 32];
 #pragma unroll
-                        for (int q = 0; q < 2; ++q) {
-                            const bool capped = S.softcap > 0.f;
-                            if (capped) cap_scores(sv[q], S.scale, S.softcap, inv_cap);
-                            const float f = capped ? 1.f : S.scale;
-                            if (bias != nullptr) {
-                                const float* sb = &s_bias[SHAPED ? warp : 0][hf][lane + PAGE - 1 - q * 32];
-#pragma unroll
-                                for (int c = 0; c < 32; ++c) sv[q][c] = __float_as_uint(fmaf(__uint_as_float(sv[q][c]), f, sb[-c]));
-                            } else if (!capped) {
-#pragma unroll
-                                for (int c = 0; c < 32; ++c) sv[q][c] = __float_as_uint(__uint_as_float(sv[q][c]) * f);
+                            for (int c = 0; c < 32; c += 2) {
+                                const float2 t = fma2(make_float2(__uint_as_float(sv[0][c]), __uint_as_float(sv[0][c + 1])), f, make_float2(sb[-c], sb[-c - 1]));
+                                sv[0][c] = __float_as_uint(t.x);
+                                sv[0][c + 1] = __float_as_uint(t.y);
                             }
+                        } else if (!capped) {
+#pragma unroll
+                            for (int c = 0; c < 32; ++c) sv[0][c] = __float_as_uint(__uint_as_float(sv[0][c]) * S.scale);
                         }
                     }
-                    if (kh + PAGE - 1 > p_first || kh < open_from) {           // some row does not see some key of the page
+                    if (kq + 32 * CW - 1 > p_first || kq < open_from) {        // some row does not see some of these keys
 #pragma unroll
-                        for (int q = 0; q < 2; ++q) {
-                            // bit c: the row sees key kh + 32 q + c, i.e. c <= last and (c >= lo or c < kp)
-                            const int last = qpos - kh - 32 * q, lo = start - kh - 32 * q, kp = keep - kh - 32 * q;
+                        for (int w = 0; w < CW; ++w) {
+                            // bit c: the row sees key kq + 32 w + c, i.e. c <= last and (c >= lo or c < kp)
+                            const int last = qpos - kq - 32 * w, lo = start - kq - 32 * w, kp = keep - kq - 32 * w;
                             const uint32_t behind = last < 0 ? 0u : 0xffffffffu >> (31 - min(last, 31));
                             const uint32_t inside = lo >= 32 ? 0u : 0xffffffffu << max(lo, 0);
                             const uint32_t kept = kp <= 0 ? 0u : 0xffffffffu >> (32 - min(kp, 32));
                             const uint32_t seen = behind & (inside | kept);
 #pragma unroll
                             for (int c = 0; c < 32; ++c)
-                                if (!(seen & (1u << c))) sv[q][c] = 0xff800000u;
+                                if (!(seen & (1u << c))) sv[w][c] = 0xff800000u;
                         }
                     }
-                    float top[4] = {fmaxf(m, floor_m), -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-                    for (int c = 0; c < PAGE; ++c) top[c % 4] = fmaxf(top[c % 4], __uint_as_float(sv[c / 32][c % 32]));
-                    const float mx = fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3]));
-                    // keep m unless the maximum grew by more than 2^8 (or nothing had been seen yet)
+                    float mx = max_of(sv[0], -INFINITY);
+                    if (CW > 1) mx = fmaxf(mx, max_of(sv[CW - 1], -INFINITY));
+                    mx = fmaxf(mx * factor, floor_m);
+                    if (x < 0) {
+                        m = fmaxf(m, mx);
+                        continue;
+                    }
+                    // keep m unless the maximum grew by more than 2^8 (or nothing had been seen yet); then by a whole power
+                    // of two, which loses nothing of what is rescaled
                     float corr = 1.0f;
                     if (m == -INFINITY) {
                         m = mx;                            // l, P and O are still zero: nothing to rescale
-                    } else if ((mx - m) * factor > RESCALE_LOG2) {
-                        corr = ex2((m - mx) * factor);
+                    } else if (mx - m > RESCALE_LOG2) {
+                        const float k = ceilf(mx - m);
+                        corr = k < 127.f ? __int_as_float((127 - (int)k) << 23) : 0.f;
                         l *= corr;
-                        m = mx;
+                        m += k;
                     }
                     if (__any_sync(0xffffffffu, corr != 1.0f)) {
                         const float2 cc = make_float2(corr, corr);
                         sum[0] = mul2(sum[0], cc);
                         sum[1] = mul2(sum[1], cc);
+                        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                        uint32_t ov[16];
                         if (i > 0) {                       // the products so far are done (s_ready)
 #pragma unroll 1
-                            for (int c0 = 0; c0 < DV; c0 += 32) {
-                                uint32_t ov[32];
-                                tmem_ld32(acc + c0, ov);
+                            for (int c0 = 0; c0 < DV; c0 += 16) {
+                                tmem_ld16(acc + c0, ov);
                                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                                for (int j = 0; j < 32; ++j) ov[j] = __float_as_uint(__uint_as_float(ov[j]) * corr);
-                                tmem_st32(acc + c0, ov);
+                                for (int j = 0; j < 16; ++j) ov[j] = __float_as_uint(__uint_as_float(ov[j]) * corr);
+                                tmem_st16(acc + c0, ov);
                             }
                         }
-                        if (hf > 0) {                      // the tile's first page as well
-                            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                            uint32_t pv[32];
-                            tmem_ld32(s_addr, pv);
+#pragma unroll 1
+                        for (int c0 = 0; c0 < q * 16; c0 += 16) {              // what the tile has of P already
+                            tmem_ld16(s_addr + c0, ov);
                             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                            for (int j = 0; j < 32; ++j) {
-                                const float2 w = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pv[j]));
+                            for (int j = 0; j < 16; ++j) {
+                                const float2 w = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&ov[j]));
                                 const __nv_bfloat162 two = __floats2bfloat162_rn(w.x * corr, w.y * corr);
-                                pv[j] = *reinterpret_cast<const uint32_t*>(&two);
+                                ov[j] = *reinterpret_cast<const uint32_t*>(&two);
                             }
-                            tmem_st32(s_addr, pv);
+                            tmem_st16(s_addr + c0, ov);
                         }
                     }
-                    const float mref = m == -INFINITY ? 0.f : m * factor;    // nothing visible yet: exponents of -inf
+                    const float mref = m == -INFINITY ? 0.f : m;             // nothing visible yet: exponents of -inf
                     const float2 ff = make_float2(factor, factor), neg = make_float2(-mref, -mref);
-                    uint32_t pk[32];
 #pragma unroll
-                    for (int e = 0; e < 32; ++e) {
-                        float2 x = fma2(make_float2(__uint_as_float(sv[e / 16][2 * e % 32]), __uint_as_float(sv[e / 16][2 * e % 32 + 1])), ff, neg);
-                        x = make_float2(ex2(x.x), ex2(x.y));
-                        sum[e % 2] = add2(sum[e % 2], x);
-                        const __nv_bfloat162 two = __floats2bfloat162_rn(x.x, x.y);
-                        pk[e] = *reinterpret_cast<const uint32_t*>(&two);
+                    for (int w = 0; w < CW; ++w) {
+                        uint32_t pk[16];
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) {
+                            float2 x = fma2(make_float2(__uint_as_float(sv[w][2 * e]), __uint_as_float(sv[w][2 * e + 1])), ff, neg);
+                            x = make_float2(ex2(x.x), ex2(x.y));
+                            sum[e % 2] = add2(sum[e % 2], x);
+                            const __nv_bfloat162 two = __floats2bfloat162_rn(x.x, x.y);
+                            pk[e] = *reinterpret_cast<const uint32_t*>(&two);
+                        }
+                        tmem_st16(s_addr + (q + w) * 16, pk);
                     }
-                    tmem_st32(s_addr + hf * 32, pk);
                 }
                 l += (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -677,30 +724,30 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             ok = __all_sync(0xffffffffu, mbar_wait(o_done(slot), (uint32_t)units & 1u, &s_abort));
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (sink != nullptr) l += ex2((floor_m - m) * factor);
+            if (sink != nullptr) l += ex2(floor_m - m);
             const float inv = 1.0f / l;
             __nv_bfloat16* dst = out + ((size_t)(u.t0[slot] + r) * S.nh + h) * DV;
-            uint32_t ov[DV / 32][32];
+#pragma unroll 1
+            for (int c0 = 0; c0 < DV; c0 += 32) {
+                uint32_t ov[32];
+                tmem_ld32(acc + c0, ov);               // every lane takes part: the load is warp-wide
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (r < u.rows[slot]) {
 #pragma unroll
-            for (int c = 0; c < DV / 32; ++c) tmem_ld32(acc + c * 32, ov[c]);  // every lane takes part: the load is warp-wide
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    for (int d = 0; d < 32; d += 8) {
+                        uint32_t packed[4];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const __nv_bfloat162 two = __floats2bfloat162_rn(__uint_as_float(ov[d + 2 * e]) * inv, __uint_as_float(ov[d + 2 * e + 1]) * inv);
+                            packed[e] = *reinterpret_cast<const uint32_t*>(&two);
+                        }
+                        *reinterpret_cast<uint4*>(dst + c0 + d) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+                    }
+                }
+            }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(o_free(slot));
-            if (r < u.rows[slot]) {
-#pragma unroll
-                for (int d = 0; d < DV; d += 8) {
-                    uint32_t packed[4];
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const int c = d + 2 * e;
-                        const __nv_bfloat162 two = __floats2bfloat162_rn(__uint_as_float(ov[c / 32][c % 32]) * inv,
-                                                                         __uint_as_float(ov[c / 32][c % 32 + 1]) * inv);
-                        packed[e] = *reinterpret_cast<const uint32_t*>(&two);
-                    }
-                    *reinterpret_cast<uint4*>(dst + d) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-                }
-            }
             ++units;
         }
     }

@@ -18,8 +18,8 @@
 //                          a layer to read
 //   tq_bias_attention      every (token, head) on its own, its visible keys cut into n_splits ranges (decode steps,
 //                          short runs; any sizes, both dtypes) + the merge of the ranges
-//   tq_bias_attention_runs runs of new tokens (prompts): a block's queries share tiles of keys and values through
-//                          shared memory
+//   tq_bias_attention_runs runs of new tokens (prompts) with keys or values of 32: a block's queries share tiles of keys
+//                          and values through shared memory (sizes of 64 and 128: csrc/attention_prefill.cu)
 #include "common.cuh"
 
 TQ_DEFINE_LAST_ERROR
@@ -1268,10 +1268,10 @@ TQ_EXPORT int tq_bias_attention_runs(const void* q, const void* cache, int act_d
     int rc = -2;
 #define BR_CASE(DK_, DV_) if (dk == DK_ && dv == DV_) rc = launch_bias_runs<DK_, DV_>(q, cache, bias_t, far, sink, cu_seqlens, \
         seq_start, page_table, table_stride, window, keep_first, cell, scale, softcap, out, n_seqs, max_run, nh, nkv, n_pages, stream);
-    BR_CASE(32, 32) BR_CASE(32, 64) BR_CASE(32, 128) BR_CASE(64, 32) BR_CASE(64, 64) BR_CASE(64, 128)
-    BR_CASE(128, 32) BR_CASE(128, 64) BR_CASE(128, 128)
+    // (keys and values of 64 or 128 each go to csrc/attention_prefill.cu)
+    BR_CASE(32, 32) BR_CASE(32, 64) BR_CASE(32, 128) BR_CASE(64, 32) BR_CASE(128, 32)
 #undef BR_CASE
-    TQ_REQUIRE(rc != -2, "bias_attention_runs: key size %d and value size %d must each be 32, 64 or 128", dk, dv);
+    TQ_REQUIRE(rc != -2, "bias_attention_runs: of key size %d and value size %d one must be 32, the other 32, 64 or 128", dk, dv);
     if (rc) return rc;
     TQ_CHECK_LAUNCH("bias_attention_runs");
     return 0;
