@@ -182,10 +182,11 @@ struct Cfg {
 
 // What a launch looks like.  A page's key row: page * kp + kv head * kg in map_k, its value row the same + v_plane in
 // map_v; the head's columns begin at kv head * kc in map_k and at v_col + kv head * vc in map_v.  table null: keys lie
-// densely, sequence s from page page_base[s] on.
+// densely, position 64 p of sequence s as page page_base[s] + p.
 struct Shape {
     int nh, nkv, n_seqs, n_qt, pairing;
-    int kp, kg, v_plane, kc, vc, v_col, k_blocks;          // k_blocks: 64-element blocks of a key that map_k holds; the rest come from map_r
+    int kp, kg, v_plane, kc, vc, v_col, k_blocks, r_col;   // k_blocks: 64-element blocks of a key that map_k holds; the rest come from
+                                                           // map_r, whose columns begin at r_col
     int table_stride, n_pages, window, keep_first, cell, far;
     float scale, softcap;
 };
@@ -310,7 +311,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     __shared__ uint32_t s_tmem_base;
     __shared__ __align__(16) uint4 s_answer;               // the hardware's answer to a request for another block
     __shared__ int s_unit[2];                              // the units this CTA takes, two in turn
-    __shared__ float s_bias[SHAPED ? 8 : 1][2][96];        // a warp's rows and a page's keys: the bias of their 95 distances
+    __shared__ float s_bias[SHAPED ? 8 : 1][2][SHAPED ? 96 : 1];        // a warp's rows and a page's keys: the bias of their 95 distances
 
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // the same for the whole warp, and known to be
 
@@ -445,7 +446,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                         const int n = page_at(u, 2 * i + pg);
                         page[pg] = page_table != nullptr
                             ? TQ_CHECKED(page_table[(size_t)u.seq * S.table_stride + TQ_CHECKED(n, S.table_stride, TQ_IDX_TABLE_COLUMN)], S.n_pages, TQ_IDX_PAGE)
-                            : page_base[u.seq] + n - u.first;
+                            : page_base[u.seq] + n;
                     }
                     // a tile in shared memory: [column block of 64 elements][128 keys][128 bytes]; a page is 64 keys of it
                     const int ks = ti % C::KST;
@@ -457,7 +458,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                             for (int c = 0; c < C::KB; ++c) {
                             const uint32_t dst = k_smem(ks) + c * (BN * 128) + pg * (PAGE * 128);
                             if (c < S.k_blocks) tma_load_2d(dst, &map_k, u.g * S.kc + c * 64, page[pg] * S.kp + u.g * S.kg, k_full(ks));
-                            else tma_load_2d(dst, &map_r, (c - S.k_blocks) * 64, page[pg] * S.kp, k_full(ks));
+                            else tma_load_2d(dst, &map_r, S.r_col + (c - S.k_blocks) * 64, page[pg] * S.kp, k_full(ks));
                         }
                     }
                     if (i == 0 && !load_q(1)) { ok = false; ++ti; break; }
@@ -864,6 +865,41 @@ TQ_EXPORT int tq_attention_prefill(const void* q, const void* cache, int planes,
     const bool shaped = softcap > 0.f || bias_t != nullptr || !(scale > 0.f);     // the other form compares unscaled scores
 #define AP_CASE(DK_, DV_) if (dk == DK_ && dv == DV_) return shaped ? launch<DK_, DV_, true>(m, S, a, stream) : launch<DK_, DV_, false>(m, S, a, stream);
     AP_CASE(64, 64) AP_CASE(64, 128) AP_CASE(128, 64) AP_CASE(128, 128)
+#undef AP_CASE
+    return -2;
+}
+
+// The same over keys and values that lie densely: kv [rows, nh * (dim + dv)] bf16, a position's keys of all heads, then its
+// values; rot [rows, rot_stride] whose columns from r_col on are the `rot` (0 or 64) last elements of every head's key.  Position
+// p of sequence s is row 64 * page_base[s] + p; rows up to the end of a position's 64 exist.  q [T, nh, dim + rot].
+TQ_EXPORT int tq_attention_prefill_dense(const void* q, const void* kv, const void* rot_rows, int rows, int rot_stride, int r_col,
+                                         const int* cu_seqlens, const int* seq_start, const int* page_base, int window, float scale,
+                                         const float* sink, void* out, int T_, int n_seqs, int max_q_len, int nh, int dim, int rot,
+                                         int dv, int* status, cudaStream_t stream) {
+    if (T_ == 0 || n_seqs == 0) return 0;
+    TQ_REQUIRE((rot == 0 || rot == 64) && (dim == 64 || dim == 128) && (dv == 64 || dv == 128) && (dim + rot < 192 || dv == 128),
+               "attention_prefill_dense: keys of %d + %d elements and values of %d", dim, rot, dv);
+    TQ_REQUIRE(rot == 0 || (r_col % 8 == 0 && rot_stride % 8 == 0 && r_col + rot <= rot_stride && ((uintptr_t)rot_rows % 16) == 0),
+               "attention_prefill_dense: the shared key columns %d of %d are not aligned", r_col, rot_stride);
+    TQ_REQUIRE(scale > 0.f, "attention_prefill_dense: scale %g", scale);
+    Shape S{};
+    S.nh = nh; S.nkv = nh; S.n_seqs = n_seqs; S.n_qt = (max_q_len + BM - 1) / BM; S.pairing = PAIR_ROWS;
+    S.kp = PAGE; S.kc = dim; S.vc = dv; S.v_col = nh * dim; S.k_blocks = dim / 64; S.r_col = r_col;
+    S.window = window; S.scale = scale;
+    int rc = check_common(S, T_, max_q_len, q, kv, kv, out, status);
+    if (rc) return rc;
+    const int dk = dim + rot;
+    Maps m;
+    rc = make_map(&m.q, q, (uint64_t)T_, (uint64_t)nh * dk, BM);
+    if (rc) return rc;
+    rc = make_map(&m.k, kv, (uint64_t)rows, (uint64_t)nh * (dim + dv), PAGE);
+    if (rc) return rc;
+    m.r = m.v = m.k;
+    if (rot) rc = make_map(&m.r, rot_rows, (uint64_t)rows, (uint64_t)rot_stride, PAGE);
+    if (rc) return rc;
+    const Args a{cu_seqlens, seq_start, nullptr, page_base, nullptr, sink, out, status};
+#define AP_CASE(DK_, DV_) if (dk == DK_ && dv == DV_) return launch<DK_, DV_, false>(m, S, a, stream);
+    AP_CASE(64, 64) AP_CASE(64, 128) AP_CASE(128, 64) AP_CASE(128, 128) AP_CASE(192, 128)
 #undef AP_CASE
     return -2;
 }

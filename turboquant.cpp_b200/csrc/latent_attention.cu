@@ -738,6 +738,56 @@ TQ_EXPORT int tq_latent_gather(const void* cache, int act_dtype, const int* tabl
     return 0;
 }
 
+// The pages of a whole step's sequences, one sequence after another, into out [pages * page_size, Dk]: of each the pages that
+// hold what its new tokens see (from position max(0, seq_start + 1 - window) on; window 0: all).  page_base[s]: the place of
+// the sequence's page 0 among them (its page p lies at page_base[s] + p).  Grid (most pages of a sequence, sequences).
+template <typename TA>
+__global__ void __launch_bounds__(256)
+latent_gather_pages_kernel(const TA* __restrict__ cache, const int* __restrict__ page_table, int table_stride, int page_size,
+                           const int* __restrict__ cu_seqlens, const int* __restrict__ seq_start, int window, int Dk,
+                           TA* __restrict__ out, int out_pages, int* __restrict__ page_base, int n_pages) {
+    tq_grid_wait();                    // everything below may read what the previous kernel wrote
+    tq_grid_launch_dependents();       // the next kernel's CTAs may move in as SMs free up
+    __shared__ int s_base, s_first, s_count;
+    const int s = blockIdx.y;
+    if (threadIdx.x < 32) {            // pages of the sequences before this one
+        int before = 0;
+        for (int i = threadIdx.x; i <= s; i += 32) {
+            const int start = seq_start[i], end = start + cu_seqlens[i + 1] - cu_seqlens[i];
+            const int first = window > 0 ? max(0, start + 1 - window) / page_size : 0, n = (end - 1) / page_size - first + 1;
+            if (i < s) before += n;
+            else { s_first = first; s_count = n; }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+        if (threadIdx.x == 0) s_base = before;
+    }
+    __syncthreads();
+    if (blockIdx.x == 0 && threadIdx.x == 0) page_base[s] = s_base - s_first;
+    const int n16 = (int)((size_t)page_size * Dk * sizeof(TA) / 16);
+    for (int p = blockIdx.x; p < s_count && s_base + p < out_pages; p += gridDim.x) {
+        const int page = TQ_CHECKED(page_table[(size_t)s * table_stride + TQ_CHECKED(s_first + p, table_stride, TQ_IDX_TABLE_COLUMN)], n_pages, TQ_IDX_PAGE);
+        const uint4* src = reinterpret_cast<const uint4*>(cache + (size_t)page * page_size * Dk);
+        uint4* dst = reinterpret_cast<uint4*>(out + (size_t)(s_base + p) * page_size * Dk);
+        for (int i = threadIdx.x; i < n16; i += blockDim.x) dst[i] = src[i];
+    }
+}
+
+TQ_EXPORT int tq_latent_gather_pages(const void* cache, int act_dtype, const int* page_table, int table_stride, int page_size,
+                                     const int* cu_seqlens, const int* seq_start, int n_seqs, int window, int Dk, void* out,
+                                     int out_pages, int* page_base, int n_pages, cudaStream_t stream) {
+    if (n_seqs == 0) return 0;
+    const int esize = act_dtype == TQ_F32 ? 4 : 2;
+    TQ_REQUIRE(n_seqs <= 65535 && out_pages >= 1 && window >= 0, "latent_gather_pages: %d sequences, %d pages", n_seqs, out_pages);
+    TQ_REQUIRE(((size_t)page_size * Dk * esize) % 16 == 0 && ((uintptr_t)cache % 16) == 0 && ((uintptr_t)out % 16) == 0,
+               "latent_gather_pages: pages of %d x %d elements are not multiples of 16 bytes", page_size, Dk);
+    TQ_DISPATCH(act_dtype, TA,
+        (tq_launch(dim3(out_pages < table_stride ? out_pages : table_stride, n_seqs), 256, 0, stream)(latent_gather_pages_kernel<TA>, (const TA*)cache, page_table,
+            table_stride, page_size, cu_seqlens, seq_start, window, Dk, (TA*)out, out_pages, page_base, n_pages)));
+    TQ_CHECK_LAUNCH("latent_gather_pages");
+    return 0;
+}
+
 // ---------------------------------------------------------------------------------------
 // scores [rows, n_keys] fp32 (row r: token r / H of the run, head r % H; column j: position k0 + j) -> weights in
 // the activation dtype: w_j = exp(s_j * scale - M) / (sum_visible exp(s * scale - M) + exp(sink_h - M)), 0 where

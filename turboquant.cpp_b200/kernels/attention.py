@@ -231,3 +231,30 @@ def prefill_rows(q: torch.Tensor, cache_layer: torch.Tensor, planes: int, cu_seq
         c_int(max_q_len), c_int(n_heads), c_int(n_kv_heads), c_int(dk), c_int(dv),
         ptr(status if status is not None else status_word(q.device)), stream()))
     return out
+
+
+def dense_usable(dtype: torch.dtype, dim: int, rot: int, vdim: int, page_size: int) -> bool:
+    """Whether the tensor-core prompt kernel takes keys of dim + rot elements (the last rot shared by the heads) and values
+    of vdim that lie densely."""
+    return dtype == torch.bfloat16 and page_size == 64 and rot in (0, 64) and dim in (64, 128) and vdim in (64, 128) \
+        and (dim + rot < 192 or vdim == 128)
+
+
+def prefill_dense(q: torch.Tensor, kv: torch.Tensor, rot_rows: torch.Tensor, r_col: int, cu_seqlens: torch.Tensor,
+                  seq_start: torch.Tensor, page_base: torch.Tensor, window: int, scale: float, sink: Optional[torch.Tensor],
+                  out: torch.Tensor, n_seqs: int, max_q_len: int, n_heads: int, dim: int, rot: int, vdim: int,
+                  status: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """The tensor-core prompt kernel over dense keys and values of every head: kv [rows, heads * (dim + vdim)], rot_rows [rows,
+    …] with the keys' shared last `rot` elements from column r_col; position p of sequence s is row 64 * page_base[s] + p."""
+    from .gemm_tc import status_word
+    for t, what in ((cu_seqlens, "cu_seqlens"), (seq_start, "seq_start"), (page_base, "page_base")):
+        want_int32(t, what)
+    if any(t.dtype != torch.bfloat16 for t in (q, kv, rot_rows, out)) or kv.shape[1] != n_heads * (dim + vdim) or rot_rows.shape[0] != kv.shape[0] \
+            or q.numel() != q.shape[0] * n_heads * (dim + rot):
+        raise KernelError("attention_prefill_dense: queries, keys, values and output must be bfloat16 and fit together")
+    lib = load_kernel("attention_prefill")
+    check("attention_prefill", lib.tq_attention_prefill_dense(
+        ptr(q), ptr(kv), ptr(rot_rows), c_int(kv.shape[0]), c_int(rot_rows.shape[1]), c_int(r_col), ptr(cu_seqlens), ptr(seq_start),
+        ptr(page_base), c_int(window), c_float(scale), ptr(sink), ptr(out), c_int(q.shape[0]), c_int(n_seqs), c_int(max_q_len),
+        c_int(n_heads), c_int(dim), c_int(rot), c_int(vdim), ptr(status if status is not None else status_word(q.device)), stream()))
+    return out

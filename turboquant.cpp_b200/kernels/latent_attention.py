@@ -96,6 +96,23 @@ def latent_gather(cache: torch.Tensor, table_row: torch.Tensor, page_size: int, 
     return out
 
 
+def latent_gather_pages(cache: torch.Tensor, page_table: torch.Tensor, page_size: int, cu_seqlens: torch.Tensor,
+                        seq_start: torch.Tensor, window: int, out: torch.Tensor, page_base: torch.Tensor) -> torch.Tensor:
+    """The pages that a step's sequences see, one sequence after another, into out [pages * page_size, row]; page_base[s]
+    (int32): where page 0 of sequence s would lie among them."""
+    for t, what in ((page_table, "the page table"), (cu_seqlens, "cu_seqlens"), (seq_start, "seq_start"), (page_base, "page_base")):
+        want_int32(t, what)
+    Dk, n_seqs = cache.shape[-1], seq_start.shape[0]
+    if out.shape[1] != Dk or out.shape[0] % page_size or out.dtype != cache.dtype or page_base.shape[0] < n_seqs or page_table.shape[0] < n_seqs:
+        raise KernelError("latent_gather_pages: the output must be [pages * page_size, row] in the cache's dtype")
+    lib = load_kernel(_LIB)
+    check(_LIB, lib.tq_latent_gather_pages(
+        ptr(cache), c_int(code(cache.dtype)), ptr(page_table), c_int(page_table.shape[1]), c_int(page_size), ptr(cu_seqlens),
+        ptr(seq_start), c_int(n_seqs), c_int(window), c_int(Dk), ptr(out), c_int(out.shape[0] // page_size), ptr(page_base),
+        c_int(cache.shape[0]), stream()))
+    return out
+
+
 def latent_softmax(scores: torch.Tensor, sink: Optional[torch.Tensor], scale: float, window: int, pos0: int, k0: int,
                    heads: int, weights: torch.Tensor) -> torch.Tensor:
     """scores float32 [tokens * heads, n_keys] of a run of tokens at positions pos0 … against positions k0 …:

@@ -12,7 +12,8 @@ With h the mixer's input, H heads, per head `dim` plain and `rot_dim` rotated qu
 
 Only [c | kr] is cached.  The products with W_uk and W_uv are moved to the query's side: q~_a = W_uk,a^T q_plain
 meets c directly, the softmax-weighted sum of the c_j is taken first and W_uv,a applied to it, so one cached row
-serves all heads as key and value, in prompts and in decoding alike.  Options: a window (position i sees j with
+serves all heads as key and value.  Prompts whose new tokens outweigh the expansion build the heads' keys and values
+from the cached rows instead (one product) and attend over those.  Options: a window (position i sees j with
 0 <= i - j < window), a learned sink per head in the softmax's denominator, reading the rows another layer
 cached (the layer then has no W_dkv), and queries that go through a latent of their own:
 
@@ -24,6 +25,7 @@ from typing import List, Optional
 
 import torch
 
+from ..kernels import attention as KA
 from ..kernels import elementwise as KE
 from ..kernels import latent_attention as KL
 from ..kernels.linear import batched_linear, linear, product
@@ -34,6 +36,9 @@ from .base import KVNeed, LayerCache, Mixer, StepContext, register_mixer
 class LatentAttentionMixer(Mixer):
     PROMPT_MIN_RUN = 32       # steps whose longest run of new tokens is at least this take the matrix-product path
     PROMPT_ROWS = 8192        # (token, head) rows of scores per block of that path
+    # steps with at most this many keys per new token build the heads' keys and values from the cached rows: a key then
+    # costs its expansion once (2 R (dim + vdim) per head) and 2 (dim + rot + vdim) per query instead of 2 (2 R + rot)
+    EXPAND_KEYS_PER_TOKEN = 32
 
     def __init__(self, prefix: str, hidden: int, heads: int, dim: int, rot_dim: int, vdim: int, kv_rank: int,
                  scale: float, eps: float, window: int = 0, position=None, own_cache: bool = True,
@@ -57,7 +62,7 @@ class LatentAttentionMixer(Mixer):
         self.keep_window = self.window if keep_window is None else int(keep_window)
         self.q_dim = self.dim + self.rot_dim
         self.q_rank = int(q_rank)            # 0: queries straight from the input
-        self.w_dq = self.w_qnorm = None
+        self.w_dq = self.w_qnorm = self.w_ukv = None
         self.w_q = self.w_dkv = self.w_norm = self.w_uk = self.w_uv_t = self.w_o = self.sink = None
 
     def weight_specs(self) -> List[WeightSpec]:
@@ -82,8 +87,12 @@ class LatentAttentionMixer(Mixer):
         self.w_q, self.w_o = store.get(p + ("uq" if self.q_rank else "q")), store.get(p + "o")
         if self.q_rank:
             self.w_dq, self.w_qnorm = store.get(p + "dq"), store.get(p + "dq.norm")
-        self.w_uk = store.get(p + "uk").view(H, self.dim, self.kv_rank)                       # q_plain [T, dim] @ [dim, R]
-        self.w_uv_t = store.get(p + "uv").view(H, self.vdim, self.kv_rank).transpose(1, 2)    # sums [T, R] @ [R, vdim]
+        uk, uv = store.take(p + "uk"), store.take(p + "uv")
+        if uk.dtype == uv.dtype:          # one matrix for both, so that a prompt builds keys and values in one product
+            self.w_ukv = torch.cat([uk, uv], dim=0).contiguous()
+            uk, uv = self.w_ukv[:H * self.dim], self.w_ukv[H * self.dim:]
+        self.w_uk = uk.view(H, self.dim, self.kv_rank)                       # q_plain [T, dim] @ [dim, R]
+        self.w_uv_t = uv.view(H, self.vdim, self.kv_rank).transpose(1, 2)    # sums [T, R] @ [R, vdim]
         if self.own_cache:
             self.w_dkv, self.w_norm = store.get(p + "dkv"), store.get(p + "dkv.norm")
         if self.has_sink:
@@ -92,7 +101,8 @@ class LatentAttentionMixer(Mixer):
             self.position.prepare(store.device)
 
     def kernels(self) -> List[str]:
-        return ["latent_attention"] + (["elementwise"] if self.q_rank else [])
+        return (["latent_attention"] + (["attention_prefill"] if getattr(self, "run_dtype", None) == torch.bfloat16 else [])
+                + (["elementwise"] if self.q_rank else []))
 
     def cache_need(self) -> KVNeed:
         return KVNeed(1, self.kv_rank + self.rot_dim, self.keep_window, planes=1)
@@ -126,6 +136,8 @@ class LatentAttentionMixer(Mixer):
         q3 = q.view(T, H, self.q_dim)
         runs = (ctx.max_q_len >= self.PROMPT_MIN_RUN and len(ctx.host_q_lens) == ctx.n_seqs
                 and len(ctx.host_seq_start) == ctx.n_seqs)
+        if runs and self._expands(ctx, cache):
+            return linear(self._attend_expanded(q3, ctx, cache), self.w_o, out_dtype=torch.float32)
         # the prompt path wants [query in the latent space | rotated part] side by side: the product writes there
         qa = torch.empty((T, H, R + self.rot_dim), dtype=act, device=xn.device) if runs else None
         q_lat = qa[:, :, :R] if runs else torch.empty((T, H, R), dtype=act, device=xn.device)
@@ -153,6 +165,33 @@ class LatentAttentionMixer(Mixer):
         partial = torch.empty(T * H * n_splits * (R + 2), dtype=torch.float32, device=q.device) if n_splits > 1 else None
         KL.latent_attention(q_lat, q, self.dim, cache.kv, self.sink, ctx.positions, ctx.seq_of_token, cache.page_table,
                             cache.page_size, self.window, self.scale, sums, H, R, self.rot_dim, n_splits, partial)
+
+    def _pages_seen(self, ctx: StepContext, page: int) -> int:
+        first = lambda start: max(0, start + 1 - self.window) // page if self.window else 0
+        return sum((start + n - 1) // page - first(start) + 1 for n, start in zip(ctx.host_q_lens, ctx.host_seq_start))
+
+    def _expands(self, ctx: StepContext, cache: LayerCache) -> bool:
+        """Whether this step builds the heads' keys and values.  Measured on B200, 16 heads of 128 + 64 / 128, rank 512, a
+        layer's time in us expanded / over the cached rows (that path's launches bound it below 1,000 tokens): 2,048 new tokens
+        in a window of 1,024: 121 / 421; 512: 128 / 231; 64 new on 1,024 held: 127 / 223; 64 on 4,000: 133 / 273; 256 on 8,000
+        (32 keys a token): 243 / 258, where the expansion's product begins to weigh."""
+        return (self.w_ukv is not None and self.w_ukv.dtype == torch.bfloat16 and cache.kv.dtype == torch.bfloat16 and self.scale > 0.0
+                and (self.kv_rank + self.rot_dim) % 8 == 0 and self.kv_rank % 8 == 0
+                and KA.dense_usable(ctx.act_dtype, self.dim, self.rot_dim, self.vdim, cache.page_size)
+                and self._pages_seen(ctx, cache.page_size) * cache.page_size <= self.EXPAND_KEYS_PER_TOKEN * ctx.n_tokens)
+
+    def _attend_expanded(self, q3, ctx: StepContext, cache: LayerCache) -> torch.Tensor:
+        """Prompts: the rows that the step's tokens see, gathered from the pages; every head's keys and values from their
+        latents in one product; the prompt kernel of the softmax attentions over those.  [T, heads * vdim]."""
+        H, R, T, dev = self.heads, self.kv_rank, q3.shape[0], q3.device
+        pages = self._pages_seen(ctx, cache.page_size)
+        rows = torch.empty((pages * cache.page_size, R + self.rot_dim), dtype=q3.dtype, device=dev)
+        page_base = torch.empty(ctx.n_seqs, dtype=torch.int32, device=dev)
+        KL.latent_gather_pages(cache.kv, cache.page_table, cache.page_size, ctx.cu_seqlens, ctx.seq_start, self.window, rows, page_base)
+        kv = linear(rows[:, :R], self.w_ukv, out_dtype=q3.dtype)
+        out = torch.empty((T, H * self.vdim), dtype=q3.dtype, device=dev)
+        return KA.prefill_dense(q3, kv, rows, R, ctx.cu_seqlens, ctx.seq_start, page_base, self.window, self.scale, self.sink, out,
+                                ctx.n_seqs, ctx.max_q_len, H, self.dim, self.rot_dim, self.vdim, status=ctx.status)
 
     def _attend_runs(self, qa, sums, ctx: StepContext, cache: LayerCache) -> None:
         """Long runs of new tokens (prompts): all heads of a block of tokens meet the same cached rows, so scores
