@@ -88,41 +88,111 @@ TQ_EXPORT int tq_bias_kv_write(const float* qkv, void* q_out, void* cache, int a
 // g / v_share of the row (v_share > 1: neighbouring key heads keep the same values; v_from_k: the row holds no values,
 // key head g / v_share as it leaves the projection is the value, dv == dk), turned by position * v_freq[m] over all dv
 // elements in the same pairing (v_freq fp32 [dv / 2]; null: as they are).
-// A warp per head (warps loop over the heads where the block has fewer); the blocks of a token share out the heads and
-// the copy of the values.  Grid (token, groups of four heads), or with norm_rows (token) with up to sixteen warps.
+// A block per token: the token's sines and cosines are computed once, a pair's angle by one thread, and read by all its heads
+// from shared memory; then a warp per query, key or value head.  What bounds it is the bytes (fp32 rows in, half of them out)
+// once the angles are shared: 4,096 tokens, 16 + 4 + 4 heads of 128, all turned, took 60.6 us with a sincosf per head and
+// pair (two per pair of a value) and takes 39 us (48 with every head passed through shared memory: 360 instructions a warp
+// and head); the bytes alone are 11.5 us.  vec: 16-byte reads and 8-byte writes (bf16), where sizes, strides and pointers allow them.
 // ---------------------------------------------------------------------------------------
 #define BA_ROT_MAX_WARPS 16
+// cos and sin of `pos * freq[i]` for i < n
+__device__ __forceinline__ void ba_angles(float2* cs, const float* __restrict__ freq, int n, float pos) {
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        float sn, c;
+        sincosf(pos * freq[i], &sn, &c);
+        cs[i] = make_float2(c, sn);
+    }
+}
+// a head's n pairs in shared memory, turned in place by the warp: (2i, 2i + 1) or (i, i + n)
+__device__ __forceinline__ void ba_turn(float* sh, const float2* cs, int n, int halves, float mag, int lane) {
+    for (int i = lane; i < n; i += 32) {
+        const int a = halves ? i : 2 * i, b = halves ? i + n : 2 * i + 1;
+        const float u = sh[a], v = sh[b];
+        sh[a] = (u * cs[i].x - v * cs[i].y) * mag;
+        sh[b] = (v * cs[i].x + u * cs[i].y) * mag;
+    }
+}
+// the same of a head of at most 128 elements that lies in the warp's registers, four neighbours a lane (n pairs: a multiple of
+// four with halves, of two without)
+__device__ __forceinline__ void ba_turn_lanes(float4& x, const float2* cs, int n, int halves, float mag, int lane) {
+    if (halves) {
+        const int step = n >> 2;
+        const bool lo = lane < step, turned = lane < 2 * step;
+        const int from = turned ? (lo ? lane + step : lane - step) : lane;
+        float4 y;
+        y.x = __shfl_sync(0xffffffffu, x.x, from);
+        y.y = __shfl_sync(0xffffffffu, x.y, from);
+        y.z = __shfl_sync(0xffffffffu, x.z, from);
+        y.w = __shfl_sync(0xffffffffu, x.w, from);
+        if (turned) {
+            const float4* t = reinterpret_cast<const float4*>(cs + 4 * (lo ? lane : lane - step));
+            const float4 a = t[0], b = t[1];
+            const float f = lo ? -1.f : 1.f;
+            x.x = (x.x * a.x + f * y.x * a.y) * mag;
+            x.y = (x.y * a.z + f * y.y * a.w) * mag;
+            x.z = (x.z * b.x + f * y.z * b.y) * mag;
+            x.w = (x.w * b.z + f * y.w * b.w) * mag;
+        }
+    } else if (2 * lane < n) {
+        const float4 t = *reinterpret_cast<const float4*>(cs + 2 * lane);
+        x = make_float4((x.x * t.x - x.y * t.y) * mag, (x.y * t.x + x.x * t.y) * mag,
+                        (x.z * t.z - x.w * t.w) * mag, (x.w * t.z + x.z * t.w) * mag);
+    }
+}
+template <typename TA> __device__ __forceinline__ void ba_store4(TA* dst, float4 v);
+template <> __device__ __forceinline__ void ba_store4<float>(float* dst, float4 v) { *reinterpret_cast<float4*>(dst) = v; }
+template <> __device__ __forceinline__ void ba_store4<__nv_bfloat16>(__nv_bfloat16* dst, float4 v) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+}
+// four elements in one access or, where the addresses are not aligned for that, in four
+template <typename TA> __device__ __forceinline__ void ba_store4(TA* dst, float4 v, int vec) {
+    if (vec) { ba_store4(dst, v); return; }
+    dst[0] = tq_from_float<TA>(v.x); dst[1] = tq_from_float<TA>(v.y); dst[2] = tq_from_float<TA>(v.z); dst[3] = tq_from_float<TA>(v.w);
+}
+__device__ __forceinline__ float4 ba_read4(const float* src, int vec) {
+    return vec ? *reinterpret_cast<const float4*>(src) : make_float4(src[0], src[1], src[2], src[3]);
+}
 template <typename TA>
-__global__ void __launch_bounds__(32 * BA_ROT_MAX_WARPS)
+__global__ void __launch_bounds__(32 * BA_ROT_MAX_WARPS, 2)
 bias_kv_write_rot_kernel(const float* __restrict__ qkv, int row_stride, TA* __restrict__ q_out, TA* __restrict__ cache,
                          const float* __restrict__ freq, int rot_dims, int halves, float mag, float unit_eps,
                          const float* __restrict__ q_norm_w, const float* __restrict__ k_norm_w, float norm_eps, int norm_rows,
                          const float* __restrict__ v_freq, int v_share, int v_from_k, float temp_coef, int temp_every,
                          const int* __restrict__ positions, const int* __restrict__ seq_of_token,
                          const int* __restrict__ page_table, int table_stride, int page_size,
-                         int nh, int nkv, int dk, int dv, int n_seqs, int n_pages) {
+                         int nh, int nkv, int dk, int dv, int n_seqs, int n_pages, int vec) {
     tq_grid_wait();                    // everything below may read what the previous kernel wrote
     tq_grid_launch_dependents();       // the next kernel's CTAs may move in as SMs free up
-    extern __shared__ float s_heads[]; // [warps][dk]
+    extern __shared__ __align__(16) float s_heads[];           // [warps][room], then the angles: rot_dims / 2, dv / 2 pairs
     __shared__ float scratch[33];
     const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
-    const int nq = nh * dk, nk = nkv * dk, nv = nkv * dv, dr = dk + dv;
+    const int nq = nh * dk, nk = nkv * dk, dr = dk + dv, room = (max(dk, dv) + 3) & ~3;
     const float* row = qkv + (size_t)t * row_stride;
     const int pos = positions[t];
+    float2* cs = reinterpret_cast<float2*>(s_heads + (size_t)n_warps * room);
+    float2* v_cs = cs + (((rot_dims >> 1) + 1) & ~1);          // 16-byte aligned
+    const int last = cache == nullptr ? nh : nh + 2 * nkv;     // without a cache the rows may hold queries only
+    auto source = [&](int head) {                              // queries, keys (which follow them in the row), values
+        if (head < nh + nkv) return row + (size_t)head * dk;
+        const int g = head - nh - nkv;
+        return row + nq + (v_from_k ? 0 : nk) + (size_t)(v_share == 1 ? g : g / v_share) * dv;
+    };
+    const int unit = halves ? 8 : 4;                           // rotated elements come in whole lanes of four, with halves in pairs of them
+    const bool k_lanes = dk % 4 == 0 && dk <= 128 && rot_dims % unit == 0, v_lanes = dv % 4 == 0 && dv <= 128 && (v_freq == nullptr || dv % unit == 0);
+    auto read = [&](int head) {                                // the lane's four elements of a head that stays in registers
+        const bool kq = head < nh + nkv;
+        return (kq ? k_lanes : v_lanes) && head < last && 4 * lane < (kq ? dk : dv) ? ba_read4(source(head) + 4 * lane, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    float4 next = read(warp);          // on its way while the angles are computed; each later head while the one before is worked on
+    ba_angles(cs, freq, rot_dims >> 1, (float)pos);
+    if (v_freq != nullptr && cache != nullptr) ba_angles(v_cs, v_freq, dv >> 1, (float)pos);
     int page = 0;                      // without a cache (a layer that only reads another's) no table is looked at
     if (cache != nullptr) {
         const int* table = page_table + (size_t)TQ_CHECKED(seq_of_token[t], n_seqs, TQ_IDX_SEQUENCE) * table_stride;
         page = TQ_CHECKED(table[TQ_CHECKED(pos / page_size, table_stride, TQ_IDX_TABLE_COLUMN)], n_pages, TQ_IDX_PAGE);
     }
     const int slot = pos % page_size;
-    if (cache != nullptr)
-        for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < nv; i += gridDim.y * blockDim.x) {
-            const int g = i / dv, e = i % dv;
-            const float* vh = row + nq + (v_from_k ? 0 : nk) + (size_t)(g / v_share) * dv;
-            const float v = v_freq ? tq_rotated(vh, e, dv & ~1, halves, v_freq, pos) : vh[e];
-            cache[(((size_t)page * nkv + g) * page_size + slot) * dr + dk + e] = tq_from_float<TA>(v);
-        }
-    const int last = cache == nullptr ? nh : nh + nkv;         // without a cache the rows may hold queries only
     float q_rs = 1.f, k_rs = 1.f;
     if (norm_rows) {                   // the same for the whole block
         if (q_norm_w != nullptr) {
@@ -136,53 +206,66 @@ bias_kv_write_rot_kernel(const float* __restrict__ qkv, int row_stride, TA* __re
             k_rs = 1.0f / sqrtf(tq_block_sum(ss, scratch) / (float)nk + norm_eps);
         }
     }
-    float* sh = s_heads + (size_t)warp * dk;
-    for (int head = blockIdx.y * n_warps + warp; head < last; head += gridDim.y * n_warps) {
-        const bool is_q = head < nh;
-        const float* src = row + (size_t)head * dk;            // keys follow the queries in the row
-        const float* nw = is_q ? q_norm_w : k_norm_w;
+    __syncthreads();                   // the angles are there
+    // heads of up to 128 elements stay in registers, four neighbours a lane; others pass through the warp's row in shared memory
+    auto lane_head = [&](int head, float4 x) {
+        const bool is_q = head < nh, is_v = head >= nh + nkv;
+        const int g = head - nh - (is_v ? nkv : 0), n = is_v ? dv : dk, e = 4 * lane;
+        const float* nw = is_v ? nullptr : is_q ? q_norm_w : k_norm_w;
         if (nw != nullptr) {
-            float rs = is_q ? q_rs : k_rs;
+            float r = is_q ? q_rs : k_rs;
+            if (norm_rows) nw += (size_t)(is_q ? head : head - nh) * dk;
+            else r = 1.0f / sqrtf(tq_warp_sum(x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w) / (float)dk + norm_eps);
+            if (e < n) x = make_float4(x.x * r * nw[e], x.y * r * nw[e + 1], x.z * r * nw[e + 2], x.w * r * nw[e + 3]);
+        }
+        if (!is_v) { if (rot_dims > 0) ba_turn_lanes(x, cs, rot_dims >> 1, halves, mag, lane); }
+        else if (v_freq != nullptr) ba_turn_lanes(x, v_cs, dv >> 1, halves, 1.0f, lane);
+        float r = 1.f;
+        if (!is_v && unit_eps > 0.f) r = 1.0f / sqrtf(tq_warp_sum(x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w) / (float)dk + unit_eps);
+        if (is_q && temp_every > 0) r *= 1.0f + temp_coef * logf((float)((pos + 1) / temp_every) + 1.0f);
+        TA* dst = is_q ? q_out + ((size_t)t * nh + head) * dk : cache + (((size_t)page * nkv + g) * page_size + slot) * dr + (is_v ? dk : 0);
+        if (e < n) ba_store4(dst + e, make_float4(x.x * r, x.y * r, x.z * r, x.w * r), vec);
+    };
+    float* sh = s_heads + (size_t)warp * room;
+    auto shared_head = [&](int head) {
+        const bool is_q = head < nh, is_v = head >= nh + nkv;
+        const int g = head - nh - (is_v ? nkv : 0), n = is_v ? dv : dk;
+        const float* src = source(head);
+        TA* dst = is_q ? q_out + ((size_t)t * nh + head) * dk : cache + (((size_t)page * nkv + g) * page_size + slot) * dr + (is_v ? dk : 0);
+        const float* nw = is_v ? nullptr : is_q ? q_norm_w : k_norm_w;
+        for (int e = lane; e < n; e += 32) sh[e] = src[e];
+        __syncwarp();
+        if (nw != nullptr) {
+            float r = is_q ? q_rs : k_rs;
             if (norm_rows) {
                 nw += (size_t)(is_q ? head : head - nh) * dk;
             } else {
                 float ss = 0.f;
-                for (int e = lane; e < dk; e += 32) { const float x = src[e]; ss += x * x; }
-                rs = 1.0f / sqrtf(tq_warp_sum(ss) / (float)dk + norm_eps);
+                for (int e = lane; e < dk; e += 32) ss += sh[e] * sh[e];
+                r = 1.0f / sqrtf(tq_warp_sum(ss) / (float)dk + norm_eps);
             }
-            for (int e = lane; e < dk; e += 32) sh[e] = src[e] * rs * nw[e];
-        } else {
-            for (int e = lane; e < dk; e += 32) sh[e] = src[e];
+            for (int e = lane; e < dk; e += 32) sh[e] = sh[e] * r * nw[e];
+            __syncwarp();
         }
+        if (!is_v) ba_turn(sh, cs, rot_dims >> 1, halves, mag, lane);
+        else if (v_freq != nullptr) ba_turn(sh, v_cs, dv >> 1, halves, 1.0f, lane);
         __syncwarp();
-        const int half = rot_dims >> 1;
-        for (int i = lane; i < half; i += 32) {                // a lane turns its pairs in place, one sincos a pair
-            const int a = halves ? i : 2 * i, b = halves ? i + half : 2 * i + 1;
-            float sn, cs;
-            sincosf((float)pos * freq[i], &sn, &cs);
-            const float u = sh[a], v = sh[b];
-            sh[a] = (u * cs - v * sn) * mag;
-            sh[b] = (v * cs + u * sn) * mag;
+        float r = 1.f;
+        if (!is_v && unit_eps > 0.f) {
+            float ss = 0.f;
+            for (int e = lane; e < dk; e += 32) ss += sh[e] * sh[e];
+            r = 1.0f / sqrtf(tq_warp_sum(ss) / (float)dk + unit_eps);
         }
-        __syncwarp();
-        float v[BA_EPL];
-        float ss = 0.f;
-#pragma unroll
-        for (int j = 0; j < BA_EPL; ++j) {
-            const int e = lane + 32 * j;
-            v[j] = e < dk ? sh[e] : 0.f;
-            ss += v[j] * v[j];
-        }
-        float rs = 1.f;
-        if (unit_eps > 0.f) rs = 1.0f / sqrtf(tq_warp_sum(ss) / (float)dk + unit_eps);
-        if (is_q && temp_every > 0) rs *= 1.0f + temp_coef * logf((float)((pos + 1) / temp_every) + 1.0f);
-        TA* dst = is_q ? q_out + ((size_t)t * nh + head) * dk : cache + (((size_t)page * nkv + (head - nh)) * page_size + slot) * dr;
-#pragma unroll
-        for (int j = 0; j < BA_EPL; ++j) {
-            const int e = lane + 32 * j;
-            if (e < dk) dst[e] = tq_from_float<TA>(v[j] * rs);
-        }
+        if (is_q && temp_every > 0) r *= 1.0f + temp_coef * logf((float)((pos + 1) / temp_every) + 1.0f);
+        for (int e = lane; e < n; e += 32) dst[e] = tq_from_float<TA>(sh[e] * r);
         __syncwarp();                  // the warp's row in shared memory is free for its next head
+    };
+#pragma unroll 1
+    for (int head = warp; head < last; head += n_warps) {
+        const float4 x = next;
+        next = read(head + n_warps);
+        if (head < nh + nkv ? k_lanes : v_lanes) lane_head(head, x);
+        else shared_head(head);
     }
 }
 
@@ -203,14 +286,18 @@ TQ_EXPORT int tq_bias_kv_write_rot(const float* qkv, int row_stride, void* q_out
                "bias_kv_write_rot: %d rotated elements of a head of %d", rot_dims, dk);
     TQ_REQUIRE(v_freq == nullptr || dv % 2 == 0, "bias_kv_write_rot: values of %d elements cannot be rotated in pairs", dv);
     TQ_REQUIRE(temp_every >= 0, "bias_kv_write_rot: a temperature that grows every %d positions", temp_every);
-    int warps = 4;
-    if (norm_rows) warps = nh + nkv >= 16 ? 16 : (nh + nkv >= 8 ? 8 : 4);
-    const dim3 grid(T_, norm_rows ? 1 : (nh + nkv + 3) / 4);
-    const size_t smem = (size_t)warps * dk * sizeof(float);
+    // long steps: blocks of eight warps, several an SM; steps of few tokens: as many warps as there are heads, a head or two each
+    const int heads = nh + (cache ? 2 * nkv : 0), most = T_ > 592 ? 8 : BA_ROT_MAX_WARPS;
+    const int room = ((dk > dv ? dk : dv) + 3) & ~3;
+    int warps = heads >= most ? most : (heads >= 8 ? 8 : 4);
+    while (warps > 1 && warps * room > 8192) warps >>= 1;    // wide values: 32 KB of rows
+    const size_t smem = (size_t)warps * room * sizeof(float) + (size_t)(rot_dims / 2 + 1 + (v_freq ? dv / 2 : 0)) * sizeof(float2);
+    const int vec = dk % 4 == 0 && dv % 4 == 0 && row_stride % 4 == 0 && ((uintptr_t)qkv & 15) == 0 && ((uintptr_t)q_out & 15) == 0
+                    && ((uintptr_t)cache & 15) == 0;
     TQ_DISPATCH(act_dtype, TA,
-        (tq_launch(grid, 32 * warps, smem, stream)(bias_kv_write_rot_kernel<TA>, qkv, row_stride, (TA*)q_out, (TA*)cache, freq, rot_dims,
+        (tq_launch(T_, 32 * warps, smem, stream)(bias_kv_write_rot_kernel<TA>, qkv, row_stride, (TA*)q_out, (TA*)cache, freq, rot_dims,
             halves, mag, unit_eps, q_norm_w, k_norm_w, norm_eps, norm_rows, v_freq, v_share, v_from_k, temp_coef, temp_every, positions,
-            seq_of_token, page_table, table_stride, page_size, nh, nkv, dk, dv, n_seqs, n_pages)));
+            seq_of_token, page_table, table_stride, page_size, nh, nkv, dk, dv, n_seqs, n_pages, vec)));
     TQ_CHECK_LAUNCH("bias_kv_write_rot");
     return 0;
 }
@@ -225,30 +312,70 @@ TQ_EXPORT int tq_bias_kv_write_rot(const float* qkv, int row_stride, void* q_out
 //                            o / sqrt(mean(o^2) + eps) * out_scale, times sigmoid of the element's gate logit.  The
 //                            maps lie as the attention kernels leave them with the maps of a key/value head's queries
 //                            side by side: head (g, map, j) at g * 2 * per + map * per + j, per = heads / kv heads.
-// A warp per (token, head), four a block.
+// diff_combine: a warp per (token, head), four a block.
 // ---------------------------------------------------------------------------------------
+// heads_unrotate_gate: a block per token, its angles shared as in bias_kv_write_rot (a sincosf per element before: 4,096 tokens,
+// 16 heads of 128, 45 us; now 15 us for 33.6 MB).
+template <typename TA> __device__ __forceinline__ float4 ba_load4(const TA* src);
+template <> __device__ __forceinline__ float4 ba_load4<float>(const float* src) { return *reinterpret_cast<const float4*>(src); }
+template <> __device__ __forceinline__ float4 ba_load4<__nv_bfloat16>(const __nv_bfloat16* src) {
+    const uint2 r = *reinterpret_cast<const uint2*>(src);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
 template <typename TA>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(32 * BA_ROT_MAX_WARPS)
 heads_unrotate_gate_kernel(const TA* __restrict__ o, const float* __restrict__ gates, int gate_stride, int gate_off,
                            const float* __restrict__ v_freq, int halves, const int* __restrict__ positions,
-                           TA* __restrict__ out, int T_, int nh, int dv) {
+                           TA* __restrict__ out, int T_, int nh, int dv, int vec) {
     tq_grid_wait();                    // everything below may read what the previous kernel wrote
     tq_grid_launch_dependents();       // the next kernel's CTAs may move in as SMs free up
-    __shared__ float s_head[4][BA_MAX_DIM];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const size_t item = (size_t)blockIdx.x * 4 + warp;
-    if (item >= (size_t)T_ * nh) return;
-    const int t = (int)(item / nh), h = (int)(item % nh);
+    __shared__ __align__(16) float s_head[BA_ROT_MAX_WARPS][BA_MAX_DIM];
+    __shared__ __align__(16) float2 cs[BA_MAX_DIM / 2];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5, t = blockIdx.x;
+    const bool lanes = vec && dv <= 128 && (v_freq == nullptr || dv % (halves ? 8 : 4) == 0);
+    float4 early[2];
+    float z[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int h = warp + i * n_warps;
+        early[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        z[i] = 0.f;
+        if (lanes && h < nh) {
+            if (4 * lane < dv) early[i] = ba_load4(o + ((size_t)t * nh + h) * dv + 4 * lane);
+            z[i] = gates[(size_t)t * gate_stride + gate_off + h];
+        }
+    }
+    if (v_freq != nullptr) {
+        ba_angles(cs, v_freq, dv >> 1, (float)-positions[t]);
+        __syncthreads();
+    }
+    if (lanes) {                       // heads of up to 128 elements stay in registers, four neighbours a lane
+        auto one_head = [&](int h, float4 x, float zh) {
+            if (v_freq != nullptr) ba_turn_lanes(x, cs, dv >> 1, halves, 1.0f, lane);
+            const float gate = 1.0f / (1.0f + expf(-zh));
+            if (4 * lane < dv) ba_store4(out + ((size_t)t * nh + h) * dv + 4 * lane, make_float4(x.x * gate, x.y * gate, x.z * gate, x.w * gate));
+        };
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+            if (warp + i * n_warps < nh) one_head(warp + i * n_warps, early[i], z[i]);
+        for (int h = warp + 2 * n_warps; h < nh; h += n_warps)
+            one_head(h, 4 * lane < dv ? ba_load4(o + ((size_t)t * nh + h) * dv + 4 * lane) : make_float4(0.f, 0.f, 0.f, 0.f),
+                     gates[(size_t)t * gate_stride + gate_off + h]);
+        return;
+    }
     float* sh = s_head[warp];
-    const TA* src = o + item * dv;
-    for (int e = lane; e < dv; e += 32) sh[e] = tq_to_float(src[e]);
-    __syncwarp();
-    const float z = gates[(size_t)t * gate_stride + gate_off + h];
-    const float gate = 1.0f / (1.0f + expf(-z));
-    const int pos = positions[t];
-    for (int e = lane; e < dv; e += 32) {
-        const float v = v_freq ? tq_rotated(sh, e, dv & ~1, halves, v_freq, -pos) : sh[e];
-        out[item * dv + e] = tq_from_float<TA>(v * gate);
+    for (int h = warp; h < nh; h += n_warps) {
+        const size_t at = ((size_t)t * nh + h) * dv;
+        for (int e = lane; e < dv; e += 32) sh[e] = tq_to_float(o[at + e]);
+        const float gate = 1.0f / (1.0f + expf(-gates[(size_t)t * gate_stride + gate_off + h]));
+        __syncwarp();
+        if (v_freq != nullptr) {
+            ba_turn(sh, cs, dv >> 1, halves, 1.0f, lane);
+            __syncwarp();
+        }
+        for (int e = lane; e < dv; e += 32) out[at + e] = tq_from_float<TA>(sh[e] * gate);
+        __syncwarp();
     }
 }
 
@@ -259,10 +386,11 @@ TQ_EXPORT int tq_heads_unrotate_gate(const void* o, int act_dtype, const float* 
     TQ_REQUIRE(nh >= 1 && dv >= 1 && dv <= BA_MAX_DIM, "heads_unrotate_gate: %d heads of %d values", nh, dv);
     TQ_REQUIRE(gate_off >= 0 && gate_off + nh <= gate_stride, "heads_unrotate_gate: the gates lie outside their rows");
     TQ_REQUIRE(v_freq == nullptr || dv % 2 == 0, "heads_unrotate_gate: values of %d elements cannot be rotated in pairs", dv);
-    const long long items = (long long)T_ * nh;
+    const int most = T_ > 592 ? 8 : BA_ROT_MAX_WARPS, warps = nh >= most ? most : (nh >= 8 ? 8 : 4);
+    const int vec = dv % 4 == 0 && ((uintptr_t)o & 15) == 0 && ((uintptr_t)out & 15) == 0;
     TQ_DISPATCH(act_dtype, TA,
-        (tq_launch((unsigned)((items + 3) / 4), 128, 0, stream)(heads_unrotate_gate_kernel<TA>, (const TA*)o, gates, gate_stride, gate_off,
-            v_freq, halves, positions, (TA*)out, T_, nh, dv)));
+        (tq_launch(T_, 32 * warps, 0, stream)(heads_unrotate_gate_kernel<TA>, (const TA*)o, gates, gate_stride, gate_off,
+            v_freq, halves, positions, (TA*)out, T_, nh, dv, vec)));
     TQ_CHECK_LAUNCH("heads_unrotate_gate");
     return 0;
 }
