@@ -17,6 +17,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "recurrence.cuh"
 
 TQ_DEFINE_LAST_ERROR
 

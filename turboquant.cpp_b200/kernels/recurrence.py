@@ -1,0 +1,50 @@
+"""Launchers of csrc/recurrence.cuh (in the library of csrc/ssm.cu): recurrences over runs of many tokens in chunks of 64, as float32 matrix products."""
+from __future__ import annotations
+
+from ctypes import c_int, c_longlong
+from typing import Sequence
+
+import torch
+
+from ..csrc.build import load_kernel
+from ._call import KernelError, check, ptr, stream, want_f32, want_int32
+from .ssm import ctypes_ptr
+
+_LIB = "ssm"
+CHUNK = 64               # csrc/recurrence.cuh L
+SIZES = (64, 128)        # key and value sizes the kernels are built for
+
+
+def chunks_of(q_lens: Sequence[int], n_tokens: int, n_seqs: int) -> int:
+    """Chunks of a step's runs (without the lengths on the host: at most)."""
+    if len(q_lens) == n_seqs:
+        return sum(-(-n // CHUNK) for n in q_lens)
+    return n_tokens // CHUNK + n_seqs
+
+
+def usable(dk: int, dv: int, rows: torch.Tensor, *offsets: int) -> bool:
+    """Whether the kernels take this shape: sizes of 64 or 128, rows and offsets of whole 16 bytes."""
+    return dk in SIZES and dv in SIZES and rows.shape[1] % 4 == 0 and all(o % 4 == 0 for o in offsets) \
+        and rows.is_contiguous() and rows.data_ptr() % 16 == 0
+
+
+def memory_chunks(rows: torch.Tensor, q_off: int, k_off: int, v_off: int, gates: torch.Tensor, state: torch.Tensor, y: torch.Tensor,
+                  dots: torch.Tensor, chunks: int, heads: int, dk: int, dv: int, cu_seqlens: torch.Tensor, slots: torch.Tensor) -> None:
+    """`kernels.ssm.memory_scan` with outputs, in chunks: state float32 [slots, heads, dv + 1, dk] (rows may be strided) is renewed,
+    y [T, heads * dv], dots [T, heads].  chunks: at least the chunks of the runs (`chunks_of`)."""
+    for t, what in ((rows, "q, k and v"), (gates, "the gates"), (state, "the state"), (y, "the output"), (dots, "the dot products")):
+        want_f32(t, what)
+    for t, what in ((cu_seqlens, "cu_seqlens"), (slots, "slots")):
+        want_int32(t, what)
+    T, n_seqs = rows.shape[0], cu_seqlens.shape[0] - 1
+    if not usable(dk, dv, rows, q_off, k_off, v_off) or tuple(state.shape[1:]) != (heads, dv + 1, dk) or not state[0].is_contiguous() \
+            or y.numel() != T * heads * dv or dots.numel() != T * heads or gates.numel() != 2 * T * heads or slots.numel() < n_seqs \
+            or max(q_off + heads * dk, k_off + heads * dk, v_off + heads * dv) > rows.shape[1]:
+        raise KernelError("memory_chunks: sizes of 64 or 128, aligned rows that hold the heads, a state row of [heads, dv + 1, dk]")
+    ends = torch.empty((chunks, heads, dv + 1, dk), dtype=torch.float32, device=rows.device)
+    decays = torch.empty((chunks, heads), dtype=torch.float32, device=rows.device)
+    lib = load_kernel(_LIB)
+    check(_LIB, lib.tq_memory_chunks(
+        ptr(rows), c_int(rows.shape[1]), c_int(q_off), c_int(k_off), c_int(v_off), ptr(gates), ctypes_ptr(state), c_longlong(state.stride(0)),
+        ptr(y), ptr(dots), ptr(ends), ptr(decays), c_int(chunks), c_int(n_seqs), c_int(heads), c_int(dk), c_int(dv), ptr(cu_seqlens),
+        ptr(slots), stream()), kernels=3)

@@ -12,7 +12,8 @@ With h the mixer's input, H heads, key size dk, value size dv:
 m only keeps the exponentials in range: with S e^m and n e^m the recurrence is linear with decay e^f.  A sequence's state
 is one float32 row: S column by column with n as one more column (the value of which is one), [H, dv + 1, dk], and m [H].
 The fused input projection [q | k | v | z | i | f] leaves the library's product as float32; everything behind it is
-float32 up to the gated norm's output.  Long runs are cut into chunks where that fills the GPU (`chunks.cut_runs`).
+float32 up to the gated norm's output.  Long runs go in chunks of 64 tokens as matrix products (`kernels.recurrence`, keys and values
+of 64 or 128), others token by token, cut into chunks where that fills the GPU (`chunks.cut_runs`).
 """
 from __future__ import annotations
 
@@ -21,6 +22,7 @@ from typing import List, Optional
 import torch
 
 from ..kernels import gemv as KG
+from ..kernels import recurrence as KR
 from ..kernels import ssm as KS
 from ..kernels.linear import linear
 from ..weights.loader import WeightSpec, WeightStore
@@ -31,6 +33,8 @@ DENOMINATOR_FLOOR = 1e-6
 
 
 class MatrixMemoryMixer(Mixer):
+    CHUNKS_MIN = 64           # steps whose longest run of new tokens is at least this take the matrix form, chunk by chunk
+
     def __init__(self, prefix: str, hidden: int, heads: int, dim: int, vdim: int, gate_cap: float, eps: float):
         if heads < 1 or vdim < 1 or not 1 <= dim <= KS.MAX_STATE:
             raise ValueError(f"matrix memory '{prefix}': {heads} heads, keys of {dim} (1..{KS.MAX_STATE}), values of {vdim}")
@@ -95,9 +99,14 @@ class MatrixMemoryMixer(Mixer):
             f32 = lambda *shape: torch.empty(shape, dtype=torch.float32, device=dev)
             gates, m, y, dots = f32(T, H, 2), f32(T, H), f32(T, self.inner), f32(T, H)
             KS.memory_gates(proj, i, f, self.i_bias, self.f_bias, self.cap, tops, gates, m, H, ctx.cu_seqlens, ctx.slots)
+            in_chunks = ctx.max_q_len >= self.CHUNKS_MIN and KR.usable(dk, dv, proj, q, k, v)
+            if in_chunks:
+                KR.memory_chunks(proj, q, k, v, gates, S, y, dots, KR.chunks_of(ctx.host_q_lens, T, ctx.n_seqs), H, dk, dv, ctx.cu_seqlens, ctx.slots)
             scan = lambda st, out, nq, cu, slots: KS.memory_scan(proj, q, k, v, gates, st, out, nq, H, dk, dv, cu, slots)
-            plan = cut_runs(ctx, H, dv + 1)
-            if plan is None:
+            plan = cut_runs(ctx, H, dv + 1) if not in_chunks else None
+            if in_chunks:
+                pass
+            elif plan is None:
                 scan(S, y, dots, ctx.cu_seqlens, ctx.slots)
             else:
                 # the chunks side by side from zero states without outputs, the states they should have started from, and
