@@ -11,8 +11,9 @@
 // fill the GPU; in chunks it is 2 + 64 (1 / dk + 1 / dv) of them, all in register-tiled products.  Everything is fp32 and
 // stays on the CUDA cores: tensor cores would round operands (three products of split tf32 parts cost what the fp32
 // units take here).  Measured, 682 + 1,366 tokens, 16 heads of 128 x 129: 289 us for both walks token by token; here 37 us for the
-// chunks' sums, 16 for the starts and 102 for the outputs (1.07 G multiply-adds, 30 us at the fp32 units' rate; the loads that
-// transpose and the fill of the last wave of blocks are the rest).
+// chunks' sums, 16 for the starts and 79 for the outputs (1.07 G multiply-adds, 30 us at the fp32 units' rate; what bounds them is shared
+// memory, twelve 128-byte reads a warp for its 32 multiply-adds a thread; 102 us with transposed stores and weights that met in one
+// bank).
 // Part of csrc/ssm.cu's library.
 //   memory_chunks   the matrix memory (a = e^gate0, b = e^gate1; n is one more column whose value is one)
 #pragma once
@@ -63,32 +64,37 @@ __device__ __forceinline__ void load_rows(float* dst, const float* __restrict__ 
         *reinterpret_cast<float4*>(dst + t * N + c) = t < n ? *reinterpret_cast<const float4*>(src + (size_t)t * stride + c) : zero4();
     }
 }
-// columns [c0, c0 + K) of R rows -> smem [K][R] (transposed); rows from n on are zeros.  Neighbouring lanes take neighbouring rows, so
-// the stores are free of conflicts; a row's 128 bytes are read by eight neighbouring iterations, out of L1.
+// K columns of R rows -> smem [K][R] (transposed); rows from n on are zeros.  A row's groups of four neighbours (along R) are shuffled
+// by the bits of k above the lowest two, so that the lanes of a warp, which read a row's columns together, store into eight
+// banks' groups instead of one; a product reads a whole group at one k, wherever it lies.
+__device__ __forceinline__ int group_at(int k, int g) { return g ^ ((k >> 2) & 15); }
 template <int K, int R>
 __device__ __forceinline__ void load_transposed(float* dst, const float* __restrict__ src, int stride, int n) {
+    constexpr int Q = K / 4;
 #pragma unroll 8
-    for (int i = threadIdx.x; i < R * (K / 4); i += THREADS) {
-        const int r = i % R, c = i / R * 4;
+    for (int i = threadIdx.x; i < R * Q; i += THREADS) {
+        const int r = i / Q, c = i % Q * 4;
         const float4 v = r < n ? *reinterpret_cast<const float4*>(src + (size_t)r * stride + c) : zero4();
-        dst[(c + 0) * R + r] = v.x;
-        dst[(c + 1) * R + r] = v.y;
-        dst[(c + 2) * R + r] = v.z;
-        dst[(c + 3) * R + r] = v.w;
+        float* at = dst + c * R + 4 * group_at(c, r >> 2) + (r & 3);
+        at[0] = v.x;
+        at[R] = v.y;
+        at[2 * R] = v.z;
+        at[3 * R] = v.w;
     }
 }
 
 // acc[4 i + r][2 j + p] += a[k][64 i + 4 ty + r] * b[k][64 j + 4 tx + 2 p, + 1] over k in [k0, k1): a [k][LDA], b [k][LDB] in shared memory
-template <int RI, int RJ, int LDA, int LDB>
+// (TA, TB: as load_transposed leaves them)
+template <int RI, int RJ, int LDA, int LDB, bool TA = false, bool TB = false>
 __device__ __forceinline__ void product(tq_f32x2 (&acc)[4 * RI][2 * RJ], const float* a, const float* b, int k0, int k1, int ty, int tx) {
 #pragma unroll 4
     for (int k = k0; k < k1; ++k) {
         float4 av[RI];
         ulonglong2 bv[RJ];
 #pragma unroll
-        for (int i = 0; i < RI; ++i) av[i] = *reinterpret_cast<const float4*>(a + k * LDA + 64 * i + 4 * ty);
+        for (int i = 0; i < RI; ++i) av[i] = *reinterpret_cast<const float4*>(a + k * LDA + 64 * i + 4 * (TA ? group_at(k, ty) : ty));
 #pragma unroll
-        for (int j = 0; j < RJ; ++j) bv[j] = *reinterpret_cast<const ulonglong2*>(b + k * LDB + 64 * j + 4 * tx);
+        for (int j = 0; j < RJ; ++j) bv[j] = *reinterpret_cast<const ulonglong2*>(b + k * LDB + 64 * j + 4 * (TB ? group_at(k, tx) : tx));
 #pragma unroll
         for (int i = 0; i < RI; ++i) {
             const float ar[4] = {av[i].x, av[i].y, av[i].z, av[i].w};
@@ -274,11 +280,11 @@ memory_outputs_kernel(const float* __restrict__ rows, int C, int q_off, int k_of
     load_transposed<DK, L>(Qt, tok + q_off + h * DK, C, c.n);
     load_transposed<DK, L>(X, tok + k_off + h * DK, C, c.n);
     __syncthreads();
-    if (tid < L) {                     // column s of D, by products in token order
+    if (tid < L) {                     // row t of D, a thread each (neighbouring threads store side by side)
         float d = 1.f;
-        for (int t = 0; t < L; ++t) {
-            if (t > tid) d *= s_a[t];
-            Pt[tid * L + t] = t >= tid ? d : 0.f;
+        for (int s = L - 1; s >= 0; --s) {
+            if (s < tid) d *= s_a[s + 1];
+            Pt[s * L + tid] = s <= tid ? d : 0.f;
         }
     } else if (tid == L) {
         float d = 1.f;
@@ -287,18 +293,17 @@ memory_outputs_kernel(const float* __restrict__ rows, int C, int q_off, int k_of
     load_transposed<64, DV>(Y, St, DK, DV);
     __syncthreads();
     {
-        tq_f32x2 p[4][2];              // q_t . k_s: rows t, columns s
+        tq_f32x2 p[4][2];              // k_s . q_t: rows s, columns t
         clear(p);
-        product<1, 1, L, L>(p, Qt, X, 0, DK, ty, tx);
+        product<1, 1, L, L, true, true>(p, X, Qt, 0, DK, ty, tx);
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
             const float4 v = four(p[r][0], p[r][1]);
-            const float x[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int s = 4 * tx + j, t = 4 * ty + r;
-                Pt[s * L + t] *= x[j] * s_b[s];
-            }
+            const float b = s_b[4 * ty + r];
+            float4* at = reinterpret_cast<float4*>(Pt + (4 * ty + r) * L + 4 * tx);
+            float4 d = *at;
+            d.x *= v.x * b; d.y *= v.y * b; d.z *= v.z * b; d.w *= v.w * b;
+            *at = d;
         }
     }
     __syncthreads();
@@ -307,12 +312,12 @@ memory_outputs_kernel(const float* __restrict__ rows, int C, int q_off, int k_of
     clear(acc);
     if (DK > 64) load_transposed<64, DV>(X, St + 64, DK, DV);
     else load_rows<DV>(X, tok + v_off + h * DV, C, c.n);
-    product<1, RJ, L, DV>(acc, Qt, Y, 0, 64, ty, tx);
+    product<1, RJ, L, DV, true, true>(acc, Qt, Y, 0, 64, ty, tx);
     __syncthreads();
     const float* Vs = X;
     if (DK > 64) {
         load_rows<DV>(Y, tok + v_off + h * DV, C, c.n);
-        product<1, RJ, L, DV>(acc, Qt + 64 * L, X, 0, 64, ty, tx);
+        product<1, RJ, L, DV, true, true>(acc, Qt + 64 * L, X, 0, 64, ty, tx);
         __syncthreads();
         Vs = Y;
     }
@@ -337,7 +342,7 @@ memory_outputs_kernel(const float* __restrict__ rows, int C, int q_off, int k_of
         const float* n0 = St + (size_t)DV * DK;
         float from = 0.f, own = 0.f;
 #pragma unroll 4
-        for (int k = 0; k < DK; ++k) from += Qt[k * L + tid] * n0[k];
+        for (int k = 0; k < DK; ++k) from += Qt[k * L + 4 * group_at(k, tid >> 2) + (tid & 3)] * n0[k];
         for (int s = 0; s <= tid; ++s) own += Pt[s * L + tid];
         dots[(size_t)(c.t0 + tid) * heads + h] = s_A[tid] * from + own;
     }
@@ -365,6 +370,7 @@ int launch_memory(const float* rows, int C, int q_off, int k_off, int v_off, con
     TQ_CHECK_LAUNCH("memory_chunks");
     return 0;
 }
+
 
 }  // namespace tq_recurrence
 
