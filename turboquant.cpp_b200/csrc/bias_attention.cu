@@ -28,6 +28,12 @@ TQ_DEFINE_LAST_ERROR
 #define BA_WARPS 4
 #define BA_EPL (BA_MAX_DIM / 32)      // elements of a key or a value per lane
 
+template <typename TA> __device__ __forceinline__ void ba_store4(TA* dst, float4 v);
+template <> __device__ __forceinline__ void ba_store4<float>(float* dst, float4 v) { *reinterpret_cast<float4*>(dst) = v; }
+template <> __device__ __forceinline__ void ba_store4<__nv_bfloat16>(__nv_bfloat16* dst, float4 v) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+}
 // ---------------------------------------------------------------------------------------
 // One block per token walks the elements of its fused row.
 // ---------------------------------------------------------------------------------------
@@ -62,6 +68,52 @@ __global__ void bias_kv_write_kernel(const float* __restrict__ qkv, TA* __restri
     }
 }
 
+// The same four neighbours at a time, for head sizes and addresses that allow it (the same bits).  Bound by its bytes: 2,048 tokens of
+// 16 x 128 + 4 x 256 floats took 14.4 us element by element, 7.2 us here; the bytes alone are 5.8 us.
+template <typename TA>
+__global__ void __launch_bounds__(256)
+bias_kv_write_vec_kernel(const float* __restrict__ qkv, TA* __restrict__ q_out, TA* __restrict__ cache,
+                         float* __restrict__ v_keep, const float* __restrict__ v_other, float lambda,
+                         const int* __restrict__ positions, const int* __restrict__ seq_of_token,
+                         const int* __restrict__ page_table, int table_stride, int page_size,
+                         int nh, int nkv, int dk, int dv, int n_seqs, int n_pages) {
+    tq_grid_wait();                    // everything below may read what the previous kernel wrote
+    tq_grid_launch_dependents();       // the next kernel's CTAs may move in as SMs free up
+    const int t = blockIdx.x;
+    const int nq = nh * dk, nk = nkv * dk, nv = nkv * dv, dr = dk + dv;
+    const float* row = qkv + (size_t)t * (nq + nk + nv);
+    const bool kv = cache != nullptr || v_keep != nullptr;
+    TA* at = nullptr;                  // the token's place in the cache, key/value head 0
+    if (kv) {
+        const int pos = positions[t];
+        const int* table = page_table + (size_t)TQ_CHECKED(seq_of_token[t], n_seqs, TQ_IDX_SEQUENCE) * table_stride;
+        const int page = TQ_CHECKED(table[TQ_CHECKED(pos / page_size, table_stride, TQ_IDX_TABLE_COLUMN)], n_pages, TQ_IDX_PAGE);
+        if (cache) at = cache + ((size_t)page * nkv * page_size + pos % page_size) * dr;
+    }
+    const int n = kv ? nq + nk + nv : nq;
+#pragma unroll 4
+    for (int i = 4 * threadIdx.x; i < n; i += 4 * 256) {
+        float4 v = *reinterpret_cast<const float4*>(row + i);
+        if (i < nq) {
+            ba_store4(q_out + (size_t)t * nq + i, v);
+            continue;
+        }
+        const int j = i - nq, x = j - nk;
+        const int g = x < 0 ? j / dk : x / dv, e = x < 0 ? j - g * dk : dk + x - g * dv;
+        if (x >= 0) {
+            if (v_other) {
+                const float4 o = *reinterpret_cast<const float4*>(v_other + (size_t)t * nv + x);
+                v.x = (1.0f - lambda) * v.x + lambda * o.x;
+                v.y = (1.0f - lambda) * v.y + lambda * o.y;
+                v.z = (1.0f - lambda) * v.z + lambda * o.z;
+                v.w = (1.0f - lambda) * v.w + lambda * o.w;
+            }
+            if (v_keep) *reinterpret_cast<float4*>(v_keep + (size_t)t * nv + x) = v;
+        }
+        if (at) ba_store4(at + (size_t)g * page_size * dr + e, v);
+    }
+}
+
 TQ_EXPORT int tq_bias_kv_write(const float* qkv, void* q_out, void* cache, int act_dtype, float* v_keep,
                                const float* v_other, float lambda, const int* positions, const int* seq_of_token,
                                const int* page_table, int table_stride, int page_size, int T_, int nh, int nkv, int dk,
@@ -69,6 +121,13 @@ TQ_EXPORT int tq_bias_kv_write(const float* qkv, void* q_out, void* cache, int a
     if (T_ == 0) return 0;
     TQ_REQUIRE(nh >= 1 && nkv >= 1 && dk >= 1 && dv >= 1, "bias_kv_write: bad sizes %d %d %d %d", nh, nkv, dk, dv);
     const int n = nh * dk + nkv * (dk + dv);
+    if (dk % 4 == 0 && dv % 4 == 0 && (((uintptr_t)qkv | (uintptr_t)q_out | (uintptr_t)cache | (uintptr_t)v_keep | (uintptr_t)v_other) & 15) == 0) {
+        TQ_DISPATCH(act_dtype, TA,
+            (tq_launch(T_, 256, 0, stream)(bias_kv_write_vec_kernel<TA>, qkv, (TA*)q_out, (TA*)cache, v_keep, v_other, lambda,
+                positions, seq_of_token, page_table, table_stride, page_size, nh, nkv, dk, dv, n_seqs, n_pages)));
+        TQ_CHECK_LAUNCH("bias_kv_write");
+        return 0;
+    }
     const int threads = n >= 1024 ? 512 : (n >= 256 ? 256 : 128);
     TQ_DISPATCH(act_dtype, TA,
         (tq_launch(T_, threads, 0, stream)(bias_kv_write_kernel<TA>, qkv, (TA*)q_out, (TA*)cache, v_keep, v_other, lambda,
@@ -138,12 +197,6 @@ __device__ __forceinline__ void ba_turn_lanes(float4& x, const float2* cs, int n
         x = make_float4((x.x * t.x - x.y * t.y) * mag, (x.y * t.x + x.x * t.y) * mag,
                         (x.z * t.z - x.w * t.w) * mag, (x.w * t.z + x.z * t.w) * mag);
     }
-}
-template <typename TA> __device__ __forceinline__ void ba_store4(TA* dst, float4 v);
-template <> __device__ __forceinline__ void ba_store4<float>(float* dst, float4 v) { *reinterpret_cast<float4*>(dst) = v; }
-template <> __device__ __forceinline__ void ba_store4<__nv_bfloat16>(__nv_bfloat16* dst, float4 v) {
-    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
-    *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
 }
 // four elements in one access or, where the addresses are not aligned for that, in four
 template <typename TA> __device__ __forceinline__ void ba_store4(TA* dst, float4 v, int vec) {
