@@ -218,17 +218,15 @@ def prefill_rows(q: torch.Tensor, cache_layer: torch.Tensor, planes: int, cu_seq
     """The tensor-core prompt kernel over a cache of two planes (keys, values) or one (rows [key | value]), with the
     options of `kernels.bias_attention.attention_runs`."""
     from .gemm_tc import status_word
-    want_int32(cu_seqlens, "cu_seqlens")
-    want_int32(seq_start, "seq_start")
-    want_int32(page_table, "page table")
+    if cu_seqlens.dtype != torch.int32 or seq_start.dtype != torch.int32 or page_table.dtype != torch.int32:
+        raise KernelError("attention_prefill: cu_seqlens, seq_start and the page table must be int32")
     if q.dtype != torch.bfloat16 or cache_layer.dtype != torch.bfloat16 or out.dtype != torch.bfloat16:
         raise KernelError("attention_prefill: queries, cache and output must be bfloat16")
-    lib = load_kernel("attention_prefill")
-    check("attention_prefill", lib.tq_attention_prefill(
-        ptr(q), ptr(cache_layer), c_int(planes), ptr(cu_seqlens), ptr(seq_start), ptr(page_table), c_int(page_table.shape[1]),
-        c_int(page_size), c_int(cache_layer.shape[0]), c_int(window), c_int(keep_first), c_int(cell), c_float(scale), c_float(softcap),
-        ptr(bias_t), c_int(0 if bias_t is None else bias_t.shape[1] - 1), ptr(sink), ptr(out), c_int(q.shape[0]), c_int(n_seqs),
-        c_int(max_q_len), c_int(n_heads), c_int(n_kv_heads), c_int(dk), c_int(dv),
+    # (plain ints are C ints to ctypes)
+    check("attention_prefill", load_kernel("attention_prefill").tq_attention_prefill(
+        ptr(q), ptr(cache_layer), planes, ptr(cu_seqlens), ptr(seq_start), ptr(page_table), page_table.shape[1], page_size,
+        cache_layer.shape[0], window, keep_first, cell, c_float(scale), c_float(softcap), ptr(bias_t), 0 if bias_t is None else bias_t.shape[1] - 1,
+        ptr(sink), ptr(out), q.shape[0], n_seqs, max_q_len, n_heads, n_kv_heads, dk, dv,
         ptr(status if status is not None else status_word(q.device)), stream()))
     return out
 

@@ -36,10 +36,10 @@ def kv_write(qkv: torch.Tensor, q_out: torch.Tensor, cache: Optional[torch.Tenso
         raise KernelError("kv_write: the cache does not fit the heads")
     lib = load_kernel(_LIB)
     check(_LIB, lib.tq_bias_kv_write(
-        ptr(qkv), ptr(q_out), ptr(cache), c_int(code(q_out.dtype)), ptr(v_keep), ptr(v_other), c_float(mix),
-        ptr(positions), ptr(seq_of_token), ptr(page_table), c_int(page_table.shape[1]), c_int(page_size), c_int(T),
-        c_int(heads), c_int(kv_heads), c_int(dk), c_int(dv), c_int(page_table.shape[0]),
-        c_int(cache.shape[0] if cache is not None else 0), stream()))
+        ptr(qkv), ptr(q_out), ptr(cache), code(q_out.dtype), ptr(v_keep), ptr(v_other), c_float(mix),
+        ptr(positions), ptr(seq_of_token), ptr(page_table), page_table.shape[1], page_size, T,
+        heads, kv_heads, dk, dv, page_table.shape[0],
+        cache.shape[0] if cache is not None else 0, stream()))
 
 
 def kv_write_rot(qkv: torch.Tensor, q_out: torch.Tensor, cache: Optional[torch.Tensor], freq: Optional[torch.Tensor],
@@ -87,11 +87,11 @@ def kv_write_rot(qkv: torch.Tensor, q_out: torch.Tensor, cache: Optional[torch.T
         raise KernelError("kv_write_rot: the cache does not fit the heads")
     lib = load_kernel(_LIB)
     check(_LIB, lib.tq_bias_kv_write_rot(
-        ptr(qkv), c_int(qkv.shape[1]), ptr(q_out), ptr(cache), c_int(code(q_out.dtype)), ptr(freq), c_int(rot_dims),
-        c_int(1 if halves else 0), c_float(mag), c_float(unit_eps), ptr(q_norm), ptr(k_norm), c_float(norm_eps),
-        c_int(1 if norm_rows else 0), ptr(v_freq), c_int(v_share), c_int(1 if values_are_keys else 0), c_float(coef), c_int(every), ptr(positions), ptr(seq_of_token), ptr(page_table),
-        c_int(page_table.shape[1]), c_int(page_size), c_int(T), c_int(heads), c_int(kv_heads), c_int(dk), c_int(dv),
-        c_int(page_table.shape[0]), c_int(cache.shape[0] if cache is not None else 0), stream()))
+        ptr(qkv), qkv.shape[1], ptr(q_out), ptr(cache), code(q_out.dtype), ptr(freq), rot_dims,
+        1 if halves else 0, c_float(mag), c_float(unit_eps), ptr(q_norm), ptr(k_norm), c_float(norm_eps),
+        1 if norm_rows else 0, ptr(v_freq), v_share, 1 if values_are_keys else 0, c_float(coef), every, ptr(positions), ptr(seq_of_token), ptr(page_table),
+        page_table.shape[1], page_size, T, heads, kv_heads, dk, dv,
+        page_table.shape[0], cache.shape[0] if cache is not None else 0, stream()))
 
 
 def heads_unrotate_gate(o: torch.Tensor, gates: torch.Tensor, gate_off: int, v_freq: Optional[torch.Tensor], halves: bool,
@@ -109,9 +109,9 @@ def heads_unrotate_gate(o: torch.Tensor, gates: torch.Tensor, gate_off: int, v_f
     if o.shape != (T, heads * dv) or out.shape != o.shape or out.dtype != o.dtype:
         raise KernelError("heads_unrotate_gate: input and output must be [T, heads * dv] of one dtype")
     lib = load_kernel(_LIB)
-    check(_LIB, lib.tq_heads_unrotate_gate(ptr(o), c_int(code(o.dtype)), ptr(gates), c_int(gates.shape[1]), c_int(gate_off),
-                                           ptr(v_freq), c_int(1 if halves else 0), ptr(positions), ptr(out), c_int(T),
-                                           c_int(heads), c_int(dv), stream()))
+    check(_LIB, lib.tq_heads_unrotate_gate(ptr(o), code(o.dtype), ptr(gates), gates.shape[1], gate_off,
+                                           ptr(v_freq), 1 if halves else 0, ptr(positions), ptr(out), T,
+                                           heads, dv, stream()))
     return out
 
 
@@ -174,7 +174,7 @@ def attention_runs(q: torch.Tensor, cache: torch.Tensor, bias_t: Optional[torch.
         far = bias_t.shape[1] - 1
     if sink is not None:
         want_f32(sink, "the sink")
-    if dk >= 64 and dv >= 64 and runs_usable(q.dtype, dk, dv, page_size):
+    if dk in (64, 128) and dv in (64, 128) and q.dtype == torch.bfloat16 and page_size == 64:
         return prefill_rows(q, cache, 1, cu_seqlens, seq_start, page_table, page_size, window, scale, out, n_seqs, max_run, heads,
                             kv_heads, dk, dv, keep_first=keep_first, cell=cell, softcap=softcap, bias_t=bias_t, sink=sink, status=status)
     lib = load_kernel(_LIB)

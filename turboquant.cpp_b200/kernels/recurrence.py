@@ -1,7 +1,7 @@
 """Launchers of csrc/recurrence.cuh (in the library of csrc/ssm.cu): recurrences over runs of many tokens in chunks of 64, as float32 matrix products."""
 from __future__ import annotations
 
-from ctypes import c_int, c_longlong
+from ctypes import c_longlong, c_void_p
 from typing import Sequence
 
 import torch
@@ -41,10 +41,11 @@ def memory_chunks(rows: torch.Tensor, q_off: int, k_off: int, v_off: int, gates:
             or y.numel() != T * heads * dv or dots.numel() != T * heads or gates.numel() != 2 * T * heads or slots.numel() < n_seqs \
             or max(q_off + heads * dk, k_off + heads * dk, v_off + heads * dv) > rows.shape[1]:
         raise KernelError("memory_chunks: sizes of 64 or 128, aligned rows that hold the heads, a state row of [heads, dv + 1, dk]")
-    ends = torch.empty((chunks, heads, dv + 1, dk), dtype=torch.float32, device=rows.device)
-    decays = torch.empty((chunks, heads), dtype=torch.float32, device=rows.device)
+    per_chunk = heads * (dv + 1) * dk
+    scratch = torch.empty(chunks * (per_chunk + heads), dtype=torch.float32, device=rows.device)      # the chunks' states, then their decays
+    at = scratch.data_ptr()
     lib = load_kernel(_LIB)
+    # (plain ints are C ints to ctypes)
     check(_LIB, lib.tq_memory_chunks(
-        ptr(rows), c_int(rows.shape[1]), c_int(q_off), c_int(k_off), c_int(v_off), ptr(gates), ctypes_ptr(state), c_longlong(state.stride(0)),
-        ptr(y), ptr(dots), ptr(ends), ptr(decays), c_int(chunks), c_int(n_seqs), c_int(heads), c_int(dk), c_int(dv), ptr(cu_seqlens),
-        ptr(slots), stream()), kernels=3)
+        ptr(rows), rows.shape[1], q_off, k_off, v_off, ptr(gates), ctypes_ptr(state), c_longlong(state.stride(0)), ptr(y), ptr(dots),
+        c_void_p(at), c_void_p(at + 4 * chunks * per_chunk), chunks, n_seqs, heads, dk, dv, ptr(cu_seqlens), ptr(slots), stream()), kernels=3)

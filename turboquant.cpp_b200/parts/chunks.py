@@ -15,12 +15,8 @@ ROUNDS = 4
 _sm_counts = {}
 
 
-def cut_runs(ctx: StepContext, heads: int, columns: int) -> Optional[Tuple[torch.Tensor, torch.Tensor, torch.Tensor]]:
-    """None, or how this step's runs are cut: (token offsets of the chunks [chunks + 1], chunk numbers [chunks], each
-    sequence's chunks [sequences + 1]) on the device.  The recurrence kernel walks a run token by token with a warp per
-    four of a head's `columns` columns of state; where those warps fill at most half of the GPU and a run is long,
-    cutting the runs fills it (ROUNDS times over, so that the last round of blocks costs little), at the price of walking
-    them once more for the states alone (half the work of a walk with outputs).  The plan depends on the step's runs and on heads and columns only, and is kept for the step's other layers."""
+def cut_size(ctx: StepContext, heads: int, columns: int) -> Optional[int]:
+    """The tokens of a chunk if this step's runs are worth cutting (see `cut_runs`), else None."""
     lens = list(ctx.host_q_lens)
     if not lens or len(lens) != ctx.n_seqs or max(lens) < 2 * MIN_CHUNK:
         return None
@@ -35,6 +31,19 @@ def cut_runs(ctx: StepContext, heads: int, columns: int) -> Optional[Tuple[torch
     size = -(-size // 16) * 16
     if max(lens) < 2 * size:
         return None
+    return size
+
+
+def cut_runs(ctx: StepContext, heads: int, columns: int) -> Optional[Tuple[torch.Tensor, torch.Tensor, torch.Tensor]]:
+    """None, or how this step's runs are cut: (token offsets of the chunks [chunks + 1], chunk numbers [chunks], each
+    sequence's chunks [sequences + 1]) on the device.  The recurrence kernel walks a run token by token with a warp per
+    four of a head's `columns` columns of state; where those warps fill at most half of the GPU and a run is long,
+    cutting the runs fills it (ROUNDS times over, so that the last round of blocks costs little), at the price of walking
+    them once more for the states alone (half the work of a walk with outputs).  The plan depends on the step's runs and on heads and columns only, and is kept for the step's other layers."""
+    size = cut_size(ctx, heads, columns)
+    if size is None:
+        return None
+    lens = list(ctx.host_q_lens)
     name = f"run_chunks_{size}"
     plan = ctx.carry.get(name) if ctx.carry is not None else None
     if plan is None:

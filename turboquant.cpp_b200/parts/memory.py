@@ -27,13 +27,16 @@ from ..kernels import ssm as KS
 from ..kernels.linear import linear
 from ..weights.loader import WeightSpec, WeightStore
 from .base import LayerCache, Mixer, StateNeed, StepContext, register_mixer
-from .chunks import cut_runs
+from .chunks import cut_runs, cut_size
 
 DENOMINATOR_FLOOR = 1e-6
 
 
 class MatrixMemoryMixer(Mixer):
-    CHUNKS_MIN = 64           # steps whose longest run of new tokens is at least this take the matrix form, chunk by chunk
+    # steps whose longest run of new tokens is at least this, or whose runs a walk would have to cut, take the matrix form; below, the
+    # walk's one launch is cheaper than three (layer on B200, walk / matrix form, us: runs of 60 to 240 tokens of four sequences
+    # 105 / 120, one run of 130: 189 / 119, of 2,048: 395 / 221)
+    CHUNKS_MIN = 256
 
     def __init__(self, prefix: str, hidden: int, heads: int, dim: int, vdim: int, gate_cap: float, eps: float):
         if heads < 1 or vdim < 1 or not 1 <= dim <= KS.MAX_STATE:
@@ -99,7 +102,7 @@ class MatrixMemoryMixer(Mixer):
             f32 = lambda *shape: torch.empty(shape, dtype=torch.float32, device=dev)
             gates, m, y, dots = f32(T, H, 2), f32(T, H), f32(T, self.inner), f32(T, H)
             KS.memory_gates(proj, i, f, self.i_bias, self.f_bias, self.cap, tops, gates, m, H, ctx.cu_seqlens, ctx.slots)
-            in_chunks = ctx.max_q_len >= self.CHUNKS_MIN and KR.usable(dk, dv, proj, q, k, v)
+            in_chunks = ((ctx.max_q_len >= self.CHUNKS_MIN or cut_size(ctx, H, dv + 1) is not None) and KR.usable(dk, dv, proj, q, k, v))
             if in_chunks:
                 KR.memory_chunks(proj, q, k, v, gates, S, y, dots, KR.chunks_of(ctx.host_q_lens, T, ctx.n_seqs), H, dk, dv, ctx.cu_seqlens, ctx.slots)
             scan = lambda st, out, nq, cu, slots: KS.memory_scan(proj, q, k, v, gates, st, out, nq, H, dk, dv, cu, slots)
