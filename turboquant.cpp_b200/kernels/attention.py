@@ -217,7 +217,9 @@ def prefill_rows(q: torch.Tensor, cache_layer: torch.Tensor, planes: int, cu_seq
                  status: Optional[torch.Tensor] = None) -> torch.Tensor:
     """The tensor-core prompt kernel over a cache of two planes (keys, values) or one (rows [key | value]), with the
     options of `kernels.bias_attention.attention_runs`."""
-    from .gemm_tc import status_word
+    if status is None:
+        from .gemm_tc import status_word
+        status = status_word(q.device)
     if cu_seqlens.dtype != torch.int32 or seq_start.dtype != torch.int32 or page_table.dtype != torch.int32:
         raise KernelError("attention_prefill: cu_seqlens, seq_start and the page table must be int32")
     if q.dtype != torch.bfloat16 or cache_layer.dtype != torch.bfloat16 or out.dtype != torch.bfloat16:
@@ -227,7 +229,7 @@ def prefill_rows(q: torch.Tensor, cache_layer: torch.Tensor, planes: int, cu_seq
         ptr(q), ptr(cache_layer), planes, ptr(cu_seqlens), ptr(seq_start), ptr(page_table), page_table.shape[1], page_size,
         cache_layer.shape[0], window, keep_first, cell, c_float(scale), c_float(softcap), ptr(bias_t), 0 if bias_t is None else bias_t.shape[1] - 1,
         ptr(sink), ptr(out), q.shape[0], n_seqs, max_q_len, n_heads, n_kv_heads, dk, dv,
-        ptr(status if status is not None else status_word(q.device)), stream()))
+        ptr(status), stream()))
     return out
 
 

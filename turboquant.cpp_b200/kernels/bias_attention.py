@@ -2,6 +2,7 @@
 positions and a sink in the softmax, over cache rows that hold a key and a value of different sizes."""
 from __future__ import annotations
 
+import os
 from ctypes import c_float, c_int
 from typing import Optional
 
@@ -150,7 +151,6 @@ RUN_SIZES = (32, 64, 128)      # key and value sizes the tensor-core kernel for 
 def runs_usable(dtype: torch.dtype, dk: int, dv: int, page_size: int) -> bool:
     """Whether the tensor-core kernel for runs of new tokens takes this shape: bfloat16, key and value sizes of 32,
     64 or 128, pages of 64 positions (TQ_BIAS_NO_MMA=1 switches it off)."""
-    import os
     return (dtype == torch.bfloat16 and dk in RUN_SIZES and dv in RUN_SIZES and page_size == 64
             and os.environ.get("TQ_BIAS_NO_MMA", "") in ("", "0"))
 

@@ -27,7 +27,7 @@ from ..kernels import ssm as KS
 from ..kernels.linear import linear
 from ..weights.loader import WeightSpec, WeightStore
 from .base import LayerCache, Mixer, StateNeed, StepContext, register_mixer
-from .chunks import cut_runs, cut_size
+from .chunks import MIN_CHUNK, cut_runs, cut_size
 
 DENOMINATOR_FLOOR = 1e-6
 
@@ -102,11 +102,12 @@ class MatrixMemoryMixer(Mixer):
             f32 = lambda *shape: torch.empty(shape, dtype=torch.float32, device=dev)
             gates, m, y, dots = f32(T, H, 2), f32(T, H), f32(T, self.inner), f32(T, H)
             KS.memory_gates(proj, i, f, self.i_bias, self.f_bias, self.cap, tops, gates, m, H, ctx.cu_seqlens, ctx.slots)
-            in_chunks = ((ctx.max_q_len >= self.CHUNKS_MIN or cut_size(ctx, H, dv + 1) is not None) and KR.usable(dk, dv, proj, q, k, v))
+            cuts = ctx.max_q_len >= 2 * MIN_CHUNK and cut_size(ctx, H, dv + 1) is not None
+            in_chunks = (cuts or ctx.max_q_len >= self.CHUNKS_MIN) and KR.usable(dk, dv, proj, q, k, v)
             if in_chunks:
                 KR.memory_chunks(proj, q, k, v, gates, S, y, dots, KR.chunks_of(ctx.host_q_lens, T, ctx.n_seqs), H, dk, dv, ctx.cu_seqlens, ctx.slots)
             scan = lambda st, out, nq, cu, slots: KS.memory_scan(proj, q, k, v, gates, st, out, nq, H, dk, dv, cu, slots)
-            plan = cut_runs(ctx, H, dv + 1) if not in_chunks else None
+            plan = cut_runs(ctx, H, dv + 1) if cuts and not in_chunks else None
             if in_chunks:
                 pass
             elif plan is None:
