@@ -53,23 +53,23 @@ def reference(m, x, held_rows, runs, held, weights, eps):
     return torch.cat(outs)
 
 
-@pytest.mark.parametrize("case", range(len(CASES)))
-def test_expanded_prompts(case, monkeypatch):
+def layer_and_step(case, seed, unused=0.0):
+    """(mixer, weights by name, input rows, the held rows, the step, its cache, whose slots that no position has taken hold `unused`)."""
     from turboquant_cpp_b200.parts import LayerCache, StepContext, make_mixer, make_position_encoding
     from turboquant_cpp_b200.weights import RandomSource, WeightStore
-    H, dim, rot, vdim, R, window, sink, runs, held = CASES[case]
+    H, dim, rot, vdim, R, window, sink, runs, held = case
     pe = make_position_encoding("rotary_scaled", dims=rot, base=10000.0, factor=2.0, original=128, fast=8.0, slow=1.0) if rot else None
     m = make_mixer("latent_attention", prefix="", hidden=256, heads=H, dim=dim, rot_dim=rot, vdim=vdim, kv_rank=R, scale=(dim + rot) ** -0.5,
                    eps=1e-5, window=window, position=pe, sink=sink)
     m.run_dtype = torch.bfloat16
-    source = RandomSource(m.weight_specs(), case, std=0.06)
+    source = RandomSource(m.weight_specs(), seed, std=0.06)
     m.bind(WeightStore(source, m.weight_specs(), DEV, torch.bfloat16))
     weights = {s.name: source.read(s.name, DEV) for s in m.weight_specs()}
-    g = torch.Generator(device=DEV).manual_seed(case)
+    g = torch.Generator(device=DEV).manual_seed(seed)
     total = [n + h for n, h in zip(runs, held)]
     counts = [-(-t // 64) for t in total]
-    order = torch.randperm(sum(counts), generator=torch.Generator().manual_seed(case)).split(counts)
-    kv = torch.zeros((sum(counts), 1, 1, 64, R + rot), dtype=torch.bfloat16, device=DEV)
+    order = torch.randperm(sum(counts), generator=torch.Generator().manual_seed(seed)).split(counts)
+    kv = torch.full((sum(counts), 1, 1, 64, R + rot), unused, dtype=torch.bfloat16, device=DEV)
     table = torch.full((len(runs), max(counts)), -1, dtype=torch.int32)
     old = []
     for i, h in enumerate(held):
@@ -86,7 +86,13 @@ def test_expanded_prompts(case, monkeypatch):
                       seq_start=i32(held), slots=i32(range(len(runs))), want_rows=i32([]), n_want=0, max_q_len=max(runs), max_kv_len=max(total),
                       act_dtype=torch.bfloat16, device=torch.device(DEV), host_q_lens=runs, host_seq_start=held,
                       status=torch.zeros(1, dtype=torch.int32, device=DEV))
-    cache = LayerCache(kv=kv, page_table=table.to(DEV), page_size=64)
+    return m, weights, x, old, ctx, LayerCache(kv=kv, page_table=table.to(DEV), page_size=64)
+
+
+@pytest.mark.parametrize("case", range(len(CASES)))
+def test_expanded_prompts(case, monkeypatch):
+    runs, held = CASES[case][-2:]
+    m, weights, x, old, ctx, cache = layer_and_step(CASES[case], case)
     want = reference(m, x, old, runs, held, weights, 1e-5)
     err = {}
     for per_token in (1 << 20, 0):       # always expanded, never
@@ -97,3 +103,16 @@ def test_expanded_prompts(case, monkeypatch):
     # the same number of roundings to bfloat16 on either path (queries, keys, values and weights here; queries in the latent
     # space, weights and weighted latents there): neither may be further off than half as much again
     assert err[1 << 20] < 1.5 * err[0] and err[1 << 20] < 8e-3, err
+
+
+@pytest.mark.parametrize("case", range(len(CASES)))
+@pytest.mark.parametrize("unused", [float("nan"), float("inf"), 3e38])
+def test_slots_that_no_position_has_taken_are_never_seen(case, unused, monkeypatch):
+    """A page keeps what its last owner left behind the new one's end: the same bits whatever that is."""
+    got = []
+    for fill in (0.0, unused):
+        m, _, x, _, ctx, cache = layer_and_step(CASES[case], case, fill)
+        monkeypatch.setattr(type(m), "EXPAND_KEYS_PER_TOKEN", 1 << 20)
+        assert m._expands(ctx, cache)
+        got.append(m.forward(x, ctx, cache))
+    assert torch.equal(got[0], got[1]) and bool(torch.isfinite(got[0]).all())

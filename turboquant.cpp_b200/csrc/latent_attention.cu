@@ -739,7 +739,9 @@ TQ_EXPORT int tq_latent_gather(const void* cache, int act_dtype, const int* tabl
 }
 
 // The pages of a whole step's sequences, one sequence after another, into out [pages * page_size, Dk]: of each the pages that
-// hold what its new tokens see (from position max(0, seq_start + 1 - window) on; window 0: all).  page_base[s]: the place of
+// hold what its new tokens see (from position max(0, seq_start + 1 - window) on; window 0: all).  Rows behind a sequence's last
+// position come out as zeros whatever the cache holds there: a page keeps what its last owner left, and the prompt kernel
+// multiplies those rows' values by weights of zero, which an infinity or NaN among them would survive.  page_base[s]: the place of
 // the sequence's page 0 among them (its page p lies at page_base[s] + p).  Grid (most pages of a sequence, sequences).
 template <typename TA>
 __global__ void __launch_bounds__(256)
@@ -748,7 +750,7 @@ latent_gather_pages_kernel(const TA* __restrict__ cache, const int* __restrict__
                            TA* __restrict__ out, int out_pages, int* __restrict__ page_base, int n_pages) {
     tq_grid_wait();                    // everything below may read what the previous kernel wrote
     tq_grid_launch_dependents();       // the next kernel's CTAs may move in as SMs free up
-    __shared__ int s_base, s_first, s_count;
+    __shared__ int s_base, s_first, s_count, s_end;
     const int s = blockIdx.y;
     if (threadIdx.x < 32) {            // pages of the sequences before this one
         int before = 0;
@@ -756,7 +758,7 @@ latent_gather_pages_kernel(const TA* __restrict__ cache, const int* __restrict__
             const int start = seq_start[i], end = start + cu_seqlens[i + 1] - cu_seqlens[i];
             const int first = window > 0 ? max(0, start + 1 - window) / page_size : 0, n = (end - 1) / page_size - first + 1;
             if (i < s) before += n;
-            else { s_first = first; s_count = n; }
+            else { s_first = first; s_count = n; s_end = end; }
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
@@ -764,12 +766,22 @@ latent_gather_pages_kernel(const TA* __restrict__ cache, const int* __restrict__
     }
     __syncthreads();
     if (blockIdx.x == 0 && threadIdx.x == 0) page_base[s] = s_base - s_first;
-    const int n16 = (int)((size_t)page_size * Dk * sizeof(TA) / 16);
+    constexpr int PER = 16 / (int)sizeof(TA);                  // elements of 16 bytes
+    const int n16 = page_size * Dk / PER;
     for (int p = blockIdx.x; p < s_count && s_base + p < out_pages; p += gridDim.x) {
+        const int live = min(page_size, s_end - (s_first + p) * page_size) * Dk;       // elements up to the sequence's end
         const int page = TQ_CHECKED(page_table[(size_t)s * table_stride + TQ_CHECKED(s_first + p, table_stride, TQ_IDX_TABLE_COLUMN)], n_pages, TQ_IDX_PAGE);
         const uint4* src = reinterpret_cast<const uint4*>(cache + (size_t)page * page_size * Dk);
         uint4* dst = reinterpret_cast<uint4*>(out + (size_t)(s_base + p) * page_size * Dk);
-        for (int i = threadIdx.x; i < n16; i += blockDim.x) dst[i] = src[i];
+        for (int i = threadIdx.x; i < n16; i += blockDim.x) {
+            union { uint4 all; TA each[PER]; } v;
+            v.all = i * PER < live ? src[i] : make_uint4(0u, 0u, 0u, 0u);
+            if (i * PER < live && (i + 1) * PER > live) {      // rows of odd sizes may end within 16 bytes
+#pragma unroll
+                for (int e = 0; e < PER; ++e) if (i * PER + e >= live) v.each[e] = tq_from_float<TA>(0.f);
+            }
+            dst[i] = v.all;
+        }
     }
 }
 
