@@ -116,3 +116,21 @@ def test_slots_that_no_position_has_taken_are_never_seen(case, unused, monkeypat
         assert m._expands(ctx, cache)
         got.append(m.forward(x, ctx, cache))
     assert torch.equal(got[0], got[1]) and bool(torch.isfinite(got[0]).all())
+
+
+def test_sequences_without_new_tokens(monkeypatch):
+    """Host and kernel count the same pages where a run is empty: the others' rows are those of the step without it."""
+    got = []
+    for runs, held in (([130, 70], [0, 40]), ([0, 130, 0, 70], [0, 0, 100, 40]), ([0, 130, 0, 70, 0], [0, 0, 0, 40, 0])):
+        m, _, x, old, ctx, cache = layer_and_step((4, 128, 64, 128, 128, 0, False, runs, held), 5)
+        live = [i for i, n in enumerate(runs) if n]
+        if not got:
+            rows, inputs = [old[i] for i in live], x
+        else:                              # the same held rows and inputs in the wider step's pages
+            for i, r in zip(live, rows):
+                at = torch.arange(r.shape[0], device=DEV)
+                cache.kv[cache.page_table[i].long()[at // 64], 0, 0, at % 64] = r
+        monkeypatch.setattr(type(m), "EXPAND_KEYS_PER_TOKEN", 1 << 20)
+        assert m._expands(ctx, cache)
+        got.append(m.forward(inputs, ctx, cache))
+    assert all(torch.equal(got[0], g) for g in got[1:])

@@ -755,8 +755,9 @@ latent_gather_pages_kernel(const TA* __restrict__ cache, const int* __restrict__
     if (threadIdx.x < 32) {            // pages of the sequences before this one
         int before = 0;
         for (int i = threadIdx.x; i <= s; i += 32) {
-            const int start = seq_start[i], end = start + cu_seqlens[i + 1] - cu_seqlens[i];
-            const int first = window > 0 ? max(0, start + 1 - window) / page_size : 0, n = (end - 1) / page_size - first + 1;
+            const int start = seq_start[i], run = cu_seqlens[i + 1] - cu_seqlens[i], end = start + run;
+            const int first = window > 0 ? max(0, start + 1 - window) / page_size : 0;
+            const int n = run > 0 ? (end - 1) / page_size - first + 1 : 0;            // a sequence without new tokens sees none
             if (i < s) before += n;
             else { s_first = first; s_count = n; s_end = end; }
         }

@@ -168,7 +168,7 @@ class LatentAttentionMixer(Mixer):
 
     def _pages_seen(self, ctx: StepContext, page: int) -> int:
         first = lambda start: max(0, start + 1 - self.window) // page if self.window else 0
-        return sum((start + n - 1) // page - first(start) + 1 for n, start in zip(ctx.host_q_lens, ctx.host_seq_start))
+        return sum((start + n - 1) // page - first(start) + 1 for n, start in zip(ctx.host_q_lens, ctx.host_seq_start) if n)
 
     def _expands(self, ctx: StepContext, cache: LayerCache) -> bool:
         """Whether this step builds the heads' keys and values.  Measured on B200, 16 heads of 128 + 64 / 128, rank 512, a
