@@ -1,6 +1,8 @@
 """The tcgen05 prompt kernel over every way its query tiles are paired and every option, against float64: runs around the
 tiles' edges (64, 128, 256 rows), sequences that hold earlier positions, grouped and ungrouped heads, windows with kept
 positions, cells, caps (scores on both sides of a quarter of the cap), distance biases, sinks."""
+import math
+
 import numpy as np
 import pytest
 import torch
@@ -93,3 +95,57 @@ def test_prompt_kernel(case, spread):
         # too (2^-8 of it); the float32 scores, |s| up to about 40, add 2^-16 of relative weight
         bound = (2.0 ** -8 + 2.0 ** -16) * mag + 2.0 ** -8 * want.abs() + 1e-6
         assert bool(((got - want).abs() <= bound).all()), float(((got - want).abs() / bound).max())
+
+
+def one_sequence(q, k, v, **options):
+    """Attention over rows of one sequence whose positions all are new: q [T, H, dk], k [T, G, dk], v [T, G, dv] -> [T, H, dv]."""
+    from turboquant_cpp_b200.kernels import bias_attention as KB
+    T, H, dk = q.shape
+    G, dv, pages = k.shape[1], v.shape[2], -(-T // 64)
+    cache = torch.zeros((pages, 1, G, 64, dk + dv), dtype=torch.bfloat16, device=DEV)
+    at = torch.arange(T, device=DEV)
+    cache[at // 64, 0, :, at % 64] = torch.cat([k, v], -1).to(torch.bfloat16)
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device=DEV)
+    out = torch.empty((T, H * dv), dtype=torch.bfloat16, device=DEV)
+    bias, sink = options.pop("bias", None), options.pop("sink", None)
+    KB.attention_runs(q.to(torch.bfloat16), cache, bias, sink, i32([0, T]), i32([0]), i32([list(range(pages))]), 64, options.pop("window", 0), 0,
+                      options.pop("scale", 1.0), out, 1, T, H, G, dk, dv, **options)
+    return out.view(T, H, dv)
+
+
+@pytest.mark.parametrize("options", [{}, {"bias": True}, {"softcap": 1e4}, {"cell": 512}])
+def test_the_largest_weight_is_not_rounded(options):
+    """A row's largest weight is exactly one in the second product, also where a later tile brings it and the maximum grows by less
+    than 2^8: with all other values zero the result is a float32 quotient, rounded once, but for the rounding of the one other weight
+    that counts in the sum."""
+    T, d, late = 400, 64, 300
+    g = torch.Generator().manual_seed(3)
+    q, k, v = torch.zeros(T, 1, d), torch.zeros(T, 1, d), torch.zeros(T, 1, d)
+    q[:, 0, 0], q[:, 0, 1] = 3.0 + 2.4 * torch.rand(T, generator=g), 1.0
+    k[late, 0, 0] = 1.0                                            # scores of 3 to 5.4
+    k[1:, 0, 1], k[late, 0, 1] = -20.0, 0.0                        # position 0: zero, all others: -20
+    v[late, 0] = 1.0 + torch.rand(d, generator=g)
+    q, v = q.to(torch.bfloat16).float(), v.to(torch.bfloat16).float()
+    options = dict(options)
+    if options.pop("bias", False):
+        options["bias"] = torch.zeros((1, 50), device=DEV)
+    got = one_sequence(q.to(DEV), k.to(DEV), v.to(DEV), **options)[late:, 0].double().cpu()
+    s = q[late:, 0, 0].double()
+    s = options["softcap"] * torch.tanh(s / options["softcap"]) if "softcap" in options else s
+    others = 1.0 + math.exp(-20) * (torch.arange(late, T, dtype=torch.float64) - 1)
+    share = (torch.exp(s) / (torch.exp(s) + others))[:, None]
+    want = share * v[late, 0].double()
+    half = torch.exp2(torch.floor(torch.log2(want)) - 8)           # half a unit in the last place of bfloat16
+    assert bool(((got - want).abs() <= half + (2.0 ** -8 * (1 - share) + 2.0 ** -18) * want).all()), float(((got - want).abs() / half).max())
+
+
+def test_the_lowest_finite_bias_leaves_a_row_its_weights():
+    """Where every key a row sees is biased by the type's lowest value the weights are equal, as they are after any other constant."""
+    T, H, d = 200, 2, 64
+    g = torch.Generator(device=DEV).manual_seed(4)
+    v = torch.randn((T, H, d), generator=g, device=DEV).to(torch.bfloat16)
+    zero = torch.zeros((T, H, d), device=DEV)
+    got = one_sequence(zero, zero, v, bias=torch.full((H, 8), torch.finfo(torch.float32).min, device=DEV)).double()
+    n = torch.arange(1, T + 1, device=DEV, dtype=torch.float64)[:, None, None]
+    want, mag = v.double().cumsum(0) / n, v.double().abs().cumsum(0) / n
+    assert bool(((got - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -20 * mag).all())

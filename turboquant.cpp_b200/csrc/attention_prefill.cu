@@ -162,6 +162,16 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16
           "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
         : "memory");
 }
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+        "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
+        ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
+          "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]),
+          "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]),
+          "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
+        : "memory");
+}
 constexpr int PAGE = 64;     // tokens per cache page
 constexpr int BN = 128;      // keys per tile = two cache pages (a unit's last tile may hold one)
 constexpr float LOG2E = 1.4426950408889634f;
@@ -295,8 +305,10 @@ __device__ __forceinline__ void cap_scores(uint32_t (&v)[32], const CapSeries& s
     }
 }
 
-// SHAPED: scores pass through a cap and/or a bias per distance before the softmax.
-template <int DK, int DV, bool SHAPED>
+// ROWS: the form of attention over rows.  Scores may pass through a cap and/or a bias per distance, and a row's largest weight is
+// exactly one at the end of each tile; the other form (plain and latent attention) takes plain scores and keeps a maximum until it is
+// outgrown by 2^8.
+template <int DK, int DV, bool ROWS>
 __global__ void __launch_bounds__(THREADS, 1)
 attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                          const __grid_constant__ CUtensorMap map_r, const __grid_constant__ CUtensorMap map_v,
@@ -311,7 +323,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     __shared__ uint32_t s_tmem_base;
     __shared__ __align__(16) uint4 s_answer;               // the hardware's answer to a request for another block
     __shared__ int s_unit[2];                              // the units this CTA takes, two in turn
-    __shared__ float s_bias[SHAPED ? 8 : 1][2][SHAPED ? 96 : 1];        // a warp's rows and a page's keys: the bias of their 95 distances
+    __shared__ float s_bias[ROWS ? 8 : 1][2][ROWS ? 96 : 1];        // a warp's rows and a page's keys: the bias of their 95 distances
 
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // the same for the whole warp, and known to be
 
@@ -563,13 +575,15 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     } else {
         // ------------------------------ softmax: a thread per query row ------------------------------
         asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
-        constexpr int CW = SHAPED ? 1 : 2;            // 32-key pieces a thread takes at a time
-        constexpr float RESCALE_LOG2 = 8.0f;          // O is rescaled when a row's maximum has grown by more than 2^8
+        constexpr int CW = ROWS ? 1 : 2;            // 32-key pieces a thread takes at a time
+        constexpr float SLACK = ROWS ? 0.f : 8.f;   // powers of two by which a row's maximum may outgrow the one its exponentials are taken against
         const int slot = warp >> 2, quarter = warp & 3, r = quarter * 32 + lane;
         const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
         const uint32_t s_addr = tmem_s(slot) + lane_addr, acc = tmem_o(slot) + lane_addr;
-        const float factor = SHAPED ? LOG2E : S.scale * LOG2E;            // from a score as it stands to an exponent of two
-        const bool capped = SHAPED && S.softcap > 0.f;
+        // plain scores become exponents of two in the multiply-add that takes the maximum off; shaped ones keep their unit until it
+        // is off, so that the largest finite values among them stay finite
+        const float factor = ROWS ? 1.0f : S.scale * LOG2E, to_log2 = ROWS ? LOG2E : 1.0f;
+        const bool capped = ROWS && S.softcap > 0.f;
         const CapSeries series = cap_series(S.scale, capped ? S.softcap : 1.f);
         int tiles = 0, units = 0, taken = 0;
         bool ok = true;
@@ -582,7 +596,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             const int keep = S.cell > 0 || S.window == 0 ? 0 : S.keep_first;   // positions below it are seen besides those from `start` on
             // a page from here on is seen whole by every row that lies behind it
             const int open_from = S.cell > 0 ? p_last - p_last % S.cell : (S.window > 0 ? p_last + 1 - S.window : 0);
-            const float* bias = SHAPED && bias_t != nullptr ? bias_t + (size_t)h * (S.far + 1) : nullptr;
+            const float* bias = ROWS && bias_t != nullptr ? bias_t + (size_t)h * (S.far + 1) : nullptr;
             float nb[6];                               // the next tile's bias values on their way to shared memory
             auto fetch_bias = [&](int i) {
 #pragma unroll
@@ -591,41 +605,66 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                     nb[j] = __ldg(bias + min(max(d, 0), S.far));
                 }
             };
-            if (SHAPED && bias != nullptr) fetch_bias(0);
-            // m: what the row's exponents of two are counted from, its maximum or up to RESCALE_LOG2 below it; l: the sum of
-            // its exponentials
-            const float floor_m = sink != nullptr ? sink[h] * LOG2E : -INFINITY;
+            if (ROWS && bias != nullptr) fetch_bias(0);
+            // m: what the row's exponents are counted from, its maximum or up to 2^SLACK below it; l: the sum of its exponentials
+            const float floor_m = sink != nullptr ? sink[h] * (ROWS ? 1.0f : LOG2E) : -INFINITY;
             float m = -INFINITY, l = 0.f;
             for (int i = 0; i < n; ++i, ++tiles) {
                 const int np = min(2, u.n_pages - 2 * i);
-                if (SHAPED && bias != nullptr) {
+                if (ROWS && bias != nullptr) {
                     __syncwarp();                      // the previous tile's values have been read
 #pragma unroll
-                    for (int j = 0; j < 6; ++j) s_bias[SHAPED ? warp : 0][j / 3][(j % 3) * 32 + lane] = nb[j];
+                    for (int j = 0; j < 6; ++j) s_bias[ROWS ? warp : 0][j / 3][(j % 3) * 32 + lane] = nb[j];
                     __syncwarp();
                     if (i + 1 < n) fetch_bias(i + 1);
                 }
                 ok = __all_sync(0xffffffffu, mbar_wait(s_ready(slot), (uint32_t)tiles & 1u, &s_abort));   // warp-uniform
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                // half a page (plain scores: a page) at a time, in one pass: shape and mask its scores, see whether they outgrow the maximum the row's
-                // exponentials are taken against, and write them, in bf16, over scores already read.  The loop is kept
-                // small: instructions come in at some 250 cycles per 128 bytes the first time and fall out of the caches
-                // that ten warps share (the tile unrolled in two passes: 1.6 times the kernel's time).
+                // half a page (plain scores: a page) at a time, twice: for the tile's maximum, which shapes and masks the scores and
+                // leaves shaped ones in place of the products, then for the weights, written in bf16 over scores already
+                // read.  The maximum comes first so that a row's largest weight can be exactly one: with it known only so far, and
+                // corrected by powers of two, the error of rows with a cap or bias against 64 bits was up to 1.3 times
+                // as large.  The loops are kept small: instructions come in at some 250 cycles per 128 bytes the first time and
+                // fall out of the caches that ten warps share (the tile unrolled in two passes: 1.6 times the kernel's time).
                 float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+                float top = -INFINITY;
 #pragma unroll 1
-                for (int x = i == 0 ? -2 * np : 0; x < 2 * np; x += CW) {
-                    const int q = x < 0 ? x + 2 * np : x;  // a unit's first tile is walked once ahead for its maximum alone
+                for (int x = -2 * np; x < 2 * np; x += CW) {
+                    const int q = x < 0 ? x + 2 * np : x;
+                    if (x == 0) {
+                        if (ROWS) asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                        const float mx = fmaxf(top * factor, floor_m);
+                        float corr = 1.0f;
+                        if (m == -INFINITY) {
+                            m = mx;                        // l and O are still zero: nothing to rescale
+                        } else if ((mx - m) * to_log2 > SLACK) {
+                            corr = ex2((m - mx) * to_log2);
+                            l *= corr;
+                            m = mx;
+                        }
+                        if (i > 0 && __any_sync(0xffffffffu, corr != 1.0f)) {  // the products so far are done (s_ready)
+#pragma unroll 1
+                            for (int c0 = 0; c0 < DV; c0 += 16) {
+                                uint32_t ov[16];
+                                tmem_ld16(acc + c0, ov);
+                                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                                for (int j = 0; j < 16; ++j) ov[j] = __float_as_uint(__uint_as_float(ov[j]) * corr);
+                                tmem_st16(acc + c0, ov);
+                            }
+                        }
+                    }
                     uint32_t sv[CW][32];
 #pragma unroll
                     for (int w = 0; w < CW; ++w) tmem_ld32(s_addr + (q + w) * 32, sv[w]);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                     const int kq = page_at(u, 2 * i + (q >> 1)) * PAGE + (q & 1) * 32;   // position of the first of these keys
-                    if (SHAPED) {
+                    if (ROWS && x < 0) {
                         if (capped) cap_scores(sv[0], series);
                         if (bias != nullptr) {
                             const float2 f = capped ? make_float2(1.f, 1.f) : make_float2(S.scale, S.scale);
-                            const float* sb = &s_bias[SHAPED ? warp : 0][q >> 1][lane + PAGE - 1 - (q & 1) * 32];
+                            const float* sb = &s_bias[ROWS ? warp : 0][q >> 1][lane + PAGE - 1 - (q & 1) * 32];
 #pragma unroll
                             for (int c = 0; c < 32; c += 2) {
                                 const float2 t = fma2(make_float2(__uint_as_float(sv[0][c]), __uint_as_float(sv[0][c + 1])), f, make_float2(sb[-c], sb[-c - 1]));
@@ -637,7 +676,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                             for (int c = 0; c < 32; ++c) sv[0][c] = __float_as_uint(__uint_as_float(sv[0][c]) * S.scale);
                         }
                     }
-                    if (kq + 32 * CW - 1 > p_first || kq < open_from) {        // some row does not see some of these keys
+                    if ((!ROWS || x < 0) && (kq + 32 * CW - 1 > p_first || kq < open_from)) {        // some row does not see some of these keys
 #pragma unroll
                         for (int w = 0; w < CW; ++w) {
                             // bit c: the row sees key kq + 32 w + c, i.e. c <= last and (c >= lo or c < kp)
@@ -651,65 +690,27 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                                 if (!(seen & (1u << c))) sv[w][c] = 0xff800000u;
                         }
                     }
-                    float mx = max_of(sv[0], -INFINITY);
-                    if (CW > 1) mx = fmaxf(mx, max_of(sv[CW - 1], -INFINITY));
-                    mx = fmaxf(mx * factor, floor_m);
                     if (x < 0) {
-                        m = fmaxf(m, mx);
+                        top = max_of(sv[0], top);
+                        if (CW > 1) top = max_of(sv[CW - 1], top);
+                        if (ROWS) tmem_st32(s_addr + q * 32, sv[0]);
                         continue;
                     }
-                    // keep m unless the maximum grew by more than 2^8 (or nothing had been seen yet); then by a whole power
-                    // of two, which loses nothing of what is rescaled
-                    float corr = 1.0f;
-                    if (m == -INFINITY) {
-                        m = mx;                            // l, P and O are still zero: nothing to rescale
-                    } else if (mx - m > RESCALE_LOG2) {
-                        const float k = ceilf(mx - m);
-                        corr = k < 127.f ? __int_as_float((127 - (int)k) << 23) : 0.f;
-                        l *= corr;
-                        m += k;
-                    }
-                    if (__any_sync(0xffffffffu, corr != 1.0f)) {
-                        const float2 cc = make_float2(corr, corr);
-                        sum[0] = mul2(sum[0], cc);
-                        sum[1] = mul2(sum[1], cc);
-                        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                        uint32_t ov[16];
-                        if (i > 0) {                       // the products so far are done (s_ready)
-#pragma unroll 1
-                            for (int c0 = 0; c0 < DV; c0 += 16) {
-                                tmem_ld16(acc + c0, ov);
-                                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                                for (int j = 0; j < 16; ++j) ov[j] = __float_as_uint(__uint_as_float(ov[j]) * corr);
-                                tmem_st16(acc + c0, ov);
-                            }
-                        }
-#pragma unroll 1
-                        for (int c0 = 0; c0 < q * 16; c0 += 16) {              // what the tile has of P already
-                            tmem_ld16(s_addr + c0, ov);
-                            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) {
-                                const float2 w = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&ov[j]));
-                                const __nv_bfloat162 two = __floats2bfloat162_rn(w.x * corr, w.y * corr);
-                                ov[j] = *reinterpret_cast<const uint32_t*>(&two);
-                            }
-                            tmem_st16(s_addr + c0, ov);
-                        }
-                    }
                     const float mref = m == -INFINITY ? 0.f : m;             // nothing visible yet: exponents of -inf
-                    const float2 ff = make_float2(factor, factor), neg = make_float2(-mref, -mref);
+                    const float2 ff = make_float2(ROWS ? to_log2 : factor, ROWS ? to_log2 : factor), neg = make_float2(-mref, -mref);
 #pragma unroll
                     for (int w = 0; w < CW; ++w) {
                         uint32_t pk[16];
 #pragma unroll
                         for (int e = 0; e < 16; ++e) {
-                            float2 x = fma2(make_float2(__uint_as_float(sv[w][2 * e]), __uint_as_float(sv[w][2 * e + 1])), ff, neg);
+                            float2 x = make_float2(__uint_as_float(sv[w][2 * e]), __uint_as_float(sv[w][2 * e + 1]));
+                            x = ROWS ? mul2(add2(x, neg), ff) : fma2(x, ff, neg);
                             x = make_float2(ex2(x.x), ex2(x.y));
-                            sum[e % 2] = add2(sum[e % 2], x);
                             const __nv_bfloat162 two = __floats2bfloat162_rn(x.x, x.y);
                             pk[e] = *reinterpret_cast<const uint32_t*>(&two);
+                            // the sum of what the second product multiplies: part of the weights' rounding cancels
+                            if (ROWS) x = make_float2(__uint_as_float(pk[e] << 16), __uint_as_float(pk[e] & 0xffff0000u));
+                            sum[e % 2] = add2(sum[e % 2], x);
                         }
                         tmem_st16(s_addr + (q + w) * 16, pk);
                     }
@@ -725,7 +726,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             ok = __all_sync(0xffffffffu, mbar_wait(o_done(slot), (uint32_t)units & 1u, &s_abort));
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (sink != nullptr) l += ex2(floor_m - m);
+            if (sink != nullptr) l += ex2((floor_m - m) * to_log2);
             const float inv = 1.0f / l;
             __nv_bfloat16* dst = out + ((size_t)(u.t0[slot] + r) * S.nh + h) * DV;
 #pragma unroll 1
@@ -800,10 +801,10 @@ struct Args {
     int* status;
 };
 
-template <int DK, int DV, bool SHAPED>
+template <int DK, int DV, bool ROWS>
 int launch(const Maps& m, const Shape& S, const Args& a, cudaStream_t stream) {
     using C = Cfg<DK, DV>;
-    auto kern = attention_prefill_kernel<DK, DV, SHAPED>;
+    auto kern = attention_prefill_kernel<DK, DV, ROWS>;
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
@@ -862,7 +863,7 @@ TQ_EXPORT int tq_attention_prefill(const void* q, const void* cache, int planes,
     if (rc) return rc;
     m.r = m.v = m.k;
     const Args a{cu_seqlens, seq_start, page_table, nullptr, bias_t, sink, out, status};
-    const bool shaped = softcap > 0.f || bias_t != nullptr || !(scale > 0.f);     // the other form compares unscaled scores
+    const bool shaped = planes == 1 || softcap > 0.f || bias_t != nullptr || !(scale > 0.f);     // (the other form compares unscaled scores)
 #define AP_CASE(DK_, DV_) if (dk == DK_ && dv == DV_) return shaped ? launch<DK_, DV_, true>(m, S, a, stream) : launch<DK_, DV_, false>(m, S, a, stream);
     AP_CASE(64, 64) AP_CASE(64, 128) AP_CASE(128, 64) AP_CASE(128, 128)
 #undef AP_CASE
