@@ -149,3 +149,37 @@ def test_the_lowest_finite_bias_leaves_a_row_its_weights():
     n = torch.arange(1, T + 1, device=DEV, dtype=torch.float64)[:, None, None]
     want, mag = v.double().cumsum(0) / n, v.double().abs().cumsum(0) / n
     assert bool(((got - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -20 * mag).all())
+
+
+def test_the_cap_beyond_a_quarter_has_the_precision_of_tanhf():
+    """Cells of two positions: an odd row's first weight is the logistic of the difference of two capped scores, and a cap of 1e6
+    shows their relative errors.  tanhf was measured to be off by 7.8e-8 (root mean square) where |x| > 1/4, fast intrinsics by
+    1.2e-7 and by more near the quarter."""
+    T, d, cap = 8192, 64, 1e6
+    g = torch.Generator().manual_seed(6)
+    q, k, v = torch.zeros(T, 1, d), torch.zeros(T, 1, d), torch.zeros(T, 1, d)
+    # scores 64 a + b / 64 of bfloat16 factors are exact in float32; a cell's two share a, its b give a difference of up to three
+    q[:, 0, 0], q[:, 0, 1] = 64.0, 1.0 / 64
+    k[:, 0, 0] = torch.round(512.0 * (0.26 + 0.1 * torch.rand(T // 2, generator=g))).repeat_interleave(2)
+    k[:, 0, 1] = torch.randint(-3, 4, (T,), generator=g).float()
+    v[0::2] = 1.0
+    scale = cap / 32768
+    got = one_sequence(q.to(DEV), k.to(DEV), v.to(DEV), scale=scale, softcap=cap, cell=2)[1::2, 0, 0].double().cpu()
+    s = cap * torch.tanh((q.double() * k.double()).sum(-1)[:, 0] * float(np.float32(scale)) / cap)
+    a, b = s[0::2], s[1::2]
+    live = (a - b).abs() < 3                                       # weights that bfloat16 holds to 2^-9 of their logit's unit
+    off = (torch.logit(got) - (a - b))[live] / (0.5 * (a + b))[live]
+    assert int(live.sum()) > 1000 and float(off.square().mean().sqrt()) < 2 ** 0.5 * 1e-7, float(off.square().mean().sqrt())
+
+
+def test_a_cap_too_small_for_the_series():
+    """Scores of zero and scores far beyond a cap of 1e-7: all weights equal."""
+    T, d = 100, 64
+    g = torch.Generator(device=DEV).manual_seed(7)
+    q, k = torch.ones((T, 1, d), device=DEV), torch.randint(0, 2, (T, 1, d), generator=g, device=DEV).float()
+    k[::2] = 0
+    v = torch.randn((T, 1, d), generator=g, device=DEV).to(torch.bfloat16)
+    got = one_sequence(q, k, v, softcap=1e-7).double()
+    n = torch.arange(1, T + 1, device=DEV, dtype=torch.float64)[:, None, None]
+    want, mag = v.double().cumsum(0) / n, v.double().abs().cumsum(0) / n
+    assert bool(((got - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -18 * mag).all())
