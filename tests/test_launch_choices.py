@@ -89,3 +89,24 @@ def test_when_the_shared_expert_rides_in_the_routed_launches():
     from turboquant_cpp_b200.parts.moe_ffn import shared_rides_with_routed
     assert [shared_rides_with_routed(T, 5632, 148) for T in (768, 1024, 1536, 2048, 8192)] == [True, True, True, False, False]
     assert not shared_rides_with_routed(512, 20480, 148)            # the larger model's shared expert fills the GPU sooner
+
+
+def test_when_a_matrix_memory_goes_in_chunks(monkeypatch):
+    """Steps that were timed in both forms: a prompt beside many sequences of one token is walked, long runs among few are not."""
+    from types import SimpleNamespace
+
+    from turboquant_cpp_b200.parts import chunks, make_mixer
+    monkeypatch.setitem(chunks._sm_counts, "cuda:0", 148)
+
+    def in_chunks(lens, heads=16, d=128):
+        m = make_mixer("matrix_memory", prefix="", hidden=64, heads=heads, dim=d, vdim=d, gate_cap=20.0, eps=1e-5)
+        ctx = SimpleNamespace(max_q_len=max(lens), n_seqs=len(lens), n_tokens=sum(lens), host_q_lens=lens, device="cuda:0")
+        return m._in_chunks(ctx, chunks.cut_size(ctx, heads, d + 1) is not None)
+    ones = lambda n: [1] * n
+    for lens in ([130], [300], [2048], [8192], [682, 1366], [1024] * 2, [2048] * 2, [2048] + ones(15), [2048] + ones(31), [4096] + ones(63)):
+        assert in_chunks(lens), lens
+    for lens in ([64], [300] * 2, [300] * 8, [256] * 64, [300] + ones(31), [512] + ones(31), [512] + ones(63), [2048] + ones(127),
+                 [300, 400, 500, 600] + ones(32), [130] + ones(15), [2048] * 2 + ones(126)):
+        assert not in_chunks(lens), lens
+    assert in_chunks([2048], heads=32) and not in_chunks([1024] + ones(31), heads=32) and not in_chunks([2048] + ones(63), heads=32)
+    assert in_chunks([2048] + ones(127), heads=4) and in_chunks([1024] * 8, heads=8, d=64) and not in_chunks([512] + ones(63), heads=8, d=64)

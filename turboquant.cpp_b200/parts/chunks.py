@@ -9,8 +9,9 @@ from ..kernels import ssm as KS
 from .base import StepContext
 
 MIN_CHUNK = 64           # the shortest chunk worth cutting a run into
-# measured on B200, 2,048 tokens, 16 heads of 128 x 129, microseconds of both walks: one run 313, 4 chunks 251, 8 chunks 225,
-# 16 chunks 212, 32 chunks 220
+# measured on B200, 2,048 tokens, 16 heads of 128 x 129, microseconds of both walks of a matrix memory (whose keys of 64 or 128 have a
+# form of their own by now, `kernels.recurrence`; retention and other sizes are walked): one run 313, 4 chunks 251, 8 chunks 225, 16
+# chunks 212, 32 chunks 220
 ROUNDS = 4
 _sm_counts = {}
 
@@ -34,13 +35,15 @@ def cut_size(ctx: StepContext, heads: int, columns: int) -> Optional[int]:
     return size
 
 
-def cut_runs(ctx: StepContext, heads: int, columns: int) -> Optional[Tuple[torch.Tensor, torch.Tensor, torch.Tensor]]:
+def cut_runs(ctx: StepContext, heads: int, columns: int,
+             size: Optional[int] = None) -> Optional[Tuple[torch.Tensor, torch.Tensor, torch.Tensor]]:
     """None, or how this step's runs are cut: (token offsets of the chunks [chunks + 1], chunk numbers [chunks], each
     sequence's chunks [sequences + 1]) on the device.  The recurrence kernel walks a run token by token with a warp per
     four of a head's `columns` columns of state; where those warps fill at most half of the GPU and a run is long,
     cutting the runs fills it (ROUNDS times over, so that the last round of blocks costs little), at the price of walking
-    them once more for the states alone (half the work of a walk with outputs).  The plan depends on the step's runs and on heads and columns only, and is kept for the step's other layers."""
-    size = cut_size(ctx, heads, columns)
+    them once more for the states alone (half the work of a walk with outputs).  The plan depends on the step's runs and on heads and columns only, and is kept for the step's other layers.  size: `cut_size`, where it is known already."""
+    if size is None:
+        size = cut_size(ctx, heads, columns)
     if size is None:
         return None
     lens = list(ctx.host_q_lens)

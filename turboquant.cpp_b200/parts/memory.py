@@ -33,10 +33,8 @@ DENOMINATOR_FLOOR = 1e-6
 
 
 class MatrixMemoryMixer(Mixer):
-    # steps whose longest run of new tokens is at least this, or whose runs a walk would have to cut, take the matrix form; below, the
-    # walk's one launch is cheaper than three (layer on B200, walk / matrix form, us: runs of 60 to 240 tokens of four sequences
-    # 105 / 120, one run of 130: 189 / 119, of 2,048: 395 / 221)
-    CHUNKS_MIN = 256
+    # uncut runs take the matrix form from this length of the longest on (see `_in_chunks`)
+    CHUNKS_MIN = 640
 
     def __init__(self, prefix: str, hidden: int, heads: int, dim: int, vdim: int, gate_cap: float, eps: float):
         if heads < 1 or vdim < 1 or not 1 <= dim <= KS.MAX_STATE:
@@ -84,6 +82,17 @@ class MatrixMemoryMixer(Mixer):
         """The fused input projection as part of a wider one."""
         self.w_in = w
 
+    def _in_chunks(self, ctx: StepContext, cuts: bool) -> bool:
+        """Whether a step's runs go in chunks of 64 tokens as matrix products, or token by token.  A chunk costs the same however
+        few tokens it holds (some 5 us a chunk of 16 heads of 128 x 129 on B200) and a walk as long as its longest run (0.3 us a
+        token of 128-element keys), so a step of one prompt and many sequences of one token is a walk.  Layer of 16 such heads, walk / chunks,
+        us: one run of 512 beside 31 of one token 175 / 259, beside 63 192 / 487; 2,048 beside 31 594 / 389, beside 63 615 / 622,
+        beside 127 651 / 1,071; 4,096 beside 63 1,174 / 776; 1,024 twice 320 / 182; 300 twice 103 / 113, four times 120 / 137
+        (there the launches count); 2,048 four times 675 / 687.  Where a walk would be cut (cuts), chunks were the faster form in every
+        step measured: one run of 130 183 / 115, of 2,048 287 / 185, of 8,192 1,022 / 718."""
+        return cuts or (ctx.max_q_len >= self.CHUNKS_MIN and 88 * ctx.max_q_len >=
+                        KR.chunks_of(ctx.host_q_lens, ctx.n_tokens, ctx.n_seqs) * self.heads * self.vdim)
+
     def forward(self, xn: torch.Tensor, ctx: StepContext, cache: LayerCache, projected: Optional[torch.Tensor] = None,
                 offset: int = 0) -> torch.Tensor:
         """projected: float32 rows of a wider product that hold this mixer's projection from column `offset`."""
@@ -102,12 +111,12 @@ class MatrixMemoryMixer(Mixer):
             f32 = lambda *shape: torch.empty(shape, dtype=torch.float32, device=dev)
             gates, m, y, dots = f32(T, H, 2), f32(T, H), f32(T, self.inner), f32(T, H)
             KS.memory_gates(proj, i, f, self.i_bias, self.f_bias, self.cap, tops, gates, m, H, ctx.cu_seqlens, ctx.slots)
-            cuts = ctx.max_q_len >= 2 * MIN_CHUNK and cut_size(ctx, H, dv + 1) is not None
-            in_chunks = (cuts or ctx.max_q_len >= self.CHUNKS_MIN) and KR.usable(dk, dv, proj, q, k, v)
+            size = cut_size(ctx, H, dv + 1) if ctx.max_q_len >= 2 * MIN_CHUNK else None
+            in_chunks = self._in_chunks(ctx, size is not None) and KR.usable(dk, dv, proj, q, k, v)
             if in_chunks:
                 KR.memory_chunks(proj, q, k, v, gates, S, y, dots, KR.chunks_of(ctx.host_q_lens, T, ctx.n_seqs), H, dk, dv, ctx.cu_seqlens, ctx.slots)
             scan = lambda st, out, nq, cu, slots: KS.memory_scan(proj, q, k, v, gates, st, out, nq, H, dk, dv, cu, slots)
-            plan = cut_runs(ctx, H, dv + 1) if cuts and not in_chunks else None
+            plan = cut_runs(ctx, H, dv + 1, size) if size is not None and not in_chunks else None
             if in_chunks:
                 pass
             elif plan is None:
