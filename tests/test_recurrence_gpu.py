@@ -75,3 +75,36 @@ def test_an_infinite_value_reaches_no_earlier_token():
         KR.memory_chunks(rows, 0, d, 2 * d, gates, state, y, dots, 2, H, d, d, i32([0, T]), i32([0]))
         res.append(y)
     assert torch.equal(res[0][:70], res[1][:70]) and not bool(torch.isfinite(res[1][70:]).any())
+
+
+def memory_step(lens, H=2, dk=64, dv=64, scratch=None, monkeypatch=None):
+    """(y, dots, state) of runs in chunks, and the bytes a step's scratch may take."""
+    from turboquant_cpp_b200.kernels import recurrence as KR
+    if scratch is not None:
+        monkeypatch.setattr(KR, "SCRATCH_BYTES", scratch)
+    T, g = sum(lens), torch.Generator(device=DEV).manual_seed(11)
+    rows = torch.randn((T, H * (2 * dk + dv)), generator=g, device=DEV)
+    gates = torch.stack([-0.2 * torch.rand((T, H), generator=g, device=DEV), -torch.rand((T, H), generator=g, device=DEV)], -1).contiguous()
+    state = torch.randn((len(lens), H, dv + 1, dk), generator=g, device=DEV)
+    y, dots = torch.empty((T, H * dv), device=DEV), torch.empty((T, H), device=DEV)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    KR.memory_chunks(rows, 0, H * dk, 2 * H * dk, gates, state, y, dots, KR.chunks_of(lens, T, len(lens)), H, dk, dv,
+                     i32(np.concatenate([[0], np.cumsum(lens)])), i32(range(len(lens))))
+    return (y, dots, state), torch.cuda.max_memory_allocated() - before
+
+
+@pytest.mark.parametrize("lens", [[700], [64, 130, 1, 300, 63], [1] * 40 + [200]])
+@pytest.mark.parametrize("at_once", [1, 2, 3, 7])
+def test_groups_of_chunks(lens, at_once, monkeypatch):
+    """The states of a few chunks at a time: the same bits, in as little scratch."""
+    whole, _ = memory_step(lens)
+    parts, _ = memory_step(lens, scratch=at_once * 4 * 2 * (65 * 64 + 1), monkeypatch=monkeypatch)
+    assert all(torch.equal(a, b) for a, b in zip(whole, parts))
+
+
+def test_the_scratch_of_a_long_run_is_bounded():
+    from turboquant_cpp_b200.kernels import recurrence as KR
+    _, used = memory_step([20000], H=8, dk=128, dv=128)           # 313 chunks of 0.5 MB
+    assert used <= KR.SCRATCH_BYTES + (1 << 20), used

@@ -6,7 +6,8 @@
 //   y_t = A_t S_0^T q_t + sum over s <= t of (q_t . k_s) D[t][s] b_s v_s
 //   S_last = A_last S_0 + sum over s of D[last][s] b_s k_s v_s^T.
 // Three launches: every chunk's own sum (the second formula from zero) side by side; the states the chunks start from, one chunk
-// after the other but every element by itself; every chunk's outputs side by side.  Token by token (csrc/ssm.cu) a walk does 2
+// after the other but every element by itself; every chunk's outputs side by side.  A long step does this for a group of chunks after
+// the other, the kept state going from group to group, so that the chunks' states take a bounded buffer.  Token by token (csrc/ssm.cu) a walk does 2
 // multiply-adds an element of the state and token, a chain of its tokens with a shuffle tree each, and long runs are walked twice to
 // fill the GPU; in chunks it is 2 + 64 (1 / dk + 1 / dv) of them, all in register-tiled products.  Everything is fp32 and
 // stays on the CUDA cores: tensor cores would round operands (three products of split tf32 parts cost what the fp32
@@ -145,10 +146,10 @@ __device__ __forceinline__ float4 four(tq_f32x2 a, tq_f32x2 b) {
     return make_float4(x.x, x.y, y.x, y.y);
 }
 
-// ---- a chunk's own sum: ends [chunk][head][dv + 1][dk] (the last row n), decays [chunk][head] -------------------------------
+// ---- a chunk's own sum, of the group from chunk0 on: ends [chunk - chunk0][head][dv + 1][dk] (the last row n), decays [..][head] ----
 template <int DK, int DV>
 __global__ void __launch_bounds__(THREADS, 2)
-memory_ends_kernel(const float* __restrict__ rows, int C, int k_off, int v_off, const float2* __restrict__ gates, int heads,
+memory_ends_kernel(const float* __restrict__ rows, int C, int k_off, int v_off, const float2* __restrict__ gates, int heads, int chunk0,
                    const int* __restrict__ cu_seqlens, int n_seqs, float* __restrict__ ends, float* __restrict__ decays) {
     tq_grid_wait();                    // everything below may read what the previous kernel wrote
     tq_grid_launch_dependents();       // the next kernel's CTAs may move in as SMs free up
@@ -158,7 +159,7 @@ memory_ends_kernel(const float* __restrict__ rows, int C, int k_off, int v_off, 
     __shared__ Chunk s_chunk;
     __shared__ float s_w[L], s_half;
     const int h = blockIdx.y;
-    const Chunk c = find_chunk(blockIdx.x, cu_seqlens, n_seqs, &s_chunk);
+    const Chunk c = find_chunk(chunk0 + blockIdx.x, cu_seqlens, n_seqs, &s_chunk);
     if (c.n == 0) return;
     const int tid = threadIdx.x, lane = tid & 31;
     load_rows<DV>(Vs, rows + (size_t)c.t0 * C + v_off + h * DV, C, c.n);
@@ -209,10 +210,10 @@ memory_ends_kernel(const float* __restrict__ rows, int C, int k_off, int v_off, 
     }
 }
 
-// ---- the states the chunks start from, in the place of their own sums; the kept state moves to the run's end ----------------
+// ---- the states the group's chunks start from, in the place of their own sums; the kept state moves to the end of the last -----
 __global__ void __launch_bounds__(256)
 chunk_starts_kernel(float* __restrict__ state, long long slot_stride, const int* __restrict__ slots, float* __restrict__ ends,
-                    const float* __restrict__ decays, int heads, int per_head, const int* __restrict__ cu_seqlens) {
+                    const float* __restrict__ decays, int heads, int per_head, int chunk0, int group, const int* __restrict__ cu_seqlens) {
     tq_grid_wait();                    // everything below may read what the previous kernel wrote
     tq_grid_launch_dependents();       // the next kernel's CTAs may move in as SMs free up
     __shared__ int s_first;
@@ -225,11 +226,12 @@ chunk_starts_kernel(float* __restrict__ state, long long slot_stride, const int*
         if (threadIdx.x == 0) s_first = before;
     }
     __syncthreads();
-    const int n = (cu_seqlens[s + 1] - cu_seqlens[s] + L - 1) / L;
-    if (e >= per_head || n == 0) return;
+    // the sequence's chunks that are in the group, counted from chunk0
+    const int from = max(s_first - chunk0, 0), to = min(s_first + (cu_seqlens[s + 1] - cu_seqlens[s] + L - 1) / L - chunk0, group), n = to - from;
+    if (e >= per_head || n <= 0) return;
     float* cell = state + (size_t)slots[s] * slot_stride + (size_t)h * per_head + e;
-    float* at = ends + ((size_t)s_first * heads + h) * per_head + e;
-    const float* d = decays + (size_t)s_first * heads + h;
+    float* at = ends + ((size_t)from * heads + h) * per_head + e;
+    const float* d = decays + (size_t)from * heads + h;
     const size_t step = (size_t)heads * per_head;
     float S = *cell;
     constexpr int AHEAD = 8;           // the sums do not depend on the chain: eight of them on their way together
@@ -254,7 +256,7 @@ chunk_starts_kernel(float* __restrict__ state, long long slot_stride, const int*
 template <int DK, int DV>
 __global__ void __launch_bounds__(THREADS, 2)
 memory_outputs_kernel(const float* __restrict__ rows, int C, int q_off, int k_off, int v_off, const float2* __restrict__ gates, int heads,
-                      const int* __restrict__ cu_seqlens, int n_seqs, const float* __restrict__ starts, float* __restrict__ y,
+                      int chunk0, const int* __restrict__ cu_seqlens, int n_seqs, const float* __restrict__ starts, float* __restrict__ y,
                       float* __restrict__ dots) {
     tq_grid_wait();                    // everything below may read what the previous kernel wrote
     tq_grid_launch_dependents();       // the next kernel's CTAs may move in as SMs free up
@@ -267,7 +269,7 @@ memory_outputs_kernel(const float* __restrict__ rows, int C, int q_off, int k_of
     __shared__ Chunk s_chunk;
     __shared__ float s_a[L], s_b[L], s_A[L];
     const int h = blockIdx.y;
-    const Chunk c = find_chunk(blockIdx.x, cu_seqlens, n_seqs, &s_chunk);
+    const Chunk c = find_chunk(chunk0 + blockIdx.x, cu_seqlens, n_seqs, &s_chunk);
     if (c.n == 0) return;
     const int tid = threadIdx.x, ty = tid / 16, tx = tid % 16;
     const float* tok = rows + (size_t)c.t0 * C;
@@ -350,7 +352,7 @@ memory_outputs_kernel(const float* __restrict__ rows, int C, int q_off, int k_of
 
 template <int DK, int DV>
 int launch_memory(const float* rows, int C, int q_off, int k_off, int v_off, const float2* gates, float* state, long long slot_stride,
-                  float* y, float* dots, float* ends, float* decays, int chunks, int n_seqs, int heads, const int* cu, const int* slots,
+                  float* y, float* dots, float* ends, float* decays, int chunks, int group, int n_seqs, int heads, const int* cu, const int* slots,
                   cudaStream_t stream) {
     constexpr int A_BYTES = L * (DK + DV) * 4, C_BYTES = (DK * L + 64 * (DK > DV ? DK : DV) + 64 * DV + L * L) * 4;
     auto ka = memory_ends_kernel<DK, DV>;
@@ -362,11 +364,14 @@ int launch_memory(const float* rows, int C, int q_off, int k_off, int v_off, con
         if (e != cudaSuccess) TQ_FAIL(-1, "memory_chunks: %d bytes of shared memory refused: %s", C_BYTES, cudaGetErrorString(e));
         configured = true;
     }
-    tq_launch(dim3(chunks, heads), THREADS, A_BYTES, stream)(ka, rows, C, k_off, v_off, gates, heads, cu, n_seqs, ends, decays);
     const int per_head = (DV + 1) * DK;
-    tq_launch(dim3((per_head + 255) / 256, n_seqs, heads), 256, 0, stream)(chunk_starts_kernel, state, slot_stride, slots, ends,
-        (const float*)decays, heads, per_head, cu);
-    tq_launch(dim3(chunks, heads), THREADS, C_BYTES, stream)(kc, rows, C, q_off, k_off, v_off, gates, heads, cu, n_seqs, (const float*)ends, y, dots);
+    for (int chunk0 = 0; chunk0 < chunks; chunk0 += group) {
+        const int n = chunks - chunk0 < group ? chunks - chunk0 : group;
+        tq_launch(dim3(n, heads), THREADS, A_BYTES, stream)(ka, rows, C, k_off, v_off, gates, heads, chunk0, cu, n_seqs, ends, decays);
+        tq_launch(dim3((per_head + 255) / 256, n_seqs, heads), 256, 0, stream)(chunk_starts_kernel, state, slot_stride, slots, ends,
+            (const float*)decays, heads, per_head, chunk0, n, cu);
+        tq_launch(dim3(n, heads), THREADS, C_BYTES, stream)(kc, rows, C, q_off, k_off, v_off, gates, heads, chunk0, cu, n_seqs, (const float*)ends, y, dots);
+    }
     TQ_CHECK_LAUNCH("memory_chunks");
     return 0;
 }
@@ -376,16 +381,16 @@ int launch_memory(const float* rows, int C, int q_off, int k_off, int v_off, con
 
 // rows fp32 [T, C] with q, k (heads x dk) and v (heads x dv) from columns that are multiples of four, gates [T, heads] pairs of
 // logarithms; state: the sequences' [heads][dv + 1][dk] at slots[s] * slot_stride, renewed; y [T, heads * dv], dots [T, heads] =
-// n . q.  ends [chunks, heads, dv + 1, dk] and decays [chunks, heads]: scratch for at least the sum of ceil(run / 64) chunks.
+// n . q.  chunks: at least the sum of ceil(run / 64); ends [group, heads, dv + 1, dk] and decays [group, heads]: scratch of a group.
 TQ_EXPORT int tq_memory_chunks(const float* rows, int C, int q_off, int k_off, int v_off, const void* gates, float* state,
-                               long long slot_stride, float* y, float* dots, float* ends, float* decays, int chunks, int n_seqs,
+                               long long slot_stride, float* y, float* dots, float* ends, float* decays, int chunks, int group, int n_seqs,
                                int heads, int dk, int dv, const int* cu_seqlens, const int* slots, cudaStream_t stream) {
     if (n_seqs == 0 || chunks == 0) return 0;
-    TQ_REQUIRE(heads >= 1 && heads <= 65535 && n_seqs <= 65535, "memory_chunks: %d heads, %d sequences", heads, n_seqs);
+    TQ_REQUIRE(heads >= 1 && heads <= 65535 && n_seqs <= 65535 && group >= 1, "memory_chunks: %d heads, %d sequences, groups of %d chunks", heads, n_seqs, group);
     TQ_REQUIRE(C % 4 == 0 && q_off % 4 == 0 && k_off % 4 == 0 && v_off % 4 == 0 && ((uintptr_t)rows & 15) == 0 && ((uintptr_t)y & 15) == 0
                && ((uintptr_t)ends & 15) == 0, "memory_chunks: rows of %d floats are not aligned to 16 bytes", C);
 #define MEM_CASE(DK_, DV_) if (dk == DK_ && dv == DV_) return tq_recurrence::launch_memory<DK_, DV_>(rows, C, q_off, k_off, v_off, (const float2*)gates, \
-        state, slot_stride, y, dots, ends, decays, chunks, n_seqs, heads, cu_seqlens, slots, stream);
+        state, slot_stride, y, dots, ends, decays, chunks, group, n_seqs, heads, cu_seqlens, slots, stream);
     MEM_CASE(64, 64) MEM_CASE(64, 128) MEM_CASE(128, 64) MEM_CASE(128, 128)
 #undef MEM_CASE
     TQ_FAIL(-2, "memory_chunks: keys of %d and values of %d elements", dk, dv);

@@ -13,6 +13,9 @@ from .ssm import ctypes_ptr
 _LIB = "ssm"
 CHUNK = 64               # csrc/recurrence.cuh L
 SIZES = (64, 128)        # key and value sizes the kernels are built for
+# the most bytes of chunks' states a step holds at a time, 126 chunks of 16 heads of 128 x 129; longer steps go in groups of equal size
+# (8,192 tokens of that layer: 718 us in one piece of 135 MB, 746 in groups of 63, 63 and 2)
+SCRATCH_BYTES = 128 << 20
 
 
 def chunks_of(q_lens: Sequence[int], n_tokens: int, n_seqs: int) -> int:
@@ -20,6 +23,12 @@ def chunks_of(q_lens: Sequence[int], n_tokens: int, n_seqs: int) -> int:
     if len(q_lens) == n_seqs:
         return sum(-(-n // CHUNK) for n in q_lens)
     return n_tokens // CHUNK + n_seqs
+
+
+def group_of(chunks: int, heads: int, dk: int, dv: int) -> int:
+    """Chunks whose states a step holds at a time."""
+    most = max(1, SCRATCH_BYTES // (4 * heads * ((dv + 1) * dk + 1)))
+    return -(-chunks // -(-chunks // most)) if chunks else 1
 
 
 def usable(dk: int, dv: int, rows: torch.Tensor, *offsets: int) -> bool:
@@ -31,7 +40,7 @@ def usable(dk: int, dv: int, rows: torch.Tensor, *offsets: int) -> bool:
 def memory_chunks(rows: torch.Tensor, q_off: int, k_off: int, v_off: int, gates: torch.Tensor, state: torch.Tensor, y: torch.Tensor,
                   dots: torch.Tensor, chunks: int, heads: int, dk: int, dv: int, cu_seqlens: torch.Tensor, slots: torch.Tensor) -> None:
     """`kernels.ssm.memory_scan` with outputs, in chunks: state float32 [slots, heads, dv + 1, dk] (rows may be strided) is renewed,
-    y [T, heads * dv], dots [T, heads].  chunks: at least the chunks of the runs (`chunks_of`)."""
+    y [T, heads * dv], dots [T, heads].  chunks: at least the chunks of the runs (`chunks_of`), in groups of `group_of`."""
     for t, what in ((rows, "q, k and v"), (gates, "the gates"), (state, "the state"), (y, "the output"), (dots, "the dot products")):
         want_f32(t, what)
     for t, what in ((cu_seqlens, "cu_seqlens"), (slots, "slots")):
@@ -41,11 +50,11 @@ def memory_chunks(rows: torch.Tensor, q_off: int, k_off: int, v_off: int, gates:
             or y.numel() != T * heads * dv or dots.numel() != T * heads or gates.numel() != 2 * T * heads or slots.numel() < n_seqs \
             or max(q_off + heads * dk, k_off + heads * dk, v_off + heads * dv) > rows.shape[1]:
         raise KernelError("memory_chunks: sizes of 64 or 128, aligned rows that hold the heads, a state row of [heads, dv + 1, dk]")
-    per_chunk = heads * (dv + 1) * dk
-    scratch = torch.empty(chunks * (per_chunk + heads), dtype=torch.float32, device=rows.device)      # the chunks' states, then their decays
+    per_chunk, group = heads * (dv + 1) * dk, group_of(chunks, heads, dk, dv)
+    scratch = torch.empty(group * (per_chunk + heads), dtype=torch.float32, device=rows.device)      # the chunks' states, then their decays
     at = scratch.data_ptr()
     lib = load_kernel(_LIB)
     # (plain ints are C ints to ctypes)
     check(_LIB, lib.tq_memory_chunks(
         ptr(rows), rows.shape[1], q_off, k_off, v_off, ptr(gates), ctypes_ptr(state), c_longlong(state.stride(0)), ptr(y), ptr(dots),
-        c_void_p(at), c_void_p(at + 4 * chunks * per_chunk), chunks, n_seqs, heads, dk, dv, ptr(cu_seqlens), ptr(slots), stream()), kernels=3)
+        c_void_p(at), c_void_p(at + 4 * group * per_chunk), chunks, group, n_seqs, heads, dk, dv, ptr(cu_seqlens), ptr(slots), stream()), kernels=3 * -(-chunks // group))
