@@ -72,3 +72,43 @@ def test_the_helper_that_waits_renews_its_pointer():
     i = text.index("void gemv_stage_x(")
     body = text[i:text.index("}", text.index("__syncthreads();", i))]
     assert body.index("tq_grid_wait()") < body.index("tq_fresh(x)") < body.index("xs + i")
+
+
+def test_shared_memory_is_asked_for_on_every_device(tmp_path):
+    """Prompts of latent attention and of matrix memories ran on any device of a process before they took kernels that need more than
+    48 KB of shared memory.  The helper they ask with, run against a CUDA runtime of the test's own: once per device and kernel,
+    again after a refusal; and those two files use nothing else."""
+    import shutil
+    import subprocess
+    for name in ("attention_prefill.cu", "recurrence.cuh"):
+        text = open(os.path.join(CSRC, name)).read()
+        assert "tq_reserve_smem(" in text and "cudaFuncSetAttribute" not in text, name
+    text = open(os.path.join(CSRC, "common.cuh")).read()
+    i = text.index("template <typename K>\ninline cudaError_t tq_reserve_smem")
+    helper = text[i:text.index("\n}\n", i) + 3]
+    program = """
+#include <atomic>
+#include <cassert>
+#include <initializer_list>
+typedef int cudaError_t;
+enum { cudaSuccess = 0, cudaFuncAttributeMaxDynamicSharedMemorySize = 8 };
+static int device = 0, calls[70], answer = 0;
+cudaError_t cudaGetDevice(int* d) { *d = device; return 0; }
+template <typename K> cudaError_t cudaFuncSetAttribute(K, int, int) { ++calls[device]; return answer; }
+""" + helper + """
+void kernel() {}
+int main() {
+    std::atomic<unsigned long long> asked{0};
+    answer = 1;
+    assert(tq_reserve_smem(kernel, 1, asked) == 1);
+    answer = 0;
+    for (int round = 0; round < 3; ++round)
+        for (int d : {0, 1, 7, 63, 64, 69}) { device = d; assert(tq_reserve_smem(kernel, 1, asked) == 0); }
+    assert(calls[0] == 2 && calls[1] == 1 && calls[7] == 1 && calls[63] == 1 && calls[64] == 3 && calls[69] == 3);
+    return 0;
+}
+"""
+    src, exe = tmp_path / "ask.cpp", tmp_path / "ask"
+    src.write_text(program)
+    subprocess.run([shutil.which("g++") or "c++", "-std=c++17", "-o", str(exe), str(src)], check=True)
+    subprocess.run([str(exe)], check=True)

@@ -807,12 +807,9 @@ template <int DK, int DV, bool ROWS>
 int launch(const Maps& m, const Shape& S, const Args& a, cudaStream_t stream) {
     using C = Cfg<DK, DV>;
     auto kern = attention_prefill_kernel<DK, DV, ROWS>;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
-        if (e != cudaSuccess) TQ_FAIL(-1, "attention_prefill: cannot reserve %d bytes of shared memory: %s", C::SMEM_BYTES, cudaGetErrorString(e));
-        configured = true;
-    }
+    static std::atomic<unsigned long long> asked{0};
+    const cudaError_t e = tq_reserve_smem(kern, C::SMEM_BYTES, asked);
+    if (e != cudaSuccess) TQ_FAIL(-1, "attention_prefill: cannot reserve %d bytes of shared memory: %s", C::SMEM_BYTES, cudaGetErrorString(e));
     // a block per unit; those that run take over the ones that have not started
     const int hs = S.pairing == PAIR_HEADS ? S.nh / 2 : S.nh, qs = S.pairing == PAIR_HEADS ? S.n_qt : (S.n_qt + 1) / 2;
     const int grid = qs * S.n_seqs * hs;

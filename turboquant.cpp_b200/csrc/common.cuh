@@ -11,6 +11,7 @@
 #include <stdio.h>
 #include <stdlib.h>
 #include <math.h>
+#include <atomic>
 
 #define TQ_EXPORT extern "C" __attribute__((visibility("default")))
 
@@ -30,6 +31,20 @@ static thread_local char tq_error_message[512] = "";
     do {                                                                     \
         if (!(cond)) TQ_FAIL(-2, __VA_ARGS__);                               \
     } while (0)
+
+// Asks for `bytes` of dynamic shared memory for a kernel on the current device: once per device, so a static `asked` per kernel
+// holds a bit for each (devices from 64 on are asked every time).
+template <typename K>
+inline cudaError_t tq_reserve_smem(K kernel, int bytes, std::atomic<unsigned long long>& asked) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const unsigned long long bit = dev < 64 ? 1ull << dev : 0;
+    if (asked.load(std::memory_order_relaxed) & bit) return cudaSuccess;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) asked.fetch_or(bit, std::memory_order_relaxed);
+    return e;
+}
 
 #define TQ_CHECK_LAUNCH(name)                                                \
     do {                                                                     \

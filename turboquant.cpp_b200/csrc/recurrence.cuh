@@ -357,13 +357,10 @@ int launch_memory(const float* rows, int C, int q_off, int k_off, int v_off, con
     constexpr int A_BYTES = L * (DK + DV) * 4, C_BYTES = (DK * L + 64 * (DK > DV ? DK : DV) + 64 * DV + L * L) * 4;
     auto ka = memory_ends_kernel<DK, DV>;
     auto kc = memory_outputs_kernel<DK, DV>;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(ka, cudaFuncAttributeMaxDynamicSharedMemorySize, A_BYTES);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(kc, cudaFuncAttributeMaxDynamicSharedMemorySize, C_BYTES);
-        if (e != cudaSuccess) TQ_FAIL(-1, "memory_chunks: %d bytes of shared memory refused: %s", C_BYTES, cudaGetErrorString(e));
-        configured = true;
-    }
+    static std::atomic<unsigned long long> asked_a{0}, asked_c{0};
+    cudaError_t e = tq_reserve_smem(ka, A_BYTES, asked_a);
+    if (e == cudaSuccess) e = tq_reserve_smem(kc, C_BYTES, asked_c);
+    if (e != cudaSuccess) TQ_FAIL(-1, "memory_chunks: %d bytes of shared memory refused: %s", C_BYTES, cudaGetErrorString(e));
     const int per_head = (DV + 1) * DK;
     for (int chunk0 = 0; chunk0 < chunks; chunk0 += group) {
         const int n = chunks - chunk0 < group ? chunks - chunk0 : group;
