@@ -183,3 +183,20 @@ def test_a_cap_too_small_for_the_series():
     n = torch.arange(1, T + 1, device=DEV, dtype=torch.float64)[:, None, None]
     want, mag = v.double().cumsum(0) / n, v.double().abs().cumsum(0) / n
     assert bool(((got - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -18 * mag).all())
+
+
+def test_queries_and_results_at_any_element():
+    """Contiguous views that begin off a 16-byte boundary, and a step without runs."""
+    from turboquant_cpp_b200.kernels import bias_attention as KB
+    T, H, d = 100, 2, 64
+    g = torch.Generator(device=DEV).manual_seed(8)
+    rand = lambda n: torch.randn(n, generator=g, device=DEV).to(torch.bfloat16)
+    cache, q0, room = rand(2 * 64 * 2 * d).view(2, 1, 1, 64, 2 * d), rand(T * H * d + 2), torch.zeros(T * H * d + 2, dtype=torch.bfloat16, device=DEV)
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device=DEV)
+    call = lambda q, out, run=T: KB.attention_runs(q, cache, None, None, i32([0, T]), i32([0]), i32([[0, 1]]), 64, 0, 0, 0.125, out, 1, run, H, 1, d, d)
+    q = q0[2:].view(T, H, d)
+    want = call(q.clone(), torch.empty((T, H * d), dtype=torch.bfloat16, device=DEV))
+    out = room[2:].view(T, H * d)
+    assert q.data_ptr() % 16 == 4 and out.data_ptr() % 16 == 4
+    assert call(q, out) is out and torch.equal(out, want) and not bool(room[:2].any())
+    assert call(q, out, run=0) is out and torch.equal(out, want)

@@ -174,9 +174,16 @@ def attention_runs(q: torch.Tensor, cache: torch.Tensor, bias_t: Optional[torch.
         far = bias_t.shape[1] - 1
     if sink is not None:
         want_f32(sink, "the sink")
+    if max_run == 0:
+        return out
     if dk in (64, 128) and dv in (64, 128) and q.dtype == torch.bfloat16 and page_size == 64:
-        return prefill_rows(q, cache, 1, cu_seqlens, seq_start, page_table, page_size, window, scale, out, n_seqs, max_run, heads,
-                            kv_heads, dk, dv, keep_first=keep_first, cell=cell, softcap=softcap, bias_t=bias_t, sink=sink, status=status)
+        # bulk copies and 16-byte stores want aligned queries and results: views that begin elsewhere go through a copy
+        if q.data_ptr() % 16:
+            q = q.clone()
+        dst = out if out.data_ptr() % 16 == 0 else torch.empty_like(out)
+        prefill_rows(q, cache, 1, cu_seqlens, seq_start, page_table, page_size, window, scale, dst, n_seqs, max_run, heads,
+                     kv_heads, dk, dv, keep_first=keep_first, cell=cell, softcap=softcap, bias_t=bias_t, sink=sink, status=status)
+        return out if dst is out else out.copy_(dst)
     lib = load_kernel(_LIB)
     check(_LIB, lib.tq_bias_attention_runs(
         ptr(q), ptr(cache), c_int(code(q.dtype)), ptr(bias_t), c_int(far), ptr(sink), ptr(cu_seqlens), ptr(seq_start),
