@@ -147,13 +147,17 @@ TQ_EXPORT int tq_bias_kv_write(const float* qkv, void* q_out, void* cache, int a
 // g / v_share of the row (v_share > 1: neighbouring key heads keep the same values; v_from_k: the row holds no values,
 // key head g / v_share as it leaves the projection is the value, dv == dk), turned by position * v_freq[m] over all dv
 // elements in the same pairing (v_freq fp32 [dv / 2]; null: as they are).
-// A block per token: the token's sines and cosines are computed once, a pair's angle by one thread, and read by all its heads
-// from shared memory; then a warp per query, key or value head.  What bounds it is the bytes (fp32 rows in, half of them out)
+// A block per token (grid y 1): the token's sines and cosines are computed once, a pair's angle by one thread, and read by all its
+// heads from shared memory; then a warp per query, key or value head.  Steps of few tokens share a token's heads out over blocks of
+// four warps (grid y), a head a warp, each block with the angles it needs: see the launcher.  What bounds it is the bytes (fp32 rows in, half of them out)
 // once the angles are shared: 4,096 tokens, 16 + 4 + 4 heads of 128, all turned, took 60.6 us with a sincosf per head and
 // pair (two per pair of a value) and takes 39 us (48 with every head passed through shared memory: 360 instructions a warp
 // and head); the bytes alone are 11.5 us.  vec: 16-byte reads and 8-byte writes (bf16), where sizes, strides and pointers allow them.
 // ---------------------------------------------------------------------------------------
 #define BA_ROT_MAX_WARPS 16
+// Steps of up to this many heads (tokens x heads) take a warp a head: 5,120 (64 tokens of 64 + 8 + 8 heads) 4.8 us against 6.7 with a
+// block a token, 6,144 (256 of 16 + 4 + 4) 5.1 against 4.7; one token of 64 + 8 + 8 heads 2.7 against 6.4
+#define BA_SPREAD_HEADS 5632
 // cos and sin of `pos * freq[i]` for i < n
 __device__ __forceinline__ void ba_angles(float2* cs, const float* __restrict__ freq, int n, float pos) {
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
@@ -237,9 +241,10 @@ bias_kv_write_rot_kernel(const float* __restrict__ qkv, int row_stride, TA* __re
         const bool kq = head < nh + nkv;
         return (kq ? k_lanes : v_lanes) && head < last && 4 * lane < (kq ? dk : dv) ? ba_read4(source(head) + 4 * lane, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
     };
-    float4 next = read(warp);          // on its way while the angles are computed; each later head while the one before is worked on
-    ba_angles(cs, freq, rot_dims >> 1, (float)pos);
-    if (v_freq != nullptr && cache != nullptr) ba_angles(v_cs, v_freq, dv >> 1, (float)pos);
+    const int head0 = blockIdx.y * n_warps, stride = gridDim.y * n_warps;
+    float4 next = read(head0 + warp);  // on its way while the angles are computed; each later head while the one before is worked on
+    if (head0 < nh + nkv) ba_angles(cs, freq, rot_dims >> 1, (float)pos);
+    if (v_freq != nullptr && cache != nullptr && (gridDim.y == 1 || head0 + n_warps > nh + nkv)) ba_angles(v_cs, v_freq, dv >> 1, (float)pos);
     int page = 0;                      // without a cache (a layer that only reads another's) no table is looked at
     if (cache != nullptr) {
         const int* table = page_table + (size_t)TQ_CHECKED(seq_of_token[t], n_seqs, TQ_IDX_SEQUENCE) * table_stride;
@@ -314,9 +319,9 @@ bias_kv_write_rot_kernel(const float* __restrict__ qkv, int row_stride, TA* __re
         __syncwarp();                  // the warp's row in shared memory is free for its next head
     };
 #pragma unroll 1
-    for (int head = warp; head < last; head += n_warps) {
+    for (int head = head0 + warp; head < last; head += stride) {
         const float4 x = next;
-        next = read(head + n_warps);
+        next = read(head + stride);
         if (head < nh + nkv ? k_lanes : v_lanes) lane_head(head, x);
         else shared_head(head);
     }
@@ -339,16 +344,19 @@ TQ_EXPORT int tq_bias_kv_write_rot(const float* qkv, int row_stride, void* q_out
                "bias_kv_write_rot: %d rotated elements of a head of %d", rot_dims, dk);
     TQ_REQUIRE(v_freq == nullptr || dv % 2 == 0, "bias_kv_write_rot: values of %d elements cannot be rotated in pairs", dv);
     TQ_REQUIRE(temp_every >= 0, "bias_kv_write_rot: a temperature that grows every %d positions", temp_every);
-    // long steps: blocks of eight warps, several an SM; steps of few tokens: as many warps as there are heads, a head or two each
+    // long steps: a block of eight warps a token, several an SM; shorter ones: sixteen warps, a head or two each; while the GPU holds a
+    // warp for every head of the step: a head a warp, over blocks of four
     const int heads = nh + (cache ? 2 * nkv : 0), most = T_ > 592 ? 8 : BA_ROT_MAX_WARPS;
     const int room = ((dk > dv ? dk : dv) + 3) & ~3;
-    int warps = heads >= most ? most : (heads >= 8 ? 8 : 4);
+    const bool spread = !norm_rows && (long long)T_ * heads <= BA_SPREAD_HEADS;      // (a norm over whole rows is a block's own)
+    int warps = spread ? 4 : (heads >= most ? most : (heads >= 8 ? 8 : 4));
     while (warps > 1 && warps * room > 8192) warps >>= 1;    // wide values: 32 KB of rows
+    const int groups = spread ? (heads + warps - 1) / warps : 1;
     const size_t smem = (size_t)warps * room * sizeof(float) + (size_t)(rot_dims / 2 + 1 + (v_freq ? dv / 2 : 0)) * sizeof(float2);
     const int vec = dk % 4 == 0 && dv % 4 == 0 && row_stride % 4 == 0 && ((uintptr_t)qkv & 15) == 0 && ((uintptr_t)q_out & 15) == 0
                     && ((uintptr_t)cache & 15) == 0;
     TQ_DISPATCH(act_dtype, TA,
-        (tq_launch(T_, 32 * warps, smem, stream)(bias_kv_write_rot_kernel<TA>, qkv, row_stride, (TA*)q_out, (TA*)cache, freq, rot_dims,
+        (tq_launch(dim3(T_, groups), 32 * warps, smem, stream)(bias_kv_write_rot_kernel<TA>, qkv, row_stride, (TA*)q_out, (TA*)cache, freq, rot_dims,
             halves, mag, unit_eps, q_norm_w, k_norm_w, norm_eps, norm_rows, v_freq, v_share, v_from_k, temp_coef, temp_every, positions,
             seq_of_token, page_table, table_stride, page_size, nh, nkv, dk, dv, n_seqs, n_pages, vec)));
     TQ_CHECK_LAUNCH("bias_kv_write_rot");
@@ -387,11 +395,12 @@ heads_unrotate_gate_kernel(const TA* __restrict__ o, const float* __restrict__ g
     __shared__ __align__(16) float2 cs[BA_MAX_DIM / 2];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5, t = blockIdx.x;
     const bool lanes = vec && dv <= 128 && (v_freq == nullptr || dv % (halves ? 8 : 4) == 0);
+    const int head0 = blockIdx.y * 2 * n_warps, stride = gridDim.y * 2 * n_warps;     // two heads a warp at a time
     float4 early[2];
     float z[2];
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-        const int h = warp + i * n_warps;
+        const int h = head0 + warp + i * n_warps;
         early[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         z[i] = 0.f;
         if (lanes && h < nh) {
@@ -411,14 +420,16 @@ heads_unrotate_gate_kernel(const TA* __restrict__ o, const float* __restrict__ g
         };
 #pragma unroll
         for (int i = 0; i < 2; ++i)
-            if (warp + i * n_warps < nh) one_head(warp + i * n_warps, early[i], z[i]);
-        for (int h = warp + 2 * n_warps; h < nh; h += n_warps)
-            one_head(h, 4 * lane < dv ? ba_load4(o + ((size_t)t * nh + h) * dv + 4 * lane) : make_float4(0.f, 0.f, 0.f, 0.f),
+            if (head0 + warp + i * n_warps < nh) one_head(head0 + warp + i * n_warps, early[i], z[i]);
+        for (int h0 = head0 + stride; h0 < nh; h0 += stride)
+            for (int h = h0 + warp; h < min(nh, h0 + 2 * n_warps); h += n_warps)
+                one_head(h, 4 * lane < dv ? ba_load4(o + ((size_t)t * nh + h) * dv + 4 * lane) : make_float4(0.f, 0.f, 0.f, 0.f),
                      gates[(size_t)t * gate_stride + gate_off + h]);
         return;
     }
     float* sh = s_head[warp];
-    for (int h = warp; h < nh; h += n_warps) {
+    for (int h0 = head0; h0 < nh; h0 += stride)
+    for (int h = h0 + warp; h < min(nh, h0 + 2 * n_warps); h += n_warps) {
         const size_t at = ((size_t)t * nh + h) * dv;
         for (int e = lane; e < dv; e += 32) sh[e] = tq_to_float(o[at + e]);
         const float gate = 1.0f / (1.0f + expf(-gates[(size_t)t * gate_stride + gate_off + h]));
@@ -441,8 +452,11 @@ TQ_EXPORT int tq_heads_unrotate_gate(const void* o, int act_dtype, const float* 
     TQ_REQUIRE(v_freq == nullptr || dv % 2 == 0, "heads_unrotate_gate: values of %d elements cannot be rotated in pairs", dv);
     const int most = T_ > 592 ? 8 : BA_ROT_MAX_WARPS, warps = nh >= most ? most : (nh >= 8 ? 8 : 4);
     const int vec = dv % 4 == 0 && ((uintptr_t)o & 15) == 0 && ((uintptr_t)out & 15) == 0;
+    // more than two heads a warp: over several blocks, where they still run all at once (64 heads, one token: 2.67 us with a sincosf per
+    // element and four heads a block, 3.38 with all heads in one block)
+    const int shares = (nh + 2 * warps - 1) / (2 * warps), groups = (long long)T_ * shares <= 592 ? shares : 1;
     TQ_DISPATCH(act_dtype, TA,
-        (tq_launch(T_, 32 * warps, 0, stream)(heads_unrotate_gate_kernel<TA>, (const TA*)o, gates, gate_stride, gate_off,
+        (tq_launch(dim3(T_, groups), 32 * warps, 0, stream)(heads_unrotate_gate_kernel<TA>, (const TA*)o, gates, gate_stride, gate_off,
             v_freq, halves, positions, (TA*)out, T_, nh, dv, vec)));
     TQ_CHECK_LAUNCH("heads_unrotate_gate");
     return 0;
