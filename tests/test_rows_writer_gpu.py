@@ -16,6 +16,8 @@ SHAPES = [  # tokens, heads, key/value heads, key size, value size, rotated elem
     (593, 16, 4, 128, 128, 128, True, True, True),
     (700, 20, 2, 200, 130, 40, True, True, True),          # through shared memory
     (650, 3, 1, 33, 7, 10, False, False, True),            # unaligned rows
+    (2, 2, 1, 64, 300, 64, True, True, False),
+    (2, 2, 1, 64, 12800, 64, False, True, True),           # 50 KB a value
 ]
 
 

@@ -224,7 +224,8 @@ bias_kv_write_rot_kernel(const float* __restrict__ qkv, int row_stride, TA* __re
     extern __shared__ __align__(16) float s_heads[];           // [warps][room], then the angles: rot_dims / 2, dv / 2 pairs
     __shared__ float scratch[33];
     const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
-    const int nq = nh * dk, nk = nkv * dk, dr = dk + dv, room = (max(dk, dv) + 3) & ~3;
+    const bool wide = dv > BA_MAX_DIM;                         // values too long for shared memory's rows: element by element
+    const int nq = nh * dk, nk = nkv * dk, dr = dk + dv, room = (max(dk, wide ? 0 : dv) + 3) & ~3;
     const float* row = qkv + (size_t)t * row_stride;
     const int pos = positions[t];
     float2* cs = reinterpret_cast<float2*>(s_heads + (size_t)n_warps * room);
@@ -244,7 +245,7 @@ bias_kv_write_rot_kernel(const float* __restrict__ qkv, int row_stride, TA* __re
     const int head0 = blockIdx.y * n_warps, stride = gridDim.y * n_warps;
     float4 next = read(head0 + warp);  // on its way while the angles are computed; each later head while the one before is worked on
     if (head0 < nh + nkv) ba_angles(cs, freq, rot_dims >> 1, (float)pos);
-    if (v_freq != nullptr && cache != nullptr && (gridDim.y == 1 || head0 + n_warps > nh + nkv)) ba_angles(v_cs, v_freq, dv >> 1, (float)pos);
+    if (v_freq != nullptr && cache != nullptr && !wide && (gridDim.y == 1 || head0 + n_warps > nh + nkv)) ba_angles(v_cs, v_freq, dv >> 1, (float)pos);
     int page = 0;                      // without a cache (a layer that only reads another's) no table is looked at
     if (cache != nullptr) {
         const int* table = page_table + (size_t)TQ_CHECKED(seq_of_token[t], n_seqs, TQ_IDX_SEQUENCE) * table_stride;
@@ -290,6 +291,10 @@ bias_kv_write_rot_kernel(const float* __restrict__ qkv, int row_stride, TA* __re
         const int g = head - nh - (is_v ? nkv : 0), n = is_v ? dv : dk;
         const float* src = source(head);
         TA* dst = is_q ? q_out + ((size_t)t * nh + head) * dk : cache + (((size_t)page * nkv + g) * page_size + slot) * dr + (is_v ? dk : 0);
+        if (is_v && wide) {
+            for (int e = lane; e < n; e += 32) dst[e] = tq_from_float<TA>(v_freq ? tq_rotated(src, e, dv, halves, v_freq, pos) : src[e]);
+            return;
+        }
         const float* nw = is_v ? nullptr : is_q ? q_norm_w : k_norm_w;
         for (int e = lane; e < n; e += 32) sh[e] = src[e];
         __syncwarp();
@@ -347,12 +352,11 @@ TQ_EXPORT int tq_bias_kv_write_rot(const float* qkv, int row_stride, void* q_out
     // long steps: a block of eight warps a token, several an SM; shorter ones: sixteen warps, a head or two each; while the GPU holds a
     // warp for every head of the step: a head a warp, over blocks of four
     const int heads = nh + (cache ? 2 * nkv : 0), most = T_ > 592 ? 8 : BA_ROT_MAX_WARPS;
-    const int room = ((dk > dv ? dk : dv) + 3) & ~3;
+    const int room = ((dk > dv || dv > BA_MAX_DIM ? dk : dv) + 3) & ~3;      // at most 16 KB of rows
     const bool spread = !norm_rows && (long long)T_ * heads <= BA_SPREAD_HEADS;      // (a norm over whole rows is a block's own)
-    int warps = spread ? 4 : (heads >= most ? most : (heads >= 8 ? 8 : 4));
-    while (warps > 1 && warps * room > 8192) warps >>= 1;    // wide values: 32 KB of rows
+    const int warps = spread ? 4 : (heads >= most ? most : (heads >= 8 ? 8 : 4));
     const int groups = spread ? (heads + warps - 1) / warps : 1;
-    const size_t smem = (size_t)warps * room * sizeof(float) + (size_t)(rot_dims / 2 + 1 + (v_freq ? dv / 2 : 0)) * sizeof(float2);
+    const size_t smem = (size_t)warps * room * sizeof(float) + (size_t)(rot_dims / 2 + 1 + (v_freq && dv <= BA_MAX_DIM ? dv / 2 : 0)) * sizeof(float2);
     const int vec = dk % 4 == 0 && dv % 4 == 0 && row_stride % 4 == 0 && ((uintptr_t)qkv & 15) == 0 && ((uintptr_t)q_out & 15) == 0
                     && ((uintptr_t)cache & 15) == 0;
     TQ_DISPATCH(act_dtype, TA,
