@@ -200,3 +200,26 @@ def test_queries_and_results_at_any_element():
     assert q.data_ptr() % 16 == 4 and out.data_ptr() % 16 == 4
     assert call(q, out) is out and torch.equal(out, want) and not bool(room[:2].any())
     assert call(q, out, run=0) is out and torch.equal(out, want)
+
+
+def test_sizes_of_any_integer_type():
+    """Counts as numpy gives them, such as the longest of an array of run lengths."""
+    from turboquant_cpp_b200.kernels import bias_attention as KB
+    T, H, d = 70, 2, 64
+    g = torch.Generator(device=DEV).manual_seed(9)
+    rand = lambda *s: torch.randn(s, generator=g, device=DEV)
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device=DEV)
+    n = lambda *v: [np.int64(x) for x in v]
+    rows, table, freq, gates = rand(T, 4 * d), i32([[0, 1]]), rand(d // 2), rand(T, H)
+    got = []
+    for f in (list, lambda v: n(*v)):
+        sizes, run, page = f([H, 1, d, d]), f([T])[0], f([64])[0]
+        q, cache, out = torch.empty((T, H, d), dtype=torch.bfloat16, device=DEV), torch.zeros((2, 1, 1, 64, 2 * d), dtype=torch.bfloat16, device=DEV), \
+            torch.empty((T, H * d), dtype=torch.bfloat16, device=DEV)
+        at = torch.arange(T, device=DEV, dtype=torch.int32), torch.zeros(T, device=DEV, dtype=torch.int32)
+        KB.kv_write(rows, q, cache, None, None, 0.0, *at, table, page, *sizes)
+        KB.attention_runs(q, cache, None, None, i32([0, T]), i32([0]), table, page, *f([0, 0]), 0.125, out, f([1])[0], run, *sizes, cell=f([0])[0])
+        KB.kv_write_rot(rows, q, cache, freq, f([d])[0], True, 0.0, *at, table, page, *sizes, v_share=f([1])[0])
+        KB.heads_unrotate_gate(out, gates, f([0])[0], None, True, at[0], out, f([H])[0], f([d])[0])
+        got.append((q, cache, out))
+    assert all(torch.equal(a, b) for a, b in zip(*got))

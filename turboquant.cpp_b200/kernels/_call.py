@@ -2,6 +2,7 @@
 from __future__ import annotations
 
 import ctypes
+from operator import index
 from typing import Optional
 
 import torch
@@ -54,6 +55,11 @@ def check(lib_name: str, rc: int, kernels: int = 1) -> None:
     if rc != 0:
         lib = load_kernel(lib_name)
         raise KernelError(lib.tq_last_error().decode("utf-8", "replace") or f"{lib_name}: error {rc}")
+
+
+def ints(*values) -> map:
+    """Whole numbers of any integer type (numpy's among them) as the plain ints that ctypes passes on without a declaration."""
+    return map(index, values)
 
 
 def want_int32(t: torch.Tensor, what: str) -> None:

@@ -8,7 +8,7 @@ from typing import Optional
 import torch
 
 from ..csrc.build import load_kernel
-from ._call import KernelError, check, code, ptr, stream, want_f32, want_int32
+from ._call import KernelError, check, code, ints, ptr, stream, want_f32, want_int32
 
 _LIB = "attention"
 MAX_HEAD_DIM = 256
@@ -224,12 +224,11 @@ def prefill_rows(q: torch.Tensor, cache_layer: torch.Tensor, planes: int, cu_seq
         raise KernelError("attention_prefill: cu_seqlens, seq_start and the page table must be int32")
     if q.dtype != torch.bfloat16 or cache_layer.dtype != torch.bfloat16 or out.dtype != torch.bfloat16:
         raise KernelError("attention_prefill: queries, cache and output must be bfloat16")
-    # (plain ints are C ints to ctypes)
     check("attention_prefill", load_kernel("attention_prefill").tq_attention_prefill(
-        ptr(q), ptr(cache_layer), planes, ptr(cu_seqlens), ptr(seq_start), ptr(page_table), page_table.shape[1], page_size,
-        cache_layer.shape[0], window, keep_first, cell, c_float(scale), c_float(softcap), ptr(bias_t), 0 if bias_t is None else bias_t.shape[1] - 1,
-        ptr(sink), ptr(out), q.shape[0], n_seqs, max_q_len, n_heads, n_kv_heads, dk, dv,
-        ptr(status), stream()))
+        ptr(q), ptr(cache_layer), planes, ptr(cu_seqlens), ptr(seq_start), ptr(page_table), page_table.shape[1],
+        *ints(page_size, cache_layer.shape[0], window, keep_first, cell), c_float(scale), c_float(softcap), ptr(bias_t),
+        0 if bias_t is None else bias_t.shape[1] - 1, ptr(sink), ptr(out),
+        *ints(q.shape[0], n_seqs, max_q_len, n_heads, n_kv_heads, dk, dv), ptr(status), stream()))
     return out
 
 

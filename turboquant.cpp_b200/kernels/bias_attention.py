@@ -9,7 +9,7 @@ from typing import Optional
 import torch
 
 from ..csrc.build import load_kernel
-from ._call import KernelError, check, code, ptr, stream, want_f32, want_int32
+from ._call import KernelError, check, code, ints, ptr, stream, want_f32, want_int32
 from .attention import prefill_rows
 
 _LIB = "bias_attention"
@@ -38,9 +38,8 @@ def kv_write(qkv: torch.Tensor, q_out: torch.Tensor, cache: Optional[torch.Tenso
     lib = load_kernel(_LIB)
     check(_LIB, lib.tq_bias_kv_write(
         ptr(qkv), ptr(q_out), ptr(cache), code(q_out.dtype), ptr(v_keep), ptr(v_other), c_float(mix),
-        ptr(positions), ptr(seq_of_token), ptr(page_table), page_table.shape[1], page_size, T,
-        heads, kv_heads, dk, dv, page_table.shape[0],
-        cache.shape[0] if cache is not None else 0, stream()))
+        ptr(positions), ptr(seq_of_token), ptr(page_table), *ints(page_table.shape[1], page_size, T, heads, kv_heads, dk, dv),
+        page_table.shape[0], cache.shape[0] if cache is not None else 0, stream()))
 
 
 def kv_write_rot(qkv: torch.Tensor, q_out: torch.Tensor, cache: Optional[torch.Tensor], freq: Optional[torch.Tensor],
@@ -88,10 +87,10 @@ def kv_write_rot(qkv: torch.Tensor, q_out: torch.Tensor, cache: Optional[torch.T
         raise KernelError("kv_write_rot: the cache does not fit the heads")
     lib = load_kernel(_LIB)
     check(_LIB, lib.tq_bias_kv_write_rot(
-        ptr(qkv), qkv.shape[1], ptr(q_out), ptr(cache), code(q_out.dtype), ptr(freq), rot_dims,
+        ptr(qkv), qkv.shape[1], ptr(q_out), ptr(cache), code(q_out.dtype), ptr(freq), *ints(rot_dims),
         1 if halves else 0, c_float(mag), c_float(unit_eps), ptr(q_norm), ptr(k_norm), c_float(norm_eps),
-        1 if norm_rows else 0, ptr(v_freq), v_share, 1 if values_are_keys else 0, c_float(coef), every, ptr(positions), ptr(seq_of_token), ptr(page_table),
-        page_table.shape[1], page_size, T, heads, kv_heads, dk, dv,
+        1 if norm_rows else 0, ptr(v_freq), *ints(v_share), 1 if values_are_keys else 0, c_float(coef), *ints(every), ptr(positions),
+        ptr(seq_of_token), ptr(page_table), *ints(page_table.shape[1], page_size, T, heads, kv_heads, dk, dv),
         page_table.shape[0], cache.shape[0] if cache is not None else 0, stream()))
 
 
@@ -110,9 +109,8 @@ def heads_unrotate_gate(o: torch.Tensor, gates: torch.Tensor, gate_off: int, v_f
     if o.shape != (T, heads * dv) or out.shape != o.shape or out.dtype != o.dtype:
         raise KernelError("heads_unrotate_gate: input and output must be [T, heads * dv] of one dtype")
     lib = load_kernel(_LIB)
-    check(_LIB, lib.tq_heads_unrotate_gate(ptr(o), code(o.dtype), ptr(gates), gates.shape[1], gate_off,
-                                           ptr(v_freq), 1 if halves else 0, ptr(positions), ptr(out), T,
-                                           heads, dv, stream()))
+    check(_LIB, lib.tq_heads_unrotate_gate(ptr(o), code(o.dtype), ptr(gates), gates.shape[1], *ints(gate_off),
+                                           ptr(v_freq), 1 if halves else 0, ptr(positions), ptr(out), *ints(T, heads, dv), stream()))
     return out
 
 

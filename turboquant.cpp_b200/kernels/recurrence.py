@@ -7,7 +7,7 @@ from typing import Sequence
 import torch
 
 from ..csrc.build import load_kernel
-from ._call import KernelError, check, ptr, stream, want_f32, want_int32
+from ._call import KernelError, check, ints, ptr, stream, want_f32, want_int32
 from .ssm import ctypes_ptr
 
 _LIB = "ssm"
@@ -54,7 +54,6 @@ def memory_chunks(rows: torch.Tensor, q_off: int, k_off: int, v_off: int, gates:
     scratch = torch.empty(group * (per_chunk + heads), dtype=torch.float32, device=rows.device)      # the chunks' states, then their decays
     at = scratch.data_ptr()
     lib = load_kernel(_LIB)
-    # (plain ints are C ints to ctypes)
     check(_LIB, lib.tq_memory_chunks(
-        ptr(rows), rows.shape[1], q_off, k_off, v_off, ptr(gates), ctypes_ptr(state), c_longlong(state.stride(0)), ptr(y), ptr(dots),
-        c_void_p(at), c_void_p(at + 4 * group * per_chunk), chunks, group, n_seqs, heads, dk, dv, ptr(cu_seqlens), ptr(slots), stream()), kernels=3 * -(-chunks // group))
+        ptr(rows), *ints(rows.shape[1], q_off, k_off, v_off), ptr(gates), ctypes_ptr(state), c_longlong(state.stride(0)), ptr(y), ptr(dots),
+        c_void_p(at), c_void_p(at + 4 * group * per_chunk), *ints(chunks, group, n_seqs, heads, dk, dv), ptr(cu_seqlens), ptr(slots), stream()), kernels=3 * -(-chunks // group))
