@@ -110,3 +110,24 @@ def test_when_a_matrix_memory_goes_in_chunks(monkeypatch):
         assert not in_chunks(lens), lens
     assert in_chunks([2048], heads=32) and not in_chunks([1024] + ones(31), heads=32) and not in_chunks([2048] + ones(63), heads=32)
     assert in_chunks([2048] + ones(127), heads=4) and in_chunks([1024] * 8, heads=8, d=64) and not in_chunks([512] + ones(63), heads=8, d=64)
+
+
+def test_expanded_latent_keys_take_a_bounded_scratch():
+    """One prompt expands whatever its length (the scores of the other path take more); many prompts with long histories do not
+    where their keys and values would take several times what that path takes."""
+    from types import SimpleNamespace
+
+    from turboquant_cpp_b200.parts import make_mixer
+    m = make_mixer("latent_attention", prefix="", hidden=64, heads=16, dim=128, rot_dim=0, vdim=128, kv_rank=512, scale=0.1, eps=1e-5)
+
+    def ok(lens, held):
+        total = [n + h for n, h in zip(lens, held)]
+        ctx = SimpleNamespace(host_q_lens=lens, n_tokens=sum(lens), max_kv_len=max(total))
+        keys = sum(-(-t // 64) * 64 for t in total)
+        fits = m._affordable(ctx, keys)
+        assert not fits or 2 * keys * 16 * 256 <= max(1 << 30, m._rows_scratch(ctx)[2])
+        return fits
+    assert ok([2048], [0]) and ok([131072], [0]) and ok([262144], [0]) and ok([512] * 64, [0] * 64) and ok([64], [1024])
+    assert not ok([512] * 64, [15000] * 64) and not ok([64], [4000])
+    m.window = 1024
+    assert ok([2048] * 64, [0] * 64)

@@ -21,7 +21,7 @@ cached (the layer then has no W_dkv), and queries that go through a latent of th
 """
 from __future__ import annotations
 
-from typing import List, Optional
+from typing import List, Optional, Tuple
 
 import torch
 
@@ -39,6 +39,7 @@ class LatentAttentionMixer(Mixer):
     # steps with at most this many keys per new token build the heads' keys and values from the cached rows: a key then
     # costs its expansion once (2 R (dim + vdim) per head) and 2 (dim + rot + vdim) per query instead of 2 (2 R + rot)
     EXPAND_KEYS_PER_TOKEN = 32
+    EXPAND_BYTES = 1 << 30    # keys and values of a step may take this, or what the path over the rows would take for its scores
 
     def __init__(self, prefix: str, hidden: int, heads: int, dim: int, rot_dim: int, vdim: int, kv_rank: int,
                  scale: float, eps: float, window: int = 0, position=None, own_cache: bool = True,
@@ -170,6 +171,14 @@ class LatentAttentionMixer(Mixer):
         first = lambda start: max(0, start + 1 - self.window) // page if self.window else 0
         return sum((start + n - 1) // page - first(start) + 1 for n, start in zip(ctx.host_q_lens, ctx.host_seq_start) if n)
 
+    def _rows_scratch(self, ctx: StepContext) -> Tuple[int, int, int]:
+        """The path over the rows: tokens of a block, the most rows of the cache one sees, bytes of its scores and weights."""
+        block = max(16, self.PROMPT_ROWS // self.heads)
+        tokens = min(block, max(ctx.host_q_lens))
+        most = min(tokens + (self.window - 1 if self.window else ctx.max_kv_len), ctx.max_kv_len)
+        most = -(-most // 64) * 64
+        return block, most, tokens * self.heads * most * (4 + 2)
+
     def _expands(self, ctx: StepContext, cache: LayerCache) -> bool:
         """Whether this step builds the heads' keys and values.  Measured on B200, 16 heads of 128 + 64 / 128, rank 512, a
         layer's time in us expanded / over the cached rows (that path's launches bound it below 1,000 tokens): 2,048 new tokens
@@ -178,7 +187,11 @@ class LatentAttentionMixer(Mixer):
         return (self.w_ukv is not None and self.w_ukv.dtype == torch.bfloat16 and cache.kv.dtype == torch.bfloat16 and self.scale > 0.0
                 and (self.kv_rank + self.rot_dim) % 8 == 0 and self.kv_rank % 8 == 0
                 and KA.dense_usable(ctx.act_dtype, self.dim, self.rot_dim, self.vdim, cache.page_size)
-                and self._pages_seen(ctx, cache.page_size) * cache.page_size <= self.EXPAND_KEYS_PER_TOKEN * ctx.n_tokens)
+                and self._affordable(ctx, self._pages_seen(ctx, cache.page_size) * cache.page_size))
+
+    def _affordable(self, ctx: StepContext, keys: int) -> bool:
+        return (keys <= self.EXPAND_KEYS_PER_TOKEN * ctx.n_tokens
+                and 2 * keys * self.heads * (self.dim + self.vdim) <= max(self.EXPAND_BYTES, self._rows_scratch(ctx)[2]))
 
     def _attend_expanded(self, q3, ctx: StepContext, cache: LayerCache) -> torch.Tensor:
         """Prompts: the rows that the step's tokens see, gathered from the pages; every head's keys and values from their
@@ -201,11 +214,9 @@ class LatentAttentionMixer(Mixer):
         sequences on the host; steps of single tokens never come here."""
         H, R, Dk = self.heads, self.kv_rank, self.kv_rank + self.rot_dim
         act, dev = qa.dtype, qa.device
-        block = max(16, self.PROMPT_ROWS // H)
         # one buffer for the gathered rows and one for the weights, sized for the widest block of the step
         longest = max(ctx.host_q_lens)
-        most = min(block, longest) + (self.window - 1 if self.window else ctx.max_kv_len)
-        most = -(-min(most, ctx.max_kv_len) // 64) * 64
+        block, most, _ = self._rows_scratch(ctx)
         rows_all = torch.empty((most, Dk), dtype=act, device=dev)
         weights_all = torch.empty(min(block, longest) * H * most, dtype=act, device=dev)
         t0 = 0
