@@ -134,3 +134,19 @@ def test_sequences_without_new_tokens(monkeypatch):
         assert m._expands(ctx, cache)
         got.append(m.forward(inputs, ctx, cache))
     assert all(torch.equal(got[0], g) for g in got[1:])
+
+
+@pytest.mark.parametrize("n_seqs", [33, 70])
+def test_many_sequences(n_seqs, monkeypatch):
+    """More sequences than a warp has lanes: each finds its own pages among the gathered ones."""
+    runs = [(1, 40, 3, 70)[s % 4] for s in range(n_seqs)]
+    held = [(0, 64, 129, 5, 63)[s % 5] for s in range(n_seqs)]
+    m, weights, x, old, ctx, cache = layer_and_step((3, 64, 64, 128, 128, 0, True, runs, held), n_seqs)
+    monkeypatch.setattr(type(m), "EXPAND_KEYS_PER_TOKEN", 1 << 20)
+    assert m._expands(ctx, cache)
+    want = reference(m, x, old, runs, held, weights, 1e-5)
+    got = m.forward(x, ctx, cache).double()
+    assert float((got - want).norm() / want.norm()) < 8e-3        # as above
+    # no sequence may hide behind the others' rows
+    for a, b in zip(got.split(runs), want.split(runs)):
+        assert float((a - b).norm() / b.norm()) < 2e-2

@@ -108,3 +108,69 @@ def test_the_scratch_of_a_long_run_is_bounded():
     from turboquant_cpp_b200.kernels import recurrence as KR
     _, used = memory_step([20000], H=8, dk=128, dv=128)           # 313 chunks of 0.5 MB
     assert used <= KR.SCRATCH_BYTES + (1 << 20), used
+
+
+@pytest.mark.parametrize("n_seqs", [33, 70])
+def test_many_sequences(n_seqs):
+    """More sequences than a warp has lanes, some of one token and some of none: the token-by-token kernel's outputs and states."""
+    from turboquant_cpp_b200.kernels import recurrence as KR, ssm as KS
+    H, d = 2, 64
+    lens = [(1, 70, 0, 3, 129, 64)[s % 6] for s in range(n_seqs)]
+    T, g = sum(lens), torch.Generator(device=DEV).manual_seed(n_seqs)
+    rows = torch.randn((T, 3 * H * d), generator=g, device=DEV)
+    gates = torch.stack([-0.2 * torch.rand((T, H), generator=g, device=DEV), -torch.rand((T, H), generator=g, device=DEV)], -1).contiguous()
+    first = torch.randn((n_seqs, H, d + 1, d), generator=g, device=DEV)
+    cu, slots = i32(np.concatenate([[0], np.cumsum(lens)])), i32(np.arange(n_seqs)[::-1].copy())
+    out = []
+    for how in ("chunks", "tokens"):
+        state, y, dots = first.clone(), torch.empty((T, H * d), device=DEV), torch.empty((T, H), device=DEV)
+        if how == "chunks":
+            KR.memory_chunks(rows, 0, H * d, 2 * H * d, gates, state, y, dots, KR.chunks_of(lens, T, n_seqs), H, d, d, cu, slots)
+        else:
+            KS.memory_scan(rows, 0, H * d, 2 * H * d, gates, state, y, dots, H, d, d, cu, slots)
+        out.append((y, dots, state))
+    for a, b in zip(*out):
+        assert float((a - b).norm() / b.norm()) < 1e-5            # float32 sums of some hundred terms in another order
+    for s, n in enumerate(lens):
+        if n == 0:
+            assert torch.equal(out[0][2][slots[s]], first[slots[s]])
+
+
+@pytest.mark.parametrize("d", [64, 128])
+def test_a_memory_layer_continues_its_runs(d, monkeypatch):
+    """The layer's own choice of form, in steps that follow one another: a chunked prompt goes on in another portion (walked or
+    chunked) and in steps of single tokens as the walk alone does."""
+    from turboquant_cpp_b200.parts import LayerCache, StepContext, chunks, make_mixer
+    from turboquant_cpp_b200.weights import RandomSource, WeightStore
+    H, n_seqs = 4, 3
+    m = make_mixer("matrix_memory", prefix="", hidden=256, heads=H, dim=d, vdim=d, gate_cap=20.0, eps=1e-5)
+    m.run_dtype = torch.float32
+    m.bind(WeightStore(RandomSource(m.weight_specs(), d, std=0.05), m.weight_specs(), DEV, torch.float32))
+    steps = [[700, 30, 1], [130, 1, 64], [200, 700, 700], [1, 1, 1], [90, 2, 60]]
+    g = torch.Generator(device=DEV).manual_seed(d)
+    xs = [torch.randn((sum(lens), 256), generator=g, device=DEV) for lens in steps]
+    got, forms = {}, []
+    for how in ("own", "walk"):
+        if how == "walk":
+            monkeypatch.setattr(type(m), "_in_chunks", lambda self, ctx, cuts: False)
+        need = m.state_need()
+        cache = LayerCache(page_size=64)
+        cache.state = torch.zeros((n_seqs,) + tuple(need.shape), dtype=need.dtype, device=DEV)
+        held, got[how] = np.zeros(n_seqs, dtype=np.int64), []
+        for lens, x in zip(steps, xs):
+            cu = np.concatenate([[0], np.cumsum(lens)])
+            seq_of = np.repeat(np.arange(n_seqs), lens)
+            pos = np.arange(cu[-1]) - cu[:-1][seq_of] + held[seq_of]
+            ctx = StepContext(n_tokens=int(cu[-1]), n_seqs=n_seqs, tokens=i32(pos), positions=i32(pos), seq_of_token=i32(seq_of), cu_seqlens=i32(cu),
+                              seq_start=i32(held), slots=i32(range(n_seqs)), want_rows=i32([]), n_want=0, max_q_len=max(lens),
+                              max_kv_len=int((held + lens).max()), act_dtype=torch.float32, device=torch.device(DEV), host_q_lens=list(lens),
+                              host_slots=list(range(n_seqs)), host_seq_start=[int(h) for h in held], status=torch.zeros(1, dtype=torch.int32, device=DEV))
+            ctx.carry = {}
+            if how == "own":
+                forms.append(max(lens) > 1 and m._in_chunks(ctx, chunks.cut_size(ctx, H, d + 1) is not None))
+            got[how].append(m.forward(x, ctx, cache))
+            held = held + lens
+        got[how].append(cache.state)
+    assert forms[0] and forms[2] and not forms[3]
+    for a, b in zip(got["own"], got["walk"]):
+        assert float((a - b).norm() / b.norm()) < 2e-5            # float32 sums in another order, through norm and closing product
