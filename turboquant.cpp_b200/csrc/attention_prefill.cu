@@ -270,12 +270,12 @@ __device__ __forceinline__ float max_of(const uint32_t (&v)[32], float from) {
 // 7.5e-7 (1.2e-7).
 // p: the series' coefficients in powers of s^2, times scale; below: the |x| up to which it serves (a cap so small against the
 // scale that they overflow: none).
-struct CapSeries { float p[5], k, scale, cap, below; };
+struct CapSeries { float p[5], k, k_low, cap, below; };
 __device__ __forceinline__ CapSeries cap_series(float scale, float cap) {
     CapSeries r;
-    r.scale = scale;
     r.cap = cap;
     r.k = scale / cap;
+    r.k_low = fmaf(-r.k, cap, scale) / cap;        // what the quotient's rounding left out: s * (k + k_low) is rounded once
     const float k2 = r.k * r.k;
     r.p[0] = scale;
     r.p[1] = -1.0f / 3.0f * k2 * scale;
@@ -303,7 +303,7 @@ __device__ __forceinline__ void cap_scores(uint32_t (&v)[32], const CapSeries& s
         }
     } else {
 #pragma unroll
-        for (int c = 0; c < 32; ++c) v[c] = __float_as_uint(s.cap * tanhf(__uint_as_float(v[c]) * s.scale / s.cap));
+        for (int c = 0; c < 32; ++c) v[c] = __float_as_uint(s.cap * tanhf(fmaf(__uint_as_float(v[c]), s.k, __uint_as_float(v[c]) * s.k_low)));
     }
 }
 
