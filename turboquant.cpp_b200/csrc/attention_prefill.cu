@@ -16,18 +16,19 @@
 // CTAs, one per SM, take units until none is left:
 //   warps 0..3    softmax of slot A, a thread per row; warps 4..7 of slot B: read S, mask, online softmax, write P
 //                 (bf16) over S in tensor memory, where the second product takes it as its left operand.  O stays in
-//                 tensor memory: it is rescaled there only when a row's maximum grows by more than 2^8 over the one
-//                 its exponentials are taken against (until then P is simply larger, at most 256, and the row's sum
-//                 carries the same factor)
+//                 tensor memory: it is rescaled there when a tile's maximum is larger than the one the row's exponentials are
+//                 taken against (attention over rows), or larger by more than 2^8 (until then P is simply larger, at most
+//                 256, and the row's sum carries the same factor)
 //   warp 8        TMA: Q of both slots, then K and V pages through rings that both slots read
 //   warp 9        owns tensor memory, issues  O += P V  of a slot's tile and right behind it  S = Q K^T  of its next
 // The two slots take turns: while one's scores are exponentiated the other's products run, which is what bounds a
 // tile pair: 2 x 16,384 exponentials at 16 a cycle and SM (2,048 cycles) beside 32 products of 128 x 128 x 16 (2,048).
-// Measured: 3,450 cycles a pair (softmax 1,950, then 1,400 until the slot's next scores are there), with a bias 5,250, with a
-// cap 6,400; with one slot (eight warps on one tile, P through shared memory, products issued by one lane) 6,000 a tile.
-// Prompts of 682 + 1,365 + 2,049 tokens, 16 heads of 128: 84.5 -> 57.5 us (16 kv heads, plain), 457 -> 80.8 us (4 kv
-// heads, cap 50) where the mma.sync kernel of csrc/bias_attention.cu served the second; 2,048 tokens, window 1,024 with a bias:
-// 97.3 -> 44.5 us.
+// Neither is reached: the tensor pipe is active 31 % of the plain form's time, the exponentials' unit as long; what remains is the turn
+// from one to the other (a slot's softmax, then its products, some 1,500 cycles).  One slot (eight warps on one tile, P
+// through shared memory, products issued by one lane) took 6,000 cycles a tile.
+// Prompts of 682 + 1,365 + 2,049 tokens, 16 heads of 128, the replaced kernels (one slot; mma.sync for rows) and this one, us: 16 kv
+// heads, plain 79 / 52; rows with 4 kv heads, plain 151 / 64, cells of 512 111 / 36, cap 50 441 / 77, cap 4 with large scores 441 / 119;
+// 2,048 tokens, window 1,024 with a bias 89 / 47.
 // Every wait on an mbarrier is bounded; a wait that runs out sets *status and the CTA
 // leaves cleanly.
 #include <cuda.h>
@@ -266,8 +267,8 @@ __device__ __forceinline__ float max_of(const uint32_t (&v)[32], float from) {
 // softcap * tanh(s * scale / softcap) of 32 scores: the odd series up to x^9, x = s * scale / softcap, where every x of the
 // warp's rows lies below a quarter (the first term left out is 9e-9 of the result there), tanhf beyond, as in the decode kernels.
 // Relative error against 64 bits, a million scores each, caps of 4 to 50: the series at most 1.1e-7 (root mean square 3.5e-8), tanhf
-// 2.4e-7 (5e-8) over the same scores and 2.9e-7 (7.8e-8) beyond a quarter, where 1 - 2 / (e^2x + 1) of fast intrinsics was off by
-// 7.5e-7 (1.2e-7).
+// 2.4e-7 (5e-8) over the same scores and 2.8e-7 (7.5e-8) beyond a quarter, where 1 - 2 / (e^2x + 1) of fast intrinsics was off by
+// 7.5e-7 (1.2e-7).  s * (k + k_low): with a division a score the code outgrew the instruction caches (500 us for the case of 119 above).
 // p: the series' coefficients in powers of s^2, times scale; below: the |x| up to which it serves (a cap so small against the
 // scale that they overflow: none).
 struct CapSeries { float p[5], k, k_low, cap, below; };
@@ -626,8 +627,8 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 // half a page (plain scores: a page) at a time, twice: for the tile's maximum, which shapes and masks the scores and
                 // leaves shaped ones in place of the products, then for the weights, written in bf16 over scores already
                 // read.  The maximum comes first so that a row's largest weight can be exactly one: with it known only so far, and
-                // corrected by powers of two, the error of rows with a cap or bias against 64 bits was up to 1.3 times
-                // as large.  The loops are kept small: instructions come in at some 250 cycles per 128 bytes the first time and
+                // corrected by powers of two, the error of rows against 64 bits was up to 1.3 times as large (here it is that of
+                // the mma.sync kernel or less).  It costs 2 to 5 us of the times above (plain 49.6, cap 50 73.7, bias 42.1).  The loops are kept small: instructions come in at some 250 cycles per 128 bytes the first time and
                 // fall out of the caches that ten warps share (the tile unrolled in two passes: 1.6 times the kernel's time).
                 float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
                 float top = -INFINITY;

@@ -10,8 +10,8 @@
 // the other, the kept state going from group to group, so that the chunks' states take a bounded buffer.  Token by token (csrc/ssm.cu) a walk does 2
 // multiply-adds an element of the state and token, a chain of its tokens with a shuffle tree each, and long runs are walked twice to
 // fill the GPU; in chunks it is 2 + 64 (1 / dk + 1 / dv) of them, all in register-tiled products.  Everything is fp32 and
-// stays on the CUDA cores: tensor cores would round operands (three products of split tf32 parts cost what the fp32
-// units take here).  Measured, 682 + 1,366 tokens, 16 heads of 128 x 129: 289 us for both walks token by token; here 37 us for the
+// stays on the CUDA cores: tensor cores round operands (two tf32 parts of each hold 22 of 24 bits; three bfloat16 parts hold all 24 in
+// six products, a form that was not built).  Measured, 682 + 1,366 tokens, 16 heads of 128 x 129: 289 us for both walks token by token; here 37 us for the
 // chunks' sums, 16 for the starts and 79 for the outputs (1.07 G multiply-adds, 30 us at the fp32 units' rate; what bounds them is shared
 // memory, twelve 128-byte reads a warp for its 32 multiply-adds a thread; 102 us with transposed stores and weights that met in one
 // bank).
