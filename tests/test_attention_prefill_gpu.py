@@ -185,6 +185,20 @@ def test_a_cap_too_small_for_the_series():
     assert bool(((got - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -18 * mag).all())
 
 
+@pytest.mark.parametrize("cap", [20.0, 7.3])
+def test_infinite_scores_are_the_cap(cap):
+    """Products that overflow float32 are capped like any other: weights e^cap and e^-cap."""
+    T, d = 100, 64
+    g = torch.Generator(device=DEV).manual_seed(10)
+    q, k = torch.zeros((T, 1, d), device=DEV), torch.zeros((T, 1, d), device=DEV)
+    q[:, 0, 0], k[:, 0, 0] = 3e38, 4.0 * (1 - 2 * torch.randint(0, 2, (T,), generator=g, device=DEV)).float()
+    v = torch.randn((T, 1, d), generator=g, device=DEV).to(torch.bfloat16)
+    got = one_sequence(q, k, v, softcap=cap).double()
+    w = torch.exp(cap * torch.sign(k[:, 0, 0]).double() - cap)[:, None, None]
+    want, mag = (w * v.double()).cumsum(0) / w.cumsum(0), (w * v.double().abs()).cumsum(0) / w.cumsum(0)
+    assert bool(((got - want).abs() <= 2.0 ** -8 * want.abs() + (2.0 ** -7 + 1e-5) * mag).all())
+
+
 def test_queries_and_results_at_any_element():
     """Contiguous views that begin off a 16-byte boundary, and a step without runs."""
     from turboquant_cpp_b200.kernels import bias_attention as KB

@@ -304,7 +304,10 @@ __device__ __forceinline__ void cap_scores(uint32_t (&v)[32], const CapSeries& s
         }
     } else {
 #pragma unroll
-        for (int c = 0; c < 32; ++c) v[c] = __float_as_uint(s.cap * tanhf(fmaf(__uint_as_float(v[c]), s.k, __uint_as_float(v[c]) * s.k_low)));
+        for (int c = 0; c < 32; ++c) {
+            const float f = __uint_as_float(v[c]), finite = fminf(fmaxf(f, -3e38f), 3e38f);      // an infinite score is the cap
+            v[c] = __float_as_uint(s.cap * tanhf(fmaf(f, s.k, finite * s.k_low)));
+        }
     }
 }
 
