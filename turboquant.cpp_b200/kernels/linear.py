@@ -2,8 +2,9 @@
 
 The reference's dense projections go through one routine that calls the platform's BLAS where
 there is one (src/engine/tq_ops.c:296-343, Accelerate at :297-306); here they go through cuBLAS
-(torch.mm).  The float32 path never uses a reduced-precision matrix mode: TF32 is switched off
-for the call and the process's setting restored after it.  Expert products do not come through here (kernels/moe.py).
+(torch.mm), but for float32 products of many tokens, which csrc/gemm_f32.cu takes.  The float32 path never uses a
+reduced-precision matrix mode: TF32 is switched off for the call and the process's setting restored after it.  Expert products
+do not come through here (kernels/moe.py).
 """
 from __future__ import annotations
 
@@ -11,6 +12,7 @@ from typing import Optional
 
 import torch
 
+from . import gemm_f32 as KF
 from ._call import KernelError
 
 
@@ -34,14 +36,16 @@ class _FullPrecision:
             m.allow_bf16_reduced_precision_reduction = self.saved[1]
 
 
-def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
+def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtype] = None, status: Optional[torch.Tensor] = None) -> torch.Tensor:
     """x [T, K] times weight [N, K] transposed -> [T, N].  A float32 weight makes the product a
-    true float32 one whatever x is; a bfloat16 weight takes bfloat16 x and accumulates in float32."""
+    true float32 one whatever x is; a bfloat16 weight takes bfloat16 x and accumulates in float32.
+    status: the step's status word, for a kernel whose bounded wait runs out; without one the product is the library's."""
     if not x.is_cuda:
         raise KernelError("linear: CUDA tensors only; there is no CPU path")
     with _FullPrecision():
         if weight.dtype == torch.float32:
-            y = torch.mm(x if x.dtype == torch.float32 else x.float(), weight.t())
+            xf = x if x.dtype == torch.float32 else x.float()
+            y = KF.gemm_f32(xf, weight, status=status) if status is not None and KF.pays(xf, weight) else torch.mm(xf, weight.t())
         elif weight.dtype == torch.bfloat16:
             xb = x if x.dtype == torch.bfloat16 else x.to(torch.bfloat16)
             if out_dtype == torch.float32:

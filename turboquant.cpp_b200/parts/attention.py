@@ -67,6 +67,8 @@ class AttentionMixer(Mixer):
             names.append("gemv")
         if getattr(self, "run_dtype", None) == torch.bfloat16 and self.head_dim in (64, 128):
             names.append("attention_prefill")
+        if getattr(self, "run_dtype", None) == torch.float32:
+            names.append("gemm_f32")
         return names
 
     def cache_need(self) -> KVNeed:
@@ -95,7 +97,7 @@ class AttentionMixer(Mixer):
                              cache.page_size, q, cache.kv if cache.writes else None, self.n_heads, self.n_kv_heads,
                              self.head_dim)
             return self._attend(q, T, act, ctx, cache)
-        qkv = linear(xn, self.w_qkv, out_dtype=act)
+        qkv = linear(xn, self.w_qkv, out_dtype=act, status=ctx.status)
         bias = self.b_qkv
         if self.position is not None and tables is None:
             # an encoding that is not a table-driven rotation: the bias first, then the encoding's own pass over
@@ -141,7 +143,7 @@ class AttentionMixer(Mixer):
                          self.window, self.scale, o, self.n_heads, self.n_kv_heads, self.head_dim)
         if KG.pays(o, self.w_o):
             return KG.gemv(o, self.w_o, torch.empty((T, self.hidden), dtype=torch.float32, device=o.device))
-        return linear(o, self.w_o, out_dtype=torch.float32)
+        return linear(o, self.w_o, out_dtype=torch.float32, status=ctx.status)
 
 
 register_mixer("attention", AttentionMixer)

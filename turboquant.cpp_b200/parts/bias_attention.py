@@ -180,7 +180,7 @@ class BiasedWindowAttentionMixer(Mixer):
         T, act, dev = xn.shape[0], ctx.act_dtype, xn.device
         if projected is not None and self.position is None and self.unit_eps == 0.0:
             raise ValueError(f"attention '{self.prefix}': rows of a wider projection need the rotating writer")
-        qkv = projected if projected is not None else linear(xn, self.w_qkv, out_dtype=torch.float32)
+        qkv = projected if projected is not None else linear(xn, self.w_qkv, out_dtype=torch.float32, status=ctx.status)
         q = torch.empty((T, self.heads, self.dim), dtype=act, device=dev)
         keep = other = None
         if self.mix_values is not None:
@@ -204,7 +204,7 @@ class BiasedWindowAttentionMixer(Mixer):
                             softcap=self.softcap, runs_min=self.RUNS_MIN)
         if KG.pays(o, self.w_o):                   # a few tokens: the output projection as a stream of its weights
             return KG.gemv(o, self.w_o, torch.empty((T, self.hidden), dtype=torch.float32, device=dev))
-        return linear(o, self.w_o, out_dtype=torch.float32)
+        return linear(o, self.w_o, out_dtype=torch.float32, status=ctx.status)
 
 
 register_mixer("window_bias_attention", BiasedWindowAttentionMixer)

@@ -105,15 +105,15 @@ class ChannelDeltaMixer(Mixer):
         st = cache.state                                                       # [max_slots, kept | S]
         kept = st[:, :self.kept_size].unflatten(1, (self.taps - 1, self.channels))
         S = st[:, self.kept_size:self.kept_size + self.heads * self.vdim * self.dim].unflatten(1, (self.heads, self.vdim, self.dim))
-        proj = linear(xn, self.w_in, out_dtype=torch.float32)                  # [T, q | k | v | beta | a1 | g1]
+        proj = linear(xn, self.w_in, out_dtype=torch.float32, status=ctx.status)                  # [T, q | k | v | beta | a1 | g1]
         qkv = torch.empty((T, self.channels), dtype=torch.float32, device=dev)
         one_each = ctx.max_q_len == 1 and ctx.n_seqs == T                     # every sequence brings one token
         if one_each:
             KS.conv_silu_step(proj, 0, self.w_conv, None, kept, qkv, ctx.slots)
         else:
             KS.conv_silu(proj, 0, self.w_conv, None, kept, qkv, ctx.seq_of_token, ctx.cu_seqlens, ctx.slots)
-        raw = linear(proj[:, self.a1_off:self.a1_off + self.rank_a], self.w_a2, out_dtype=torch.float32)      # raw decays
-        gate = linear(proj[:, self.g1_off:self.g1_off + self.rank_g], self.w_g2, out_dtype=torch.float32)
+        raw = linear(proj[:, self.a1_off:self.a1_off + self.rank_a], self.w_a2, out_dtype=torch.float32, status=ctx.status)      # raw decays
+        gate = linear(proj[:, self.g1_off:self.g1_off + self.rank_g], self.w_g2, out_dtype=torch.float32, status=ctx.status)
         o = torch.empty((T, self.inner), dtype=ctx.act_dtype, device=dev)
         if one_each:
             KS.delta_step(qkv, 0, self.qk_size, 2 * self.qk_size, proj, self.b_off, raw, 0, self.dt_bias, self.a_log, gate, 0, True,
@@ -127,7 +127,7 @@ class ChannelDeltaMixer(Mixer):
             KS.gated_group_norm(y, gate, 0, self.w_norm, self.heads, self.eps, o, gate_after=True, sigmoid_gate=True)
         if KG.pays(o, self.w_o):
             return KG.gemv(o, self.w_o, torch.empty((T, self.hidden), dtype=torch.float32, device=dev))
-        return linear(o, self.w_o, out_dtype=torch.float32)
+        return linear(o, self.w_o, out_dtype=torch.float32, status=ctx.status)
 
 
 register_mixer("channel_delta", ChannelDeltaMixer)
@@ -200,7 +200,7 @@ class HeadDeltaMixer(Mixer):
         st = cache.state                                                       # [max_slots, kept | S]
         kept = st[:, :self.kept_size].unflatten(1, (self.taps - 1, self.channels))
         S = st[:, self.kept_size:self.kept_size + self.state_size].unflatten(1, (H, dv, dk))
-        proj = projected if projected is not None else linear(xn, self.w_in, out_dtype=torch.float32)
+        proj = projected if projected is not None else linear(xn, self.w_in, out_dtype=torch.float32, status=ctx.status)
         b, a, z = offset + self.b_off, offset + self.a_off, offset + self.g_off
         qkv = torch.empty((T, self.channels), dtype=torch.float32, device=dev)
         o = torch.empty((T, self.inner), dtype=ctx.act_dtype, device=dev)
@@ -217,7 +217,7 @@ class HeadDeltaMixer(Mixer):
             KS.gated_group_norm(y, proj, z, self.w_norm, H, self.eps, o, gate_after=True)
         if KG.pays(o, self.w_o):
             return KG.gemv(o, self.w_o, torch.empty((T, self.hidden), dtype=torch.float32, device=dev))
-        return linear(o, self.w_o, out_dtype=torch.float32)
+        return linear(o, self.w_o, out_dtype=torch.float32, status=ctx.status)
 
 
 register_mixer("head_delta", HeadDeltaMixer)

@@ -39,10 +39,10 @@ class SwiGLUFeedForward(FeedForward):
         return {"matmul": (wb(self.w_gate_up) + wb(self.w_down), 6.0 * n_tokens * self.hidden * self.intermediate)}
 
     def forward(self, xn: torch.Tensor, ctx: StepContext) -> torch.Tensor:
-        gu = linear(xn, self.w_gate_up, out_dtype=torch.float32)     # gate and up stay fp32 until the product
+        gu = linear(xn, self.w_gate_up, out_dtype=torch.float32, status=ctx.status)     # gate and up stay fp32 until the product
         h = torch.empty((xn.shape[0], self.intermediate), dtype=ctx.act_dtype, device=xn.device)
         K.silu_mul(gu, h)
-        return linear(h, self.w_down, out_dtype=torch.float32)
+        return linear(h, self.w_down, out_dtype=torch.float32, status=ctx.status)
 
 
 register_feed_forward("swiglu", SwiGLUFeedForward)
@@ -89,10 +89,10 @@ class GluFeedForward(FeedForward):
         return {"matmul": (wb(self.w_gate_up) + wb(self.w_down), 6.0 * n_tokens * self.hidden * self.intermediate)}
 
     def forward(self, xn: torch.Tensor, ctx: StepContext, leave_bias: bool = False) -> torch.Tensor:
-        gu = linear(xn, self.w_gate_up, out_dtype=torch.float32)
+        gu = linear(xn, self.w_gate_up, out_dtype=torch.float32, status=ctx.status)
         h = torch.empty((xn.shape[0], self.intermediate), dtype=ctx.act_dtype, device=xn.device)
         K.glu_mul(gu, h, self.glu, bias=self.gate_up_bias)
-        y = linear(h, self.w_down, out_dtype=torch.float32)
+        y = linear(h, self.w_down, out_dtype=torch.float32, status=ctx.status)
         if self.down_bias is not None and not leave_bias:
             K.add_bias(y, self.down_bias)
         return y
@@ -134,13 +134,13 @@ class ReluSquaredFeedForward(FeedForward):
         return {"matmul": (wb(self.w_up) + wb(self.w_down), 4.0 * n_tokens * self.hidden * self.intermediate)}
 
     def forward(self, xn: torch.Tensor, ctx: StepContext, leave_bias: bool = False) -> torch.Tensor:
-        u = linear(xn, self.w_up, out_dtype=torch.float32)          # fp32 until the activation has been taken
+        u = linear(xn, self.w_up, out_dtype=torch.float32, status=ctx.status)          # fp32 until the activation has been taken
         h = torch.empty((xn.shape[0], self.intermediate), dtype=ctx.act_dtype, device=xn.device)
         if self.up_bias is not None:
             K.bias_map(u, self.up_bias, h, K.MAP_RELU_SQUARED)
         else:
             K.map_elements(u, h, K.MAP_RELU_SQUARED)
-        y = linear(h, self.w_down, out_dtype=torch.float32)
+        y = linear(h, self.w_down, out_dtype=torch.float32, status=ctx.status)
         if self.down_bias is not None and not leave_bias:
             K.add_bias(y, self.down_bias)
         return y

@@ -48,10 +48,10 @@ def _fuse(ws: List[torch.Tensor]) -> torch.Tensor:
     return torch.cat([w.to(dt) for w in ws], dim=0).contiguous()
 
 
-def _output(o: torch.Tensor, w_o: torch.Tensor, hidden: int) -> torch.Tensor:
+def _output(o: torch.Tensor, w_o: torch.Tensor, hidden: int, ctx: StepContext) -> torch.Tensor:
     if KG.pays(o, w_o):                   # a few tokens: the output projection as a stream of its weights
         return KG.gemv(o, w_o, torch.empty((o.shape[0], hidden), dtype=torch.float32, device=o.device))
-    return linear(o, w_o, out_dtype=torch.float32)
+    return linear(o, w_o, out_dtype=torch.float32, status=ctx.status)
 
 
 class RotatedValueAttentionMixer(Mixer):
@@ -120,7 +120,7 @@ class RotatedValueAttentionMixer(Mixer):
 
     def forward(self, xn: torch.Tensor, ctx: StepContext, cache: LayerCache) -> torch.Tensor:
         T, act, dev = xn.shape[0], ctx.act_dtype, xn.device
-        rows = linear(xn, self.w_in, out_dtype=torch.float32)                   # [q | k | v | gate logits]
+        rows = linear(xn, self.w_in, out_dtype=torch.float32, status=ctx.status)                   # [q | k | v | gate logits]
         q = torch.empty((T, self.heads, self.dim), dtype=act, device=dev)
         pe = self.position
         halves = pe.halves if pe is not None else True
@@ -131,7 +131,7 @@ class RotatedValueAttentionMixer(Mixer):
         o = paged_attention(q, cache, ctx, self.heads, self.kv_heads, self.dim, self.vdim, self.scale, window=self.window,
                             softcap=self.softcap, runs_min=self.RUNS_MIN)
         KB.heads_unrotate_gate(o, rows, self.gate_off, self.v_freq, halves, ctx.positions, o, self.heads, self.vdim)
-        return _output(o, self.w_o, self.hidden)
+        return _output(o, self.w_o, self.hidden, ctx)
 
 
 register_mixer("rotated_value_attention", RotatedValueAttentionMixer)
@@ -202,7 +202,7 @@ class DifferentialAttentionMixer(Mixer):
         if cache.writes != self.own_cache:
             raise RuntimeError(f"attention '{self.prefix}': the layer {'keeps' if self.own_cache else 'reads'} a cache, "
                                f"the model's schedule says otherwise")
-        rows = linear(xn, self.w_in, out_dtype=torch.float32)                   # [q | k | v | gate logits] or [q | gate logits]
+        rows = linear(xn, self.w_in, out_dtype=torch.float32, status=ctx.status)                   # [q | k | v | gate logits] or [q | gate logits]
         H2, G2 = 2 * self.heads, 2 * self.kv_heads
         q = torch.empty((T, H2, self.dim), dtype=act, device=dev)
         KB.kv_write_rot(rows, q, cache.kv if cache.writes else None, None, 0, True, 0.0, ctx.positions, ctx.seq_of_token,
@@ -211,7 +211,7 @@ class DifferentialAttentionMixer(Mixer):
         o = torch.empty((T, self.heads * self.vdim), dtype=act, device=dev)
         KB.diff_combine(maps, rows, self.q_size + self.kv_size, self.lam, self.eps, 1.0 - self.diff, o, self.heads,
                         self.kv_heads, self.vdim)
-        return _output(o, self.w_o, self.hidden)
+        return _output(o, self.w_o, self.hidden, ctx)
 
 
 register_mixer("differential_attention", DifferentialAttentionMixer)

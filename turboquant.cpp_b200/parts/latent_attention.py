@@ -124,12 +124,12 @@ class LatentAttentionMixer(Mixer):
         T, H, R, act = xn.shape[0], self.heads, self.kv_rank, ctx.act_dtype
         if self.q_rank:
             # the queries' latent: projection in float32, RMS norm with its weight, rounded to the activation dtype
-            cq = KE.rmsnorm(linear(xn, self.w_dq, out_dtype=torch.float32), self.w_qnorm, self.eps,
+            cq = KE.rmsnorm(linear(xn, self.w_dq, out_dtype=torch.float32, status=ctx.status), self.w_qnorm, self.eps,
                             torch.empty((T, self.q_rank), dtype=act, device=xn.device))
-            q = linear(cq, self.w_q, out_dtype=act)
+            q = linear(cq, self.w_q, out_dtype=act, status=ctx.status)
         else:
-            q = linear(xn, self.w_q, out_dtype=act)                                    # [T, H * (dim + rot_dim)]
-        dkv = linear(xn, self.w_dkv, out_dtype=torch.float32) if self.own_cache else None
+            q = linear(xn, self.w_q, out_dtype=act, status=ctx.status)                                    # [T, H * (dim + rot_dim)]
+        dkv = linear(xn, self.w_dkv, out_dtype=torch.float32, status=ctx.status) if self.own_cache else None
         freq, mag = (self.position.freq, self.position.mag) if self.position is not None and self.position.dims else (None, 1.0)
         # norm of the latent, the two rotations and the cache write in one launch
         KL.latent_prepare(q, dkv, self.w_norm, self.eps, freq, mag, ctx.positions, ctx.seq_of_token, cache.page_table,
@@ -138,7 +138,7 @@ class LatentAttentionMixer(Mixer):
         runs = (ctx.max_q_len >= self.PROMPT_MIN_RUN and len(ctx.host_q_lens) == ctx.n_seqs
                 and len(ctx.host_seq_start) == ctx.n_seqs)
         if runs and self._expands(ctx, cache):
-            return linear(self._attend_expanded(q3, ctx, cache), self.w_o, out_dtype=torch.float32)
+            return linear(self._attend_expanded(q3, ctx, cache), self.w_o, out_dtype=torch.float32, status=ctx.status)
         # the prompt path wants [query in the latent space | rotated part] side by side: the product writes there
         qa = torch.empty((T, H, R + self.rot_dim), dtype=act, device=xn.device) if runs else None
         q_lat = qa[:, :, :R] if runs else torch.empty((T, H, R), dtype=act, device=xn.device)
@@ -155,7 +155,7 @@ class LatentAttentionMixer(Mixer):
             self._attend_tokens(q, q_lat, sums, ctx, cache)
         v = torch.empty((T, H, self.vdim), dtype=act, device=xn.device)
         batched_linear(sums.transpose(0, 1), self.w_uv_t, v.transpose(0, 1))
-        return linear(v.view(T, H * self.vdim), self.w_o, out_dtype=torch.float32)
+        return linear(v.view(T, H * self.vdim), self.w_o, out_dtype=torch.float32, status=ctx.status)
 
     def _attend_tokens(self, q, q_lat, sums, ctx: StepContext, cache: LayerCache) -> None:
         """Every token on its own: the kernel walks its keys (decode steps, short runs).  Reads device tensors of
@@ -201,7 +201,7 @@ class LatentAttentionMixer(Mixer):
         rows = torch.empty((pages * cache.page_size, R + self.rot_dim), dtype=q3.dtype, device=dev)
         page_base = torch.empty(ctx.n_seqs, dtype=torch.int32, device=dev)
         KL.latent_gather_pages(cache.kv, cache.page_table, cache.page_size, ctx.cu_seqlens, ctx.seq_start, self.window, rows, page_base)
-        kv = linear(rows[:, :R], self.w_ukv, out_dtype=q3.dtype)
+        kv = linear(rows[:, :R], self.w_ukv, out_dtype=q3.dtype, status=ctx.status)
         out = torch.empty((T, H * self.vdim), dtype=q3.dtype, device=dev)
         return KA.prefill_dense(q3, kv, rows, R, ctx.cu_seqlens, ctx.seq_start, page_base, self.window, self.scale, self.sink, out,
                                 ctx.n_seqs, ctx.max_q_len, H, self.dim, self.rot_dim, self.vdim, status=ctx.status)

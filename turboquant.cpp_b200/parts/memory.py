@@ -97,7 +97,7 @@ class MatrixMemoryMixer(Mixer):
                 offset: int = 0) -> torch.Tensor:
         """projected: float32 rows of a wider product that hold this mixer's projection from column `offset`."""
         T, dev, H, dk, dv = xn.shape[0], xn.device, self.heads, self.dim, self.vdim
-        proj = projected if projected is not None else linear(xn, self.w_in, out_dtype=torch.float32)
+        proj = projected if projected is not None else linear(xn, self.w_in, out_dtype=torch.float32, status=ctx.status)
         q, k = offset, offset + self.qk
         v, z = k + self.qk, k + self.qk + self.inner
         i, f = z + self.inner, z + self.inner + H
@@ -135,7 +135,7 @@ class MatrixMemoryMixer(Mixer):
                                 dot_scale=dk ** -0.5, floor=DENOMINATOR_FLOOR)
         if KG.pays(o, self.w_o):
             return KG.gemv(o, self.w_o, torch.empty((T, self.hidden), dtype=torch.float32, device=dev))
-        return linear(o, self.w_o, out_dtype=torch.float32)
+        return linear(o, self.w_o, out_dtype=torch.float32, status=ctx.status)
 
 
 register_mixer("matrix_memory", MatrixMemoryMixer)

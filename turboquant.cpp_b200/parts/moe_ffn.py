@@ -299,12 +299,12 @@ class MoEFeedForward(FeedForward):
                     # unpacked weights (float32 runs, sizes the tensor-core kernel does not take) and more rows than
                     # one pass of the exact weight-stream kernel holds: the shared expert is a dense feed-forward, and
                     # the library's products serve it as they serve the dense layers
-                    gu = linear(xn, self.ws13[0], out_dtype=torch.float32)
+                    gu = linear(xn, self.ws13[0], out_dtype=torch.float32, status=ctx.status)
                     if self.gated:
                         KE.glu_mul(gu, hs, self.shared_glu)
                     else:
                         KE.map_elements(gu, hs, self.map)
-                    y_shared = linear(hs, self.ws2[0], out_dtype=torch.float32)
+                    y_shared = linear(hs, self.ws2[0], out_dtype=torch.float32, status=ctx.status)
                     return
                 self._product(xn, self.ws13, hs, None, True, stile, ctx.status, glu=self.shared_glu)
                 splits = 1

@@ -105,7 +105,7 @@ class NormedAttentionMixer(Mixer):
     def forward(self, xn: torch.Tensor, ctx: StepContext, cache: LayerCache, projected: Optional[torch.Tensor] = None) -> torch.Tensor:
         """projected: float32 rows of a wider product that begin with this mixer's projection."""
         T, act, dev = xn.shape[0], ctx.act_dtype, xn.device
-        rows = projected if projected is not None else linear(xn, self.w_in, out_dtype=torch.float32)
+        rows = projected if projected is not None else linear(xn, self.w_in, out_dtype=torch.float32, status=ctx.status)
         q = torch.empty((T, self.heads, self.dim), dtype=act, device=dev)
         pe = self.position if self.position is not None and self.position.dims else None
         KB.kv_write_rot(rows, q, cache.kv if cache.writes else None, pe.freq if pe is not None else None,
@@ -117,7 +117,7 @@ class NormedAttentionMixer(Mixer):
                             sink=self.sink, runs_min=self.RUNS_MIN)
         if self.has_gate:
             KB.elements_gate(o, rows, self.gate_off, o)
-        return _output(o, self.w_o, self.hidden)
+        return _output(o, self.w_o, self.hidden, ctx)
 
 
 register_mixer("normed_attention", NormedAttentionMixer)

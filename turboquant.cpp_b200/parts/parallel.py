@@ -83,7 +83,7 @@ class ParallelMixer(Mixer):
         branches' norms and their weighted sum in its own pass."""
         left_in, right_in = {}, {}
         if self.w_in is not None:
-            proj = linear(xn, self.w_in, out_dtype=torch.float32)
+            proj = linear(xn, self.w_in, out_dtype=torch.float32, status=ctx.status)
             left_in, right_in = {"projected": proj}, {"projected": proj, "offset": self.left.input_weight().shape[0]}
         runs_apart = xn.numel() >= self.SIDE_MIN_ELEMENTS and not (self.left.runs_alone or self.right.runs_alone)
         if self.SIDE_BY_SIDE and (ctx.max_q_len == 1 or runs_apart):

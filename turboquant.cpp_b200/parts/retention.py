@@ -92,7 +92,7 @@ class RetentionMixer(Mixer):
                 offset: int = 0) -> torch.Tensor:
         """projected: float32 rows of a wider product that hold this mixer's [q | k | v | g] from column `offset`."""
         T, dev = xn.shape[0], xn.device
-        proj = projected if projected is not None else linear(xn, self.w_in, out_dtype=torch.float32)
+        proj = projected if projected is not None else linear(xn, self.w_in, out_dtype=torch.float32, status=ctx.status)
         S = cache.state.unflatten(1, (self.heads, self.vdim, self.dim))          # column by column
         pe = self.position
         if ctx.max_q_len == 1 and ctx.n_seqs == T and T * self.heads >= self.STEP_MIN_BLOCKS:
@@ -102,7 +102,7 @@ class RetentionMixer(Mixer):
                               pe.freq if pe is not None and pe.dims else None, pe.dims if pe is not None else 0,
                               pe is not None and pe.halves, self.k_scale, ctx.positions, S, ctx.slots, self.decay, g,
                               self.heads, self.dim, self.vdim, self.eps)
-            return linear(g, self.w_o, out_dtype=torch.float32)
+            return linear(g, self.w_o, out_dtype=torch.float32, status=ctx.status)
         xbc = torch.empty((T, self.inner + 2 * self.qk), dtype=torch.float32, device=dev)
         KS.retention_prepare(proj, offset, offset + self.qk, offset + 2 * self.qk, xbc,
                              pe.freq if pe is not None and pe.dims else None, pe.dims if pe is not None else 0,
@@ -126,7 +126,7 @@ class RetentionMixer(Mixer):
             scan(starts, y)
         g = torch.empty((T, self.inner), dtype=ctx.act_dtype, device=dev)
         KS.gated_group_norm(y, proj, offset + 2 * self.qk + self.inner, None, self.heads, self.eps, g, gate_after=True)
-        return linear(g, self.w_o, out_dtype=torch.float32)
+        return linear(g, self.w_o, out_dtype=torch.float32, status=ctx.status)
 
 
 register_mixer("retention", RetentionMixer)

@@ -74,7 +74,7 @@ class Mamba2Mixer(Mixer):
         st = cache.state                                                       # [max_slots, kept | S]
         kept = st[:, :self.kept_size].unflatten(1, (self.taps - 1, self.channels))
         S = st[:, self.kept_size:].unflatten(1, (self.heads, self.vdim, self.n_state))     # column by column
-        proj = linear(xn, self.w_in, out_dtype=torch.float32)                  # [T, z | x | B | C | dt]
+        proj = linear(xn, self.w_in, out_dtype=torch.float32, status=ctx.status)                  # [T, z | x | B | C | dt]
         xbc = torch.empty((T, self.channels), dtype=torch.float32, device=dev)
         KS.conv_silu(proj, self.inner, self.w_conv, self.b_conv, kept, xbc, ctx.seq_of_token, ctx.cu_seqlens, ctx.slots)
         y = torch.empty((T, self.inner), dtype=torch.float32, device=dev)
@@ -82,7 +82,7 @@ class Mamba2Mixer(Mixer):
                     self.heads, self.vdim, self.n_state, self.groups, ctx.cu_seqlens, ctx.slots)
         g = torch.empty((T, self.inner), dtype=ctx.act_dtype, device=dev)
         KS.gated_group_norm(y, proj, 0, self.w_norm, self.norm_groups, self.eps, g)
-        return linear(g, self.w_o, out_dtype=torch.float32)
+        return linear(g, self.w_o, out_dtype=torch.float32, status=ctx.status)
 
 
 register_mixer("mamba2", Mamba2Mixer)

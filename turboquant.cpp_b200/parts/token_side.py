@@ -55,10 +55,10 @@ class TokenSideInput(Part):
         T, dev = x.shape[0], x.device
         exact = ctx.act_dtype == torch.float32
         h = x if exact else (cast if cast is not None else K.map_elements(x, torch.empty(x.shape, dtype=ctx.act_dtype, device=dev)))
-        z = linear(h, self.w_gate, out_dtype=torch.float32)
+        z = linear(h, self.w_gate, out_dtype=torch.float32, status=ctx.status)
         g = torch.empty((T, self.dim), dtype=ctx.act_dtype, device=dev)
         K.glu_table_rows(z, ctx.tokens, self.table, self.col0, g, self.glu)
-        y = linear(g, self.w_proj, out_dtype=torch.float32)
+        y = linear(g, self.w_proj, out_dtype=torch.float32, status=ctx.status)
         w = getattr(then, "weight", None)
         if w is not None and w.dtype == self.w_norm.dtype:
             out = torch.empty(x.shape, dtype=ctx.act_dtype, device=dev)
