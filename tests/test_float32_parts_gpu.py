@@ -1,8 +1,9 @@
-"""float32 products on the tensor cores (operands as three bfloat16 values) against float64: around the tiles'
+"""float32 products and float32 prompt attention on the tensor cores (operands as three bfloat16 values) against float64: around the tiles'
 edges (16, 32, 64, 128, 256), with weights that are bfloat16 values and that are not, with infinities and NaN, and the rule that
 chooses the product."""
 import math
 
+import numpy as np
 import pytest
 import torch
 
@@ -58,3 +59,58 @@ def test_which_products_it_takes():
         assert not KF.pays(a, b)
         torch.testing.assert_close(linear(a, b, status=status), torch.mm(a, b.t()), rtol=0, atol=0)
     assert int(status) == 0
+
+
+CASES = [  # H, G, head size, page, runs, held, window
+    (4, 2, 128, 64, [1, 31, 32, 33, 64, 65], [0, 0, 31, 40, 0, 7], 0),
+    (6, 3, 64, 64, [127, 300], [0, 100], 0),
+    (4, 1, 64, 48, [200, 20], [13, 0], 70),              # a tile of keys lies in two pages
+    (2, 2, 128, 16, [129, 65], [0, 500], 33),
+    (16, 16, 128, 64, [700], [0], 0),
+]
+
+
+@pytest.mark.parametrize("case", range(len(CASES)))
+@pytest.mark.parametrize("spread", [1.0, 6.0])
+def test_attention_f32(case, spread):
+    from test_attention_prefill_gpu import attend
+    from turboquant_cpp_b200.kernels import attention as KA
+    H, G, hd, page, runs, held, window = CASES[case]
+    g = torch.Generator(device=DEV).manual_seed(case)
+    r = lambda *s: torch.randn(s, generator=g, device=DEV)
+    i32 = lambda a: torch.tensor(np.asarray(a), dtype=torch.int32, device=DEV)
+    T, cu = sum(runs), np.concatenate([[0], np.cumsum(runs)])
+    counts = [-(-(a + b) // page) for a, b in zip(runs, held)]
+    order, table, at = np.random.RandomState(0).permutation(sum(counts)), np.full((len(runs), max(counts)), -1), 0
+    cache = torch.full((sum(counts), 2, G, page, hd), 1e30, device=DEV)         # what lies behind a sequence's end
+    q, rows = spread * r(T, H, hd), []
+    for i, c in enumerate(counts):
+        table[i, :c] = order[at:at + c]
+        at += c
+        n = runs[i] + held[i]
+        rows.append((r(n, G, hd), r(n, G, hd)))
+        pos = torch.arange(n, device=DEV)
+        where = i32(table[i]).long()[pos // page]
+        cache[where, 0, :, pos % page], cache[where, 1, :, pos % page] = rows[i]
+    out = torch.full((T, H * hd), math.nan, device=DEV)
+    run = lambda: KA.attention_tiled(q, cache, i32(cu), i32(held), i32(table), page, window, hd ** -0.5, out, len(runs), H, G, hd)
+    run()
+    for i in range(len(runs)):
+        mine = slice(cu[i], cu[i + 1])
+        want, mag = attend(q[mine].double(), rows[i][0].double(), rows[i][1].double(), held[i], hd ** -0.5, window, 0, 0, 0.0, None, None)
+        # a score is off by about its products' 2^-21 and its sums' 2^-20, of the size of |q| |k| / sqrt(hd); so is a weight, relatively
+        size = q[mine].double().norm(dim=2).max() * rows[i][0].double().norm(dim=2).max() * hd ** -0.5
+        assert bool(((out[mine].view(-1, H, hd).double() - want).abs() <= mag * (2.0 ** -20 * size + 2.0 ** -18)).all())
+    # a key of -inf has no weight; a value of inf shows in the rows that see it, a NaN too, and in no others
+    first = int(table[0, 0])
+    cache[first, 0, 0, 0] = 0.0
+    cache[first, 0, 0, 0, 1] = -math.inf
+    q[..., 1] = q[..., 1].abs() + 0.1
+    run()
+    assert bool(out[cu[0] + 1:cu[1]].isfinite().all()) if held[0] == 0 else True
+    cache[int(table[-1, 0]), 1, 0, 0, 0] = math.inf
+    run()
+    sees = (torch.arange(runs[-1], device=DEV) + held[-1] < window) if window else torch.ones(runs[-1], dtype=torch.bool, device=DEV)
+    got = out[cu[-2]:].view(-1, H, hd)[:, :H // G, 0]
+    if len(runs) > 1:
+        assert bool(((got == math.inf) == sees[:, None]).all()) and bool(out[:cu[1]].isfinite().logical_not().sum() <= H * hd)

@@ -171,18 +171,29 @@ def attention_split(q: torch.Tensor, cache_layer: torch.Tensor, positions: torch
     return out
 
 
+F32_HEAD_DIMS = (64, 128)
+
+
 def attention_tiled(q: torch.Tensor, cache_layer: torch.Tensor, cu_seqlens: torch.Tensor, seq_start: torch.Tensor,
                     page_table: torch.Tensor, page_size: int, window: int, scale: float, out: torch.Tensor,
                     n_seqs: int, n_heads: int, n_kv_heads: int, head_dim: int) -> torch.Tensor:
-    """Causal attention of whole runs of new tokens in exact fp32 arithmetic on CUDA cores: 32 queries share every
-    tile of keys and values through shared memory.  For float32 runs and for head sizes the tensor-core prompt
-    kernel does not take.  Rows as in attention_prefill."""
+    """Causal attention of whole runs of new tokens in float32 arithmetic, queries sharing every tile of keys and values through shared
+    memory.  For float32 runs and for head sizes the bfloat16 prompt kernel does not take.  Rows as in attention_prefill.
+    float32 heads of 64 and 128 go to the tensor cores in three bfloat16 parts (csrc/attention_f32.cu), everything else to the fp32
+    units."""
     T = q.shape[0]
     want_int32(cu_seqlens, "cu_seqlens")
     want_int32(seq_start, "seq_start")
     want_int32(page_table, "page table")
     if head_dim % 4:
         raise KernelError(f"attention_tiled: head size {head_dim} must be a multiple of 4")
+    if (q.dtype == torch.float32 and cache_layer.dtype == q.dtype and head_dim in F32_HEAD_DIMS
+            and q.data_ptr() % 16 == 0 and cache_layer.data_ptr() % 16 == 0 and out.data_ptr() % 8 == 0):
+        lib = load_kernel("attention_f32")
+        check("attention_f32", lib.tq_attention_f32(
+            ptr(q), ptr(cache_layer), ptr(cu_seqlens), ptr(seq_start), ptr(page_table), c_int(page_table.shape[1]), c_int(page_size), c_int(window),
+            c_float(scale), ptr(out), c_int(T), c_int(n_seqs), c_int(n_heads), c_int(n_kv_heads), c_int(head_dim), c_int(cache_layer.shape[0]), stream()))
+        return out
     lib = load_kernel(_LIB)
     check(_LIB, lib.tq_attention_tiled(ptr(q), ptr(cache_layer), c_int(code(q.dtype)), ptr(cu_seqlens), ptr(seq_start),
                                        ptr(page_table), c_int(page_table.shape[1]), c_int(page_size), c_int(window),

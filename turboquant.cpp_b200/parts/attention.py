@@ -68,7 +68,7 @@ class AttentionMixer(Mixer):
         if getattr(self, "run_dtype", None) == torch.bfloat16 and self.head_dim in (64, 128):
             names.append("attention_prefill")
         if getattr(self, "run_dtype", None) == torch.float32:
-            names.append("gemm_f32")
+            names += ["gemm_f32"] + (["attention_f32"] if self.head_dim in KA.F32_HEAD_DIMS else [])
         return names
 
     def cache_need(self) -> KVNeed:
