@@ -125,15 +125,27 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr) {
 __device__ __forceinline__ uint32_t umma_idesc(int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
 }
-__device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+// One lane of the warp, the same each time.  The products and their commits are issued under its predicate by code the whole warp
+// runs, so that their operands stay in uniform registers: from a one-lane branch each of them costs over a hundred cycles of
+// moving its descriptors there, more than a product of some hundred token rows.
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+    return e;
 }
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+__device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate, uint32_t elected) {
+    asm volatile(
+        "{\n\t.reg .pred p, e;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 e, %5, 0;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(elected) : "memory");
+}
+__device__ __forceinline__ void umma_commit(uint32_t bar, uint32_t elected) {
+    asm volatile(
+        "{\n\t.reg .pred e;\n\t"
+        "setp.ne.b32 e, %1, 0;\n\t"
+        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar), "r"(elected) : "memory");
 }
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
     asm volatile(
@@ -173,17 +185,21 @@ __device__ __forceinline__ void tma_load_block_pair(uint32_t dst, const CUtensor
         ::"r"(dst), "l"((uint64_t)map), "r"(cluster_bar), "r"(0), "r"(0), "r"(kb), "r"(tile), "l"(policy) : "memory");
 }
 // one product of the pair: M = 256 (128 weight rows from each CTA), the token rows half from each CTA
-__device__ __forceinline__ void umma_pair(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void umma_pair(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate, uint32_t elected) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p, e;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+        "setp.ne.b32 e, %5, 0;\n\t"
+        "@e tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(elected) : "memory");
 }
 // arrives on the barrier at this address in both CTAs of the pair once the products issued so far are done
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-                 ::"r"(bar), "h"((uint16_t)3) : "memory");
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar, uint32_t elected) {
+    asm volatile(
+        "{\n\t.reg .pred e;\n\t"
+        "setp.ne.b32 e, %2, 0;\n\t"
+        "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
+        ::"r"(bar), "h"((uint16_t)3), "r"(elected) : "memory");
 }
 
 // silu(gate) * up.  A bfloat16 result keeps 8 bits, so the fast exponential and division (a few units in
@@ -497,7 +513,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer (the pair's first CTA issues for both) ----------------
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
+            const uint32_t elected = elect_one(), tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
+            const uint64_t a_desc = umma_desc(a_tile(0)), b_desc = umma_desc(b_tile(0));          // descriptors count in 16 bytes
+            auto wait = [&](uint32_t bar, uint32_t parity) { return (bool)__all_sync(0xffffffffu, mbar_wait(bar, parity, &s_abort)); };
             int sa = 0, sb = 0, it = 0;      // weight slot (and barrier) and token slot of the next block
             uint32_t phase = 0;
             bool ok = true;
@@ -515,28 +534,29 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 // N of the products: this tile's rows; pairs: M = 256, 128 weight rows from each CTA
                 const uint32_t idesc = umma_idesc((t.count + 15) & ~15) + (PAIR ? ((uint32_t)(BM >> 4) << 24) : 0u);
                 const int b = it & 1;
-                const uint32_t acc = tmem_base + (uint32_t)(b * T::ACC_COLS);
+                const uint32_t acc = tmem + (uint32_t)(b * T::ACC_COLS);
                 // the epilogue must have drained this accumulator (two tiles ago)
-                if (it >= 2) ok = mbar_wait(acc_empty(b), (uint32_t)((it >> 1) - 1) & 1u, &s_abort);
+                if (it >= 2) ok = wait(acc_empty(b), (uint32_t)((it >> 1) - 1) & 1u);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 for (int kb = kb0; kb < kb1; ++kb) {
-                    ok = mbar_wait(full_bar(sa), phase, &s_abort);
+                    ok = wait(full_bar(sa), phase);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint64_t ad = a_desc + (uint64_t)(sa * (T::A_BYTES / 16)), bd = b_desc + (uint64_t)(sb * (T::B_BYTES / 16));
 #pragma unroll
                     for (int k = 0; k < BK / UMMA_K; ++k) {
                         const uint32_t accum = (kb > kb0 || k > 0) ? 1u : 0u;
-                        const uint64_t ad = umma_desc(a_tile(sa) + k * UMMA_K * 2), bd = umma_desc(b_tile(sb) + k * UMMA_K * 2);
-                        if (PAIR) umma_pair(acc, ad, bd, idesc, accum); else umma(acc, ad, bd, idesc, accum);
+                        if (PAIR) umma_pair(acc, ad + k * (UMMA_K * 2 / 16), bd + k * (UMMA_K * 2 / 16), idesc, accum, elected);
+                        else umma(acc, ad + k * (UMMA_K * 2 / 16), bd + k * (UMMA_K * 2 / 16), idesc, accum, elected);
                     }
                     // the slots are free (in both CTAs) once these MMAs have read them
-                    if (PAIR) umma_commit_pair(done_bar(sa)); else umma_commit(done_bar(sa));
+                    if (PAIR) umma_commit_pair(done_bar(sa), elected); else umma_commit(done_bar(sa), elected);
                     if (++sa == SA) { sa = 0; phase ^= 1u; }
                     if (++sb == SB) sb = 0;
                 }
                 // this tile's accumulator is complete once all MMAs are done
-                if (ok) { if (PAIR) umma_commit_pair(acc_full(b)); else umma_commit(acc_full(b)); }
+                if (ok) { if (PAIR) umma_commit_pair(acc_full(b), elected); else umma_commit(acc_full(b), elected); }
             }
         }
     } else {
