@@ -18,7 +18,7 @@ def inputs(T, N, K, exact_weights, seed=0):
 
 
 def bound(x, w):
-    """What a result may be off by, of the sum of |x| |w|: products left out 2^-21; the tensor cores cut bits off (2^-23 each) at 4
+    """What a result may be off by, of the sum of |x| |w|: products left out 2^-26 (2^-21 if the parts were cut, not rounded); the tensor cores cut bits off (2^-23 each) at 4
     additions of 16 products and inside each, 8 in all; K / 64 + 1 rounded additions of 2^-24."""
     return (x.double().abs() @ w.double().abs().t()) * (2.0 ** -21 + 8 * 2.0 ** -23 + (x.shape[1] / 64 + 1) * 2.0 ** -24)
 
@@ -34,7 +34,7 @@ def test_gemm_f32(T, N, K, tokens, exact_weights):
     want = x.double() @ w.double().t()
     assert bool(((y.double() - want).abs() <= bound(x, w)).all())
     library = torch.mm(x, w.t())
-    if K >= MIN_K:                        # as accurate as a float32 sum wherever it is chosen; a sum of 32 has fewer roundings than this has parts
+    if K >= MIN_K:                        # as accurate as a float32 sum wherever it is chosen; sums of fewer elements have as few roundings as this
         assert (y.double() - want).norm() <= 1.05 * (library.double() - want).norm() + 1e-12
     # rows of a wider tensor, infinities and NaN: where they are, and nowhere else
     wide = torch.zeros((T, K + 8), device=DEV)

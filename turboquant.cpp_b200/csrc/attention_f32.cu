@@ -6,7 +6,7 @@
 // other head sizes, csrc/attention.cu, takes 4.6 times that); as six bfloat16 products they are 6,600 of mma.sync (960 multiply-adds a
 // cycle and SM measured), whose operands a warp reads once for 16 rows.
 // 16 heads of 128, one prompt: 82 us for 700 tokens (287 before), 19 for 100 (47), 420 for 2,048 (1,662); errors against 64 bits
-// 1.9e-7 (3.6e-7), queries of spread 5 3.4e-7 (1.05e-6).  What bounds it: the tensor cores are active 49 % of the time, the rest is a warp's
+// 1.5e-7 (3.6e-7), queries of spread 5 3.1e-7 (1.05e-6).  What bounds it: the tensor cores are active 49 % of the time, the rest is a warp's
 // own chain of splitting, products and exponentials, two warps a scheduler (their sums take 255 registers).
 //   A CTA takes 64 consecutive new tokens of one sequence and one query head, a warp of either half of it 16 of them.  Queries, scaled,
 //   lie in shared memory in three parts.  The halves take every other 32 keys each, with sums of their own that are put together
@@ -24,46 +24,6 @@ namespace {
 
 constexpr int BQ = 64, BKEYS = 32, WARPS = 4, HALVES = 2, THREADS = 32 * WARPS * HALVES;
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void ldm4(uint32_t (&r)[4], uint32_t addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
-}
-__device__ __forceinline__ void ldm4t(uint32_t (&r)[4], uint32_t addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
-}
-__device__ __forceinline__ void mma_more(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
-// the first product of a sum
-__device__ __forceinline__ void mma0(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
-                 : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
-}
-template <bool FIRST> __device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    if (FIRST) mma0(c, a, b0, b1); else mma_more(c, a, b0, b1);
-}
-// six products of 16 rows and four groups of eight columns: h h' to `big`, the rest to `small`; b[part][two groups].  A sum is
-// met again after four products, as many as its latency.
-template <bool FIRST_BIG, bool FIRST>
-__device__ __forceinline__ void six(float (&big)[4][4], float (&small)[4][4], const uint32_t (&ah)[4], const uint32_t (&am)[4], const uint32_t (&al)[4],
-                                    const uint32_t (&b)[3][2][4]) {
-#define TQ_ALL(FIRST_, to, a, part)                                                                                       \
-    _Pragma("unroll") for (int u = 0; u < 4; ++u) mma<FIRST_>(to[u], a, b[part][u >> 1][2 * (u & 1)], b[part][u >> 1][2 * (u & 1) + 1]);
-    TQ_ALL(FIRST_BIG, big, ah, 0)
-    TQ_ALL(FIRST, small, al, 0)
-    TQ_ALL(false, small, am, 1)
-    TQ_ALL(false, small, ah, 2)
-    TQ_ALL(false, small, am, 0)
-    TQ_ALL(false, small, ah, 1)
-#undef TQ_ALL
-}
-
-// Rows of HD bfloat16 in shared memory, their 16-byte pieces shuffled by the row's lowest three bits: eight neighbouring rows' pieces
-// of one column, and a row's pieces, lie in different banks.
-template <int HD> __device__ __forceinline__ uint32_t piece(int row, int c) { return (uint32_t)(row * (HD * 2) + ((c ^ (row & 7)) << 4)); }
-
 template <int HD>
 struct Cfg {
     static constexpr int Q_PART = BQ * HD * 2, K_PART = BKEYS * HD * 2;
@@ -71,16 +31,6 @@ struct Cfg {
     static constexpr int SMEM_BYTES = 3 * Q_PART + HALVES * HALF;
     static_assert(BQ * (HD + 4) * 4 <= HALF, "the second half's sums take the place of its keys");
 };
-
-// one row of HD floats, four a lane, scaled and split into the row of three parts
-template <int HD>
-__device__ __forceinline__ void put_row(uint32_t at, int part, int row, int d, float4 v) {
-    const TqSplit4 s = tq_split4(v);
-    const uint32_t a = at + piece<HD>(row, d >> 3) + (d & 4) * 2;
-    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(a), "r"(s.h.x), "r"(s.h.y) : "memory");
-    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(a + part), "r"(s.m.x), "r"(s.m.y) : "memory");
-    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(a + 2 * part), "r"(s.l.x), "r"(s.l.y) : "memory");
-}
 
 __device__ __forceinline__ void half_sync(int half) { asm volatile("bar.sync %0, %1;" ::"r"(half + 1), "n"(32 * WARPS) : "memory"); }
 // 16 bytes, or as many zeros
@@ -120,7 +70,7 @@ attention_f32_kernel(const float* __restrict__ q, const float* __restrict__ cach
         const int page = TQ_CHECKED(table[TQ_CHECKED(p / page_size, table_stride, TQ_IDX_TABLE_COLUMN)], n_pages, TQ_IDX_PAGE);
         return cache + (((size_t)page * 2 * nkv + g) * page_size + p % page_size) * HD;
     };
-    const uint32_t sq = smem_u32(smem), sk = sq + 3 * C::Q_PART + half * C::HALF, sv = sk + 3 * C::K_PART;
+    const uint32_t sq = tq_smem_u32(smem), sk = sq + 3 * C::Q_PART + half * C::HALF, sv = sk + 3 * C::K_PART;
     const uint32_t raw = sv + 3 * C::K_PART + (threadIdx.x & (32 * WARPS - 1)) * 16;
     constexpr int LANES = HD / 4, RPW = 32 / LANES;           // lanes of a row, rows a warp brings at a time
     const int sub = lane / LANES, d4 = lane % LANES * 4;
@@ -128,7 +78,7 @@ attention_f32_kernel(const float* __restrict__ q, const float* __restrict__ cach
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (r < rows) v = *reinterpret_cast<const float4*>(q + ((size_t)(t_first + r) * nh + h) * HD + d4);
         v.x *= scale; v.y *= scale; v.z *= scale; v.w *= scale;
-        put_row<HD>(sq, C::Q_PART, r, d4, v);
+        tq_put4<HD>(sq, C::Q_PART, r, d4, v);
     }
     // the thread's rows: two, of the accumulators' layout (lane / 4 and 8 below)
     const int row_a = warp * 16 + (lane >> 2), pos_a = pos0 + row_a, pos_b = pos_a + 8;
@@ -173,7 +123,7 @@ attention_f32_kernel(const float* __restrict__ q, const float* __restrict__ cach
         for (int i = 0; i < 2 * EACH; ++i) {
             float4 v;
             asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(raw + i * (32 * WARPS * 16)) : "memory");
-            put_row<HD>(i < EACH ? sk : sv, C::K_PART, (i % EACH * WARPS + warp) * RPW + sub, d4, v);
+            tq_put4<HD>(i < EACH ? sk : sv, C::K_PART, (i % EACH * WARPS + warp) * RPW + sub, d4, v);
         }
         bring(k0 + HALVES * BKEYS);
         half_sync(half);
@@ -189,19 +139,16 @@ attention_f32_kernel(const float* __restrict__ q, const float* __restrict__ cach
 #pragma unroll
                         for (int e = 0; e < 4; ++e) first[j][e] = s[j][e];
                 }
-                uint32_t ah[4], am[4], al[4];
-                const uint32_t aq = sq + piece<HD>(a_row, 2 * k + a_c);
-                ldm4(ah, aq);
-                ldm4(am, aq + C::Q_PART);
-                ldm4(al, aq + 2 * C::Q_PART);
-                uint32_t b[3][2][4];
+                uint32_t a[3][4], b[3][2][4];
 #pragma unroll
-                for (int part = 0; part < 3; ++part)
+                for (int part = 0; part < 3; ++part) {
+                    tq_ldm4(a[part], sq + part * C::Q_PART + tq_piece<HD>(a_row, 2 * k + a_c));
 #pragma unroll
-                    for (int jp = 0; jp < 2; ++jp) ldm4(b[part][jp], sk + part * C::K_PART + piece<HD>(16 * jp + b_row, 2 * k + b_c));
-                if (k == 0) six<true, true>(s, rest, ah, am, al, b);
-                else if (k == 4) six<true, false>(s, rest, ah, am, al, b);
-                else six<false, false>(s, rest, ah, am, al, b);
+                    for (int jp = 0; jp < 2; ++jp) tq_ldm4(b[part][jp], sk + part * C::K_PART + tq_piece<HD>(16 * jp + b_row, 2 * k + b_c));
+                }
+                if (k == 0) tq_six<4, true, true>(s, rest, a, b);
+                else if (k == 4) tq_six<4, true, false>(s, rest, a, b);
+                else tq_six<4, false, false>(s, rest, a, b);
             }
 #pragma unroll
             for (int j = 0; j < 4; ++j)
@@ -232,14 +179,15 @@ attention_f32_kernel(const float* __restrict__ q, const float* __restrict__ cach
             l[r] *= corr[r];
             m[r] = top[r];
         }
-        uint32_t ph[2][4], pm[2][4], pl[2][4];                                   // weights as left operands, 16 keys each
+        uint32_t p[2][3][4];                                                     // weights as left operands, 16 keys each
 #pragma unroll
         for (int j = 0; j < 4; ++j)
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
                 const float e0 = top[r] == -INFINITY ? 0.f : expf(s[j][2 * r] - top[r]), e1 = top[r] == -INFINITY ? 0.f : expf(s[j][2 * r + 1] - top[r]);
                 l[r] += e0 + e1;
-                tq_split2(e0, e1, ph[j >> 1][2 * (j & 1) + r], pm[j >> 1][2 * (j & 1) + r], pl[j >> 1][2 * (j & 1) + r]);
+                const int at = 2 * (j & 1) + r;
+                tq_split2(e0, e1, p[j >> 1][0][at], p[j >> 1][1][at], p[j >> 1][2][at]);
             }
 #pragma unroll
         for (int j4 = 0; j4 < HD / 32; ++j4) {                                   // 32 elements of the output at a time
@@ -250,9 +198,9 @@ attention_f32_kernel(const float* __restrict__ q, const float* __restrict__ cach
 #pragma unroll
                 for (int part = 0; part < 3; ++part)
 #pragma unroll
-                    for (int jp = 0; jp < 2; ++jp) ldm4t(b[part][jp], sv + part * C::K_PART + piece<HD>(16 * k + v_row, 4 * j4 + 2 * jp + v_c));
-                if (k == 0) six<true, true>(t, rest, ph[k], pm[k], pl[k], b);
-                else six<false, false>(t, rest, ph[k], pm[k], pl[k], b);
+                    for (int jp = 0; jp < 2; ++jp) tq_ldm4t(b[part][jp], sv + part * C::K_PART + tq_piece<HD>(16 * k + v_row, 4 * j4 + 2 * jp + v_c));
+                if (k == 0) tq_six<4, true, true>(t, rest, p[k], b);
+                else tq_six<4, false, false>(t, rest, p[k], b);
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u)

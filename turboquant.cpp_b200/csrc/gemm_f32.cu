@@ -10,7 +10,7 @@
 //   warps 8..15   add the accumulator of the largest products, h h', to sums in their registers every two blocks and write the result
 // The tensor cores' own sums cut bits off at every addition, so a chain of products over all of K is off by more than a
 // float32 sum is (K 2,048: 2.2e-6 of the result; the library's sum 8.1e-7); sums of 64 elements added up in rounded float32 are
-// off by less (2.0e-7, with bfloat16 weights 1.3e-7).  The smaller products, 2^-8 of the result and less, stay in one accumulator
+// off by less (1.3e-7).  The smaller products, 2^-8 of the result and less, stay in one accumulator
 // for all of K, and the other accumulator is read in the time they take: it costs nothing.
 // 700 tokens, K 2,048: 79 us for 6,144 rows (65 with bfloat16 weights; the library's fp32 product 309), 47 for 2,048 (145).  What bounds it is
 // the splitting, some 1,200 cycles a block of 32 elements for 720 (three products) or 1,440 (six) of the tensor cores at 240 tokens.

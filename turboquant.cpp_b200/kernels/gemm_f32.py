@@ -17,8 +17,7 @@ MIN_TOKENS = 9
 # tokens x 2,048, 41 / 42 at 96, 42 / 57 at 192, 47 / 145 at 700; 41 / 41 at 17 x 6,144, 42 / 54 at 33, 79 / 309 at 700; 41 / 38 at 128 x
 # 1,024, 41 / 42 at 192.  K 512: 15 / 13 at 64 x 2,048, 15 / 19 at 192.  K 5,632: 101 / 95 at 64 x 2,048, 102 / 105 at 128.
 MIN_RESULTS = 200_000
-# Below this a plain sum has so few roundings that the products left out here show (K 32: 3.1e-5 against 2.8e-5 in all, K 64: 1.1e-7 against
-# 1.4e-7 of the result).
+# Below this a product is a few launches' time either way.
 MIN_K = 64
 
 
