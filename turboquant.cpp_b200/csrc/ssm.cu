@@ -1292,6 +1292,65 @@ delta_prepare_kernel(const float* __restrict__ xqkv, int C, int q_off, int k_off
     }
 }
 
+// The same with one decay per head, keys of up to 128 elements in whole 16 bytes: four elements a lane, read once, the two norms' sums side
+// by side, and a lane per head for the decays and betas (a warp each otherwise).  2,048 tokens of 16 heads of 128: 23 us before, 12.5
+// now for 67 MB (10 at the copy rate).
+__global__ void __launch_bounds__(128)
+delta_prepare_vec_kernel(const float* __restrict__ xqkv, int C, int q_off, int k_off, const float* __restrict__ proj, int P, int b_off,
+                         const float* __restrict__ a_raw, int A, int a_off, const float* __restrict__ dt_bias, const float* __restrict__ a_log,
+                         float* __restrict__ rows, int R, int heads, int kv_heads, int dk, float unit_eps, float q_scale) {
+    tq_grid_wait();                    // everything below may read what the previous kernel wrote
+    tq_grid_launch_dependents();       // the next kernel's CTAs may move in as SMs free up
+    const int lane = threadIdx.x & 31, item = blockIdx.y * 4 + (threadIdx.x >> 5);
+    const size_t t = blockIdx.x;
+    float* out = rows + t * R;
+    const int g_at = 2 * kv_heads * dk, kq_at = g_at + heads, b_at = kq_at + kv_heads;
+    if (item < kv_heads) {
+        const int e = 4 * lane;
+        float4 k = make_float4(0.f, 0.f, 0.f, 0.f), q = k;
+        if (e < dk) {
+            k = *reinterpret_cast<const float4*>(xqkv + t * C + k_off + (size_t)item * dk + e);
+            q = *reinterpret_cast<const float4*>(xqkv + t * C + q_off + (size_t)item * dk + e);
+        }
+        float ssk = k.x * k.x + k.y * k.y + k.z * k.z + k.w * k.w, ssq = q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            ssk += __shfl_xor_sync(0xffffffffu, ssk, o);
+            ssq += __shfl_xor_sync(0xffffffffu, ssq, o);
+        }
+        const float rk = 1.0f / sqrtf(ssk + unit_eps), rq = q_scale / sqrtf(ssq + unit_eps);
+        k.x *= rk; k.y *= rk; k.z *= rk; k.w *= rk;
+        q.x *= rq; q.y *= rq; q.z *= rq; q.w *= rq;
+        if (e < dk) {
+            *reinterpret_cast<float4*>(out + (size_t)item * dk + e) = k;
+            *reinterpret_cast<float4*>(out + (size_t)(kv_heads + item) * dk + e) = q;
+        }
+        // k.q of the vectors as they are written
+        const float kq = tq_warp_sum(k.x * q.x + k.y * q.y + k.z * q.z + k.w * q.w);
+        if (lane == 0) out[kq_at + item] = kq;
+    } else {
+        const int h = (item - kv_heads) * 32 + lane;
+        if (h < heads) {
+            const float z = a_raw[t * A + a_off + h] + dt_bias[h];
+            const float sp = z > 20.f ? z : log1pf(expf(z));
+            out[g_at + h] = expf(-expf(a_log[h]) * sp);
+            out[b_at + h] = 1.0f / (1.0f + expf(-proj[t * P + b_off + h]));
+        }
+    }
+}
+
+// Which of the two: the second where the rows and offsets are whole 16 bytes.
+static void launch_delta_prepare(const float* xqkv, int C, int q_off, int k_off, const float* proj, int P, int b_off, const float* a_raw, int A,
+                                 int a_off, int dper, const float* dt_bias, const float* a_log, float* rows, int R, int T_, int heads,
+                                 int kv_heads, int dk, float unit_eps, float q_scale, cudaStream_t stream) {
+    if (dper == 1 && dk % 4 == 0 && dk <= 128 && C % 4 == 0 && q_off % 4 == 0 && k_off % 4 == 0 && ((uintptr_t)xqkv & 15) == 0 && ((uintptr_t)rows & 15) == 0)
+        tq_launch(dim3(T_, (kv_heads + (heads + 31) / 32 + 3) / 4), 128, 0, stream)(delta_prepare_vec_kernel, xqkv, C, q_off, k_off, proj, P, b_off, a_raw,
+            A, a_off, dt_bias, a_log, rows, R, heads, kv_heads, dk, unit_eps, q_scale);
+    else
+        tq_launch(dim3(T_, (kv_heads + heads + 3) / 4), 128, 0, stream)(delta_prepare_kernel, xqkv, C, q_off, k_off, proj, P, b_off, a_raw, A,
+            a_off, dper, dt_bias, a_log, rows, R, T_, heads, kv_heads, dk, unit_eps, q_scale);
+}
+
 __device__ __forceinline__ void delta_copy4(float* smem_dst, const float* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(smem_dst)), "l"(src) : "memory");
 }
@@ -1467,6 +1526,20 @@ TQ_EXPORT int tq_delta_rows_width(int heads, int kv_heads, int dk, int dper) {
     return (2 * kv_heads * dk + heads * dper + kv_heads + heads + 3) / 4 * 4;
 }
 
+// delta_prepare alone, for the recurrence in chunks (csrc/delta_chunks.cu).  Arguments as below.
+TQ_EXPORT int tq_delta_prepare(const float* xqkv, int C, int q_off, int k_off, const float* proj, int P, int b_off, const float* a_raw, int A,
+                               int a_off, int dper, const float* dt_bias, const float* a_log, float* rows, int T_, int heads, int kv_heads, int dk,
+                               float unit_eps, float q_scale, cudaStream_t stream) {
+    if (T_ == 0) return 0;
+    TQ_REQUIRE(heads >= 1 && kv_heads >= 1 && heads % kv_heads == 0 && heads <= 65535 && dk >= 1, "delta_prepare: %d heads on %d query/key heads of %d", heads, kv_heads, dk);
+    TQ_REQUIRE(q_off >= 0 && k_off >= 0 && q_off + kv_heads * dk <= C && k_off + kv_heads * dk <= C && (dper == dk || dper == 1) && b_off >= 0
+               && b_off + heads <= P && a_off >= 0 && a_off + heads * dper <= A && rows != nullptr, "delta_prepare: the heads lie outside their rows");
+    launch_delta_prepare(xqkv, C, q_off, k_off, proj, P, b_off, a_raw, A, a_off, dper, dt_bias, a_log, rows,
+                         tq_delta_rows_width(heads, kv_heads, dk, dper), T_, heads, kv_heads, dk, unit_eps, q_scale, stream);
+    TQ_CHECK_LAUNCH("delta_prepare");
+    return 0;
+}
+
 // The two launches; `rows` is scratch of T * tq_delta_rows_width() floats.  Arguments as for tq_delta_scan.
 TQ_EXPORT int tq_delta_scan_runs(const float* xqkv, int C, int q_off, int k_off, int v_off, const float* proj, int P, int b_off,
                                  const float* a_raw, int A, int a_off, int dper, const float* dt_bias, const float* a_log, float* rows,
@@ -1483,8 +1556,8 @@ TQ_EXPORT int tq_delta_scan_runs(const float* xqkv, int C, int q_off, int k_off,
     TQ_REQUIRE(rows != nullptr, "delta_scan_runs: no scratch for the prepared rows");
     const int R = tq_delta_rows_width(heads, kv_heads, dk, dper);
     const bool head_decay = dper == 1;       // keys of one channel: the same either way
-    tq_launch(dim3(T_, (kv_heads + heads + 3) / 4), 128, 0, stream)(delta_prepare_kernel, xqkv, C, q_off, k_off, proj, P, b_off, a_raw, A,
-        a_off, dper, dt_bias, a_log, rows, R, T_, heads, kv_heads, dk, unit_eps, q_scale);
+    launch_delta_prepare(xqkv, C, q_off, k_off, proj, P, b_off, a_raw, A, a_off, dper, dt_bias, a_log, rows, R, T_, heads, kv_heads, dk, unit_eps,
+                         q_scale, stream);
     TQ_CHECK_LAUNCH("delta_prepare");
     const int rpl = dk <= 64 ? 8 : (dk <= 128 ? 16 : 32);
     const int tc = rpl <= 16 ? 16 : 8;

@@ -1,13 +1,15 @@
-"""Launchers of csrc/recurrence.cuh (in the library of csrc/ssm.cu): recurrences over runs of many tokens in chunks of 64, as float32 matrix products."""
+"""Recurrences over runs of many tokens in chunks of 64, as float32 matrix products: the matrix memory (csrc/recurrence.cuh, in the library of
+csrc/ssm.cu) and the delta rule with one decay per head (csrc/delta_chunks.cu)."""
 from __future__ import annotations
 
-from ctypes import c_longlong, c_void_p
-from typing import Sequence
+from ctypes import c_float, c_int, c_longlong, c_void_p
+from typing import Optional, Sequence
 
 import torch
 
 from ..csrc.build import load_kernel
 from ._call import KernelError, check, ints, ptr, stream, want_f32, want_int32
+from .gemm_tc import status_word
 from .ssm import ctypes_ptr
 
 _LIB = "ssm"
@@ -57,3 +59,42 @@ def memory_chunks(rows: torch.Tensor, q_off: int, k_off: int, v_off: int, gates:
     check(_LIB, lib.tq_memory_chunks(
         ptr(rows), *ints(rows.shape[1], q_off, k_off, v_off), ptr(gates), ctypes_ptr(state), c_longlong(state.stride(0)), ptr(y), ptr(dots),
         c_void_p(at), c_void_p(at + 4 * group * per_chunk), *ints(chunks, group, n_seqs, heads, dk, dv), ptr(cu_seqlens), ptr(slots), stream()), kernels=3 * -(-chunks // group))
+
+
+def delta_bytes(group: int, heads: int, kv_heads: int, dk: int, dv: int) -> int:
+    """Bytes of scratch that a group of the delta rule's chunks takes (csrc/delta_chunks.cu)."""
+    lib = load_kernel("delta_chunks")
+    lib.tq_delta_chunks_bytes.restype = c_longlong
+    return int(lib.tq_delta_chunks_bytes(*ints(group, heads, kv_heads, dk, dv)))
+
+
+def delta_chunks(xqkv: torch.Tensor, q_off: int, k_off: int, v_off: int, proj: torch.Tensor, b_off: int, a_raw: torch.Tensor, a_off: int,
+                 dt_bias: torch.Tensor, a_log: torch.Tensor, state: torch.Tensor, y: torch.Tensor, chunks: int, heads: int, kv_heads: int, dk: int,
+                 dv: int, unit_eps: float, q_scale: float, cu_seqlens: torch.Tensor, slots: torch.Tensor,
+                 status: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """`kernels.ssm.delta_scan_runs` with one decay per head, in chunks: dk and dv 64 or 128 (`usable`); chunks: at least the chunks of the
+    runs (`chunks_of`), as many at a time as SCRATCH_BYTES hold."""
+    for t, what in ((xqkv, "q, k and v"), (proj, "the projection"), (a_raw, "the raw decays"), (dt_bias, "the decays' bias"),
+                    (a_log, "the decay rates"), (state, "the state"), (y, "the output")):
+        want_f32(t, what)
+    for t, what in ((cu_seqlens, "cu_seqlens"), (slots, "slots")):
+        want_int32(t, what)
+    T, n_seqs = xqkv.shape[0], cu_seqlens.shape[0] - 1
+    if not usable(dk, dv, xqkv, v_off) or tuple(state.shape[1:]) != (heads, dv, dk) or not state[0].is_contiguous() or y.numel() != T * heads * dv \
+            or dt_bias.numel() != heads or a_log.numel() != heads or slots.numel() < n_seqs or y.data_ptr() % 16:
+        raise KernelError("delta_chunks: sizes of 64 or 128, aligned rows, one decay per head, a state row of [heads, vdim, dim]")
+    lib = load_kernel(_LIB)
+    rows = torch.empty((T, int(lib.tq_delta_rows_width(*ints(heads, kv_heads, dk, 1)))), dtype=torch.float32, device=xqkv.device)
+    check(_LIB, lib.tq_delta_prepare(
+        ptr(xqkv), *ints(xqkv.shape[1], q_off, k_off), ptr(proj), *ints(proj.shape[1], b_off), ptr(a_raw), *ints(a_raw.shape[1], a_off, 1), ptr(dt_bias),
+        ptr(a_log), ptr(rows), *ints(T, heads, kv_heads, dk), c_float(unit_eps), c_float(q_scale), stream()))
+    if chunks == 0:
+        return y
+    most = max(1, SCRATCH_BYTES // delta_bytes(1, heads, kv_heads, dk, dv))
+    group = -(-chunks // -(-chunks // most))
+    scratch = torch.empty(delta_bytes(group, heads, kv_heads, dk, dv), dtype=torch.uint8, device=xqkv.device)
+    check("delta_chunks", load_kernel("delta_chunks").tq_delta_chunks(
+        ptr(rows), c_int(rows.shape[1]), ptr(xqkv), *ints(xqkv.shape[1], v_off), ctypes_ptr(state), c_longlong(state.stride(0)), ptr(y), ptr(scratch),
+        *ints(chunks, group, n_seqs, heads, kv_heads, dk, dv), ptr(cu_seqlens), ptr(slots), ptr(status if status is not None else status_word(xqkv.device)),
+        stream()), kernels=3 * -(-chunks // group))
+    return y

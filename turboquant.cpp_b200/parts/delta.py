@@ -26,6 +26,7 @@ from typing import List, Optional
 import torch
 
 from ..kernels import gemv as KG
+from ..kernels import recurrence as KR
 from ..kernels import ssm as KS
 from ..kernels.linear import linear
 from ..weights.loader import WeightSpec, WeightStore
@@ -192,6 +193,16 @@ class HeadDeltaMixer(Mixer):
         """The fused input projection as part of a wider one."""
         self.w_in = w
 
+    def _in_chunks(self, ctx: StepContext) -> bool:
+        """Whether a step's runs go in chunks of 64 tokens as matrix products, or token by token: by the times of either on B200, us.  A walk is
+        as long as its longest run, or as all its tokens where its blocks (16 columns of a head's state) are more than the SMs; chunks
+        are a chain of a link per chunk, likewise, and work per chunk and head beside it.  Walk / chunks, 16 heads of 128: one run of
+        2,048 337 / 187, 1,000 and 1,048 together 257 / 192, 64 26 / 44; 8 heads: four runs of 300 82 / 81, one of 128 30 / 46; 4 heads: 512
+        88 / 57, 300 and 257 58 / 51."""
+        n, wide = KR.chunks_of(ctx.host_q_lens, ctx.n_tokens, ctx.n_seqs), self.heads * -(-self.vdim // 16) / 148
+        walk = 12 + 0.158 * max(ctx.max_q_len, 0.88 * ctx.n_tokens * wide)
+        return walk > 36 + 2.45 * max(-(-ctx.max_q_len // KR.CHUNK), n * wide) + 0.136 * n * self.heads
+
     def forward(self, xn: torch.Tensor, ctx: StepContext, cache: LayerCache, projected: Optional[torch.Tensor] = None,
                 offset: int = 0) -> torch.Tensor:
         """projected: float32 rows of a wider product that hold this mixer's projection from column `offset`."""
@@ -211,9 +222,14 @@ class HeadDeltaMixer(Mixer):
         else:
             KS.conv_silu(proj, offset, self.w_conv, None, kept, qkv, ctx.seq_of_token, ctx.cu_seqlens, ctx.slots)
             y = torch.empty((T, self.inner), dtype=torch.float32, device=dev)
-            scan = KS.delta_scan_runs if ctx.max_q_len >= self.RUNS_MIN else KS.delta_scan
-            scan(qkv, 0, self.qk_size, 2 * self.qk_size, proj, b, proj, a, self.dt_bias, self.a_log, S, y, H, G, dk, dv, UNIT_EPS,
-                 dk ** -0.5, ctx.cu_seqlens, ctx.slots)
+            if KR.usable(dk, dv, qkv, 2 * self.qk_size) and self._in_chunks(ctx):
+                KR.delta_chunks(qkv, 0, self.qk_size, 2 * self.qk_size, proj, b, proj, a, self.dt_bias, self.a_log, S, y,
+                                KR.chunks_of(ctx.host_q_lens, T, ctx.n_seqs), H, G, dk, dv, UNIT_EPS, dk ** -0.5, ctx.cu_seqlens, ctx.slots,
+                                status=ctx.status)
+            else:
+                scan = KS.delta_scan_runs if ctx.max_q_len >= self.RUNS_MIN else KS.delta_scan
+                scan(qkv, 0, self.qk_size, 2 * self.qk_size, proj, b, proj, a, self.dt_bias, self.a_log, S, y, H, G, dk, dv, UNIT_EPS,
+                     dk ** -0.5, ctx.cu_seqlens, ctx.slots)
             KS.gated_group_norm(y, proj, z, self.w_norm, H, self.eps, o, gate_after=True)
         if KG.pays(o, self.w_o):
             return KG.gemv(o, self.w_o, torch.empty((T, self.hidden), dtype=torch.float32, device=dev))
