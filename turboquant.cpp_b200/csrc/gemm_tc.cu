@@ -732,7 +732,9 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mxt,
         if (room < (PAIR ? 2 : 1)) room = PAIR ? 2 : 1;
     }
     const int grid = (int)(want < room ? want : room);
-    tq_launch(grid, T::THREADS, T::SMEM_BYTES, stream, PAIR ? 2 : 1)(kern, mw, mx, mxt, (TO*)out, te, tr, tc, nt, R, N, K,
+    // Pairs fill the GPU one CTA an SM: launched early they would hold the SMs that the kernels they wait for, and other streams', still need
+    // (2,048 tokens through 60 experts with a shared one on a second stream: 421 us with them early, 403 without).
+    tq_launch(grid, T::THREADS, T::SMEM_BYTES, stream, PAIR ? 2 : 1, !PAIR)(kern, mw, mx, mxt, (TO*)out, te, tr, tc, nt, R, N, K,
         /* stream_weights: on average at most one token tile per group */ ((te != nullptr && (long long)R <= (long long)G * BN) ? 1 : 0) | (early_weights ? 2 : 0), status,
         k_splits, act, map, second);
     TQ_CHECK_LAUNCH("gemm_tc");
