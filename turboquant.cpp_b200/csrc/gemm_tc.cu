@@ -732,10 +732,8 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mxt,
         if (room < (PAIR ? 2 : 1)) room = PAIR ? 2 : 1;
     }
     const int grid = (int)(want < room ? want : room);
-    // Pairs fill the GPU one CTA an SM: launched early they would hold the SMs that the kernels they wait for, and other streams', still need
-    // (2,048 tokens through 60 experts with a shared one on a second stream: 421 us with them early, 403 without).
-    tq_launch(grid, T::THREADS, T::SMEM_BYTES, stream, PAIR ? 2 : 1, !PAIR)(kern, mw, mx, mxt, (TO*)out, te, tr, tc, nt, R, N, K,
-        /* stream_weights: on average at most one token tile per group */ ((te != nullptr && (long long)R <= (long long)G * BN) ? 1 : 0) | (early_weights ? 2 : 0), status,
+    tq_launch(grid, T::THREADS, T::SMEM_BYTES, stream, PAIR ? 2 : 1, early_weights != 2)(kern, mw, mx, mxt, (TO*)out, te, tr, tc, nt, R, N, K,
+        /* stream_weights: on average at most one token tile per group */ ((te != nullptr && (long long)R <= (long long)G * BN) ? 1 : 0) | (early_weights == 1 ? 2 : 0), status,
         k_splits, act, map, second);
     TQ_CHECK_LAUNCH("gemm_tc");
     return 0;
@@ -754,7 +752,8 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mxt,
 // CTAs the GPU runs at once.  k_splits > 1 (plain products, fp32 out): out is [k_splits][R][N], slice s holding the
 // partial sums over the s-th share of K; the caller adds them up.  early_weights: the caller vouches that W, the
 // tile arrays and n_tiles were final before the kernel ahead of this one in the stream started; the weight stream then
-// starts without waiting for that kernel (programmatic dependent launch), the token rows wait for it as always.
+// starts without waiting for that kernel (programmatic dependent launch), the token rows wait for it as always.  2: the launch starts
+// only when the kernel ahead has ended (where another stream's kernels need the SMs that its waiting CTAs would hold).
 // map: a function of each output element of a plain product (TQ_MAP_*).
 TQ_EXPORT int tq_gemm_tc(const void* X, const void* W, void* out, int out_dtype, const int* tile_expert,
                          const int* tile_row0, const int* tile_count, const int* n_tiles, int max_tiles, int bn,

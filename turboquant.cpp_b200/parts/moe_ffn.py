@@ -223,13 +223,13 @@ class MoEFeedForward(FeedForward):
     EXACT_SHARED_ROWS = 2        # rows of the shared expert that the exact weight-stream kernel takes in one pass
     EXACT_FEW_ROWS = int(os.environ.get("TQ_EXACT_FEW_ROWS", "64"))      # steps of up to this many tokens take the exact kernels' weight-stream form
 
-    def _product(self, x, w, out, layout, inner, token_tile, status=None, early=False, glu=None):
+    def _product(self, x, w, out, layout, inner, token_tile, status=None, early=False, glu=None, late=False):
         """Tensor cores for weights packed at load time (bfloat16, 16-byte rows), the exact CUDA-core
         kernel otherwise.  inner: the product(s) ahead of the activation, which rides on it.  early: this is a down projection right behind its gate/up product in the stream: its
         weights and the layout were there before that product started, so it may stream weights while that runs."""
         swiglu, map = inner and self.gated, self.map if inner and not self.gated else KE.MAP_COPY
         if isinstance(w, KT.PackedWeights):
-            return KT.gemm_tc(x, w, out, layout, token_tile, status=status, early_weights=early and self.EARLY_WEIGHTS, glu=glu, map=map)
+            return KT.gemm_tc(x, w, out, layout, token_tile, status=status, early_weights=early and self.EARLY_WEIGHTS, glu=glu, map=map, late=late)
         # the exact kernels: tiles of a few rows (decode steps) stream the weights; a group's tile holds at most the
         # step's tokens, and the one-group product (the shared expert) all of them
         rows = x.shape[0]
@@ -281,6 +281,10 @@ class MoEFeedForward(FeedForward):
         # router runs beside it.  (Measured on B200, tokens/s with the router first / with the shared expert first:
         # A2.7B sizes batch 8: 2,214 / 2,287, batch 16: 3,228 / 3,147; 57B-A14B sizes batch 1: 177 / 190, batch 8: 602 / 586.)
         shared_after = small and (T * k >= self.n_experts if self.SHARED_AFTER_ROUTER is None else self.SHARED_AFTER_ROUTER)
+        # Long prompts, whose products fill the GPU one CTA an SM on either stream: launched early, a product's waiting CTAs would hold SMs that the
+        # other stream's kernels still need.  (2,048 tokens, 60 experts of 1,408 and a shared one of 5,632: 421 us with early launches, 403
+        # without; with early launches of some of the products only 414 to 422.)
+        apart = self.ws13 is not None and not dual and tile >= KT.PAIR_MIN_TILE
 
         def select(logits):
             KM.router_select_corrected(logits, self.w_correction, k, self.norm_topk, self.renorm_floor, self.n_groups,
@@ -306,7 +310,7 @@ class MoEFeedForward(FeedForward):
                         KE.map_elements(gu, hs, self.map)
                     y_shared = linear(hs, self.ws2[0], out_dtype=torch.float32, status=ctx.status)
                     return
-                self._product(xn, self.ws13, hs, None, True, stile, ctx.status, glu=self.shared_glu)
+                self._product(xn, self.ws13, hs, None, True, stile, ctx.status, glu=self.shared_glu, late=apart)
                 splits = 1
                 if isinstance(self.ws2, KT.PackedWeights):
                     splits = shared_down_shares(T, self.n_experts, k, self.intermediate, S, H, stile, KA_resident(dev),
@@ -315,7 +319,7 @@ class MoEFeedForward(FeedForward):
                 if splits > 1:
                     KT.gemm_tc(hs, self.ws2, y_shared, None, stile, status=ctx.status, k_splits=splits, early_weights=self.EARLY_WEIGHTS)
                 else:
-                    self._product(hs, self.ws2, y_shared, None, False, stile, ctx.status, early=True)
+                    self._product(hs, self.ws2, y_shared, None, False, stile, ctx.status, early=True, late=apart)
             # hs and y_shared were allocated on the side stream; both live until this function returns,
             # after the main stream has joined the side stream again, and the side stream's next use
             # starts with a wait on the main stream: no cross-stream reuse hazard
@@ -333,7 +337,7 @@ class MoEFeedForward(FeedForward):
                 # long steps (prompts): the logits of all tokens as one tensor-core product (bf16 x bf16 products
                 # are exact in fp32 and the sum is fp32), then the selection kernel
                 logits = torch.empty((T, self.n_experts + 1), dtype=torch.float32, device=dev)
-                KT.gemm_tc(xn, self.w_router_packed, logits, None, KT.token_tile_for(T, 1), status=ctx.status)
+                KT.gemm_tc(xn, self.w_router_packed, logits, None, KT.token_tile_for(T, 1), status=ctx.status, late=apart)
                 if self.w_router_bias is not None:
                     KE.scale_bias_cols(logits, 1.0, self.w_router_bias, cols=self.n_experts)
                 if self.corrected:
@@ -367,8 +371,8 @@ class MoEFeedForward(FeedForward):
                             glu=self.glu, glu2=self.shared_glu)
             KT.gemm_tc_dual(h_rows, self.w2, y_rows, layout, hs, self.ws2, y_shared, tile, ctx.status, first)
         else:
-            self._product(x_rows, self.w13, h_rows, layout, True, tile, ctx.status, glu=self.glu)
-            self._product(h_rows, self.w2, y_rows, layout, False, tile, ctx.status, early=True)
+            self._product(x_rows, self.w13, h_rows, layout, True, tile, ctx.status, glu=self.glu, late=apart)
+            self._product(h_rows, self.w2, y_rows, layout, False, tile, ctx.status, early=True, late=apart)
         if side is not None:
             torch.cuda.current_stream().wait_stream(side)
         if leave_rows and y_shared is None:
