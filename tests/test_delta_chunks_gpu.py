@@ -109,3 +109,23 @@ def test_which_steps_go_in_chunks():
     step = lambda lens: SimpleNamespace(host_q_lens=lens, n_tokens=sum(lens), n_seqs=len(lens), max_q_len=max(lens))
     assert m._in_chunks(step([2048])) and m._in_chunks(step([1000, 1048])) and m._in_chunks(step([8192]))
     assert not m._in_chunks(step([64])) and not m._in_chunks(step([200])) and not m._in_chunks(step([2048] + [1] * 63)) and not m._in_chunks(step([2] * 64))
+
+
+@pytest.mark.parametrize("what", ["key", "value"])
+def test_a_matrix_memory_s_token_that_is_not_finite(what):
+    """In chunks a token's output depends on no later token, and other heads on neither."""
+    from turboquant_cpp_b200.kernels import recurrence as KR
+    H, dk, dv, lens, at = 2, 128, 64, [150, 70], 77
+    g = torch.Generator(device=DEV).manual_seed(1)
+    rows, gates = torch.randn((220, H * (2 * dk + dv)), generator=g, device=DEV), -torch.rand((220, H, 2), generator=g, device=DEV)
+    out = []
+    for bad in (0.5, float("nan"), float("inf")):
+        rows[at, (H * dk if what == "key" else 2 * H * dk) + 3] = bad
+        state, y, dots = torch.ones((2, H, dv + 1, dk), device=DEV), torch.empty((220, H * dv), device=DEV), torch.empty((220, H), device=DEV)
+        KR.memory_chunks(rows, 0, H * dk, 2 * H * dk, gates, state, y, dots, KR.chunks_of(lens, 220, 2), H, dk, dv, i32([0, 150, 220]), i32([0, 1]))
+        out.append((y.view(220, H, dv), dots, state))
+    for y, dots, state in out[1:]:
+        for new, old in ((y, out[0][0]), (dots, out[0][1])):
+            assert torch.equal(new[:at], old[:at]) and torch.equal(new[150:], old[150:]) and torch.equal(new[:, 1], old[:, 1])
+        assert torch.equal(state[1], out[0][2][1]) and torch.equal(state[0, 1], out[0][2][0, 1])
+        assert not bool(y[at:150, 0, 3].isfinite().any()) and not bool(state[0, 0, 3].isfinite().all())

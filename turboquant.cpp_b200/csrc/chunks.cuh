@@ -1,10 +1,11 @@
-// Runs of many tokens in chunks of 64: which tokens a chunk holds.
+// Runs of many tokens in chunks of 64: which tokens a chunk holds, its decays, and where the lanes' shares of its products lie.
 #pragma once
 #include "common.cuh"
 
 namespace tq_recurrence {
 
 constexpr int L = 64;          // tokens of a chunk
+constexpr int LD = 65;         // row stride of a 64 x 64 float32 matrix in shared memory
 
 // Chunks are numbered sequence after sequence; a sequence has ceil(run / 64).
 struct Chunk { int seq, t0, n, in_seq; };      // in_seq: its place among the sequence's; n = 0: there is no such chunk
@@ -32,6 +33,36 @@ __device__ __forceinline__ Chunk find_chunk(int chunk, const int* __restrict__ c
     }
     __syncthreads();
     return *s_chunk;
+}
+
+__device__ __forceinline__ float4 zero4() { return make_float4(0.f, 0.f, 0.f, 0.f); }
+// NaN if one of the four is not finite, else 0
+__device__ __forceinline__ float odd(float4 v) { return fmaf(v.x, 0.f, fmaf(v.y, 0.f, fmaf(v.z, 0.f, v.w * 0.f))); }
+// row of an accumulator's or left operand's lane, right operand's address parts: [n][k] rows, [k][n] rows
+struct Lane {
+    int a_row, a_c, b_row, b_c, t_row, t_c, v_row, v_c, r, c;
+    __device__ __forceinline__ explicit Lane(int lane)
+        : a_row(lane & 15), a_c(lane >> 4),                                      // left operand [m][k]
+          b_row(((lane >> 4) << 3) + (lane & 7)), b_c((lane >> 3) & 1),          // right operand lying as [n][k]
+          t_row(lane & 15), t_c(lane >> 4),                                      // right operand lying as [k][n]
+          v_row(((lane >> 4) << 3) + (lane & 7)), v_c((lane >> 3) & 1),          // left operand lying as [k][m]
+          r(lane >> 2), c(2 * (lane & 3)) {}
+};
+
+// D[t][s] (zero for s > t) to m, A_t to s_A, D[last] to s_D; g beyond the chunk's tokens is one
+__device__ __forceinline__ void decays(float* m, const float* s_g, float* s_A, float* s_D) {
+    const int t = threadIdx.x;
+    if (t < L) {
+        float d = 1.f;
+        for (int s = L - 1; s >= 0; --s) {
+            if (s < t) d *= s_g[s + 1];
+            m[t * LD + s] = s <= t ? d : 0.f;
+            if (t == L - 1 && s_D) s_D[s] = d;
+        }
+    } else if (t == L) {
+        float d = 1.f;
+        for (int i = 0; i < L; ++i) { d *= s_g[i]; s_A[i] = d; }
+    }
 }
 
 }  // namespace tq_recurrence

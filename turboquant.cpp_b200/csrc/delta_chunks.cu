@@ -28,11 +28,9 @@ TQ_DEFINE_LAST_ERROR
 
 namespace {
 
-using tq_recurrence::Chunk;
-using tq_recurrence::L;
-using tq_recurrence::find_chunk;
+using namespace tq_recurrence;
 
-constexpr int THREADS = 128, CHAIN_WARPS = 4, LD = 65;          // LD: row stride of the 64 x 64 float32 matrices in shared memory
+constexpr int THREADS = 128, CHAIN_WARPS = 4;
 constexpr int T_PART = L * L * 2;
 constexpr int XLD = 72;                                         // row stride of the warps' shares of K S: four rows' pairs in different banks
 constexpr uint32_t WAIT_LIMIT = 1u << 20;                       // polls of an mbarrier before a wait gives up ...
@@ -59,36 +57,6 @@ constexpr int N_A = 0, N_BETA = L, N_D = 2 * L, N_LAST = 3 * L, N_BAD = 3 * L + 
 
 // What a token brings, as delta_prepare lays it out: [k: G x dk | q: G x dk | g: H | k.q: G | beta: H]
 struct Rows { const float* at; int stride, heads, kv_heads; };
-
-__device__ __forceinline__ float4 zero4() { return make_float4(0.f, 0.f, 0.f, 0.f); }
-// NaN if one of the four is not finite, else 0
-__device__ __forceinline__ float odd(float4 v) { return fmaf(v.x, 0.f, fmaf(v.y, 0.f, fmaf(v.z, 0.f, v.w * 0.f))); }
-// row of an accumulator's or left operand's lane, right operand's address parts: [n][k] rows, [k][n] rows
-struct Lane {
-    int a_row, a_c, b_row, b_c, t_row, t_c, v_row, v_c, r, c;
-    __device__ __forceinline__ explicit Lane(int lane)
-        : a_row(lane & 15), a_c(lane >> 4),                                      // left operand [m][k]
-          b_row(((lane >> 4) << 3) + (lane & 7)), b_c((lane >> 3) & 1),          // right operand lying as [n][k]
-          t_row(lane & 15), t_c(lane >> 4),                                      // right operand lying as [k][n]
-          v_row(((lane >> 4) << 3) + (lane & 7)), v_c((lane >> 3) & 1),          // left operand lying as [k][m]
-          r(lane >> 2), c(2 * (lane & 3)) {}
-};
-
-// D[t][s] (zero for s > t) to m, A_t to s_A, D[last] to s_D; g beyond the chunk's tokens is one
-__device__ __forceinline__ void decays(float* m, const float* s_g, float* s_A, float* s_D) {
-    const int t = threadIdx.x;
-    if (t < L) {
-        float d = 1.f;
-        for (int s = L - 1; s >= 0; --s) {
-            if (s < t) d *= s_g[s + 1];
-            m[t * LD + s] = s <= t ? d : 0.f;
-            if (t == L - 1 && s_D) s_D[s] = d;
-        }
-    } else if (t == L) {
-        float d = 1.f;
-        for (int i = 0; i < L; ++i) { d *= s_g[i]; s_A[i] = d; }
-    }
-}
 
 template <int DK, int DV>
 __global__ void __launch_bounds__(THREADS, 2)
@@ -122,21 +90,28 @@ delta_solve_kernel(Rows rows, const float* __restrict__ xv, int C, int v_off, Sc
         if (!fine) atomicMin(&s_bad, tid);
     }
     {
-        constexpr int Q = DK / 4;
-#pragma unroll 8
-        for (int i = tid; i < L * Q; i += THREADS) {
-            const int t = i / Q, d = i % Q * 4;
-            float4 v = t < c.n ? *reinterpret_cast<const float4*>(tok + (size_t)t * rows.stride + g * DK + d) : zero4();
-            if (odd(v) != 0.f) { atomicMin(&s_bad, t); v = zero4(); }
-            tq_put4<DK>(sk, F::K_PART, t, d, v);
+        constexpr int KQ = DK / 4, KN = L * KQ / THREADS, VQ = DV / 4, VN = L * VQ / THREADS;
+        float4 k4[KN], v4[VN];         // all of them asked for before the first is used
+#pragma unroll
+        for (int i = 0; i < KN; ++i) {
+            const int t = (i * THREADS + tid) / KQ;
+            k4[i] = t < c.n ? *reinterpret_cast<const float4*>(tok + (size_t)t * rows.stride + g * DK + tid % KQ * 4) : zero4();
         }
-    }
-    {
-        constexpr int Q = DV / 4;
-        const float* v0 = xv + (size_t)c.t0 * C + v_off + h * DV;
-#pragma unroll 8
-        for (int i = tid; i < c.n * Q; i += THREADS)
-            if (odd(*reinterpret_cast<const float4*>(v0 + (size_t)(i / Q) * C + i % Q * 4)) != 0.f) atomicMin(&s_bad, i / Q);
+        const float* v0 = xv + (size_t)c.t0 * C + v_off + h * DV + tid % VQ * 4;
+#pragma unroll
+        for (int i = 0; i < VN; ++i) {
+            const int t = (i * THREADS + tid) / VQ;
+            v4[i] = t < c.n ? *reinterpret_cast<const float4*>(v0 + (size_t)t * C) : zero4();
+        }
+#pragma unroll
+        for (int i = 0; i < KN; ++i) {
+            const int t = (i * THREADS + tid) / KQ;
+            if (odd(k4[i]) != 0.f) { atomicMin(&s_bad, t); k4[i] = zero4(); }
+            tq_put4<DK>(sk, F::K_PART, t, tid % KQ * 4, k4[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < VN; ++i)
+            if (odd(v4[i]) != 0.f) atomicMin(&s_bad, (i * THREADS + tid) / VQ);
     }
     for (int i = tid; i < L * LD; i += THREADS) T[i] = 0.f;
     __syncthreads();
@@ -517,12 +492,15 @@ delta_outputs_kernel(Rows rows, Scratch in, float* __restrict__ y, int chunk0, c
             const float a = tid < c.n ? tok[(size_t)tid * rows.stride + 2 * rows.kv_heads * DK + h] : 1.f;
             s_g[tid] = isfinite(a) ? a : 1.f;
         }
-        constexpr int Q = DK / 4;
-#pragma unroll 8
-        for (int i = tid; i < L * Q; i += THREADS) {
-            const int t = i / Q, d = i % Q * 4;
-            tq_put4<DK>(sq, F::K_PART, t, d, t < c.n ? *reinterpret_cast<const float4*>(tok + (size_t)t * rows.stride + (rows.kv_heads + g) * DK + d) : zero4());
+        constexpr int Q = DK / 4, QN = L * Q / THREADS;
+        float4 q4[QN];                 // all of them asked for before the first is used
+#pragma unroll
+        for (int i = 0; i < QN; ++i) {
+            const int t = (i * THREADS + tid) / Q;
+            q4[i] = t < c.n ? *reinterpret_cast<const float4*>(tok + (size_t)t * rows.stride + (rows.kv_heads + g) * DK + tid % Q * 4) : zero4();
         }
+#pragma unroll
+        for (int i = 0; i < QN; ++i) tq_put4<DK>(sq, F::K_PART, (i * THREADS + tid) / Q, tid % Q * 4, q4[i]);
         asm volatile("cp.async.wait_all;" ::: "memory");
     }
     __syncthreads();

@@ -1,139 +1,60 @@
-// Recurrences over runs of many tokens in chunks of 64, as matrix products in fp32.  A state S [dk, dv] per head with a decay
-// and a write per token,
-//   S_t = a_t S_(t-1) + b_t k_t v_t^T,   y_t = S_t^T q_t,
+// The matrix memory over runs of many tokens in chunks of 64 as float32 matrix products on the tensor cores, operands as three bfloat16
+// values each (split3.cuh).  A state S [dk, dv] per head with a decay and a write per token,
+//   S_t = a_t S_(t-1) + b_t k_t v_t^T,   y_t = S_t^T q_t       (a = e^gate0, b = e^gate1; n is one more column whose value is one)
 // is linear in the state it starts from: with D[t][s] = a_(s+1) ... a_t (products in token order; D[t][t] = 1) and
 // A_t = a_first ... a_t, inside a chunk that starts from S_0
 //   y_t = A_t S_0^T q_t + sum over s <= t of (q_t . k_s) D[t][s] b_s v_s
 //   S_last = A_last S_0 + sum over s of D[last][s] b_s k_s v_s^T.
 // Three launches: every chunk's own sum (the second formula from zero) side by side; the states the chunks start from, one chunk
 // after the other but every element by itself; every chunk's outputs side by side.  A long step does this for a group of chunks after
-// the other, the kept state going from group to group, so that the chunks' states take a bounded buffer.  Token by token (csrc/ssm.cu) a walk does 2
-// multiply-adds an element of the state and token, a chain of its tokens with a shuffle tree each, and long runs are walked twice to
-// fill the GPU; in chunks it is 2 + 64 (1 / dk + 1 / dv) of them, all in register-tiled products.  Everything is fp32 and
-// stays on the CUDA cores: tensor cores round operands (two tf32 parts of each hold 22 of 24 bits; three bfloat16 parts hold all 24 in
-// six products, a form that was not built).  Measured, 682 + 1,366 tokens, 16 heads of 128 x 129: 289 us for both walks token by token; here 37 us for the
-// chunks' sums, 16 for the starts and 79 for the outputs (1.07 G multiply-adds, 30 us at the fp32 units' rate; what bounds them is shared
-// memory, twelve 128-byte reads a warp for its 32 multiply-adds a thread; 102 us with transposed stores and weights that met in one
-// bank).
+// the other, the kept state going from group to group, so that the chunks' states take a bounded buffer.  Token by token (csrc/ssm.cu)
+// a walk does 2 multiply-adds an element of the state and token, a chain of its tokens with a shuffle tree each, and long runs are
+// walked twice to fill the GPU; in chunks it is 2 + 64 (1 / dk + 1 / dv) of them, all in products.
+// Everything is kept and added up in float32; products are six bfloat16 ones whose largest are summed over at most 64 elements.
+// 682 + 1,366 tokens, 16 heads of 128 x 129: 33 us for the chunks' sums, 17 for the starts and 54 for the outputs (as products on the
+// fp32 units 37, 16 and 79, bound by what they read of shared memory; token by token 289).  With one CTA an SM the outputs take 89; what bounds
+// either kernel with two is a warp's own chain of loads, splitting and products, the tensor cores are active 32 to 40 % of the time.
+// A value that is not finite takes no part in earlier tokens' outputs; the token's own and all later ones are NaN in its group of 32 columns.
 // Part of csrc/ssm.cu's library.
-//   memory_chunks   the matrix memory (a = e^gate0, b = e^gate1; n is one more column whose value is one)
 #pragma once
+#include "split3.cuh"
 #include "chunks.cuh"
 
 namespace tq_recurrence {
 
-constexpr int THREADS = 256;   // 16 x 16: a thread holds 4 x 4 blocks of a product, 64 apart in rows and columns
+constexpr int THREADS = 128;
 
-__device__ __forceinline__ float4 zero4() { return make_float4(0.f, 0.f, 0.f, 0.f); }
+template <int DK, int DV>
+struct MemoryCfg {
+    static constexpr int K_PART = L * DK * 2, V_PART = L * DV * 2;
+    static constexpr int ENDS_BYTES = 3 * (K_PART + V_PART);
+    static constexpr int SQ_PART = 32 * DK * 2, VQ_PART = L * 32 * 2;                // 32 columns of a state and of the values
+    static constexpr int WORK = 3 * (K_PART > SQ_PART + VQ_PART ? K_PART : SQ_PART + VQ_PART);
+    static constexpr int OUT_BYTES = 3 * K_PART + WORK + L * LD * 4;
+};
 
-// rows [n tokens][N] at src (stride floats apart) -> smem [64][N], zeros behind the last
-template <int N>
-__device__ __forceinline__ void load_rows(float* dst, const float* __restrict__ src, int stride, int n) {
-    constexpr int Q = N / 4;
-#pragma unroll
-    for (int i = threadIdx.x; i < L * Q; i += THREADS) {
-        const int t = i / Q, c = i % Q * 4;
-        *reinterpret_cast<float4*>(dst + t * N + c) = t < n ? *reinterpret_cast<const float4*>(src + (size_t)t * stride + c) : zero4();
-    }
-}
-// K columns of R rows -> smem [K][R] (transposed); rows from n on are zeros.  A row's groups of four neighbours (along R) are shuffled
-// by the bits of k above the lowest two, so that the lanes of a warp, which read a row's columns together, store into eight
-// banks' groups instead of one; a product reads a whole group at one k, wherever it lies.
-__device__ __forceinline__ int group_at(int k, int g) { return g ^ ((k >> 2) & 15); }
-template <int K, int R>
-__device__ __forceinline__ void load_transposed(float* dst, const float* __restrict__ src, int stride, int n) {
-    constexpr int Q = K / 4;
-#pragma unroll 8
-    for (int i = threadIdx.x; i < R * Q; i += THREADS) {
-        const int r = i / Q, c = i % Q * 4;
-        const float4 v = r < n ? *reinterpret_cast<const float4*>(src + (size_t)r * stride + c) : zero4();
-        float* at = dst + c * R + 4 * group_at(c, r >> 2) + (r & 3);
-        at[0] = v.x;
-        at[R] = v.y;
-        at[2 * R] = v.z;
-        at[3 * R] = v.w;
-    }
-}
+// Rows of 32 bfloat16, their four 16-byte pieces shuffled by bits 1 and 2 of the row: eight neighbouring rows' pieces of one column lie in
+// different banks
+__device__ __forceinline__ uint32_t piece32(int row, int c) { return (uint32_t)(row * 64 + ((c ^ ((row >> 1) & 3)) << 4)); }
 
-// acc[4 i + r][2 j + p] += a[k][64 i + 4 ty + r] * b[k][64 j + 4 tx + 2 p, + 1] over k in [k0, k1): a [k][LDA], b [k][LDB] in shared memory
-// (TA, TB: as load_transposed leaves them)
-template <int RI, int RJ, int LDA, int LDB, bool TA = false, bool TB = false>
-__device__ __forceinline__ void product(tq_f32x2 (&acc)[4 * RI][2 * RJ], const float* a, const float* b, int k0, int k1, int ty, int tx) {
-#pragma unroll 4
-    for (int k = k0; k < k1; ++k) {
-        float4 av[RI];
-        ulonglong2 bv[RJ];
-#pragma unroll
-        for (int i = 0; i < RI; ++i) av[i] = *reinterpret_cast<const float4*>(a + k * LDA + 64 * i + 4 * (TA ? group_at(k, ty) : ty));
-#pragma unroll
-        for (int j = 0; j < RJ; ++j) bv[j] = *reinterpret_cast<const ulonglong2*>(b + k * LDB + 64 * j + 4 * (TB ? group_at(k, tx) : tx));
-#pragma unroll
-        for (int i = 0; i < RI; ++i) {
-            const float ar[4] = {av[i].x, av[i].y, av[i].z, av[i].w};
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const tq_f32x2 x = tq_pack2(ar[r], ar[r]);
-#pragma unroll
-                for (int j = 0; j < RJ; ++j) {
-                    acc[4 * i + r][2 * j] = tq_fma2(x, bv[j].x, acc[4 * i + r][2 * j]);
-                    acc[4 * i + r][2 * j + 1] = tq_fma2(x, bv[j].y, acc[4 * i + r][2 * j + 1]);
-                }
-            }
-        }
-    }
-}
-// acc[r][..] += sum over s <= t of Pt[s][t] Vs[s][..] for the thread's rows t = 4 ty + r: the tokens ahead of the warp's eight
-// rows as a product, those eight one by one, so that a token never meets a later one's values, whatever they are
-template <int RJ, int LDA, int LDB>
-__device__ __forceinline__ void add_earlier(tq_f32x2 (&acc)[4][2 * RJ], const float* Pt, const float* Vs, int ty, int tx) {
-    const int first = 8 * (ty >> 1);
-    product<1, RJ, LDA, LDB>(acc, Pt, Vs, 0, first, ty, tx);
-#pragma unroll 2
-    for (int s = first; s < first + 8; ++s) {
-        const float4 p = *reinterpret_cast<const float4*>(Pt + s * LDA + 4 * ty);
-        const float pr[4] = {p.x, p.y, p.z, p.w};
-#pragma unroll
-        for (int j = 0; j < RJ; ++j) {
-            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(Vs + s * LDB + 64 * j + 4 * tx);
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-                if (s <= 4 * ty + r) {
-                    const tq_f32x2 x = tq_pack2(pr[r], pr[r]);
-                    acc[r][2 * j] = tq_fma2(x, v.x, acc[r][2 * j]);
-                    acc[r][2 * j + 1] = tq_fma2(x, v.y, acc[r][2 * j + 1]);
-                }
-        }
-    }
-}
-template <int M, int N>
-__device__ __forceinline__ void clear(tq_f32x2 (&acc)[M][N]) {
-#pragma unroll
-    for (int i = 0; i < M; ++i)
-#pragma unroll
-        for (int j = 0; j < N; ++j) acc[i][j] = 0ull;
-}
-__device__ __forceinline__ float4 four(tq_f32x2 a, tq_f32x2 b) {
-    const float2 x = tq_unpack2(a), y = tq_unpack2(b);
-    return make_float4(x.x, x.y, y.x, y.y);
-}
-
-// ---- a chunk's own sum, of the group from chunk0 on: ends [chunk - chunk0][head][dv + 1][dk] (the last row n), decays [..][head] ----
+// ---- a chunk's own sum, of the group from chunk0 on: ends [chunk - chunk0][head][dv + 1][dk] (the last row n), last [..][head] ----
 template <int DK, int DV>
 __global__ void __launch_bounds__(THREADS, 2)
 memory_ends_kernel(const float* __restrict__ rows, int C, int k_off, int v_off, const float2* __restrict__ gates, int heads, int chunk0,
-                   const int* __restrict__ cu_seqlens, int n_seqs, float* __restrict__ ends, float* __restrict__ decays) {
+                   const int* __restrict__ cu_seqlens, int n_seqs, float* __restrict__ ends, float* __restrict__ last) {
     tq_grid_wait();                    // everything below may read what the previous kernel wrote
     tq_grid_launch_dependents();       // the next kernel's CTAs may move in as SMs free up
-    extern __shared__ __align__(16) float smem[];
-    float* Ks = smem;                  // [64][DK], times the weight of its token
-    float* Vs = smem + L * DK;         // [64][DV]
+    using F = MemoryCfg<DK, DV>;
+    extern __shared__ __align__(128) uint8_t smem[];
+    const uint32_t sk = tq_smem_u32(smem), sv = sk + 3 * F::K_PART;                // K; V times the weight of its token
     __shared__ Chunk s_chunk;
     __shared__ float s_w[L], s_half;
     const int h = blockIdx.y;
     const Chunk c = find_chunk(chunk0 + blockIdx.x, cu_seqlens, n_seqs, &s_chunk);
     if (c.n == 0) return;
-    const int tid = threadIdx.x, lane = tid & 31;
-    load_rows<DV>(Vs, rows + (size_t)c.t0 * C + v_off + h * DV, C, c.n);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const Lane ln(lane);
+    const float* tok = rows + (size_t)c.t0 * C;
     if (tid < L) {                     // D[last][s] b_s: what is left of token s at the chunk's end
         const float2 g = tid < c.n ? gates[(size_t)(c.t0 + tid) * heads + h] : make_float2(0.f, -INFINITY);
         float a = expf(g.x), down = a;
@@ -143,40 +64,69 @@ memory_ends_kernel(const float* __restrict__ rows, int C, int k_off, int v_off, 
         if (lane == 31) after = 1.f;
         s_w[tid] = after * expf(g.y);
         if (tid == L / 2) s_half = down;
-        if (tid == 0) decays[(size_t)blockIdx.x * heads + h] = down;       // the first half's; completed below
+        if (tid == 0) last[(size_t)blockIdx.x * heads + h] = down;         // the first half's; completed below
+    }
+    constexpr int KQ = DK / 4, VQ = DV / 4, KN = L * KQ / THREADS, VN = L * VQ / THREADS;
+    float4 v4[VN];                     // on their way while K is split
+    {
+        float4 k4[KN];
+#pragma unroll
+        for (int i = 0; i < KN; ++i) {
+            const int t = (i * THREADS + tid) / KQ;
+            k4[i] = t < c.n ? *reinterpret_cast<const float4*>(tok + (size_t)t * C + k_off + h * DK + tid % KQ * 4) : zero4();
+        }
+#pragma unroll
+        for (int i = 0; i < VN; ++i) {
+            const int t = (i * THREADS + tid) / VQ;
+            v4[i] = t < c.n ? *reinterpret_cast<const float4*>(tok + (size_t)t * C + v_off + h * DV + tid % VQ * 4) : zero4();
+        }
+#pragma unroll
+        for (int i = 0; i < KN; ++i) tq_put4<DK>(sk, F::K_PART, (i * THREADS + tid) / KQ, tid % KQ * 4, k4[i]);
     }
     __syncthreads();
     if (tid < L / 2) s_w[tid] *= s_half;
-    if (tid == 0) decays[(size_t)blockIdx.x * heads + h] *= s_half;
+    if (tid == 0) last[(size_t)blockIdx.x * heads + h] *= s_half;
     __syncthreads();
-    {
-        constexpr int Q = DK / 4;
-        const float* src = rows + (size_t)c.t0 * C + k_off + h * DK;
 #pragma unroll
-        for (int i = tid; i < L * Q; i += THREADS) {
-            const int t = i / Q, e = i % Q * 4;
-            float4 v = t < c.n ? *reinterpret_cast<const float4*>(src + (size_t)t * C + e) : zero4();
-            const float w = s_w[t];
-            v.x *= w; v.y *= w; v.z *= w; v.w *= w;
-            *reinterpret_cast<float4*>(Ks + t * DK + e) = v;
-        }
+    for (int i = 0; i < VN; ++i) {
+        const int t = (i * THREADS + tid) / VQ;
+        const float w = s_w[t];
+        v4[i].x *= w; v4[i].y *= w; v4[i].z *= w; v4[i].w *= w;
+        tq_put4<DV>(sv, F::V_PART, t, tid % VQ * 4, v4[i]);
     }
     __syncthreads();
-    constexpr int RI = DV / 64, RJ = DK / 64;
-    const int ty = tid / 16, tx = tid % 16;
-    tq_f32x2 acc[4 * RI][2 * RJ];
-    clear(acc);
-    product<RI, RJ, DV, DK>(acc, Vs, Ks, 0, L, ty, tx);
     float* out = ends + ((size_t)blockIdx.x * heads + h) * (DV + 1) * DK;
+    constexpr int MT = DV / 64;        // groups of 16 columns a warp takes
+    for (int d4 = 0; d4 < DK / 32; ++d4) {
+        float big[MT][4][4], small[MT][4][4];
 #pragma unroll
-    for (int i = 0; i < 4 * RI; ++i)
+        for (int k = 0; k < L / 16; ++k) {
+            uint32_t b[3][2][4];
 #pragma unroll
-        for (int j = 0; j < RJ; ++j)
-            *reinterpret_cast<float4*>(out + (size_t)(i / 4 * 64 + 4 * ty + i % 4) * DK + 64 * j + 4 * tx) = four(acc[i][2 * j], acc[i][2 * j + 1]);
+            for (int p = 0; p < 3; ++p)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) tq_ldm4t(b[p][j], sk + p * F::K_PART + tq_piece<DK>(16 * k + ln.t_row, 4 * d4 + 2 * j + ln.t_c));
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt) {
+                uint32_t a[3][4];
+#pragma unroll
+                for (int p = 0; p < 3; ++p) tq_ldm4t(a[p], sv + p * F::V_PART + tq_piece<DV>(16 * k + ln.v_row, 2 * (warp * MT + mt) + ln.v_c));
+                if (k == 0) tq_six<4, true, true>(big[mt], small[mt], a, b); else tq_six<4, false, false>(big[mt], small[mt], a, b);
+            }
+        }
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int r = 0; r < 2; ++r)
+                    *reinterpret_cast<float2*>(out + (size_t)(16 * (warp * MT + mt) + ln.r + 8 * r) * DK + 32 * d4 + 8 * u + ln.c) =
+                        make_float2(big[mt][u][2 * r] + small[mt][u][2 * r], big[mt][u][2 * r + 1] + small[mt][u][2 * r + 1]);
+    }
     if (tid < DK) {
         float n = 0.f;
-#pragma unroll 8
-        for (int s = 0; s < L; ++s) n += Ks[s * DK + tid];
+#pragma unroll 16
+        for (int s = 0; s < c.n; ++s) n = fmaf(s_w[s], tok[(size_t)s * C + k_off + h * DK + tid], n);
         out[(size_t)DV * DK + tid] = n;
     }
 }
@@ -184,7 +134,7 @@ memory_ends_kernel(const float* __restrict__ rows, int C, int k_off, int v_off, 
 // ---- the states the group's chunks start from, in the place of their own sums; the kept state moves to the end of the last -----
 __global__ void __launch_bounds__(256)
 chunk_starts_kernel(float* __restrict__ state, long long slot_stride, const int* __restrict__ slots, float* __restrict__ ends,
-                    const float* __restrict__ decays, int heads, int per_head, int chunk0, int group, const int* __restrict__ cu_seqlens) {
+                    const float* __restrict__ last, int heads, int per_head, int chunk0, int group, const int* __restrict__ cu_seqlens) {
     tq_grid_wait();                    // everything below may read what the previous kernel wrote
     tq_grid_launch_dependents();       // the next kernel's CTAs may move in as SMs free up
     __shared__ int s_first;
@@ -202,7 +152,7 @@ chunk_starts_kernel(float* __restrict__ state, long long slot_stride, const int*
     if (e >= per_head || n <= 0) return;
     float* cell = state + (size_t)slots[s] * slot_stride + (size_t)h * per_head + e;
     float* at = ends + ((size_t)from * heads + h) * per_head + e;
-    const float* d = decays + (size_t)from * heads + h;
+    const float* d = last + (size_t)from * heads + h;
     const size_t step = (size_t)heads * per_head;
     float S = *cell;
     constexpr int AHEAD = 8;           // the sums do not depend on the chain: eight of them on their way together
@@ -224,6 +174,8 @@ chunk_starts_kernel(float* __restrict__ state, long long slot_stride, const int*
 }
 
 // ---- a chunk's outputs ----------------------------------------------------------------------------------------------------------
+// A warp has 16 tokens; the weights of the chunk's own tokens stay in its registers, the columns come 32 at a time while the 32 ahead
+// are multiplied.
 template <int DK, int DV>
 __global__ void __launch_bounds__(THREADS, 2)
 memory_outputs_kernel(const float* __restrict__ rows, int C, int q_off, int k_off, int v_off, const float2* __restrict__ gates, int heads,
@@ -231,134 +183,222 @@ memory_outputs_kernel(const float* __restrict__ rows, int C, int q_off, int k_of
                       float* __restrict__ dots) {
     tq_grid_wait();                    // everything below may read what the previous kernel wrote
     tq_grid_launch_dependents();       // the next kernel's CTAs may move in as SMs free up
-    extern __shared__ __align__(16) float smem[];
-    constexpr int BUF = 64 * (DK > DV ? DK : DV);
-    float* Qt = smem;                  // [DK][64]
-    float* X = Qt + DK * L;            // keys [DK][64], then the second 64 rows of the state [64][DV] (DK 128) or the values
-    float* Y = X + BUF;                // the state's first 64 rows [64][DV], then (DK 128) the values [64][DV]
-    float* Pt = Y + 64 * DV;           // [s][t]: D[t][s], then the weight of value s in output t
+    using F = MemoryCfg<DK, DV>;
+    extern __shared__ __align__(128) uint8_t smem[];
+    const uint32_t sq = tq_smem_u32(smem), sk = sq + 3 * F::K_PART, sv = sk + 3 * F::SQ_PART;   // Q; K, then 32 columns of the state and of V
+    float* m = reinterpret_cast<float*>(smem + 3 * F::K_PART + F::WORK);
     __shared__ Chunk s_chunk;
-    __shared__ float s_a[L], s_b[L], s_A[L];
+    // (Two CTAs an SM fit with 2 KB to spare: every 256 bytes count.  The b lie in the unused column of m, n . q where the a were.)
+    __shared__ float s_a[L], s_A[L];
+    __shared__ int s_bad[2];           // of the 32 columns at hand: the first token whose value is not finite
     const int h = blockIdx.y;
     const Chunk c = find_chunk(chunk0 + blockIdx.x, cu_seqlens, n_seqs, &s_chunk);
     if (c.n == 0) return;
-    const int tid = threadIdx.x, ty = tid / 16, tx = tid % 16;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const Lane ln(lane);
     const float* tok = rows + (size_t)c.t0 * C;
     const float* St = starts + ((size_t)blockIdx.x * heads + h) * (DV + 1) * DK;     // [column][dk]
     if (tid < L) {
         const float2 g = tid < c.n ? gates[(size_t)(c.t0 + tid) * heads + h] : make_float2(0.f, -INFINITY);
         s_a[tid] = expf(g.x);
-        s_b[tid] = expf(g.y);
+        m[tid * LD + L] = expf(g.y);
     }
-    load_transposed<DK, L>(Qt, tok + q_off + h * DK, C, c.n);
-    load_transposed<DK, L>(X, tok + k_off + h * DK, C, c.n);
-    __syncthreads();
-    if (tid < L) {                     // row t of D, a thread each (neighbouring threads store side by side)
-        float d = 1.f;
-        for (int s = L - 1; s >= 0; --s) {
-            if (s < tid) d *= s_a[s + 1];
-            Pt[s * L + tid] = s <= tid ? d : 0.f;
-        }
-    } else if (tid == L) {
-        float d = 1.f;
-        for (int t = 0; t < L; ++t) { d *= s_a[t]; s_A[t] = d; }
-    }
-    load_transposed<64, DV>(Y, St, DK, DV);
-    __syncthreads();
+    if (tid == 0) s_bad[0] = L;
+    constexpr int KQ = DK / 4, KN = L * KQ / THREADS;
+    float from[KN];
     {
-        tq_f32x2 p[4][2];              // k_s . q_t: rows s, columns t
-        clear(p);
-        product<1, 1, L, L, true, true>(p, X, Qt, 0, DK, ty, tx);
+        float4 q4[KN], k4[KN];         // all of them asked for before the first is used
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const float4 v = four(p[r][0], p[r][1]);
-            const float b = s_b[4 * ty + r];
-            float4* at = reinterpret_cast<float4*>(Pt + (4 * ty + r) * L + 4 * tx);
-            float4 d = *at;
-            d.x *= v.x * b; d.y *= v.y * b; d.z *= v.z * b; d.w *= v.w * b;
-            *at = d;
+        for (int i = 0; i < KN; ++i) {
+            const int t = (i * THREADS + tid) / KQ, e = tid % KQ * 4;
+            const float* at = tok + (size_t)t * C + h * DK + e;
+            q4[i] = t < c.n ? *reinterpret_cast<const float4*>(at + q_off) : zero4();
+            k4[i] = t < c.n ? *reinterpret_cast<const float4*>(at + k_off) : zero4();
+        }
+        const float4 n4 = *reinterpret_cast<const float4*>(St + (size_t)DV * DK + tid % KQ * 4);       // the column whose value is one
+#pragma unroll
+        for (int i = 0; i < KN; ++i) {
+            const int t = (i * THREADS + tid) / KQ, e = tid % KQ * 4;
+            tq_put4<DK>(sq, F::K_PART, t, e, q4[i]);
+            tq_put4<DK>(sk, F::K_PART, t, e, k4[i]);
+            from[i] = fmaf(q4[i].x, n4.x, fmaf(q4[i].y, n4.y, fmaf(q4[i].z, n4.z, q4[i].w * n4.w)));
+#pragma unroll
+            for (int o = KQ / 2; o > 0; o >>= 1) from[i] += __shfl_xor_sync(0xffffffffu, from[i], o);
         }
     }
     __syncthreads();
-    constexpr int RJ = DV / 64;
-    tq_f32x2 acc[4][2 * RJ];
-    clear(acc);
-    if (DK > 64) load_transposed<64, DV>(X, St + 64, DK, DV);
-    else load_rows<DV>(X, tok + v_off + h * DV, C, c.n);
-    product<1, RJ, L, DV, true, true>(acc, Qt, Y, 0, 64, ty, tx);
+    decays(m, s_a, s_A, nullptr);
+    // the first 32 columns of the state and of the values are on their way meanwhile
+    constexpr int SN = 32 * DK / 4 / THREADS, VN = L * 8 / THREADS;
+    float4 ns[SN], nv[VN];
+    auto ask = [&](int q) {
+        const float4* s_at = reinterpret_cast<const float4*>(St + (size_t)32 * q * DK) + tid;
+#pragma unroll
+        for (int i = 0; i < SN; ++i) ns[i] = s_at[i * THREADS];
+#pragma unroll
+        for (int i = 0; i < VN; ++i) {
+            const int t = (i * THREADS + tid) >> 3, e = (tid & 7) * 4;
+            nv[i] = t < c.n ? *reinterpret_cast<const float4*>(tok + (size_t)t * C + v_off + h * DV + 32 * q + e) : zero4();
+        }
+    };
+    ask(0);
     __syncthreads();
-    const float* Vs = X;
-    if (DK > 64) {
-        load_rows<DV>(Y, tok + v_off + h * DV, C, c.n);
-        product<1, RJ, L, DV, true, true>(acc, Qt + 64 * L, X, 0, 64, ty, tx);
+    if (tid % KQ == 0)
+#pragma unroll
+        for (int i = 0; i < KN; ++i) s_a[(i * THREADS + tid) / KQ] = from[i];
+    uint32_t P[L / 16][3][4];          // (Q K^T) o D times b as left operands
+    float own[2] = {0.f, 0.f};         // their sums: n of the chunk's own tokens
+    for (int grp = 0; grp < 2; ++grp) {
+        float big[4][4], small[4][4], first[4][4];
+        if (grp <= warp >> 1) {
+#pragma unroll
+            for (int k = 0; k < DK / 16; ++k) {
+                if (k == 4)
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) first[u][e] = big[u][e];
+                uint32_t a[3][4], b[3][2][4];
+#pragma unroll
+                for (int p = 0; p < 3; ++p) {
+                    tq_ldm4(a[p], sq + p * F::K_PART + tq_piece<DK>(16 * warp + ln.a_row, 2 * k + ln.a_c));
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) tq_ldm4(b[p][j], sk + p * F::K_PART + tq_piece<DK>(32 * grp + 16 * j + ln.b_row, 2 * k + ln.b_c));
+                }
+                if (k == 0) tq_six<4, true, true>(big, small, a, b);
+                else if (k == 4) tq_six<4, true, false>(big, small, a, b);
+                else tq_six<4, false, false>(big, small, a, b);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const int t = 16 * warp + ln.r + 8 * r, s = 32 * grp + 8 * u + ln.c;
+                // a token never meets a later one, whatever that is
+                auto val = [&](int e) {
+                    const int at = s + (e & 1);
+                    return at > t ? 0.f : m[t * LD + at] * m[at * LD + L] * ((DK > 64 ? first[u][e] + big[u][e] : big[u][e]) + small[u][e]);
+                };
+                const float x = val(2 * r), z = val(2 * r + 1);
+                own[r] += x + z;
+                const int at = 2 * (u & 1) + r;
+                if (grp == 0) tq_split2(x, z, P[u >> 1][0][at], P[u >> 1][1][at], P[u >> 1][2][at]);
+                else tq_split2(x, z, P[2 + (u >> 1)][0][at], P[2 + (u >> 1)][1][at], P[2 + (u >> 1)][2][at]);
+            }
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        own[r] += __shfl_xor_sync(0xffffffffu, own[r], 1);
+        own[r] += __shfl_xor_sync(0xffffffffu, own[r], 2);
+    }
+    const float A[2] = {s_A[16 * warp + ln.r], s_A[16 * warp + ln.r + 8]};
+    for (int q = 0; q < DV / 32; ++q) {
+        __syncthreads();               // what was there has been used
+        if (q == 0 && ln.c == 0)       // n . q
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const int t = 16 * warp + ln.r + 8 * r;
+                if (t < c.n) dots[(size_t)(c.t0 + t) * heads + h] = s_A[t] * s_a[t] + own[r];
+            }
+#pragma unroll
+        for (int i = 0; i < SN; ++i) { const int at = (i * THREADS + tid) * 4; tq_put4<DK>(sk, F::SQ_PART, at / DK, at % DK, ns[i]); }
+#pragma unroll
+        for (int i = 0; i < VN; ++i) {
+            const int t = (i * THREADS + tid) >> 3, e = (tid & 7) * 4;
+            if (odd(nv[i]) != 0.f) { atomicMin(&s_bad[q & 1], t); nv[i] = zero4(); }
+            const TqSplit4 v = tq_split4(nv[i]);
+            const uint32_t at = sv + piece32(t, e >> 3) + (e & 4) * 2;
+            asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(v.h.x), "r"(v.h.y) : "memory");
+            asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at + F::VQ_PART), "r"(v.m.x), "r"(v.m.y) : "memory");
+            asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at + 2 * F::VQ_PART), "r"(v.l.x), "r"(v.l.y) : "memory");
+        }
+        if (q + 1 < DV / 32) ask(q + 1);
         __syncthreads();
-        Vs = Y;
-    }
+        if (tid == 0) s_bad[(q + 1) & 1] = L;
+        float big[4][4], small[4][4], o[4][4];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const float A = s_A[4 * ty + r];
-        const tq_f32x2 AA = tq_pack2(A, A);
+        for (int k = 0; k < DK / 16; ++k) {
+            if (k == 4)
 #pragma unroll
-        for (int j = 0; j < 2 * RJ; ++j) acc[r][j] = tq_mul2(acc[r][j], AA);
-    }
-    add_earlier<RJ, L, DV>(acc, Pt, Vs, ty, tx);
+                for (int u = 0; u < 4; ++u)
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const int t = 4 * ty + r;
-        if (t < c.n)
+                    for (int e = 0; e < 4; ++e) o[u][e] = big[u][e];
+            uint32_t a[3][4], b[3][2][4];
 #pragma unroll
-            for (int j = 0; j < RJ; ++j)
-                *reinterpret_cast<float4*>(y + ((size_t)(c.t0 + t) * heads + h) * DV + 64 * j + 4 * tx) = four(acc[r][2 * j], acc[r][2 * j + 1]);
-    }
-    // n . q: the column whose value is one
-    if (tid < c.n) {
-        const float* n0 = St + (size_t)DV * DK;
-        float from = 0.f, own = 0.f;
-#pragma unroll 4
-        for (int k = 0; k < DK; ++k) from += Qt[k * L + 4 * group_at(k, tid >> 2) + (tid & 3)] * n0[k];
-        for (int s = 0; s <= tid; ++s) own += Pt[s * L + tid];
-        dots[(size_t)(c.t0 + tid) * heads + h] = s_A[tid] * from + own;
+            for (int p = 0; p < 3; ++p) {
+                tq_ldm4(a[p], sq + p * F::K_PART + tq_piece<DK>(16 * warp + ln.a_row, 2 * k + ln.a_c));
+#pragma unroll
+                for (int j = 0; j < 2; ++j) tq_ldm4(b[p][j], sk + p * F::SQ_PART + tq_piece<DK>(16 * j + ln.b_row, 2 * k + ln.b_c));
+            }
+            if (k == 0) tq_six<4, true, true>(big, small, a, b);
+            else if (k == 4) tq_six<4, true, false>(big, small, a, b);
+            else tq_six<4, false, false>(big, small, a, b);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) o[u][e] = A[e >> 1] * ((DK > 64 ? o[u][e] + big[u][e] : big[u][e]) + small[u][e]);
+#pragma unroll
+        for (int k = 0; k < L / 16; ++k) {
+            if (k > warp) break;       // later tokens
+            uint32_t b[3][2][4];
+#pragma unroll
+            for (int p = 0; p < 3; ++p)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) tq_ldm4t(b[p][j], sv + p * F::VQ_PART + piece32(16 * k + ln.t_row, 2 * j + ln.t_c));
+            if (k == 0) tq_six<4, true, true>(big, small, P[k], b); else tq_six<4, false, false>(big, small, P[k], b);
+        }
+        const int bad = *(volatile int*)&s_bad[q & 1];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const int t = 16 * warp + ln.r + 8 * r;
+            float* at = y + ((size_t)(c.t0 + t) * heads + h) * DV + 32 * q + ln.c;
+            if (t < c.n)
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    auto sum = [&](int e) { return t < bad ? o[u][e] + (big[u][e] + small[u][e]) : NAN; };
+                    *reinterpret_cast<float2*>(at + 8 * u) = make_float2(sum(2 * r), sum(2 * r + 1));
+                }
+        }
     }
 }
 
 template <int DK, int DV>
-int launch_memory(const float* rows, int C, int q_off, int k_off, int v_off, const float2* gates, float* state, long long slot_stride,
-                  float* y, float* dots, float* ends, float* decays, int chunks, int group, int n_seqs, int heads, const int* cu, const int* slots,
-                  cudaStream_t stream) {
-    constexpr int A_BYTES = L * (DK + DV) * 4, C_BYTES = (DK * L + 64 * (DK > DV ? DK : DV) + 64 * DV + L * L) * 4;
-    auto ka = memory_ends_kernel<DK, DV>;
-    auto kc = memory_outputs_kernel<DK, DV>;
-    static std::atomic<unsigned long long> asked_a{0}, asked_c{0};
-    cudaError_t e = tq_reserve_smem(ka, A_BYTES, asked_a);
-    if (e == cudaSuccess) e = tq_reserve_smem(kc, C_BYTES, asked_c);
-    if (e != cudaSuccess) TQ_FAIL(-1, "memory_chunks: %d bytes of shared memory refused: %s", C_BYTES, cudaGetErrorString(e));
+int launch_memory(const float* rows, int C, int q_off, int k_off, int v_off, const float2* gates, float* state, long long slot_stride, float* y,
+           float* dots, float* ends, float* last, int chunks, int group, int n_seqs, int heads, const int* cu, const int* slots, cudaStream_t stream) {
+    using F = MemoryCfg<DK, DV>;
+    static std::atomic<unsigned long long> asked[2];
+    cudaError_t e = tq_reserve_smem(memory_ends_kernel<DK, DV>, F::ENDS_BYTES, asked[0]);
+    if (e == cudaSuccess) e = tq_reserve_smem(memory_outputs_kernel<DK, DV>, F::OUT_BYTES, asked[1]);
+    if (e != cudaSuccess) TQ_FAIL(-1, "memory_chunks: %d bytes of shared memory refused: %s", F::OUT_BYTES, cudaGetErrorString(e));
     const int per_head = (DV + 1) * DK;
     for (int chunk0 = 0; chunk0 < chunks; chunk0 += group) {
         const int n = chunks - chunk0 < group ? chunks - chunk0 : group;
-        tq_launch(dim3(n, heads), THREADS, A_BYTES, stream)(ka, rows, C, k_off, v_off, gates, heads, chunk0, cu, n_seqs, ends, decays);
+        tq_launch(dim3(n, heads), THREADS, F::ENDS_BYTES, stream)(memory_ends_kernel<DK, DV>, rows, C, k_off, v_off, gates, heads, chunk0, cu, n_seqs, ends, last);
         tq_launch(dim3((per_head + 255) / 256, n_seqs, heads), 256, 0, stream)(chunk_starts_kernel, state, slot_stride, slots, ends,
-            (const float*)decays, heads, per_head, chunk0, n, cu);
-        tq_launch(dim3(n, heads), THREADS, C_BYTES, stream)(kc, rows, C, q_off, k_off, v_off, gates, heads, chunk0, cu, n_seqs, (const float*)ends, y, dots);
+            (const float*)last, heads, per_head, chunk0, n, cu);
+        tq_launch(dim3(n, heads), THREADS, F::OUT_BYTES, stream)(memory_outputs_kernel<DK, DV>, rows, C, q_off, k_off, v_off, gates, heads, chunk0, cu,
+            n_seqs, (const float*)ends, y, dots);
     }
     TQ_CHECK_LAUNCH("memory_chunks");
     return 0;
 }
 
-
 }  // namespace tq_recurrence
 
 // rows fp32 [T, C] with q, k (heads x dk) and v (heads x dv) from columns that are multiples of four, gates [T, heads] pairs of
 // logarithms; state: the sequences' [heads][dv + 1][dk] at slots[s] * slot_stride, renewed; y [T, heads * dv], dots [T, heads] =
-// n . q.  chunks: at least the sum of ceil(run / 64); ends [group, heads, dv + 1, dk] and decays [group, heads]: scratch of a group.
+// n . q.  chunks: at least the sum of ceil(run / 64); ends [group, heads, dv + 1, dk] and last [group, heads]: scratch of a group.
 TQ_EXPORT int tq_memory_chunks(const float* rows, int C, int q_off, int k_off, int v_off, const void* gates, float* state,
-                               long long slot_stride, float* y, float* dots, float* ends, float* decays, int chunks, int group, int n_seqs,
+                               long long slot_stride, float* y, float* dots, float* ends, float* last, int chunks, int group, int n_seqs,
                                int heads, int dk, int dv, const int* cu_seqlens, const int* slots, cudaStream_t stream) {
     if (n_seqs == 0 || chunks == 0) return 0;
     TQ_REQUIRE(heads >= 1 && heads <= 65535 && n_seqs <= 65535 && group >= 1, "memory_chunks: %d heads, %d sequences, groups of %d chunks", heads, n_seqs, group);
     TQ_REQUIRE(C % 4 == 0 && q_off % 4 == 0 && k_off % 4 == 0 && v_off % 4 == 0 && ((uintptr_t)rows & 15) == 0 && ((uintptr_t)y & 15) == 0
                && ((uintptr_t)ends & 15) == 0, "memory_chunks: rows of %d floats are not aligned to 16 bytes", C);
 #define MEM_CASE(DK_, DV_) if (dk == DK_ && dv == DV_) return tq_recurrence::launch_memory<DK_, DV_>(rows, C, q_off, k_off, v_off, (const float2*)gates, \
-        state, slot_stride, y, dots, ends, decays, chunks, group, n_seqs, heads, cu_seqlens, slots, stream);
+        state, slot_stride, y, dots, ends, last, chunks, group, n_seqs, heads, cu_seqlens, slots, stream);
     MEM_CASE(64, 64) MEM_CASE(64, 128) MEM_CASE(128, 64) MEM_CASE(128, 128)
 #undef MEM_CASE
     TQ_FAIL(-2, "memory_chunks: keys of %d and values of %d elements", dk, dv);

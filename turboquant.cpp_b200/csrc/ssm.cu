@@ -16,7 +16,6 @@
 //   delta_scan, ...    the delta rule with a decay per key channel or per head (their own headers below)
 #include <type_traits>
 
-#include "common.cuh"
 #include "recurrence.cuh"
 
 TQ_DEFINE_LAST_ERROR

@@ -1,5 +1,5 @@
-"""Recurrences over runs of many tokens in chunks of 64, as float32 matrix products: the matrix memory (csrc/recurrence.cuh, in the library of
-csrc/ssm.cu) and the delta rule with one decay per head (csrc/delta_chunks.cu)."""
+"""Recurrences over runs of many tokens in chunks of 64, as float32 matrix products: the matrix memory (csrc/recurrence.cuh, in the
+library of csrc/ssm.cu) and the delta rule with one decay per head (csrc/delta_chunks.cu)."""
 from __future__ import annotations
 
 from ctypes import c_float, c_int, c_longlong, c_void_p
@@ -13,7 +13,7 @@ from .gemm_tc import status_word
 from .ssm import ctypes_ptr
 
 _LIB = "ssm"
-CHUNK = 64               # csrc/recurrence.cuh L
+CHUNK = 64               # csrc/chunks.cuh L
 SIZES = (64, 128)        # key and value sizes the kernels are built for
 # the most bytes of chunks' states a step holds at a time, 126 chunks of 16 heads of 128 x 129; longer steps go in groups of equal size
 # (8,192 tokens of that layer: 718 us in one piece of 135 MB, 746 in groups of 63, 63 and 2)
