@@ -151,8 +151,8 @@ TQ_EXPORT int tq_bias_kv_write(const float* qkv, void* q_out, void* cache, int a
 // heads from shared memory; then a warp per query, key or value head.  Steps of few tokens share a token's heads out over blocks of
 // four warps (grid y), a head a warp, each block with the angles it needs: see the launcher.  What bounds it is the bytes (fp32 rows in, half of them out)
 // once the angles are shared: 4,096 tokens, 16 + 4 + 4 heads of 128, all turned, took 60.6 us with a sincosf per head and
-// pair (two per pair of a value) and takes 39 us (48 with every head passed through shared memory: 360 instructions a warp
-// and head); the bytes alone are 11.5 us.  vec: 16-byte reads and 8-byte writes (bf16), where sizes, strides and pointers allow them.
+// pair (two per pair of a value) and 37 us so (48 with every head passed through shared memory: 360 instructions a warp
+// and head); the bytes alone are 11.5 us.  Long steps take the kernel below it where they can.  vec: 16-byte reads and 8-byte writes (bf16), where sizes, strides and pointers allow them.
 // ---------------------------------------------------------------------------------------
 #define BA_ROT_MAX_WARPS 16
 // Steps of up to this many heads (tokens x heads) take a warp a head: 5,120 (64 tokens of 64 + 8 + 8 heads) 4.8 us against 6.7 with a
@@ -332,6 +332,152 @@ bias_kv_write_rot_kernel(const float* __restrict__ qkv, int row_stride, TA* __re
     }
 }
 
+// Long steps whose heads stay in registers (sizes up to 128 in whole lanes, no norm over whole rows): a warp per token, or per some of a
+// token's heads where the tokens are few.  The lane's sines and cosines are in its registers for all of them, no block waits for a
+// token's angles or its page, and four heads of a kind are worked on side by side while the next four are on their way.  4,096 tokens of
+// 16 + 4 + 4 heads of 128, 75.5 MB: 21 us, with a block a token (the kernel above) 37; 2,048 tokens 14.1 / 19.7, 300 4.4 / 7.6; head after
+// head 30 (the sums over the lanes and the roots wait for one another).  11.5 us are the bytes at the copy rate; the rest is instructions.
+struct BaTurn { float c[4], s[4]; };   // of the lane's four elements (neighbours: of its two pairs)
+// n angles pos * freq[i] of a head, by way of the warp's n pairs in shared memory
+__device__ __forceinline__ BaTurn ba_lane_turn(float2* cs, const float* __restrict__ freq, int n, int halves, float pos, int lane) {
+    BaTurn t;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) { t.c[k] = 1.f; t.s[k] = 0.f; }
+    __syncwarp();
+    for (int i = lane; i < n; i += 32) {
+        float sn, c;
+        sincosf(pos * freq[i], &sn, &c);
+        cs[i] = make_float2(c, sn);
+    }
+    __syncwarp();
+    const int step = n >> 2;
+    if (halves ? lane < 2 * step : 2 * lane < n) {
+        const int first = halves ? 4 * (lane < step ? lane : lane - step) : 2 * lane;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (halves || k < 2) { const float2 v = cs[first + k]; t.c[k] = v.x; t.s[k] = v.y; }
+    }
+    return t;
+}
+// ba_turn_lanes with the angles in registers
+__device__ __forceinline__ void ba_turn_regs(float4& x, const BaTurn& t, int n, int halves, float mag, int lane) {
+    if (halves) {
+        const int step = n >> 2;
+        const bool lo = lane < step, turned = lane < 2 * step;
+        const int from = turned ? (lo ? lane + step : lane - step) : lane;
+        float4 y;
+        y.x = __shfl_sync(0xffffffffu, x.x, from);
+        y.y = __shfl_sync(0xffffffffu, x.y, from);
+        y.z = __shfl_sync(0xffffffffu, x.z, from);
+        y.w = __shfl_sync(0xffffffffu, x.w, from);
+        if (turned) {
+            const float f = lo ? -1.f : 1.f;
+            x.x = (x.x * t.c[0] + f * y.x * t.s[0]) * mag;
+            x.y = (x.y * t.c[1] + f * y.y * t.s[1]) * mag;
+            x.z = (x.z * t.c[2] + f * y.z * t.s[2]) * mag;
+            x.w = (x.w * t.c[3] + f * y.w * t.s[3]) * mag;
+        }
+    } else if (2 * lane < n) {
+        x = make_float4((x.x * t.c[0] - x.y * t.s[0]) * mag, (x.y * t.c[0] + x.x * t.s[0]) * mag,
+                        (x.z * t.c[1] - x.w * t.s[1]) * mag, (x.w * t.c[1] + x.z * t.s[1]) * mag);
+    }
+}
+constexpr int TURN_WARPS = 4, TURN_AHEAD = 4;      // of a block; heads worked on together
+constexpr int TURN_FULL = 8192;                    // warps that a token's heads are shared out for: 4,096 tokens 21.0 us, with 4,096 warps 22.3, 12,288 23.4
+template <typename TA>
+__global__ void __launch_bounds__(32 * TURN_WARPS)
+bias_kv_turn_kernel(const float* __restrict__ qkv, int row_stride, TA* __restrict__ q_out, TA* __restrict__ cache, const float* __restrict__ freq,
+                    int rot_dims, int halves, float mag, float unit_eps, const float* __restrict__ q_norm_w, const float* __restrict__ k_norm_w,
+                    float norm_eps, const float* __restrict__ v_freq, int v_share, int v_from_k, float temp_coef, int temp_every,
+                    const int* __restrict__ positions, const int* __restrict__ seq_of_token, const int* __restrict__ page_table, int table_stride,
+                    int page_size, int T_, int nh, int nkv, int dk, int dv, int n_seqs, int n_pages, int per) {
+    tq_grid_wait();                    // everything below may read what the previous kernel wrote
+    tq_grid_launch_dependents();       // the next kernel's CTAs may move in as SMs free up
+    __shared__ __align__(16) float2 s_cs[TURN_WARPS][64];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = blockIdx.x * TURN_WARPS + warp, e = 4 * lane;
+    if (t >= T_) return;
+    const int nq = nh * dk, nk = nkv * dk, dr = dk + dv, last = min(cache == nullptr ? nh : nh + 2 * nkv, ((int)blockIdx.y + 1) * per);
+    const float* row = qkv + (size_t)t * row_stride;
+    const int pos = positions[t];
+    auto read = [&](int head) {
+        if (head >= last || e >= (head < nh + nkv ? dk : dv)) return make_float4(0.f, 0.f, 0.f, 0.f);
+        if (head < nh + nkv) return *reinterpret_cast<const float4*>(row + (size_t)head * dk + e);
+        const int g = head - nh - nkv;
+        return *reinterpret_cast<const float4*>(row + nq + (v_from_k ? 0 : nk) + (size_t)(v_share == 1 ? g : g / v_share) * dv + e);
+    };
+    int head = blockIdx.y * per;
+    float4 next[TURN_AHEAD];
+#pragma unroll
+    for (int i = 0; i < TURN_AHEAD; ++i) next[i] = read(head + i);
+    TA* cached = nullptr;              // the token's slot, key/value head 0
+    if (cache != nullptr && last > nh) {
+        const int* table = page_table + (size_t)TQ_CHECKED(seq_of_token[t], n_seqs, TQ_IDX_SEQUENCE) * table_stride;
+        const int page = TQ_CHECKED(table[TQ_CHECKED(pos / page_size, table_stride, TQ_IDX_TABLE_COLUMN)], n_pages, TQ_IDX_PAGE);
+        cached = cache + ((size_t)page * nkv * page_size + pos % page_size) * dr;
+    }
+    BaTurn turn, v_turn;
+    if (rot_dims > 0 && head < nh + nkv) turn = ba_lane_turn(s_cs[warp], freq, rot_dims >> 1, halves, (float)pos, lane);
+    if (v_freq != nullptr && last > nh + nkv) v_turn = ba_lane_turn(s_cs[warp], v_freq, dv >> 1, halves, (float)pos, lane);
+    const float temp = temp_every > 0 ? 1.0f + temp_coef * logf((float)((pos + 1) / temp_every) + 1.0f) : 1.f;
+    float4 qw = make_float4(1.f, 1.f, 1.f, 1.f), kw = qw;
+    if (q_norm_w != nullptr && e < dk) qw = make_float4(q_norm_w[e], q_norm_w[e + 1], q_norm_w[e + 2], q_norm_w[e + 3]);
+    if (k_norm_w != nullptr && e < dk) kw = make_float4(k_norm_w[e], k_norm_w[e + 1], k_norm_w[e + 2], k_norm_w[e + 3]);
+    const float inv_dk = 1.0f / (float)dk;
+    // four heads of a kind, or some of them, side by side: their sums over the lanes do not wait for one another
+    auto heads = [&](float4 (&x)[TURN_AHEAD], int at, int n, bool is_q, bool is_v) {
+        auto sums = [&](float (&ss)[TURN_AHEAD]) {
+#pragma unroll
+            for (int i = 0; i < TURN_AHEAD; ++i) ss[i] = x[i].x * x[i].x + x[i].y * x[i].y + x[i].z * x[i].z + x[i].w * x[i].w;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                for (int i = 0; i < TURN_AHEAD; ++i) ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], o);
+        };
+        float ss[TURN_AHEAD];
+        if (!is_v && (is_q ? q_norm_w : k_norm_w) != nullptr) {
+            const float4 w = is_q ? qw : kw;
+            sums(ss);
+#pragma unroll
+            for (int i = 0; i < TURN_AHEAD; ++i) {
+                const float r = 1.0f / sqrtf(ss[i] * inv_dk + norm_eps);
+                x[i] = make_float4(x[i].x * r * w.x, x[i].y * r * w.y, x[i].z * r * w.z, x[i].w * r * w.w);
+            }
+        }
+        if (is_v ? v_freq != nullptr : rot_dims > 0) {
+#pragma unroll
+            for (int i = 0; i < TURN_AHEAD; ++i) {
+                if (is_v) ba_turn_regs(x[i], v_turn, dv >> 1, halves, 1.0f, lane); else ba_turn_regs(x[i], turn, rot_dims >> 1, halves, mag, lane);
+            }
+        }
+        float r[TURN_AHEAD];
+#pragma unroll
+        for (int i = 0; i < TURN_AHEAD; ++i) r[i] = is_q ? temp : 1.f;
+        if (!is_v && unit_eps > 0.f) {
+            sums(ss);
+#pragma unroll
+            for (int i = 0; i < TURN_AHEAD; ++i) r[i] *= 1.0f / sqrtf(ss[i] * inv_dk + unit_eps);
+        }
+        if (e < (is_v ? dv : dk)) {
+            const int g = at - nh - (is_v ? nkv : 0), step = is_q ? dk : page_size * dr;
+            TA* dst = (is_q ? q_out + ((size_t)t * nh + at) * dk : cached + (size_t)g * step + (is_v ? dk : 0)) + e;
+#pragma unroll
+            for (int i = 0; i < TURN_AHEAD; ++i)
+                if (i < n) ba_store4(dst + (size_t)i * step, make_float4(x[i].x * r[i], x[i].y * r[i], x[i].z * r[i], x[i].w * r[i]));
+        }
+    };
+#pragma unroll 1
+    while (head < last) {              // up to four heads, none of another kind behind them
+        const int ends = head < nh ? nh : head < nh + nkv ? nh + nkv : last, n = min(min(ends, last) - head, TURN_AHEAD);
+        float4 now[TURN_AHEAD];
+#pragma unroll
+        for (int i = 0; i < TURN_AHEAD; ++i) now[i] = next[i];
+#pragma unroll
+        for (int i = 0; i < TURN_AHEAD; ++i) next[i] = read(head + n + i);
+        heads(now, head, n, head < nh, head >= nh + nkv);
+        head += n;
+    }
+}
+
 // qkv: fp32 rows of row_stride floats that begin with [q | k | v] (v: nkv / v_share heads; none with v_from_k); freq: fp32
 // [rot_dims / 2] (null with rot_dims 0).
 TQ_EXPORT int tq_bias_kv_write_rot(const float* qkv, int row_stride, void* q_out, void* cache, int act_dtype,
@@ -359,6 +505,17 @@ TQ_EXPORT int tq_bias_kv_write_rot(const float* qkv, int row_stride, void* q_out
     const size_t smem = (size_t)warps * room * sizeof(float) + (size_t)(rot_dims / 2 + 1 + (v_freq && dv <= BA_MAX_DIM ? dv / 2 : 0)) * sizeof(float2);
     const int vec = dk % 4 == 0 && dv % 4 == 0 && row_stride % 4 == 0 && ((uintptr_t)qkv & 15) == 0 && ((uintptr_t)q_out & 15) == 0
                     && ((uintptr_t)cache & 15) == 0;
+    const int unit = halves ? 8 : 4;
+    if (vec && !norm_rows && !spread && dk <= 128 && dv <= 128 && rot_dims % unit == 0 && (v_freq == nullptr || dv % unit == 0)) {
+        // a token's heads are shared out, four or a multiple of it a warp, while the warps are fewer than TURN_FULL
+        const int shares = T_ >= TURN_FULL ? 1 : TURN_FULL / T_, per = shares >= (heads + 3) / 4 ? 4 : ((heads + shares - 1) / shares + 3) / 4 * 4;
+        TQ_DISPATCH(act_dtype, TA,
+            (tq_launch(dim3((T_ + TURN_WARPS - 1) / TURN_WARPS, (heads + per - 1) / per), 32 * TURN_WARPS, 0, stream)(bias_kv_turn_kernel<TA>, qkv, row_stride,
+                (TA*)q_out, (TA*)cache, freq, rot_dims, halves, mag, unit_eps, q_norm_w, k_norm_w, norm_eps, v_freq, v_share, v_from_k, temp_coef,
+                temp_every, positions, seq_of_token, page_table, table_stride, page_size, T_, nh, nkv, dk, dv, n_seqs, n_pages, per)));
+        TQ_CHECK_LAUNCH("bias_kv_write_rot");
+        return 0;
+    }
     TQ_DISPATCH(act_dtype, TA,
         (tq_launch(dim3(T_, groups), 32 * warps, smem, stream)(bias_kv_write_rot_kernel<TA>, qkv, row_stride, (TA*)q_out, (TA*)cache, freq, rot_dims,
             halves, mag, unit_eps, q_norm_w, k_norm_w, norm_eps, norm_rows, v_freq, v_share, v_from_k, temp_coef, temp_every, positions,
@@ -447,6 +604,47 @@ heads_unrotate_gate_kernel(const TA* __restrict__ o, const float* __restrict__ g
     }
 }
 
+// Long steps: a warp per token, or per some of its heads, as above.  16 heads of 128: 4,096 tokens 10.3 us (13.0 with a block a token), 2,048
+// 6.4 (7.6), 1,500 6.2 (5.9).
+template <typename TA>
+__global__ void __launch_bounds__(32 * TURN_WARPS)
+heads_unturn_gate_kernel(const TA* __restrict__ o, const float* __restrict__ gates, int gate_stride, int gate_off, const float* __restrict__ v_freq,
+                         int halves, const int* __restrict__ positions, TA* __restrict__ out, int T_, int nh, int dv, int per) {
+    tq_grid_wait();                    // everything below may read what the previous kernel wrote
+    tq_grid_launch_dependents();       // the next kernel's CTAs may move in as SMs free up
+    __shared__ __align__(16) float2 s_cs[TURN_WARPS][64];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = blockIdx.x * TURN_WARPS + warp, e = 4 * lane;
+    if (t >= T_) return;
+    const int last = min(nh, ((int)blockIdx.y + 1) * per);
+    const TA* src = o + (size_t)t * nh * dv + e;
+    const float* gate = gates + (size_t)t * gate_stride + gate_off;
+    auto read = [&](int h) { return h < last && e < dv ? ba_load4(src + (size_t)h * dv) : make_float4(0.f, 0.f, 0.f, 0.f); };
+    int h = blockIdx.y * per;
+    float4 next[TURN_AHEAD];
+    float z[TURN_AHEAD];
+#pragma unroll
+    for (int i = 0; i < TURN_AHEAD; ++i) { next[i] = read(h + i); z[i] = h + i < last ? gate[h + i] : 0.f; }
+    BaTurn turn;
+    if (v_freq != nullptr) turn = ba_lane_turn(s_cs[warp], v_freq, dv >> 1, halves, (float)-positions[t], lane);
+#pragma unroll 1
+    for (; h < last; h += TURN_AHEAD) {
+        float4 now[TURN_AHEAD];
+        float zn[TURN_AHEAD];
+#pragma unroll
+        for (int i = 0; i < TURN_AHEAD; ++i) { now[i] = next[i]; zn[i] = z[i]; }
+#pragma unroll
+        for (int i = 0; i < TURN_AHEAD; ++i) { next[i] = read(h + TURN_AHEAD + i); z[i] = h + TURN_AHEAD + i < last ? gate[h + TURN_AHEAD + i] : 0.f; }
+#pragma unroll
+        for (int i = 0; i < TURN_AHEAD; ++i) {
+            if (h + i >= last) break;  // the same for the whole warp
+            float4 x = now[i];
+            if (v_freq != nullptr) ba_turn_regs(x, turn, dv >> 1, halves, 1.0f, lane);
+            const float g = 1.0f / (1.0f + expf(-zn[i]));
+            if (e < dv) ba_store4(out + ((size_t)t * nh + h + i) * dv + e, make_float4(x.x * g, x.y * g, x.z * g, x.w * g));
+        }
+    }
+}
+
 TQ_EXPORT int tq_heads_unrotate_gate(const void* o, int act_dtype, const float* gates, int gate_stride, int gate_off,
                                      const float* v_freq, int halves, const int* positions, void* out, int T_, int nh, int dv,
                                      cudaStream_t stream) {
@@ -456,6 +654,14 @@ TQ_EXPORT int tq_heads_unrotate_gate(const void* o, int act_dtype, const float* 
     TQ_REQUIRE(v_freq == nullptr || dv % 2 == 0, "heads_unrotate_gate: values of %d elements cannot be rotated in pairs", dv);
     const int most = T_ > 592 ? 8 : BA_ROT_MAX_WARPS, warps = nh >= most ? most : (nh >= 8 ? 8 : 4);
     const int vec = dv % 4 == 0 && ((uintptr_t)o & 15) == 0 && ((uintptr_t)out & 15) == 0;
+    if (vec && T_ >= 1792 && dv <= 128 && (v_freq == nullptr || dv % (halves ? 8 : 4) == 0)) {
+        const int shares = T_ >= 4096 ? 1 : 4096 / T_, per = shares >= (nh + 3) / 4 ? 4 : ((nh + shares - 1) / shares + 3) / 4 * 4;
+        TQ_DISPATCH(act_dtype, TA,
+            (tq_launch(dim3((T_ + TURN_WARPS - 1) / TURN_WARPS, (nh + per - 1) / per), 32 * TURN_WARPS, 0, stream)(heads_unturn_gate_kernel<TA>, (const TA*)o, gates,
+                gate_stride, gate_off, v_freq, halves, positions, (TA*)out, T_, nh, dv, per)));
+        TQ_CHECK_LAUNCH("heads_unrotate_gate");
+        return 0;
+    }
     // more than two heads a warp: over several blocks, where they still run all at once (64 heads, one token: 2.67 us with a sincosf per
     // element and four heads a block, 3.38 with all heads in one block)
     const int shares = (nh + 2 * warps - 1) / (2 * warps), groups = (long long)T_ * shares <= 592 ? shares : 1;
