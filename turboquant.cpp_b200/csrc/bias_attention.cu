@@ -1401,16 +1401,29 @@ bias_attention_runs_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloa
 }
 
 // ---------------------------------------------------------------------------------------
-// Token form on tensor cores, bfloat16, for several query heads per key/value head: the sixteen rows of
-// mma.sync m16n8k16 are up to sixteen heads of one (token, key/value head).  Grid (token, key/value head x chunks of
-// 16 heads, key range), four warps; the visible positions are walked in tiles of 16 absolute positions (a tile lies
+// Token form on tensor cores, bfloat16, for several query heads per key/value head.  The keys are the rows of
+// mma.sync m16n8k16 and the heads its columns: S^T = K q^T, O^T = V^T P^T, eight heads of one (token, key/value head) a
+// product (heads as rows would leave the rows past the group's heads to be computed for nothing, in the softmax too),
+// sixteen with NT 2.  P^T turns from accumulator to operand with movmatrix.  Grid (token, key/value head x chunks of
+// 8 NT heads, key range), four warps; the visible positions are walked in tiles of 16 absolute positions (a tile lies
 // in one page: one contiguous piece of the cache), the kept first tiles and then the window's; warp w takes every
-// fourth tile of the block's range through a two-stage cp.async ring of its own.  Scores, mask, bias and online
-// softmax on the accumulator fragments as in the kernel for runs; the warps' states are joined through shared
-// memory in warp order, the ranges' by bias_attention_merge.  The page size is a multiple of 16.
+// fourth tile of the block's range through a cp.async ring of its own, a tile's page looked up while the tiles
+// before it are on their way.  The warps' states are joined through shared memory in warp order, the ranges' by
+// bias_attention_merge.  The page size is a multiple of 16.
+// Bound by the rows: 64 tokens x 4 key/value heads x 4 heads, 2,049 keys of 128 + 128 (269 MB, 41 us at 6.5 TB/s) take 44 us in one
+// range, 51.5 + 4.7 in three with heads as rows (730 instructions a tile of 16 keys there, 350 here).  Two stages and three blocks
+// an SM (203 KB of rings), not three stages and two blocks: 30.2 us against 30.7 for 1,024 keys, 49.2 against 51.0 for 2,048 (events
+// around one launch), 43.0 against 51.2 at 96 tokens; only where the last round of blocks is nearly empty do three stages win
+// (128 tokens, 512 blocks for 444 places: 102 against 92).
 // ---------------------------------------------------------------------------------------
 #define BH_K 16
-template <int DK, int DV>
+#define BH_STAGES 2
+__device__ __forceinline__ uint32_t bh_turn(uint32_t x) {      // an 8 x 8 tile of 16-bit values, transposed over the warp
+    uint32_t y;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
+    return y;
+}
+template <int DK, int DV, int NT>
 __global__ void __launch_bounds__(BA_WARPS * 32, 3)
 bias_attention_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ cache,
                             const float* __restrict__ bias_t, int far, const float* __restrict__ sink,
@@ -1420,16 +1433,16 @@ bias_attention_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bflo
                             int n_splits, int nh, int nkv, int n_seqs, int n_pages) {
     tq_grid_wait();                    // everything below may read what the previous kernel wrote
     tq_grid_launch_dependents();       // the next kernel's CTAs may move in as SMs free up
-    constexpr int DR = DK + DV, LD = DR + 8;
+    constexpr int DR = DK + DV, LD = DR + 8, HEADS = 8 * NT, LO = DV + 4;
     constexpr int STAGE = BH_K * LD;                         // elements of a warp's stage
     extern __shared__ __align__(16) uint8_t bh_smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    __nv_bfloat16* ring = reinterpret_cast<__nv_bfloat16*>(bh_smem) + (size_t)warp * 2 * STAGE;
+    __nv_bfloat16* ring = reinterpret_cast<__nv_bfloat16*>(bh_smem) + (size_t)warp * BH_STAGES * STAGE;
     const int G_all = nh / nkv;
-    const int chunks = (G_all + 15) / 16;
+    const int chunks = (G_all + HEADS - 1) / HEADS;
     const int t = blockIdx.x, g = blockIdx.y / chunks, chunk = blockIdx.y - g * chunks, split = blockIdx.z;
-    const int h0 = g * G_all + chunk * 16;
-    const int G = min(16, G_all - chunk * 16);
+    const int h0 = g * G_all + chunk * HEADS;
+    const int G = min(HEADS, G_all - chunk * HEADS);
     const int pos = positions[t];
     const int* table = page_table + (size_t)TQ_CHECKED(seq_of_token[t], n_seqs, TQ_IDX_SEQUENCE) * table_stride;
     if (cell > 0) { window = pos % cell + 1; keep_first = 0; }
@@ -1440,128 +1453,154 @@ bias_attention_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bflo
     const int per = (n_tiles + n_splits - 1) / n_splits;
     const int i0 = split * per, i1 = min(n_tiles, i0 + per);
 
-    auto load_tile = [&](int i, int stage) {
-        const int p0 = (i < kept ? i : first + (i - kept)) * BH_K;
-        const int page = TQ_CHECKED(table[TQ_CHECKED(p0 / page_size, table_stride, TQ_IDX_TABLE_COLUMN)], n_pages, TQ_IDX_PAGE);
-        const __nv_bfloat16* src = cache + (((size_t)max(page, 0) * nkv + g) * page_size + p0 % page_size) * DR;
+    auto base_of = [&](int i) { return (i < kept ? i : first + (i - kept)) * BH_K; };
+    auto rows_of = [&](int i) {                              // where the cache holds tile i's rows
+        const int p0 = base_of(i), column = p0 / page_size;
+        const int page = TQ_CHECKED(table[TQ_CHECKED(column, table_stride, TQ_IDX_TABLE_COLUMN)], n_pages, TQ_IDX_PAGE);
+        return cache + (((size_t)max(page, 0) * nkv + g) * page_size + (p0 - column * page_size)) * DR;
+    };
+    auto load_tile = [&](const __nv_bfloat16* src, int stage) {
         __nv_bfloat16* dst = ring + (size_t)stage * STAGE;
         constexpr int CPR = DR / 8;
-        for (int c = lane; c < BH_K * CPR; c += 32) {
-            const int r = c / CPR, k = c % CPR;
+#pragma unroll
+        for (int j = 0; j < (BH_K * CPR) / 32; ++j) {
+            const int c = j * 32 + lane, r = c / CPR, k = c % CPR;
             br_copy16(dst + r * LD + k * 8, src + r * DR + k * 8);
         }
     };
-    if (i0 + warp < i1) load_tile(i0 + warp, 0);
-    asm volatile("cp.async.commit_group;" ::: "memory");
+#pragma unroll
+    for (int j = 0; j < BH_STAGES - 1; ++j) {                // one commit per stage, also past the end: the count is uniform
+        if (i0 + warp + j * BA_WARPS < i1) load_tile(rows_of(i0 + warp + j * BA_WARPS), j);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    int next = i0 + warp + (BH_STAGES - 1) * BA_WARPS;       // the tile whose rows are looked up next
+    const __nv_bfloat16* ahead = next < i1 ? rows_of(next) : nullptr;
 
-    const int r_lo = lane >> 2, r_hi = r_lo + 8;             // the thread's two rows: heads h0 + r
-    uint32_t qf[DK / 16][4];
-    {
-        const __nv_bfloat16* q_lo = q + ((size_t)t * nh + h0 + r_lo) * DK + (lane & 3) * 2;
-        const __nv_bfloat16* q_hi = q + ((size_t)t * nh + h0 + r_hi) * DK + (lane & 3) * 2;
+    const int col = (lane & 3) * 2;                          // the thread's two columns of an accumulator: heads col, col + 1
+    uint32_t qf[NT][DK / 16][2];
+    const float* bias_of[NT][2];
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+        const int h = nt * 8 + (lane >> 2);
+        const __nv_bfloat16* q_h = q + ((size_t)t * nh + h0 + h) * DK + col;
 #pragma unroll
         for (int ks = 0; ks < DK / 16; ++ks) {
-            qf[ks][0] = r_lo < G ? *reinterpret_cast<const uint32_t*>(q_lo + ks * 16) : 0u;
-            qf[ks][1] = r_hi < G ? *reinterpret_cast<const uint32_t*>(q_hi + ks * 16) : 0u;
-            qf[ks][2] = r_lo < G ? *reinterpret_cast<const uint32_t*>(q_lo + ks * 16 + 8) : 0u;
-            qf[ks][3] = r_hi < G ? *reinterpret_cast<const uint32_t*>(q_hi + ks * 16 + 8) : 0u;
+            qf[nt][ks][0] = h < G ? *reinterpret_cast<const uint32_t*>(q_h + ks * 16) : 0u;
+            qf[nt][ks][1] = h < G ? *reinterpret_cast<const uint32_t*>(q_h + ks * 16 + 8) : 0u;
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int hb = nt * 8 + col + e;
+            bias_of[nt][e] = bias_t && hb < G ? bias_t + (size_t)(h0 + hb) * (far + 1) : nullptr;
         }
     }
-    const float* b_lo = bias_t && r_lo < G ? bias_t + (size_t)(h0 + r_lo) * (far + 1) : nullptr;
-    const float* b_hi = bias_t && r_hi < G ? bias_t + (size_t)(h0 + r_hi) * (far + 1) : nullptr;
-    float m_lo = -INFINITY, m_hi = -INFINITY, l_lo = 0.f, l_hi = 0.f;
-    float o[DV / 8][4];
+    float m[NT][2], l[NT][2], o[NT][DV / 16][4];
 #pragma unroll
-    for (int n = 0; n < DV / 8; ++n) { o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f; }
+    for (int nt = 0; nt < NT; ++nt) {
+        m[nt][0] = m[nt][1] = -INFINITY; l[nt][0] = l[nt][1] = 0.f;
+#pragma unroll
+        for (int n = 0; n < DV / 16; ++n) { o[nt][n][0] = o[nt][n][1] = o[nt][n][2] = o[nt][n][3] = 0.f; }
+    }
 
-    int stage = 0;
+    int stage = 0, fill = BH_STAGES - 1;
+    const int mi = lane >> 3;
     for (int i = i0 + warp; i < i1; i += BA_WARPS) {
-        if (i + BA_WARPS < i1) load_tile(i + BA_WARPS, stage ^ 1);
+        if (ahead != nullptr) load_tile(ahead, fill);
         asm volatile("cp.async.commit_group;" ::: "memory");
-        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        next += BA_WARPS;
+        ahead = next < i1 ? rows_of(next) : nullptr;
+        asm volatile("cp.async.wait_group %0;" ::"n"(BH_STAGES - 1) : "memory");
         __syncwarp();                                       // every lane's pieces of this tile have landed
         const __nv_bfloat16* tile = ring + (size_t)stage * STAGE;
-        const int p_base = (i < kept ? i : first + (i - kept)) * BH_K;
-        float s[2][4];
+        float s[NT][4], s2[NT][4];                          // even and odd steps of 16: two chains of products
 #pragma unroll
-        for (int n = 0; n < 2; ++n) { s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f; }
-        const int mi = lane >> 3;
+        for (int nt = 0; nt < NT; ++nt) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) s[nt][c] = s2[nt][c] = 0.f;
+        }
+        const __nv_bfloat16* keys = tile + ((mi & 1) * 8 + (lane & 7)) * LD + (mi >> 1) * 8;
 #pragma unroll
         for (int ks = 0; ks < DK / 16; ++ks) {
-            uint32_t b[4];
-            br_ldsm4(b, tile + ((mi >> 1) * 8 + (lane & 7)) * LD + ks * 16 + (mi & 1) * 8);
-            br_mma(s[0], qf[ks], b[0], b[1]);
-            br_mma(s[1], qf[ks], b[2], b[3]);
-        }
-        float mx_lo = -INFINITY, mx_hi = -INFINITY;
+            uint32_t a[4];
+            br_ldsm4(a, keys + ks * 16);
 #pragma unroll
-        for (int n = 0; n < 2; ++n) {
+            for (int nt = 0; nt < NT; ++nt) br_mma(ks & 1 ? s2[nt] : s[nt], a, qf[nt][ks][0], qf[nt][ks][1]);
+        }
+        const int p_base = base_of(i) + (lane >> 2);        // the thread's keys: p_base, p_base + 8
+        bool see[2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const int p = p_base + r * 8, d = pos - p;
+            see[r] = d >= 0 && (window == 0 || d < window || p < keep_first);
+        }
+        uint32_t b[NT][2], rest[NT][2];                     // the weights' operand: rounded, and what rounding left
+        float shrink[NT][2];
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-                const int p = p_base + n * 8 + (lane & 3) * 2 + (c & 1);
-                const int d = pos - p;
-                const bool see = d >= 0 && (window == 0 || d < window || p < keep_first);
-                const float* bh = (c & 2) ? b_hi : b_lo;
-                float v = s[n][c] * scale;
+                float v = (s[nt][c] + s2[nt][c]) * scale;
                 if (softcap > 0.f) v = softcap * tanhf(v / softcap);
-                if (bh && see) v += __ldg(bh + min(d, far));
-                v = see ? v : -INFINITY;
-                s[n][c] = v;
-                if (c & 2) mx_hi = fmaxf(mx_hi, v); else mx_lo = fmaxf(mx_lo, v);
+                if (bias_of[nt][c & 1] && see[c >> 1]) v += __ldg(bias_of[nt][c & 1] + min(pos - p_base - (c >> 1) * 8, far));
+                s[nt][c] = see[c >> 1] ? v : -INFINITY;
+            }
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                float mx = fmaxf(s[nt][e], s[nt][2 + e]);
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+                const float next_m = fmaxf(m[nt][e], mx), u = next_m == -INFINITY ? 0.f : next_m;
+                shrink[nt][e] = __expf(m[nt][e] - u);
+                m[nt][e] = next_m;
+                s[nt][e] = __expf(s[nt][e] - u);
+                s[nt][2 + e] = __expf(s[nt][2 + e] - u);
+                l[nt][e] = l[nt][e] * shrink[nt][e] + (s[nt][e] + s[nt][2 + e]);
+            }
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const uint32_t w = br_pack(s[nt][2 * r], s[nt][2 * r + 1]);
+                b[nt][r] = bh_turn(w);
+                rest[nt][r] = bh_turn(br_pack(s[nt][2 * r] - __uint_as_float(w << 16), s[nt][2 * r + 1] - __uint_as_float(w & 0xffff0000u)));
             }
         }
-        mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 1));
-        mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 2));
-        mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 1));
-        mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 2));
-        const float mn_lo = fmaxf(m_lo, mx_lo), mn_hi = fmaxf(m_hi, mx_hi);
-        const float u_lo = mn_lo == -INFINITY ? 0.f : mn_lo, u_hi = mn_hi == -INFINITY ? 0.f : mn_hi;
-        const float c_lo = __expf(m_lo - u_lo), c_hi = __expf(m_hi - u_hi);
-        m_lo = mn_lo; m_hi = mn_hi;
-        l_lo *= c_lo; l_hi *= c_hi;
+        const __nv_bfloat16* values = tile + ((mi >> 1) * 8 + (lane & 7)) * LD + DK + (mi & 1) * 8;
 #pragma unroll
-        for (int n = 0; n < DV / 8; ++n) { o[n][0] *= c_lo; o[n][1] *= c_lo; o[n][2] *= c_hi; o[n][3] *= c_hi; }
+        for (int n = 0; n < DV / 16; ++n) {
+            uint32_t a[4];
+            br_ldsm4_t(a, values + n * 16);
 #pragma unroll
-        for (int n = 0; n < 2; ++n) {
-            s[n][0] = __expf(s[n][0] - u_lo); s[n][1] = __expf(s[n][1] - u_lo);
-            s[n][2] = __expf(s[n][2] - u_hi); s[n][3] = __expf(s[n][3] - u_hi);
-            l_lo += s[n][0] + s[n][1];
-            l_hi += s[n][2] + s[n][3];
+            for (int nt = 0; nt < NT; ++nt) {
+                o[nt][n][0] *= shrink[nt][0]; o[nt][n][1] *= shrink[nt][1];
+                o[nt][n][2] *= shrink[nt][0]; o[nt][n][3] *= shrink[nt][1];
+                br_mma(o[nt][n], a, b[nt][0], b[nt][1]);
+                br_mma(o[nt][n], a, rest[nt][0], rest[nt][1]);
+            }
         }
-        uint32_t a[4];
-        a[0] = br_pack(s[0][0], s[0][1]);
-        a[1] = br_pack(s[0][2], s[0][3]);
-        a[2] = br_pack(s[1][0], s[1][1]);
-        a[3] = br_pack(s[1][2], s[1][3]);
-#pragma unroll
-        for (int n = 0; n < DV / 8; n += 2) {
-            uint32_t b[4];
-            br_ldsm4_t(b, tile + ((mi & 1) * 8 + (lane & 7)) * LD + DK + (n + (mi >> 1)) * 8);
-            br_mma(o[n], a, b[0], b[1]);
-            br_mma(o[n + 1], a, b[2], b[3]);
-        }
-        __syncwarp();                                       // the stage is filled again two tiles on
-        stage ^= 1;
+        __syncwarp();                                       // the stage is filled with the next pass's tile
+        fill = stage;
+        stage = stage + 1 == BH_STAGES ? 0 : stage + 1;
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 1);
-    l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 2);
-    l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 1);
-    l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 2);
-    // the warps' states meet in shared memory (the rings are done with): [warp][row] max and sum, [warp][row][DV]
+    // the warps' states meet in shared memory (the rings are done with): [warp][head] max and sum, [warp][head][LO]
     __syncthreads();
     float* s_m = reinterpret_cast<float*>(bh_smem);
-    float* s_l = s_m + BA_WARPS * 16;
-    float* s_o = s_l + BA_WARPS * 16;
-    if ((lane & 3) == 0) {
-        s_m[warp * 16 + r_lo] = m_lo; s_l[warp * 16 + r_lo] = l_lo;
-        s_m[warp * 16 + r_hi] = m_hi; s_l[warp * 16 + r_hi] = l_hi;
-    }
+    float* s_l = s_m + BA_WARPS * HEADS;
+    float* s_o = s_l + BA_WARPS * HEADS;
 #pragma unroll
-    for (int n = 0; n < DV / 8; ++n) {
-        float* lo = s_o + ((size_t)warp * 16 + r_lo) * DV + n * 8 + (lane & 3) * 2;
-        float* hi = s_o + ((size_t)warp * 16 + r_hi) * DV + n * 8 + (lane & 3) * 2;
-        lo[0] = o[n][0]; lo[1] = o[n][1]; hi[0] = o[n][2]; hi[1] = o[n][3];
+    for (int nt = 0; nt < NT; ++nt) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int row = warp * HEADS + nt * 8 + col + e;
+            float sum = l[nt][e];
+            sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 8);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+            if (lane < 4) { s_m[row] = m[nt][e]; s_l[row] = sum; }
+            float* dst = s_o + (size_t)row * LO + (lane >> 2);
+#pragma unroll
+            for (int n = 0; n < DV / 16; ++n) { dst[n * 16] = o[nt][n][e]; dst[n * 16 + 8] = o[nt][n][2 + e]; }
+        }
     }
     __syncthreads();
     for (int idx = threadIdx.x; idx < G * DV; idx += blockDim.x) {
@@ -1569,13 +1608,13 @@ bias_attention_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bflo
         const bool with_sink = sink != nullptr && split == 0;
         float M = with_sink ? sink[h0 + r] : -INFINITY;
 #pragma unroll
-        for (int w = 0; w < BA_WARPS; ++w) M = fmaxf(M, s_m[w * 16 + r]);
+        for (int w = 0; w < BA_WARPS; ++w) M = fmaxf(M, s_m[w * HEADS + r]);
         float L = with_sink ? expf(sink[h0 + r] - M) : 0.f, a = 0.f;
 #pragma unroll
         for (int w = 0; w < BA_WARPS; ++w) {
-            const float f = s_m[w * 16 + r] == -INFINITY ? 0.f : expf(s_m[w * 16 + r] - M);
-            L += s_l[w * 16 + r] * f;
-            a += s_o[((size_t)w * 16 + r) * DV + d] * f;
+            const float f = s_m[w * HEADS + r] == -INFINITY ? 0.f : expf(s_m[w * HEADS + r] - M);
+            L += s_l[w * HEADS + r] * f;
+            a += s_o[((size_t)w * HEADS + r) * LO + d] * f;
         }
         if (n_splits == 1) {
             out[((size_t)t * nh + h0 + r) * DV + d] = __float2bfloat16_rn(a / L);
@@ -1587,14 +1626,14 @@ bias_attention_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bflo
     }
 }
 
-template <int DK, int DV>
+template <int DK, int DV, int NT>
 int launch_bias_heads(const void* q, const void* cache, const float* bias_t, int far, const float* sink, const int* positions,
                       const int* seq_of_token, const int* page_table, int table_stride, int page_size, int window,
                       int keep_first, int cell, float scale, float softcap, void* out, float* partial, int n_splits, int T_, int nh, int nkv,
                       int n_seqs, int n_pages, cudaStream_t stream) {
-    auto kern = bias_attention_heads_kernel<DK, DV>;
-    const int ring = BA_WARPS * 2 * BH_K * (DK + DV + 8) * (int)sizeof(__nv_bfloat16);
-    const int merge = (BA_WARPS * 16 * 2 + BA_WARPS * 16 * DV) * (int)sizeof(float);
+    auto kern = bias_attention_heads_kernel<DK, DV, NT>;
+    const int ring = BA_WARPS * BH_STAGES * BH_K * (DK + DV + 8) * (int)sizeof(__nv_bfloat16);
+    const int merge = BA_WARPS * 8 * NT * (2 + DV + 4) * (int)sizeof(float);
     const int smem = ring > merge ? ring : merge;
     static bool configured = false;
     if (!configured) {
@@ -1602,7 +1641,7 @@ int launch_bias_heads(const void* q, const void* cache, const float* bias_t, int
         if (e != cudaSuccess) TQ_FAIL(-1, "bias_attention_heads: %d bytes of shared memory refused: %s", smem, cudaGetErrorString(e));
         configured = true;
     }
-    const int chunks = (nh / nkv + 15) / 16;
+    const int chunks = (nh / nkv + 8 * NT - 1) / (8 * NT);
     dim3 grid(T_, nkv * chunks, n_splits);
     tq_launch(grid, BA_WARPS * 32, smem, stream)(kern, (const __nv_bfloat16*)q, (const __nv_bfloat16*)cache, bias_t, far, sink,
         positions, seq_of_token, page_table, table_stride, page_size, window, keep_first, cell, scale, softcap, (__nv_bfloat16*)out, partial,
@@ -1623,9 +1662,9 @@ TQ_EXPORT int tq_bias_attention_heads(const void* q, const void* cache, const fl
                "bias_attention_heads: %d ranges or %d key/value heads exceed the grid limit", n_splits, nkv);
     TQ_REQUIRE(n_splits == 1 || partial != nullptr, "bias_attention_heads: %d ranges need scratch for their states", n_splits);
     int rc = -2;
-#define BH_CASE(DK_, DV_) if (dk == DK_ && dv == DV_) rc = launch_bias_heads<DK_, DV_>(q, cache, bias_t, far, sink, positions, \
-        seq_of_token, page_table, table_stride, page_size, window, keep_first, cell, scale, softcap, out, partial, n_splits, T_, nh, nkv,  \
-        n_seqs, n_pages, stream);
+#define BH_CASE(DK_, DV_) if (dk == DK_ && dv == DV_) rc = (nh / nkv <= 8 ? launch_bias_heads<DK_, DV_, 1> : launch_bias_heads<DK_, DV_, 2>)( \
+        q, cache, bias_t, far, sink, positions, seq_of_token, page_table, table_stride, page_size, window, keep_first, cell, scale, softcap,  \
+        out, partial, n_splits, T_, nh, nkv, n_seqs, n_pages, stream);
     BH_CASE(32, 32) BH_CASE(32, 64) BH_CASE(32, 128) BH_CASE(64, 32) BH_CASE(64, 64) BH_CASE(64, 128)
     BH_CASE(128, 32) BH_CASE(128, 64) BH_CASE(128, 128)
 #undef BH_CASE

@@ -217,20 +217,18 @@ def heads_form(dtype: torch.dtype, dk: int, dv: int, per_kv: int, page_size: int
 HEADS_FORM_MIN = 2
 
 
-def splits_for(n_tokens: int, blocks_per_token: int, longest: int, device, unit: int = 8) -> int:
-    """Ranges the visible keys of a token are cut into.  A block's four warps walk its range in units of `unit` keys
-    (16 in the tensor-core form); three blocks run on an SM at once.  The count that gives the fewest rounds of
-    blocks times units per warp, a block's fixed cost (its queries, the merge) counted as two units, and never fewer
-    than a unit per warp: a step of few tokens is cut until it fills the GPU, a large batch so that its last round
-    of blocks is full.  (Measured on B200 at 64 tokens x 4 key/value heads x 1,028 keys of 128 + 128, tensor-core
-    form: one range 45.2 us, 2 ranges 50.2 + 3.4 us for the merge, 3: 41.9 + 4.6, 5: 44.7 + 5.1, 7: 53.3 + 6.5, 13: 64.4 + 8.1.)  The ranges are joined in range order, so a launch shape always gives the same bits; logits
-    agree across shapes to rounding."""
+def splits_for(n_tokens: int, blocks_per_token: int, longest: int, device) -> int:
+    """Ranges the visible keys of a token are cut into.  A block's four warps walk its range in units of 8 keys; three
+    blocks run on an SM at once.  The count that gives the fewest rounds of blocks times units per warp, a block's fixed
+    cost (its queries, the merge) counted as two units, and never fewer than a unit per warp: a step of few tokens is
+    cut until it fills the GPU, a large batch so that its last round of blocks is full.  The ranges are joined in range
+    order, so a launch shape always gives the same bits; logits agree across shapes to rounding."""
     import os
     forced = os.environ.get("TQ_BIAS_SPLITS", "")
     if forced:
         return max(1, min(64, int(forced)))
     slots = 3 * torch.cuda.get_device_properties(device).multi_processor_count
-    units = -(-max(1, longest) // unit)
+    units = -(-max(1, longest) // 8)
     best, best_cost = 1, float("inf")
     for s in range(1, min(64, max(1, units // 4)) + 1):
         per_block = -(-(-(-units // s)) // 4) + 2
@@ -239,6 +237,22 @@ def splits_for(n_tokens: int, blocks_per_token: int, longest: int, device, unit:
         if cost < best_cost:
             best, best_cost = s, cost
     return best
+
+
+def heads_splits_for(n_tokens: int, blocks_per_token: int, longest: int, row: int, device) -> int:
+    """The same count for the tensor-core form, whose blocks keep up with memory once there are two on an SM (rows of
+    256 elements; four for rows of 128, whose tiles are half as long): ranges only fill the GPU up to there, and none
+    is so short that a warp has fewer than four tiles of 16 keys.  (Measured on B200, events around one launch, 4
+    key/value heads x 4 heads, 128 + 128, 2,048 keys: 8 tokens 36.7 us in one range, 20.5 in 4, 18.5 in 8, 24.6 in 16; 24
+    tokens 36.9, 28.7 in 3, 34.8 in 6; 32 tokens 36.9, 32.8 in 2, 43.0 in 4; 64 tokens 49.2, 67.3 in 2, 58.6 in 3; 96
+    tokens 75.8, 77.8 in 2.  64 + 64: 32 tokens 32.8, 22.6 in 4, 28.7 in 8; 64 tokens 35.7, 34.1 in 2, 41.0 in 3.)"""
+    import os
+    forced = os.environ.get("TQ_BIAS_SPLITS", "")
+    if forced:
+        return max(1, min(64, int(forced)))
+    places = 2 * torch.cuda.get_device_properties(device).multi_processor_count * 256 // max(128, row)
+    tiles = -(-max(1, longest) // 16)
+    return max(1, min(64, places // max(1, n_tokens * blocks_per_token), tiles // 16))
 
 
 def attention(q: torch.Tensor, cache: torch.Tensor, bias: Optional[torch.Tensor], sink: Optional[torch.Tensor],

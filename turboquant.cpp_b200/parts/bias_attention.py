@@ -70,12 +70,13 @@ def paged_attention(q: torch.Tensor, cache: LayerCache, ctx: StepContext, heads:
     per_kv = heads // kv_heads
     gc = KB.group_heads(act, dim, vdim, per_kv)
     blocks = kv_heads * -(-per_kv // gc) if gc else heads
-    unit = 8
     if KB.heads_form(act, dim, vdim, per_kv, cache.page_size):
-        blocks, unit = kv_heads * -(-per_kv // 16), 16
+        n_splits = KB.heads_splits_for(T, kv_heads * -(-per_kv // 16), longest, dim + vdim, dev)
+    else:
+        n_splits = KB.splits_for(T, blocks, longest, dev)
     return KB.attention(q, cache.kv, bias, sink, ctx.positions, ctx.seq_of_token, cache.page_table, cache.page_size,
                         window, keep_first, scale, o, heads, kv_heads, dim, vdim,
-                        n_splits=KB.splits_for(T, blocks, longest, dev, unit), bias_t=bias_t, softcap=softcap, cell=cell)
+                        n_splits=n_splits, bias_t=bias_t, softcap=softcap, cell=cell)
 
 
 class BiasedWindowAttentionMixer(Mixer):
