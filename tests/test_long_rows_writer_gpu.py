@@ -54,3 +54,31 @@ def test_values_turned_back(T, H, dv, halves):
     pos = torch.randint(0, 300, (T,), generator=g, device=DEV, dtype=torch.int32)
     want = turned(o.double().view(T, H, dv), -pos, freq, halves) * torch.sigmoid(gates[:, 2:2 + H].double())[..., None]
     close(KB.heads_unrotate_gate(o, gates, 2, freq, halves, pos, o, H, dv).view(T, H, dv), want)
+
+
+@pytest.mark.parametrize("halves", [True, False])
+@pytest.mark.parametrize("dk,dv,dims", [(128, 128, 128), (96, 64, 32)])
+def test_a_token_s_rows_do_not_depend_on_the_step_s_size(halves, dk, dv, dims):
+    """The kernels of long steps and of small ones write the same bits."""
+    from turboquant_cpp_b200.kernels import bias_attention as KB
+    H, G, T, part = 6, 2, 1800, 50
+    g = torch.Generator(device=DEV).manual_seed(dk)
+    rand = lambda *s: torch.randn(s, generator=g, device=DEV)
+    rows, pos = rand(T, (H + G) * dk + G * dv), torch.arange(T, device=DEV, dtype=torch.int32)
+    freq, v_freq, qw, kw = rand(dims // 2).abs(), rand(dv // 2).abs(), 1 + 0.1 * rand(dk), 1 + 0.1 * rand(dk)
+    o, gates = rand(T, H * dv), rand(T, H)
+    pages = -(-T // 64)
+    table = torch.arange(pages, device=DEV, dtype=torch.int32).view(1, pages)
+
+    def run(steps):
+        cache, out = torch.zeros((pages, 1, G, 64, dk + dv), device=DEV), []
+        for a in range(0, T, steps):
+            n = slice(a, a + steps)
+            q = torch.empty((rows[n].shape[0], H, dk), device=DEV)
+            KB.kv_write_rot(rows[n], q, cache, freq, dims, halves, 1e-5, pos[n], torch.zeros_like(pos[n]), table, 64, H, G, dk, dv, mag=1.1, q_norm=qw,
+                            k_norm=kw, norm_eps=1e-5, v_freq=v_freq, temperature=(0.1, 50))
+            out.append(torch.cat([q.flatten(1), KB.heads_unrotate_gate(o[n], gates[n], 0, v_freq, halves, pos[n], torch.empty_like(o[n]), H, dv)], 1))
+        return torch.cat(out), cache
+
+    for a, b in zip(run(T), run(part)):
+        assert torch.equal(a, b)

@@ -175,6 +175,9 @@ __device__ __forceinline__ void ba_turn(float* sh, const float2* cs, int n, int 
         sh[b] = (v * cs[i].x + u * cs[i].y) * mag;
     }
 }
+// One element of a turned pair in registers, own * c + other * s, with the roundings spelled out: a token's rows come out the same
+// to the bit whichever kernel its step's size takes (left to the compiler, the kernels of long steps rounded own * c first).
+__device__ __forceinline__ float ba_turned(float own, float c, float other, float s) { return fmaf(own, c, other * s); }
 // the same of a head of at most 128 elements that lies in the warp's registers, four neighbours a lane (n pairs: a multiple of
 // four with halves, of two without)
 __device__ __forceinline__ void ba_turn_lanes(float4& x, const float2* cs, int n, int halves, float mag, int lane) {
@@ -191,15 +194,15 @@ __device__ __forceinline__ void ba_turn_lanes(float4& x, const float2* cs, int n
             const float4* t = reinterpret_cast<const float4*>(cs + 4 * (lo ? lane : lane - step));
             const float4 a = t[0], b = t[1];
             const float f = lo ? -1.f : 1.f;
-            x.x = (x.x * a.x + f * y.x * a.y) * mag;
-            x.y = (x.y * a.z + f * y.y * a.w) * mag;
-            x.z = (x.z * b.x + f * y.z * b.y) * mag;
-            x.w = (x.w * b.z + f * y.w * b.w) * mag;
+            x.x = ba_turned(x.x, a.x, f * y.x, a.y) * mag;
+            x.y = ba_turned(x.y, a.z, f * y.y, a.w) * mag;
+            x.z = ba_turned(x.z, b.x, f * y.z, b.y) * mag;
+            x.w = ba_turned(x.w, b.z, f * y.w, b.w) * mag;
         }
     } else if (2 * lane < n) {
         const float4 t = *reinterpret_cast<const float4*>(cs + 2 * lane);
-        x = make_float4((x.x * t.x - x.y * t.y) * mag, (x.y * t.x + x.x * t.y) * mag,
-                        (x.z * t.z - x.w * t.w) * mag, (x.w * t.z + x.z * t.w) * mag);
+        x = make_float4(ba_turned(x.x, t.x, -x.y, t.y) * mag, ba_turned(x.y, t.x, x.x, t.y) * mag,
+                        ba_turned(x.z, t.z, -x.w, t.w) * mag, ba_turned(x.w, t.z, x.z, t.w) * mag);
     }
 }
 // four elements in one access or, where the addresses are not aligned for that, in four
@@ -372,14 +375,14 @@ __device__ __forceinline__ void ba_turn_regs(float4& x, const BaTurn& t, int n, 
         y.w = __shfl_sync(0xffffffffu, x.w, from);
         if (turned) {
             const float f = lo ? -1.f : 1.f;
-            x.x = (x.x * t.c[0] + f * y.x * t.s[0]) * mag;
-            x.y = (x.y * t.c[1] + f * y.y * t.s[1]) * mag;
-            x.z = (x.z * t.c[2] + f * y.z * t.s[2]) * mag;
-            x.w = (x.w * t.c[3] + f * y.w * t.s[3]) * mag;
+            x.x = ba_turned(x.x, t.c[0], f * y.x, t.s[0]) * mag;
+            x.y = ba_turned(x.y, t.c[1], f * y.y, t.s[1]) * mag;
+            x.z = ba_turned(x.z, t.c[2], f * y.z, t.s[2]) * mag;
+            x.w = ba_turned(x.w, t.c[3], f * y.w, t.s[3]) * mag;
         }
     } else if (2 * lane < n) {
-        x = make_float4((x.x * t.c[0] - x.y * t.s[0]) * mag, (x.y * t.c[0] + x.x * t.s[0]) * mag,
-                        (x.z * t.c[1] - x.w * t.s[1]) * mag, (x.w * t.c[1] + x.z * t.s[1]) * mag);
+        x = make_float4(ba_turned(x.x, t.c[0], -x.y, t.s[0]) * mag, ba_turned(x.y, t.c[0], x.x, t.s[0]) * mag,
+                        ba_turned(x.z, t.c[1], -x.w, t.s[1]) * mag, ba_turned(x.w, t.c[1], x.z, t.s[1]) * mag);
     }
 }
 constexpr int TURN_WARPS = 4, TURN_AHEAD = 4;      // of a block; heads worked on together
@@ -422,7 +425,9 @@ bias_kv_turn_kernel(const float* __restrict__ qkv, int row_stride, TA* __restric
     float4 qw = make_float4(1.f, 1.f, 1.f, 1.f), kw = qw;
     if (q_norm_w != nullptr && e < dk) qw = make_float4(q_norm_w[e], q_norm_w[e + 1], q_norm_w[e + 2], q_norm_w[e + 3]);
     if (k_norm_w != nullptr && e < dk) kw = make_float4(k_norm_w[e], k_norm_w[e + 1], k_norm_w[e + 2], k_norm_w[e + 3]);
+    const bool exact = (dk & (dk - 1)) == 0;       // then the product with 1 / dk is the quotient
     const float inv_dk = 1.0f / (float)dk;
+    auto mean = [&](float ss) { return exact ? ss * inv_dk : ss / (float)dk; };
     // four heads of a kind, or some of them, side by side: their sums over the lanes do not wait for one another
     auto heads = [&](float4 (&x)[TURN_AHEAD], int at, int n, bool is_q, bool is_v) {
         auto sums = [&](float (&ss)[TURN_AHEAD]) {
@@ -439,7 +444,7 @@ bias_kv_turn_kernel(const float* __restrict__ qkv, int row_stride, TA* __restric
             sums(ss);
 #pragma unroll
             for (int i = 0; i < TURN_AHEAD; ++i) {
-                const float r = 1.0f / sqrtf(ss[i] * inv_dk + norm_eps);
+                const float r = 1.0f / sqrtf(mean(ss[i]) + norm_eps);
                 x[i] = make_float4(x[i].x * r * w.x, x[i].y * r * w.y, x[i].z * r * w.z, x[i].w * r * w.w);
             }
         }
@@ -455,7 +460,7 @@ bias_kv_turn_kernel(const float* __restrict__ qkv, int row_stride, TA* __restric
         if (!is_v && unit_eps > 0.f) {
             sums(ss);
 #pragma unroll
-            for (int i = 0; i < TURN_AHEAD; ++i) r[i] *= 1.0f / sqrtf(ss[i] * inv_dk + unit_eps);
+            for (int i = 0; i < TURN_AHEAD; ++i) r[i] *= 1.0f / sqrtf(mean(ss[i]) + unit_eps);
         }
         if (e < (is_v ? dv : dk)) {
             const int g = at - nh - (is_v ? nkv : 0), step = is_q ? dk : page_size * dr;
