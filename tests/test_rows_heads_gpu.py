@@ -47,3 +47,28 @@ def test_tokens_of_several_sequences_against_float64(per_kv, dk, dv, window, kee
         # the weights and the result are rounded to bfloat16 (2^-9 each, the weights' errors averaging out), sums are float32
         err = (out.view(T, H, dv).double() - want).norm() / want.norm()
         assert err < 2 * 2.0 ** -9, (n_splits, float(err))
+
+
+@pytest.mark.parametrize("per_kv,dk,dv", [(4, 128, 128), (16, 64, 64)])
+@pytest.mark.parametrize("n_splits", [1, 3])
+def test_infinite_and_nan_values_stay_in_their_column(per_kv, dk, dv, n_splits):
+    """A value of infinity makes its own element of the sums that infinity, a NaN a NaN, and nothing else changes: the weights reach the
+    product in two parts, neither of which may turn an infinity round or meet it with a zero."""
+    from turboquant_cpp_b200.kernels import bias_attention as KB
+    g = torch.Generator(device=DEV).manual_seed(per_kv)
+    n, G, H = 200, 2, 2 * per_kv
+    cache = torch.randn((4, G, PAGE, dk + dv), generator=g, device=DEV).to(torch.bfloat16)
+    q = torch.randn((1, H, dk), generator=g, device=DEV).to(torch.bfloat16)
+    q[0, 0] = 0                                              # weights of exactly one: their second part is nothing
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device=DEV)
+
+    def run():
+        out = torch.empty((1, H * dv), dtype=torch.bfloat16, device=DEV)
+        KB.attention(q, cache, None, None, i32([n - 1]), i32([0]), i32([[2, 0, 3, 1]]), PAGE, 0, 0, dk ** -0.5, out, H, G, dk, dv, n_splits=n_splits)
+        return out.view(H, dv)
+
+    clean = run()
+    cache[0, :, 5, dk + 1], cache[0, :, 5, dk + 2], cache[0, :, 5, dk + 3] = math.inf, -math.inf, math.nan
+    got = run()
+    assert bool((got[:, 1] == math.inf).all()) and bool((got[:, 2] == -math.inf).all()) and bool(got[:, 3].isnan().all())
+    assert torch.equal(got[:, 4:], clean[:, 4:]) and torch.equal(got[:, 0], clean[:, 0])

@@ -1428,6 +1428,12 @@ __device__ __forceinline__ uint32_t bh_turn(uint32_t x) {      // an 8 x 8 tile 
     asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
     return y;
 }
+// What the upper 16 bits of a weight leave, which is not negative; more than zero where the weight is, so that an infinite value
+// times both parts is that infinity and not a NaN (2^-126 of a value is nothing beside a sum of weights of one or more).
+__device__ __forceinline__ float bh_rest(float w) {
+    const float upper = __uint_as_float(__float_as_uint(w) & 0xffff0000u), left = w - upper;
+    return upper > 0.f ? fmaxf(left, 1.17549435e-38f) : left;
+}
 template <int DK, int DV, int NT>
 __global__ void __launch_bounds__(BA_WARPS * 32, 3)
 bias_attention_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ cache,
@@ -1538,7 +1544,7 @@ bias_attention_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bflo
             const int p = p_base + r * 8, d = pos - p;
             see[r] = d >= 0 && (window == 0 || d < window || p < keep_first);
         }
-        uint32_t b[NT][2], rest[NT][2];                     // the weights' operand: rounded, and what rounding left
+        uint32_t b[NT][2], rest[NT][2];                     // the weights' operand: their upper bits, and the rest
         float shrink[NT][2];
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
@@ -1564,9 +1570,9 @@ bias_attention_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bflo
             }
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
-                const uint32_t w = br_pack(s[nt][2 * r], s[nt][2 * r + 1]);
+                const uint32_t w = __byte_perm(__float_as_uint(s[nt][2 * r]), __float_as_uint(s[nt][2 * r + 1]), 0x7632);
                 b[nt][r] = bh_turn(w);
-                rest[nt][r] = bh_turn(br_pack(s[nt][2 * r] - __uint_as_float(w << 16), s[nt][2 * r + 1] - __uint_as_float(w & 0xffff0000u)));
+                rest[nt][r] = bh_turn(br_pack(bh_rest(s[nt][2 * r]), bh_rest(s[nt][2 * r + 1])));
             }
         }
         const __nv_bfloat16* values = tile + ((mi >> 1) * 8 + (lane & 7)) * LD + DK + (mi & 1) * 8;
