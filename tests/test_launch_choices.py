@@ -131,3 +131,21 @@ def test_expanded_latent_keys_take_a_bounded_scratch():
     assert not ok([512] * 64, [15000] * 64) and not ok([64], [4000])
     m.window = 1024
     assert ok([2048] * 64, [0] * 64)
+
+
+def test_ranges_of_the_tensor_core_rows_form(monkeypatch):
+    """Few tokens are cut finer than to fill the GPU alone, many or short ones are not; never more than 64 ranges."""
+    from types import SimpleNamespace
+
+    import torch
+
+    from turboquant_cpp_b200.kernels import bias_attention as KB
+    monkeypatch.setattr(torch.cuda, "get_device_properties", lambda device: SimpleNamespace(multi_processor_count=148))
+    monkeypatch.delenv("TQ_BIAS_SPLITS", raising=False)
+    ranges = lambda tokens, keys, row=256: KB.heads_splits_for(tokens, 4, keys, row, None, 16)
+    assert [ranges(4, n) for n in (100, 256, 500, 1000, 2048, 4096)] == [1, 4, 4, 8, 8, 16]
+    assert [ranges(t, 2048) for t in (1, 8, 16, 24, 32, 64)] == [8, 8, 4, 4, 2, 1]
+    assert [ranges(t, 500) for t in (8, 24, 32, 64)] == [4, 4, 2, 1] and ranges(4, 256, 128) == 1
+    for t in (1, 3, 17, 200, 5000):
+        for n in (0, 1, 15, 16, 400, 100000):
+            assert 1 <= ranges(t, n) <= 64

@@ -239,20 +239,31 @@ def splits_for(n_tokens: int, blocks_per_token: int, longest: int, device) -> in
     return best
 
 
-def heads_splits_for(n_tokens: int, blocks_per_token: int, longest: int, row: int, device) -> int:
+def heads_splits_for(n_tokens: int, blocks_per_token: int, longest: int, row: int, device, heads: int = 0) -> int:
     """The same count for the tensor-core form, whose blocks keep up with memory once there are two on an SM (rows of
-    256 elements; four for rows of 128, whose tiles are half as long): ranges only fill the GPU up to there, and none
-    is so short that a warp has fewer than four tiles of 16 keys.  (Measured on B200, events around one launch, 4
-    key/value heads x 4 heads, 128 + 128, 2,048 keys: 8 tokens 36.7 us in one range, 20.5 in 4, 18.5 in 8, 24.6 in 16; 24
-    tokens 36.9, 28.7 in 3, 34.8 in 6; 32 tokens 36.9, 32.8 in 2, 43.0 in 4; 64 tokens 49.2, 67.3 in 2, 58.6 in 3; 96
-    tokens 75.8, 77.8 in 2.  64 + 64: 32 tokens 32.8, 22.6 in 4, 28.7 in 8; 64 tokens 35.7, 34.1 in 2, 41.0 in 3.)"""
+    256 elements; four for rows of 128, whose tiles are half as long): ranges fill the GPU up to there, none so short that a
+    warp has fewer than four tiles of 16 keys.  Where a GPU is far from full, a walk shortened further still outweighs the
+    ranges' states and their merge: then the largest power of two up to 1.13 sqrt(tiles), up to three blocks an SM and
+    3,072 states (`heads`: query heads of a token; 1.5 where a block has more than eight of them).  Below 32 tiles (16 for a few blocks of rows of 256) one range.  (Measured on
+    B200 in a graph, rows in the L2, 4 key/value heads x 4 heads, 128 + 128, us: 4 tokens of 500 keys 10.3 in one range, 9.2 in 2, 7.3
+    in 4, 7.3 in 8; of 1,000 17.7, 12.8, 9.2, 8.1, 10.2 in 16; of 4,096 61.1, 13.6 in 8, 14.1 in 16, 20.5 in 32; 1 token of 2,048 10.2
+    in 8, 9.6 in 16, 11.8 in 32; 24 tokens of 1,000 17.8, 14.4 in 3, 13.6 in 4, 18.0 in 8; 32 tokens of 500 10.6, 11.5 in 2, of 2,048
+    33.8, 28.1 in 2, 37.9 in 4; 64 tokens of 1,000 28.7, 37.3 in 2.  16 heads on one: 1 token of 2,048 14.6 in 8, 13.8 in 16.)"""
+    import math
     import os
     forced = os.environ.get("TQ_BIAS_SPLITS", "")
     if forced:
         return max(1, min(64, int(forced)))
-    places = 2 * torch.cuda.get_device_properties(device).multi_processor_count * 256 // max(128, row)
+    sms, blocks = torch.cuda.get_device_properties(device).multi_processor_count, max(1, n_tokens * blocks_per_token)
     tiles = -(-max(1, longest) // 16)
-    return max(1, min(64, places // max(1, n_tokens * blocks_per_token), tiles // 16))
+    fill = max(1, min(64, 2 * sms * 256 // max(128, row) // blocks, tiles // 16))
+    if tiles < 16 or (tiles < 32 and (blocks > 32 or row <= 128)):
+        return fill
+    wide = heads > 8 * blocks_per_token                    # two products of eight heads a tile: a walk takes 1.35 times as long
+    short = min(int((1.5 if wide else 1.13) * math.sqrt(tiles)), (3 if row > 128 else 4) * sms // blocks, 3072 // max(1, n_tokens * heads), 32)
+    if short < 2 or (short < 4 and tiles < 48):
+        return fill
+    return max(fill, 1 << (short.bit_length() - 1))
 
 
 def attention(q: torch.Tensor, cache: torch.Tensor, bias: Optional[torch.Tensor], sink: Optional[torch.Tensor],

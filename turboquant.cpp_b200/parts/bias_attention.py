@@ -71,7 +71,7 @@ def paged_attention(q: torch.Tensor, cache: LayerCache, ctx: StepContext, heads:
     gc = KB.group_heads(act, dim, vdim, per_kv)
     blocks = kv_heads * -(-per_kv // gc) if gc else heads
     if KB.heads_form(act, dim, vdim, per_kv, cache.page_size):
-        n_splits = KB.heads_splits_for(T, kv_heads * -(-per_kv // 16), longest, dim + vdim, dev)
+        n_splits = KB.heads_splits_for(T, kv_heads * -(-per_kv // 16), longest, dim + vdim, dev, heads)
     else:
         n_splits = KB.splits_for(T, blocks, longest, dev)
     return KB.attention(q, cache.kv, bias, sink, ctx.positions, ctx.seq_of_token, cache.page_table, cache.page_size,
