@@ -112,3 +112,17 @@ int main() {
     src.write_text(program)
     subprocess.run([shutil.which("g++") or "c++", "-std=c++17", "-o", str(exe), str(src)], check=True)
     subprocess.run([str(exe)], check=True)
+
+
+def test_arrivals_in_another_cta_name_their_scope():
+    """An arrival without a scope is a release inside the arriving CTA alone: whoever waits in another CTA is not promised to see
+    what was written before it.  An arrival on another CTA's barrier says `cluster`, and releases unless no data goes with it."""
+    found = 0
+    for name in sorted(os.listdir(CSRC)):
+        if name.endswith((".cu", ".cuh")):
+            with open(os.path.join(CSRC, name), encoding="utf-8") as f:
+                for op in re.findall(r"mbarrier\.arrive[\w.:]*", f.read()):
+                    if "shared::cluster" in op:
+                        found += 1
+                        assert re.search(r"\.(release|relaxed)\.cluster\.", op), (name, op)
+    assert found >= 2

@@ -8,14 +8,17 @@
 //   warps 0..7    split them and store the parts as K-major tiles of 32 elements, 64-byte swizzle
 //   warp 16       issues the products (the first CTA's for both)
 //   warps 8..15   add the accumulator of the largest products, h h', to sums in their registers every two blocks and write the result
+//   warps 18, 19  of the second CTA: tell the first that its parts are stored, every other block each.  What the splitting warps wrote is
+//                 seen in the other CTA only behind a release at the cluster's scope, and that takes most of a block's time
 // The tensor cores' own sums cut bits off at every addition, so a chain of products over all of K is off by more than a
 // float32 sum is (K 2,048: 2.2e-6 of the result; the library's sum 8.1e-7); sums of 64 elements added up in rounded float32 are
 // off by less (1.3e-7).  The smaller products, 2^-8 of the result and less, stay in one accumulator
 // for all of K, and the other accumulator is read in the time they take: it costs nothing.
-// 700 tokens, K 2,048: 79 us for 6,144 rows (65 with bfloat16 weights; the library's fp32 product 309), 47 for 2,048 (145).  What bounds it is
+// 700 tokens, K 2,048: 80 us for 6,144 rows (65 with bfloat16 weights; the library's fp32 product 309), 47 for 2,048 (145).  What bounds it is
 // the splitting, some 1,200 cycles a block of 32 elements for 720 (three products) or 1,440 (six) of the tensor cores at 240 tokens.
-// What a block cost otherwise: 450 cycles more with arrivals that release at the cluster's scope, 500 more with two
-// stages of parts instead of three; two groups of splitting warps taking every other block: nothing gained.
+// What a block cost otherwise: 450 cycles more with splitting warps that release at the cluster's scope themselves, 240 with one warp
+// that tells of all blocks, 120 to 230 with three stages of parts where more fit; two groups of splitting warps taking every other
+// block: nothing gained.
 // Every result that is not finite is computed again as a plain sum, so infinities and NaN come out as fmaf leaves them.
 // Waits on mbarriers are bounded: one that runs out sets a flag, every role leaves, and *status is set.
 #include <cuda.h>
@@ -35,11 +38,17 @@ constexpr int CONV_REGS = 56, DRAIN_REGS = 168, MMA_REGS = 24, LAUNCH_REGS = 96;
 static_assert(32 * (CONV_WARPS * CONV_REGS + DRAIN_WARPS * DRAIN_REGS + 4 * MMA_REGS) <= THREADS * LAUNCH_REGS, "more registers than the block is launched with");
 constexpr int ROWS_EACH = 8;                   // rows of a block that a thread splits four elements of
 constexpr int PART = BM * BK * 2;              // one part of one operand of a block
-constexpr int STAGE = 6 * PART;                // weights h, m, l, tokens h, m, l
-constexpr int STAGES = 3;
-constexpr int RAW = 2 * BM * BK * 4;           // a block as it comes
 constexpr int RAWS = 2;
-constexpr int SMEM_BYTES = STAGES * STAGE + RAWS * RAW + 1024 /* alignment */;
+// Shared memory by the tokens of a tile: a block's parts (weights h, m, l, tokens h, m, l), blocks as they come, and as many stages
+// of parts as fit beside those
+constexpr int SMEM_BYTES = 226 * 1024, MAX_STAGES = 6;
+__host__ __device__ constexpr int stage_bytes(int n) { return 3 * PART + 3 * (n / 2) * BK * 2; }
+__host__ __device__ constexpr int raw_bytes(int n) { return BM * BK * 4 + (n / 2) * BK * 4; }
+__host__ __device__ constexpr int stages_of(int n) {
+    const int fit = (SMEM_BYTES - 1024 /* alignment */ - RAWS * raw_bytes(n)) / stage_bytes(n);
+    return fit < MAX_STAGES ? fit : MAX_STAGES;
+}
+static_assert(stages_of(MAX_TOKENS) >= 3, "shared memory");
 constexpr int GROUP = 2;                       // blocks whose h h' the tensor cores add up: 64 elements
 constexpr uint32_t WAIT_LIMIT = 1u << 20;      // polls of an mbarrier before a wait gives up ...
 constexpr uint64_t WAIT_NS = 2000000000ull;    // ... or two seconds
@@ -91,9 +100,9 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
-// for a barrier that says no more than that shared memory was read, or was written and fenced for the tensor cores
-__device__ __forceinline__ void mbar_arrive_near(uint32_t cluster_bar) {
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+// ... without any data: for a barrier that only says that tensor memory has been read
+__device__ __forceinline__ void mbar_arrive_order(uint32_t cluster_bar) {
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -157,7 +166,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     __shared__ int s_abort;
     __shared__ uint32_t s_tmem_base;
     __shared__ uint32_t s_low;         // the weights so far were not all bfloat16 values (the first CTA's)
-    __shared__ __align__(8) uint64_t s_bars[2 * STAGES + 3 + 2 * RAWS];
+    __shared__ __align__(8) uint64_t s_bars[3 * MAX_STAGES + 3 + 2 * RAWS];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t rank = blockIdx.x & 1;
     const int tile = blockIdx.x >> 1;
@@ -165,18 +174,21 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     const int count = min(n, T - t0);
     const int blocks = (K + BK - 1) / BK;
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t raw0 = base + STAGES * STAGE;
+    const int stages = stages_of(n), stage = stage_bytes(n), raw = raw_bytes(n), x_part = n / 2 * BK * 2;
+    const uint32_t raw0 = base + stages * stage;
     auto full_bar = [&](int s) { return smem_u32(&s_bars[s]); };                    // parts stored (the first CTA's)
-    auto done_bar = [&](int s) { return smem_u32(&s_bars[STAGES + s]); };           // ... and used
-    const uint32_t sum_full = smem_u32(&s_bars[2 * STAGES]), sum_empty = sum_full + 8, all_done = sum_full + 16;
+    auto done_bar = [&](int s) { return smem_u32(&s_bars[MAX_STAGES + s]); };       // ... and used
+    const uint32_t sum_full = smem_u32(&s_bars[2 * MAX_STAGES]), sum_empty = sum_full + 8, all_done = sum_full + 16;
     auto raw_full = [&](int r) { return all_done + 8 + 8u * r; };                   // this CTA's: brought
     auto raw_done = [&](int r) { return all_done + 8 + 8u * (RAWS + r); };          // ... and split
+    auto stored_bar = [&](int s) { return all_done + 8 + 8u * (2 * RAWS + s); };    // the second CTA's own: parts stored
     const int half = n / 2, x0 = t0 + (int)rank * half;                             // this CTA's tokens of the tile
 
     if (tid == 0) {
         s_abort = 0;
         s_low = 0;
-        for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), 2 * CONV_WARPS); mbar_init(done_bar(s), 1); }
+        // the first CTA's warps and, for all of the second's, one that passes it on
+        for (int s = 0; s < stages; ++s) { mbar_init(full_bar(s), CONV_WARPS + 1); mbar_init(done_bar(s), 1); mbar_init(stored_bar(s), CONV_WARPS); }
         mbar_init(sum_full, 1);
         mbar_init(sum_empty, 2 * DRAIN_WARPS);
         mbar_init(all_done, 1);
@@ -197,16 +209,16 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         // ---- both operands: split, stored ----
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(CONV_REGS));
         const int c = tid & 7, r0 = tid >> 3;
-        const uint32_t full0 = map_to_cta(full_bar(0), 0);
-        auto full_in_first = [&](int s) { return full0 + 8u * s; };
         bool told = false;
         // a row's 64 bytes hold four pieces of 16, their places shuffled by bits 1 and 2 of the row; the lanes' rows are 32 apart
         const uint32_t at = (uint32_t)r0 * 64 + (uint32_t)(((c >> 1) ^ ((r0 >> 1) & 3)) * 16 + (c & 1) * 8);
+        int s = 0;
+        uint32_t phase = 1;                                              // of the stage's last use
         for (int kb = 0; kb < blocks; ++kb) {
-            const int s = kb % STAGES, rs = kb % RAWS;
+            const int rs = kb % RAWS;
             if (!mbar_wait(raw_full(rs), (uint32_t)(kb / RAWS) & 1u, &s_abort)) break;
-            if (kb >= STAGES && !mbar_wait(done_bar(s), (uint32_t)(kb / STAGES - 1) & 1u, &s_abort)) break;
-            const uint32_t src = raw0 + rs * RAW + (uint32_t)r0 * (BK * 4) + c * 16, dst = base + s * STAGE + at;
+            if (kb >= stages && !mbar_wait(done_bar(s), phase, &s_abort)) break;
+            const uint32_t src = raw0 + rs * raw + (uint32_t)r0 * (BK * 4) + c * 16, dst = base + s * stage + at;
             uint32_t low = 0;
             float4 v[ROWS_EACH];
 #pragma unroll
@@ -218,25 +230,23 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             for (int i = 0; i < ROWS_EACH; ++i)
                 if (i < 4 || r0 + 32 * (i - 4) < half) {
                     const TqSplit4 p = tq_split4(v[i]);
-                    const uint32_t d = dst + (i < 4 ? 0 : 3 * PART) + (i & 3) * (32 * 64);
+                    const uint32_t d = dst + (i < 4 ? 0 : 3 * PART) + (i & 3) * (32 * 64), part = i < 4 ? PART : x_part;
                     asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(d), "r"(p.h.x), "r"(p.h.y) : "memory");
-                    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(d + PART), "r"(p.m.x), "r"(p.m.y) : "memory");
-                    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(d + 2 * PART), "r"(p.l.x), "r"(p.l.y) : "memory");
+                    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(d + part), "r"(p.m.x), "r"(p.m.y) : "memory");
+                    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(d + 2 * part), "r"(p.l.x), "r"(p.l.y) : "memory");
                     if (i < 4) low |= p.m.x | p.m.y | p.l.x | p.l.y;
                 }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tensor cores read through the other proxy
             const bool tell = !told && __any_sync(0xffffffffu, low != 0);
             __syncwarp();
             if (lane == 0) {
-                if (tell) {                                               // once a warp; the wider release costs half a microsecond
+                if (tell)                                                 // once a warp
                     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(map_to_cta(smem_u32(&s_low), 0)), "r"(1u) : "memory");
-                    mbar_arrive_cluster(full_in_first(s));
-                } else {
-                    mbar_arrive_near(full_in_first(s));
-                }
+                mbar_arrive(rank == 0 ? full_bar(s) : stored_bar(s));
                 mbar_arrive(raw_done(rs));
             }
             told |= tell;
+            if (++s == stages) { s = 0; phase ^= 1u; }
         }
     } else if (warp < CONV_WARPS + DRAIN_WARPS) {
         // ---- sums: lane = weight row, every other 16 tokens ----
@@ -271,7 +281,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             add(0);
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive_near(map_to_cta(sum_empty, 0));
+            if (lane == 0) mbar_arrive_order(map_to_cta(sum_empty, 0));
         }
         if (ok) ok = __all_sync(0xffffffffu, mbar_wait(all_done, 0u, &s_abort));
         if (ok) {
@@ -309,15 +319,16 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         if (warp == CONV_WARPS + DRAIN_WARPS && rank == 0) {
             const uint32_t elected = elect_one(), idesc = umma_idesc(n), sums = __shfl_sync(0xffffffffu, tmem, 0), rest = sums + MAX_TOKENS;
             const uint64_t desc0 = umma_desc(base);                          // descriptors count in 16 bytes
-            auto wait = [&](uint32_t bar, uint32_t parity) { return (bool)__all_sync(0xffffffffu, mbar_wait(bar, parity, &s_abort)); };
+            auto wait = [&](uint32_t bar, uint32_t parity) { return (bool)__all_sync(0xffffffffu, mbar_wait<true>(bar, parity, &s_abort)); };
+            int s = 0;
+            uint32_t phase = 0;
             for (int kb = 0; kb < blocks; ++kb) {
-                const int s = kb % STAGES;
-                if (!__all_sync(0xffffffffu, mbar_wait<true>(full_bar(s), (uint32_t)(kb / STAGES) & 1u, &s_abort))) break;
+                if (!wait(full_bar(s), phase)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const bool low = __shfl_sync(0xffffffffu, *(volatile uint32_t*)&s_low, 0) != 0;
-                const uint64_t wd = desc0 + (uint64_t)(s * (STAGE / 16)), xd = wd + 3 * PART / 16;
+                const uint64_t wd = desc0 + (uint64_t)(s * (stage / 16)), xd = wd + 3 * PART / 16;
                 auto times = [&](uint32_t d, int pw, int px, int k, uint32_t accumulate) {
-                    umma_pair(d, wd + (pw * (PART / 16) + k * 2), xd + (px * (PART / 16) + k * 2), idesc, accumulate, elected);
+                    umma_pair(d, wd + (pw * (PART / 16) + k * 2), xd + (px * (x_part / 16) + k * 2), idesc, accumulate, elected);
                 };
 #pragma unroll
                 for (int k = 0; k < BK / UMMA_K; ++k) times(rest, 0, 2, k, kb > 0 || k > 0 ? 1u : 0u);
@@ -341,6 +352,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 umma_commit_pair(done_bar(s), elected);
                 if (kb % GROUP == GROUP - 1 || kb == blocks - 1) umma_commit_pair(sum_full, elected);
                 if (kb == blocks - 1) umma_commit_pair(all_done, elected);
+                if (++s == stages) { s = 0; phase ^= 1u; }
             }
         } else if (warp == CONV_WARPS + DRAIN_WARPS + 1 && lane == 0) {
             // ---- both operands' blocks, zeros behind their ends ----
@@ -349,12 +361,22 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 const int r = issued % RAWS;
                 if (issued >= RAWS && !mbar_wait(raw_done(r), (uint32_t)(issued / RAWS - 1) & 1u, &s_abort)) break;
                 mbar_expect_tx(raw_full(r), (uint32_t)((BM + half) * BK * 4));
-                tma_load_2d(raw0 + r * RAW, &map_w, issued * BK, n0, raw_full(r));
-                tma_load_2d(raw0 + r * RAW + BM * BK * 4, &map_x, issued * BK, x0, raw_full(r));
+                tma_load_2d(raw0 + r * raw, &map_w, issued * BK, n0, raw_full(r));
+                tma_load_2d(raw0 + r * raw + BM * BK * 4, &map_x, issued * BK, x0, raw_full(r));
             }
             if (s_abort)                                   // no copy lands after the CTA is gone
                 for (int j = max(issued - RAWS, 0); j < issued; ++j)
                     for (uint32_t i = 0; i < WAIT_LIMIT && !mbar_try_wait(raw_full(j % RAWS), (uint32_t)(j / RAWS) & 1u); ++i) {}
+        } else if (warp >= CONV_WARPS + DRAIN_WARPS + 2 && rank == 1 && lane == 0) {
+            // ---- the second CTA's parts are stored (each writer fenced its own for the tensor cores); every other block each ----
+            const uint32_t first = map_to_cta(full_bar(0), 0);
+            int s = warp - (CONV_WARPS + DRAIN_WARPS + 2);
+            uint32_t phase = 0;
+            for (int kb = s; kb < blocks; kb += 2) {
+                if (!mbar_wait(stored_bar(s), phase, &s_abort)) break;
+                mbar_arrive_cluster(first + 8u * s);
+                if ((s += 2) >= stages) { s -= stages; phase ^= 1u; }
+            }
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
