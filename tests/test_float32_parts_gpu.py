@@ -61,6 +61,16 @@ def test_which_products_it_takes():
     assert int(status) == 0
 
 
+def test_a_build_that_cannot_launch_leaves_the_products_to_the_library(monkeypatch):
+    from turboquant_cpp_b200.kernels import gemm_f32 as KF
+    from turboquant_cpp_b200.kernels.linear import linear
+    x, w = inputs(256, 1024, 512, False)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    assert KF.runs() and KF.pays(x, w)
+    monkeypatch.setattr(KF, "runs", lambda: False)
+    assert not KF.pays(x, w) and torch.equal(linear(x, w, status=status), torch.mm(x, w.t()))
+
+
 CASES = [  # H, G, head size, page, runs, held, window
     (4, 2, 128, 64, [1, 31, 32, 33, 64, 65], [0, 0, 31, 40, 0, 7], 0),
     (6, 3, 64, 64, [127, 300], [0, 100], 0),

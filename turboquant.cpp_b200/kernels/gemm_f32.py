@@ -2,6 +2,7 @@
 from __future__ import annotations
 
 from ctypes import c_int, c_longlong, c_void_p
+from functools import lru_cache
 from typing import Optional
 
 import torch
@@ -21,6 +22,13 @@ MIN_RESULTS = 200_000
 MIN_K = 64
 
 
+@lru_cache(maxsize=None)
+def runs() -> bool:
+    """Whether the library on hand can launch the kernel: its warpgroups share out the registers that this repository's compiler gives
+    it, and another compiler may give it fewer."""
+    return bool(load_kernel(_LIB).tq_gemm_f32_runs())
+
+
 def pays(x: torch.Tensor, w: torch.Tensor) -> bool:
     """float32 x [T, K] (rows on 16-byte boundaries) and w [N, K] that this kernel takes and is the faster one for."""
     T, K = x.shape
@@ -28,7 +36,7 @@ def pays(x: torch.Tensor, w: torch.Tensor) -> bool:
             and w.dim() == 2 and w.shape[1] == K and w.is_contiguous() and x.stride(1) == 1 and x.stride(0) % 4 == 0 and x.stride(0) >= K
             and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
             and x.device == w.device and x.device.index == torch.cuda.current_device()
-            and not (torch.is_grad_enabled() and (x.requires_grad or w.requires_grad)))
+            and not (torch.is_grad_enabled() and (x.requires_grad or w.requires_grad)) and runs())
 
 
 def gemm_f32(x: torch.Tensor, w: torch.Tensor, tokens: int = 0, status: Optional[torch.Tensor] = None) -> torch.Tensor:
