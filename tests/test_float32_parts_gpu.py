@@ -58,6 +58,9 @@ def test_which_products_it_takes():
     for a, b in ((x[:100], w), (x[:, :62], w[:, :62]), (strided, w), (x.t().contiguous().t(), w), (x, w.t().contiguous().t()), (x.clone().requires_grad_(), w)):
         assert not KF.pays(a, b)
         torch.testing.assert_close(linear(a, b, status=status), torch.mm(a, b.t()), rtol=0, atol=0)
+    for (T, N, K), taken in {(16, 20480, 128): False, (64, 20480, 128): False, (65, 20480, 128): True, (16, 20480, 256): True, (4096, 64, 64): True,
+                             (8, 30000, 512): False}.items():
+        assert KF.pays(torch.empty((T, K), device=DEV), torch.empty((N, K), device=DEV)) == taken, (T, N, K)
     assert int(status) == 0
 
 

@@ -20,6 +20,11 @@ MIN_TOKENS = 9
 MIN_RESULTS = 200_000
 # Below this a product is a few launches' time either way.
 MIN_K = 64
+# Sums shorter than LONG_K of FEW_TOKENS or fewer are the library's: the tiles' setting up is more than what they compute.  us, here / library:
+# K 64, 40,960 rows 16 / 11 at 16 tokens, 19 / 17 at 64, 20 / 21 at 65; K 128, 20,480 rows 14 / 12 at 32, 16 / 20 at 65, 40,960 rows 20 / 15 at
+# 16, 24 / 31 at 65; K 512, 20,480 rows 26 / 27 at 16, 30 / 41 at 64.  Few weight rows are no reason: 4,096 tokens, K 64, 64 rows 15 / 15, K
+# 512 16 / 15, K 2,048 44 / 42, K 5,632 130 / 139.
+LONG_K, FEW_TOKENS = 256, 64
 
 
 @lru_cache(maxsize=None)
@@ -32,7 +37,8 @@ def runs() -> bool:
 def pays(x: torch.Tensor, w: torch.Tensor) -> bool:
     """float32 x [T, K] (rows on 16-byte boundaries) and w [N, K] that this kernel takes and is the faster one for."""
     T, K = x.shape
-    return (T >= MIN_TOKENS and T * w.shape[0] >= MIN_RESULTS and K % 4 == 0 and K >= MIN_K and x.dtype == torch.float32 and w.dtype == torch.float32
+    return (T >= MIN_TOKENS and T * w.shape[0] >= MIN_RESULTS and K % 4 == 0 and K >= MIN_K and (K >= LONG_K or T > FEW_TOKENS)
+            and x.dtype == torch.float32 and w.dtype == torch.float32
             and w.dim() == 2 and w.shape[1] == K and w.is_contiguous() and x.stride(1) == 1 and x.stride(0) % 4 == 0 and x.stride(0) >= K
             and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
             and x.device == w.device and x.device.index == torch.cuda.current_device()
