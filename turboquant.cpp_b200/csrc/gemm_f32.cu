@@ -442,6 +442,7 @@ TQ_EXPORT int tq_gemm_f32(const float* x, long long ldx, const float* w, float* 
         // cycles: 1,090 at 32 tokens, 1,160 at 96, 1,700 at 240 before the result's writing was shortened)
         long long best = 0;
         for (int k = (T + MAX_TOKENS - 1) / MAX_TOKENS; k <= (T + 15) / 16; ++k) {
+            if (n != 0 && (long long)m_tiles * (T / (T / k + 16)) / 74 * (256 + 16) >= best) break;       // at least as many tiles, of 16 tokens or more
             const int each = ((T + k - 1) / k + 15) / 16 * 16;
             const long long waves = ((long long)m_tiles * ((T + each - 1) / each) + 73) / 74, cost = waves * (256 + each);
             if (n == 0 || cost < best) { n = each; best = cost; }
