@@ -84,7 +84,8 @@ def test_groups_of_chunks(monkeypatch):
 @pytest.mark.parametrize("what", ["key", "value", "beta", "decay", "query"])
 @pytest.mark.parametrize("bad", [float("nan"), float("inf")])
 def test_a_token_that_is_not_finite(what, bad):
-    """Earlier tokens and other heads are what they were; the token and, but for a query, all behind it and the state are not finite."""
+    """Earlier tokens and other heads are what they were; the token and, but for a query, all behind it and the state are not finite, of a
+    value its own column alone.  Token by token the same places are lost."""
     lens, H, G, dk, dv, at = [200, 90], 2, 2, 64, 64, 77
     d = data(lens, H, G, dk, dv)
     clean = run("chunks", d, lens, H, G, dk, dv, [0, 1])
@@ -97,9 +98,32 @@ def test_a_token_that_is_not_finite(what, bad):
     y, was = y.view(-1, H, dv), clean[0].view(-1, H, dv)
     assert torch.equal(y[:at], was[:at]) and torch.equal(y[:, 1], was[:, 1]) and torch.equal(y[200:], was[200:])
     assert torch.equal(state[0, 1], clean[1][0, 1]) and torch.equal(state[1], clean[1][1])
-    gone = slice(at, at + 1) if what == "query" else slice(at, 200)
-    assert not bool(y[gone, 0].isfinite().any())
-    assert torch.equal(state[0, 0], clean[1][0, 0]) if what == "query" else not bool(state[0, 0].isfinite().any())
+    lost, lost_state = torch.zeros_like(y[:, 0], dtype=torch.bool), torch.zeros_like(state[0, 0], dtype=torch.bool)
+    tokens, columns = slice(at, at + 1 if what == "query" else 200), slice(5, 6) if what == "value" else slice(None)
+    lost[tokens, columns] = True
+    if what != "query":
+        lost_state[columns] = True
+    assert not bool(y[:, 0][lost].isfinite().any()) and torch.equal(y[:, 0][~lost], was[:, 0][~lost])
+    assert not bool(state[0, 0][lost_state].isfinite().any()) and torch.equal(state[0, 0][~lost_state], clean[1][0, 0][~lost_state])
+    walked, walked_state = run("walk", d, lens, H, G, dk, dv, [0, 1])
+    assert torch.equal(walked.isfinite(), y.isfinite().view(walked.shape)) and torch.equal(walked_state.isfinite(), state.isfinite())
+
+
+@pytest.mark.parametrize("dk,dv", [(64, 128), (128, 128)])
+def test_values_that_are_not_finite_in_several_columns_and_chunks(dk, dv):
+    """Both ends of a value, several tokens of one chunk and another chunk's first and last token."""
+    lens, H, G = [330], 2, 1
+    d = data(lens, H, G, dk, dv)
+    clean = run("chunks", d, lens, H, G, dk, dv, [0])
+    places = [(0, 1), (63, 0), (64, 17), (70, dv - 1), (66, 40), (100, 40), (127, 33), (329, 2)]
+    for t, c in places:
+        d[0][t, 4 + 2 * G * dk + dv + c] = float("nan")           # the second head
+    y, state = run("chunks", d, lens, H, G, dk, dv, [0])
+    y, was, lost = y.view(-1, H, dv), clean[0].view(-1, H, dv), torch.zeros((330, H, dv), dtype=torch.bool, device=DEV)
+    for t, c in places:
+        lost[t:, 1, c] = True
+    assert bool(y[lost].isnan().all()) and torch.equal(y[~lost], was[~lost])
+    assert bool(state[0][lost[-1]].isnan().all()) and torch.equal(state[0][~lost[-1]], clean[1][0][~lost[-1]])
 
 
 def test_which_steps_go_in_chunks():

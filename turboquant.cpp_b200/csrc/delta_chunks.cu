@@ -18,8 +18,9 @@
 // Chains that were longer: W = T diag(beta A) K in the place of K S, a product less but 96 KB, 2.1 us and a third more work beside the chain;
 // the same with keys brought in float32 and split by four more warps 2.9.
 // A long step does this for a group of chunks after the other, the kept state going from group to group.
-// A token whose key, value, decay or beta is not finite leaves the tokens ahead of it in its chunk as they are (it takes no part in
-// the products); its own output, all later ones and the state are NaN for that head.
+// What is not finite leaves the tokens ahead of it in its chunk as they are (it takes no part in the products).  A key, decay or
+// beta: the token's own output, all later ones and the state are NaN for that head.  An element of a value: the same for its own column,
+// and no other.
 // Everything is kept and added up in float32; products are six bfloat16 ones whose largest are summed over at most 64 elements.
 #include "split3.cuh"
 #include "chunks.cuh"
@@ -52,15 +53,15 @@ struct Cfg {
 // [dv][dk]; a row of numbers.
 struct Scratch { uint8_t *k, *t; float *u, *s, *d; };
 constexpr int T_IMAGE = 3 * T_PART;
-constexpr int N_A = 0, N_BETA = L, N_D = 2 * L, N_LAST = 3 * L, N_BAD = 3 * L + 1, N_ROW = 3 * L + 4;    // A, beta, D[last], A_last, the first token
-                                                                                                         // that is not finite (64: none)
+constexpr int N_A = 0, N_BETA = L, N_D = 2 * L, N_LAST = 3 * L, N_BAD = 3 * L + 1;      // A, beta, D[last], A_last, the first token that is
+constexpr int N_COLS = 3 * L + 4, N_ROW = N_COLS + 128;                                // not finite (64: none) and, per column, the first value
 
 // What a token brings, as delta_prepare lays it out: [k: G x dk | q: G x dk | g: H | k.q: G | beta: H]
 struct Rows { const float* at; int stride, heads, kv_heads; };
 
 template <int DK, int DV>
 __global__ void __launch_bounds__(THREADS, 2)
-delta_solve_kernel(Rows rows, const float* __restrict__ xv, int C, int v_off, Scratch out, int chunk0, const int* __restrict__ cu_seqlens, int n_seqs) {
+delta_solve_kernel(Rows rows, Scratch out, int chunk0, const int* __restrict__ cu_seqlens, int n_seqs) {
     tq_grid_wait();                    // everything below may read what the previous kernel wrote
     tq_grid_launch_dependents();       // the next kernel's CTAs may move in as SMs free up
     using F = Cfg<DK, DV>;
@@ -90,18 +91,12 @@ delta_solve_kernel(Rows rows, const float* __restrict__ xv, int C, int v_off, Sc
         if (!fine) atomicMin(&s_bad, tid);
     }
     {
-        constexpr int KQ = DK / 4, KN = L * KQ / THREADS, VQ = DV / 4, VN = L * VQ / THREADS;
-        float4 k4[KN], v4[VN];         // all of them asked for before the first is used
+        constexpr int KQ = DK / 4, KN = L * KQ / THREADS;
+        float4 k4[KN];                 // all of them asked for before the first is used
 #pragma unroll
         for (int i = 0; i < KN; ++i) {
             const int t = (i * THREADS + tid) / KQ;
             k4[i] = t < c.n ? *reinterpret_cast<const float4*>(tok + (size_t)t * rows.stride + g * DK + tid % KQ * 4) : zero4();
-        }
-        const float* v0 = xv + (size_t)c.t0 * C + v_off + h * DV + tid % VQ * 4;
-#pragma unroll
-        for (int i = 0; i < VN; ++i) {
-            const int t = (i * THREADS + tid) / VQ;
-            v4[i] = t < c.n ? *reinterpret_cast<const float4*>(v0 + (size_t)t * C) : zero4();
         }
 #pragma unroll
         for (int i = 0; i < KN; ++i) {
@@ -109,9 +104,6 @@ delta_solve_kernel(Rows rows, const float* __restrict__ xv, int C, int v_off, Sc
             if (odd(k4[i]) != 0.f) { atomicMin(&s_bad, t); k4[i] = zero4(); }
             tq_put4<DK>(sk, F::K_PART, t, tid % KQ * 4, k4[i]);
         }
-#pragma unroll
-        for (int i = 0; i < VN; ++i)
-            if (odd(v4[i]) != 0.f) atomicMin(&s_bad, (i * THREADS + tid) / VQ);
     }
     for (int i = tid; i < L * LD; i += THREADS) T[i] = 0.f;
     __syncthreads();
@@ -278,7 +270,7 @@ delta_chain_kernel(Scratch io, const float* __restrict__ xv, int C, int v_off, f
     constexpr int KS = F::K_STAGES, TS = F::T_STAGES;
     const uint32_t base = (tq_smem_u32(smem_raw) + 127u) & ~127u, tbase = base + KS * F::IMAGE, zp = tbase + TS * T_IMAGE, up = zp + 3 * F::U_PART;
     float* X = reinterpret_cast<float*>(smem_raw + (up + 3 * F::U_PART - tq_smem_u32(smem_raw)));      // the warps' shares of K S, [warp][16 columns][64 tokens]
-    __shared__ int s_first, s_abort;
+    __shared__ int s_first, s_abort, s_cols[2][16];           // s_cols: a link's first value that is not finite, per column
     __shared__ __align__(8) uint64_t s_bars[2 * (F::K_STAGES + F::T_STAGES)];
     const int s = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * 16, g = h / (heads / kv_heads);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -291,6 +283,7 @@ delta_chain_kernel(Scratch io, const float* __restrict__ xv, int C, int v_off, f
         for (int i = lane; i < s; i += 32) before += (cu_seqlens[i + 1] - cu_seqlens[i] + L - 1) / L;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+        s_cols[lane >> 4][lane & 15] = L;
         if (lane == 0) {
             s_first = before;
             s_abort = 0;
@@ -398,14 +391,23 @@ delta_chain_kernel(Scratch io, const float* __restrict__ xv, int C, int v_off, f
                     float2 x[CHAIN_WARPS];
 #pragma unroll
                     for (int w = 0; w < CHAIN_WARPS; ++w) x[w] = *reinterpret_cast<const float2*>(X + (w * 16 + ln.r + 8 * r) * XLD + s0 + 8 * u);
-                    auto z = [&](float v, float b, float a, float ks) { return b * ((isfinite(v) ? v : 0.f) - a * ks); };
-                    tq_put2<L>(zp, F::U_PART, ln.r + 8 * r, s0 + 8 * u, z(V[u][2 * r], beta[u].x, A[u].x, (x[0].x + x[1].x) + (x[2].x + x[3].x)),
-                               z(V[u][2 * r + 1], beta[u].y, A[u].y, (x[0].y + x[1].y) + (x[2].y + x[3].y)));
+                    auto z = [&](int e, float b, float a, float ks) {
+                        float v = V[u][2 * r + e];
+                        if (!isfinite(v)) { atomicMin(&s_cols[i & 1][ln.r + 8 * r], s0 + 8 * u + e); v = 0.f; }
+                        return b * (v - a * ks);
+                    };
+                    tq_put2<L>(zp, F::U_PART, ln.r + 8 * r, s0 + 8 * u, z(0, beta[u].x, A[u].x, (x[0].x + x[1].x) + (x[2].x + x[3].x)),
+                               z(1, beta[u].y, A[u].y, (x[0].y + x[1].y) + (x[2].y + x[3].y)));
                 }
             const float2 d_left[2] = {left[0], left[1]};
-            const float d_last = bad < (float)L ? NAN : last;        // a token that is not finite: so is the state behind it
+            const float left_last = bad < (float)L ? NAN : last;     // a token that is not finite: so is the state behind it
             if (i + 1 < n) ask(i + 1);
             chain_sync();
+            const float d_last[2] = {s_cols[i & 1][ln.r] < L ? NAN : left_last, s_cols[i & 1][ln.r + 8] < L ? NAN : left_last};
+            if (tid < 16) {
+                io.d[unit * N_ROW + N_COLS + v0 + tid] = (float)s_cols[i & 1][tid];
+                s_cols[(i + 1) & 1][tid] = L;
+            }
             {   // U^T = Z^T T^T.  (T is lower triangular, but the last warp needs all of its row, and
                 // the others would wait for it)
                 float big[2][4], small[2][2][4];
@@ -453,7 +455,7 @@ delta_chain_kernel(Scratch io, const float* __restrict__ xv, int C, int v_off, f
 #pragma unroll
                 for (int u = 0; u < NT; ++u)
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) S[u][e] = d_last * S[u][e] + (big[u][e] + small[u][e]);
+                    for (int e = 0; e < 4; ++e) S[u][e] = d_last[e >> 1] * S[u][e] + (big[u][e] + small[u][e]);
             }
         }
 #pragma unroll
@@ -518,6 +520,10 @@ delta_outputs_kernel(Rows rows, Scratch in, float* __restrict__ y, int chunk0, c
     };
     ask(0);
     __syncthreads();
+    // per column the first value that is not finite, in the place of the decays, which have been used (two CTAs an SM fit with no room for more)
+    uint8_t* cols = reinterpret_cast<uint8_t*>(s_g);
+    const int bad = (int)in.d[unit * N_ROW + N_BAD];
+    if (tid < DV) cols[tid] = (uint8_t)min(bad, (int)in.d[unit * N_ROW + N_COLS + tid]);
     uint32_t P[L / 16][3][4];          // D o Q K^T as left operands
     for (int grp = 0; grp < 2; ++grp) {
         float big[4][4], small[4][4], first[4][4];
@@ -555,7 +561,6 @@ delta_outputs_kernel(Rows rows, Scratch in, float* __restrict__ y, int chunk0, c
     }
     const uint32_t su = sk + 3 * F::SQ_PART;
     const float A[2] = {s_A[16 * warp + ln.r], s_A[16 * warp + ln.r + 8]};
-    const int bad = (int)in.d[unit * N_ROW + N_BAD];
     for (int q = 0; q < DV / 32; ++q) {
         __syncthreads();               // what was there has been used
 #pragma unroll
@@ -604,7 +609,7 @@ delta_outputs_kernel(Rows rows, Scratch in, float* __restrict__ y, int chunk0, c
             if (t < c.n)
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    auto sum = [&](int e) { return t < bad ? o[u][e] + (big[u][e] + small[u][e]) : NAN; };
+                    auto sum = [&](int e) { return t < cols[32 * q + 8 * u + ln.c + (e & 1)] ? o[u][e] + (big[u][e] + small[u][e]) : NAN; };
                     *reinterpret_cast<float2*>(at + 8 * u) = make_float2(sum(2 * r), sum(2 * r + 1));
                 }
         }
@@ -622,7 +627,7 @@ int launch(const Rows& rows, const float* xv, int C, int v_off, const Scratch& s
     if (e != cudaSuccess) TQ_FAIL(-1, "delta_chunks: %d bytes of shared memory refused: %s", F::CHAIN_BYTES, cudaGetErrorString(e));
     for (int chunk0 = 0; chunk0 < chunks; chunk0 += group) {
         const int n = chunks - chunk0 < group ? chunks - chunk0 : group;
-        tq_launch(dim3(n, rows.heads), THREADS, F::SOLVE_BYTES, stream)(delta_solve_kernel<DK, DV>, rows, xv, C, v_off, scratch, chunk0, cu, n_seqs);
+        tq_launch(dim3(n, rows.heads), THREADS, F::SOLVE_BYTES, stream)(delta_solve_kernel<DK, DV>, rows, scratch, chunk0, cu, n_seqs);
         tq_launch(dim3(n_seqs, rows.heads, DV / 16), 32 * (CHAIN_WARPS + 1), F::CHAIN_BYTES, stream)(delta_chain_kernel<DK, DV>, scratch, xv, C, v_off, state,
             slot_stride, slots, rows.heads, rows.kv_heads, chunk0, n, cu, status);
         tq_launch(dim3(n, rows.heads), THREADS, F::OUT_BYTES, stream)(delta_outputs_kernel<DK, DV>, rows, scratch, y, chunk0, cu, n_seqs);
