@@ -135,21 +135,38 @@ def test_which_steps_go_in_chunks():
     assert not m._in_chunks(step([64])) and not m._in_chunks(step([200])) and not m._in_chunks(step([2048] + [1] * 63)) and not m._in_chunks(step([2] * 64))
 
 
-@pytest.mark.parametrize("what", ["key", "value"])
-def test_a_matrix_memory_s_token_that_is_not_finite(what):
-    """In chunks a token's output depends on no later token, and other heads on neither."""
-    from turboquant_cpp_b200.kernels import recurrence as KR
-    H, dk, dv, lens, at = 2, 128, 64, [150, 70], 77
+@pytest.mark.parametrize("what", ["query", "key", "value"])
+@pytest.mark.parametrize("dk,dv", [(64, 64), (128, 64), (128, 128)])
+def test_a_matrix_memory_s_token_that_is_not_finite(what, dk, dv):
+    """In chunks a token's output depends on no later token, other heads on neither, and a value reaches its own column only.  Token by
+    token the same places are lost."""
+    from turboquant_cpp_b200.kernels import recurrence as KR, ssm as KS
+    H, lens, at, column = 2, [150, 70], 77, 35
     g = torch.Generator(device=DEV).manual_seed(1)
     rows, gates = torch.randn((220, H * (2 * dk + dv)), generator=g, device=DEV), -torch.rand((220, H, 2), generator=g, device=DEV)
-    out = []
+    new = lambda: (torch.ones((2, H, dv + 1, dk), device=DEV), torch.empty((220, H * dv), device=DEV), torch.empty((220, H), device=DEV))
+    offsets, cu, slots, out = (0, H * dk, 2 * H * dk), i32([0, 150, 220]), i32([0, 1]), []
     for bad in (0.5, float("nan"), float("inf")):
-        rows[at, (H * dk if what == "key" else 2 * H * dk) + 3] = bad
-        state, y, dots = torch.ones((2, H, dv + 1, dk), device=DEV), torch.empty((220, H * dv), device=DEV), torch.empty((220, H), device=DEV)
-        KR.memory_chunks(rows, 0, H * dk, 2 * H * dk, gates, state, y, dots, KR.chunks_of(lens, 220, 2), H, dk, dv, i32([0, 150, 220]), i32([0, 1]))
+        rows[at, {"query": 0, "key": H * dk, "value": 2 * H * dk}[what] + column] = bad
+        if bad != 0.5:
+            rows[100, 2 * H * dk + 40] = bad                      # the same chunk, another column
+        (state, y, dots), (w_state, w_y, w_dots) = new(), new()
+        KR.memory_chunks(rows, *offsets, gates, state, y, dots, KR.chunks_of(lens, 220, 2), H, dk, dv, cu, slots)
+        KS.memory_scan(rows, *offsets, gates, w_state, w_y, w_dots, H, dk, dv, cu, slots)
+        for a, b in ((y, w_y), (dots, w_dots), (state, w_state)):
+            assert torch.equal(a.isfinite(), b.isfinite())
         out.append((y.view(220, H, dv), dots, state))
-    for y, dots, state in out[1:]:
-        for new, old in ((y, out[0][0]), (dots, out[0][1])):
-            assert torch.equal(new[:at], old[:at]) and torch.equal(new[150:], old[150:]) and torch.equal(new[:, 1], old[:, 1])
-        assert torch.equal(state[1], out[0][2][1]) and torch.equal(state[0, 1], out[0][2][0, 1])
-        assert not bool(y[at:150, 0, 3].isfinite().any()) and not bool(state[0, 0, 3].isfinite().all())
+    lost = torch.zeros_like(out[0][0], dtype=torch.bool)
+    lost[at:at + 1 if what == "query" else 150, 0, slice(column, column + 1) if what == "value" else slice(None)] = True
+    lost[100:150, 0, 40] = True
+    lost_dots, lost_state = torch.zeros_like(out[0][1], dtype=torch.bool), torch.zeros_like(out[0][2], dtype=torch.bool)
+    if what != "value":
+        lost_dots[at:at + 1 if what == "query" else 150, 0] = True
+    lost_state[0, 0, 40] = True
+    if what == "value":
+        lost_state[0, 0, column] = True
+    if what == "key":
+        lost_state[0, 0, :, column] = True
+    for case in out[1:]:
+        for got, was, where in zip(case, out[0], (lost, lost_dots, lost_state)):
+            assert not bool(got[where].isfinite().any()) and torch.equal(got[~where], was[~where])

@@ -14,7 +14,8 @@
 // 682 + 1,366 tokens, 16 heads of 128 x 129: 33 us for the chunks' sums, 17 for the starts and 54 for the outputs (as products on the
 // fp32 units 37, 16 and 79, bound by what they read of shared memory; token by token 289).  With one CTA an SM the outputs take 89; what bounds
 // either kernel with two is a warp's own chain of loads, splitting and products, the tensor cores are active 32 to 40 % of the time.
-// A value that is not finite takes no part in earlier tokens' outputs; the token's own and all later ones are NaN in its group of 32 columns.
+// An element of a value that is not finite takes no part in earlier tokens' outputs; the token's own and all later ones are NaN in its
+// column, and in no other.
 // Part of csrc/ssm.cu's library.
 #pragma once
 #include "split3.cuh"
@@ -306,7 +307,11 @@ memory_outputs_kernel(const float* __restrict__ rows, int C, int q_off, int k_of
 #pragma unroll
         for (int i = 0; i < VN; ++i) {
             const int t = (i * THREADS + tid) >> 3, e = (tid & 7) * 4;
-            if (odd(nv[i]) != 0.f) { atomicMin(&s_bad[q & 1], t); nv[i] = zero4(); }
+            if (odd(nv[i]) != 0.f) {
+                atomicMin(&s_bad[q & 1], t);
+                auto held = [](float v) { return isfinite(v) ? v : 0.f; };
+                nv[i] = make_float4(held(nv[i].x), held(nv[i].y), held(nv[i].z), held(nv[i].w));
+            }
             const TqSplit4 v = tq_split4(nv[i]);
             const uint32_t at = sv + piece32(t, e >> 3) + (e & 4) * 2;
             asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(v.h.x), "r"(v.h.y) : "memory");
@@ -357,10 +362,20 @@ memory_outputs_kernel(const float* __restrict__ rows, int C, int q_off, int k_of
             if (t < c.n)
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    auto sum = [&](int e) { return t < bad ? o[u][e] + (big[u][e] + small[u][e]) : NAN; };
+                    auto sum = [&](int e) { return o[u][e] + (big[u][e] + small[u][e]); };
                     *reinterpret_cast<float2*>(at + 8 * u) = make_float2(sum(2 * r), sum(2 * r + 1));
                 }
         }
+        if (bad < L)                   // the columns that have such a value, from its token on: the values are looked at once more
+#pragma unroll 1
+            for (int i = 0; i < 8; ++i) {
+                const int column = h * DV + 32 * q + 8 * (i >> 1) + ln.c + (i & 1);
+                bool lost = false;
+                for (int t = bad; t < c.n; ++t) {
+                    lost |= !isfinite(tok[(size_t)t * C + v_off + column]);
+                    if (lost && t >> 4 == warp && (t & 7) == ln.r) y[(size_t)(c.t0 + t) * heads * DV + column] = NAN;
+                }
+            }
     }
 }
 
