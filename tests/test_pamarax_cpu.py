@@ -26,7 +26,7 @@ def test_cache_and_state_needs_follow_the_layers():
     assert [s.shape if s else None for s in model.state_needs()] == \
         [None, (3 * 13 * 8 + 3,), (2 * (2 * 2 * 8 + 4 * 12) + 4 * 12 * 8,), (2 * 7 * 20 + 2,), (1 * (2 * 2 * 16 + 2 * 8) + 2 * 8 * 16,)]
     assert model.capturable() and all(e.cache_of is None for e in model.schedule)
-    assert set(model.kernels()) == {"elementwise", "bias_attention", "ssm"}
+    assert set(model.kernels()) == {"elementwise", "bias_attention", "gemm_f32", "ssm"}
 
 
 def test_optional_keys_may_be_missing():

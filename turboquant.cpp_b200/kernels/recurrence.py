@@ -33,9 +33,14 @@ def group_of(chunks: int, heads: int, dk: int, dv: int) -> int:
     return -(-chunks // -(-chunks // most)) if chunks else 1
 
 
+def takes(dk: int, dv: int) -> bool:
+    """Whether the kernels are built for keys and values of these sizes."""
+    return dk in SIZES and dv in SIZES
+
+
 def usable(dk: int, dv: int, rows: torch.Tensor, *offsets: int) -> bool:
     """Whether the kernels take this shape: sizes of 64 or 128, rows and offsets of whole 16 bytes."""
-    return dk in SIZES and dv in SIZES and rows.shape[1] % 4 == 0 and all(o % 4 == 0 for o in offsets) \
+    return takes(dk, dv) and rows.shape[1] % 4 == 0 and all(o % 4 == 0 for o in offsets) \
         and rows.is_contiguous() and rows.data_ptr() % 16 == 0
 
 

@@ -67,9 +67,9 @@ class AttentionMixer(Mixer):
             names.append("gemv")
         if getattr(self, "run_dtype", None) == torch.bfloat16 and self.head_dim in (64, 128):
             names.append("attention_prefill")
-        if getattr(self, "run_dtype", None) == torch.float32:
-            names += ["gemm_f32"] + (["attention_f32"] if self.head_dim in KA.F32_HEAD_DIMS else [])
-        return names
+        if getattr(self, "run_dtype", None) == torch.float32 and self.head_dim in KA.F32_HEAD_DIMS:
+            names.append("attention_f32")
+        return names + self.product_kernels(self.hidden, self.q_size)
 
     def cache_need(self) -> KVNeed:
         return KVNeed(self.n_kv_heads, self.head_dim, self.window)

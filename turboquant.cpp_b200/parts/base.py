@@ -39,6 +39,7 @@ from typing import Any, Callable, Dict, List, Optional, Sequence, Tuple
 
 import torch
 
+from ..kernels.gemm_f32 import MIN_K
 from ..weights.loader import WeightSpec, WeightStore
 
 
@@ -158,6 +159,13 @@ class Part:
     def kernels(self) -> List[str]:
         """Kernel files (csrc/<name>.cu) this part launches; they are built before the first step."""
         return []
+
+    def product_kernels(self, *inner: int) -> List[str]:
+        """What `kernels.linear.linear` may launch for the part's products: csrc/gemm_f32.cu where weights are float32, in a float32 run or
+        because a checkpoint's are (then known once they are bound).  inner: the lengths of the products' sums."""
+        takes = lambda k: k >= MIN_K and k % 4 == 0
+        bound = any(isinstance(t, torch.Tensor) and t.dtype == torch.float32 and t.dim() in (2, 3) and takes(t.shape[-1]) for t in vars(self).values())
+        return ["gemm_f32"] if bound or (getattr(self, "run_dtype", None) == torch.float32 and any(map(takes, inner))) else []
 
     def step_work(self, n_tokens: int, kv_tokens: int) -> Dict[str, Tuple[float, float]]:
         """What a step of n_tokens tokens over sequences that hold kv_tokens tokens together has to do in this

@@ -154,7 +154,8 @@ class BiasedWindowAttentionMixer(Mixer):
             self.mix = float(store.get(p + "vmix").float().item())
 
     def kernels(self) -> List[str]:
-        return ["bias_attention"] + (["attention_prefill", "gemv"] if getattr(self, "run_dtype", None) == torch.bfloat16 else [])
+        return (["bias_attention"] + (["attention_prefill", "gemv"] if getattr(self, "run_dtype", None) == torch.bfloat16 else [])
+                + self.product_kernels(self.hidden, self.heads * self.vdim))
 
     def cache_need(self) -> KVNeed:
         return KVNeed(self.kv_heads, self.dim + self.vdim, self.window, planes=1, keep_first=self.keep_first)

@@ -88,7 +88,8 @@ class ChannelDeltaMixer(Mixer):
         self.g1_off = self.a1_off + self.rank_a
 
     def kernels(self) -> List[str]:
-        return ["ssm"] + (["gemv"] if getattr(self, "run_dtype", None) == torch.bfloat16 else [])
+        return (["ssm"] + (["gemv"] if getattr(self, "run_dtype", None) == torch.bfloat16 else [])
+                + self.product_kernels(self.hidden, self.rank_a, self.rank_g, self.inner))
 
     def state_need(self) -> StateNeed:
         return StateNeed((self.kept_size + self.heads * self.vdim * self.dim,), torch.float32)
@@ -175,7 +176,8 @@ class HeadDeltaMixer(Mixer):
         self.w_o = store.get(p + "o")
 
     def kernels(self) -> List[str]:
-        return ["ssm"] + (["gemv"] if getattr(self, "run_dtype", None) == torch.bfloat16 else [])
+        return (["ssm"] + (["delta_chunks"] if KR.takes(self.dim, self.vdim) else [])
+                + (["gemv"] if getattr(self, "run_dtype", None) == torch.bfloat16 else []) + self.product_kernels(self.hidden, self.inner))
 
     def state_need(self) -> StateNeed:
         return StateNeed((self.kept_size + self.state_size,), torch.float32)

@@ -32,7 +32,7 @@ class SwiGLUFeedForward(FeedForward):
         self.w_down = store.get(p + "down_proj.weight")
 
     def kernels(self) -> List[str]:
-        return ["elementwise"]
+        return ["elementwise"] + self.product_kernels(self.hidden, self.intermediate)
 
     def step_work(self, n_tokens, kv_tokens):
         wb = lambda w: 0 if w is None else w.numel() * w.element_size()
@@ -82,7 +82,7 @@ class GluFeedForward(FeedForward):
             self.down_bias = store.take(p + self.names[2] + ".b").float().contiguous()
 
     def kernels(self) -> List[str]:
-        return ["elementwise"]
+        return ["elementwise"] + self.product_kernels(self.hidden, self.intermediate)
 
     def step_work(self, n_tokens, kv_tokens):
         wb = lambda w: 0 if w is None else w.numel() * w.element_size()
@@ -127,7 +127,7 @@ class ReluSquaredFeedForward(FeedForward):
             self.up_bias, self.down_bias = store.get(self.prefix + self.up_name + ".b"), store.get(self.prefix + self.down_name + ".b")
 
     def kernels(self) -> List[str]:
-        return ["elementwise"]
+        return ["elementwise"] + self.product_kernels(self.hidden, self.intermediate)
 
     def step_work(self, n_tokens, kv_tokens):
         wb = lambda w: 0 if w is None else w.numel() * w.element_size()

@@ -105,7 +105,8 @@ class RotatedValueAttentionMixer(Mixer):
             self.v_freq = f.to(torch.float32).to(store.device).contiguous()
 
     def kernels(self) -> List[str]:
-        return ["bias_attention"] + (["attention_prefill", "gemv"] if getattr(self, "run_dtype", None) == torch.bfloat16 else [])
+        return (["bias_attention"] + (["attention_prefill", "gemv"] if getattr(self, "run_dtype", None) == torch.bfloat16 else [])
+                + self.product_kernels(self.hidden, self.heads * self.vdim))
 
     def cache_need(self) -> KVNeed:
         return KVNeed(self.kv_heads, self.dim + self.vdim, self.window, planes=1)
@@ -183,7 +184,8 @@ class DifferentialAttentionMixer(Mixer):
         self.lam = math.exp(float((l["lq1"] * l["lk1"]).sum())) - math.exp(float((l["lq2"] * l["lk2"]).sum())) + self.diff
 
     def kernels(self) -> List[str]:
-        return ["bias_attention"] + (["attention_prefill", "gemv"] if getattr(self, "run_dtype", None) == torch.bfloat16 else [])
+        return (["bias_attention"] + (["attention_prefill", "gemv"] if getattr(self, "run_dtype", None) == torch.bfloat16 else [])
+                + self.product_kernels(self.hidden, self.heads * self.vdim))
 
     def cache_need(self) -> KVNeed:
         return KVNeed(2 * self.kv_heads, self.dim + self.vdim, self.keep, planes=1)

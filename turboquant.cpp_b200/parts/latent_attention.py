@@ -103,7 +103,7 @@ class LatentAttentionMixer(Mixer):
 
     def kernels(self) -> List[str]:
         return (["latent_attention"] + (["attention_prefill"] if getattr(self, "run_dtype", None) == torch.bfloat16 else [])
-                + (["elementwise"] if self.q_rank else []))
+                + (["elementwise"] if self.q_rank else []) + self.product_kernels(self.hidden, self.q_rank, self.kv_rank, self.heads * self.vdim))
 
     def cache_need(self) -> KVNeed:
         return KVNeed(1, self.kv_rank + self.rot_dim, self.keep_window, planes=1)

@@ -63,7 +63,8 @@ class MatrixMemoryMixer(Mixer):
         self.w_norm, self.w_o = store.get(p + "norm"), store.get(p + "o")
 
     def kernels(self) -> List[str]:
-        return ["ssm"] + (["gemv"] if getattr(self, "run_dtype", None) == torch.bfloat16 else [])
+        return (["ssm"] + (["gemv"] if getattr(self, "run_dtype", None) == torch.bfloat16 else [])
+                + self.product_kernels(self.hidden, self.inner))
 
     def state_need(self) -> StateNeed:
         return StateNeed((self.state_size + self.heads,), torch.float32)

@@ -201,7 +201,7 @@ class MoEFeedForward(FeedForward):
         dt = self.w13.dtype if self.w13 is not None else getattr(self, "run_dtype", torch.bfloat16)
         if dt == torch.bfloat16:
             names.append("gemm_tc")       # float32 runs never launch the tensor-core kernel
-        return names
+        return names + (self.product_kernels(self.hidden, self.shared_intermediate) if self.shared_intermediate else [])
 
     def step_work(self, n_tokens, kv_tokens):
         E, k, H, I, S = self.n_experts, self.top_k, self.hidden, self.intermediate, self.shared_intermediate

@@ -81,7 +81,8 @@ class NormedAttentionMixer(Mixer):
             self.position.prepare(store.device)
 
     def kernels(self) -> List[str]:
-        return ["bias_attention"] + (["attention_prefill", "gemv"] if getattr(self, "run_dtype", None) == torch.bfloat16 else [])
+        return (["bias_attention"] + (["attention_prefill", "gemv"] if getattr(self, "run_dtype", None) == torch.bfloat16 else [])
+                + self.product_kernels(self.hidden, self.heads * self.vdim))
 
     def cache_need(self) -> KVNeed:
         return KVNeed(self.kv_heads, self.dim + self.vdim, self.window, planes=1)

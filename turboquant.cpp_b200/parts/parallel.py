@@ -64,7 +64,7 @@ class ParallelMixer(Mixer):
                 self.right.take_input_weight(self.w_in[a.shape[0]:])
 
     def kernels(self) -> List[str]:
-        return ["elementwise"] + self.left.kernels() + self.right.kernels()
+        return ["elementwise"] + self.left.kernels() + self.right.kernels() + self.product_kernels()
 
     def cache_need(self) -> Optional[KVNeed]:
         return self.left.cache_need() or self.right.cache_need()

@@ -66,7 +66,7 @@ class RetentionMixer(Mixer):
             self.position.prepare(store.device)
 
     def kernels(self) -> List[str]:
-        return ["ssm"]
+        return ["ssm"] + self.product_kernels(self.hidden, self.inner)
 
     def state_need(self) -> StateNeed:
         return StateNeed((self.heads * self.vdim * self.dim,), torch.float32)

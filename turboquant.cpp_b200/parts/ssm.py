@@ -58,7 +58,7 @@ class Mamba2Mixer(Mixer):
         self.w_norm = store.get(p + "norm")
 
     def kernels(self) -> List[str]:
-        return ["ssm"]
+        return ["ssm"] + self.product_kernels(self.hidden, self.inner)
 
     def state_need(self) -> StateNeed:
         return StateNeed((self.kept_size + self.heads * self.n_state * self.vdim,), torch.float32)

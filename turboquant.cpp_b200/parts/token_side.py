@@ -42,7 +42,7 @@ class TokenSideInput(Part):
         self.w_gate, self.w_proj, self.w_norm = store.get(p + "gate"), store.get(p + "proj"), store.get(p + "norm")
 
     def kernels(self) -> List[str]:
-        return ["elementwise"]
+        return ["elementwise"] + self.product_kernels(self.hidden, self.dim)
 
     def step_work(self, n_tokens, kv_tokens):
         wb = lambda w: 0 if w is None else w.numel() * w.element_size()
