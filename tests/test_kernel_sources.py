@@ -126,3 +126,13 @@ def test_arrivals_in_another_cta_name_their_scope():
                         found += 1
                         assert re.search(r"\.(release|relaxed)\.cluster\.", op), (name, op)
     assert found >= 2
+
+
+def test_shared_memory_is_asked_for_on_every_device():
+    """A kernel's shared memory limit belongs to a device: what was asked for is remembered per device (common.cuh), never in a flag of
+    the process, or a second GPU's launches are refused."""
+    for name in sorted(os.listdir(CSRC)):
+        if name.endswith((".cu", ".cuh")):
+            with open(os.path.join(CSRC, name), encoding="utf-8") as f:
+                text = f.read()
+            assert "cudaFuncAttributeMaxDynamicSharedMemorySize" not in text or name == "common.cuh", name

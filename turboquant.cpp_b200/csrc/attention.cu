@@ -844,12 +844,9 @@ TQ_EXPORT int tq_attention_split(const void* q, const void* cache, int act_dtype
         do {                                                                                                    \
             auto kern = attention_gqa_kernel<HD_>;                                                              \
             constexpr int smem = gqa_smem_bytes<HD_>();                                                         \
-            static bool configured = false;                                                                     \
-            if (!configured) {                                                                                  \
-                cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);  \
-                if (e != cudaSuccess) TQ_FAIL(-1, "attention_split: %d bytes of shared memory refused: %s", smem, cudaGetErrorString(e)); \
-                configured = true;                                                                              \
-            }                                                                                                   \
+            static std::atomic<unsigned long long> asked{0};                                                   \
+            const cudaError_t e = tq_reserve_smem(kern, smem, asked);                                          \
+            if (e != cudaSuccess) TQ_FAIL(-1, "attention_split: %d bytes of shared memory refused: %s", smem, cudaGetErrorString(e)); \
             tq_launch(dim3(T_, nkv, n_splits), GQA_WARPS * 32, smem, stream)(kern,                              \
                 (const __nv_bfloat16*)q, (const __nv_bfloat16*)cache, positions, seq_of_token, page_table, table_stride, \
                 page_size, window, scale, partial, n_splits, arrived, (__nv_bfloat16*)out, nh, nkv, n_seqs, n_pages, early_keys); \
@@ -867,12 +864,9 @@ TQ_EXPORT int tq_attention_split(const void* q, const void* cache, int act_dtype
     do {                                                                                                        \
         auto kern = attention_split_kernel<TA, LPK, GC, STAGES>;                                                \
         constexpr int ring = split_ring_bytes<TA, LPK, STAGES>();                                               \
-        static bool configured = false;                                                                         \
-        if (ring > 0 && !configured) {                                                                          \
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ring);      \
-            if (e != cudaSuccess) TQ_FAIL(-1, "attention_split: %d bytes of shared memory refused: %s", ring, cudaGetErrorString(e)); \
-            configured = true;                                                                                  \
-        }                                                                                                       \
+        static std::atomic<unsigned long long> asked{0};                                                       \
+        const cudaError_t e = ring > 0 ? tq_reserve_smem(kern, ring, asked) : cudaSuccess;                     \
+        if (e != cudaSuccess) TQ_FAIL(-1, "attention_split: %d bytes of shared memory refused: %s", ring, cudaGetErrorString(e)); \
         tq_launch(grid, SPLIT_WARPS * 32, ring, stream)(kern,                                                   \
             (const TA*)q, (const TA*)cache, positions, seq_of_token, page_table, table_stride, page_size, window, \
             scale, partial, n_splits, arrived, (TA*)out, nh, nkv, n_seqs, n_pages, early_keys);                 \
@@ -1135,12 +1129,9 @@ TQ_EXPORT int tq_attention_tiled(const void* q, const void* cache, int act_dtype
 #define TILED_LAUNCH(TA, EPL)                                                                                   \
     do {                                                                                                        \
         auto kern = attention_tiled_kernel<TA, EPL>;                                                            \
-        static size_t configured = 0;                                                                           \
-        if (smem > 48 * 1024 && smem > configured) {                                                            \
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-            if (e != cudaSuccess) TQ_FAIL(-1, "attention_tiled: %zu bytes of shared memory refused: %s", smem, cudaGetErrorString(e)); \
-            configured = smem;                                                                                  \
-        }                                                                                                       \
+        static TqSmemAsked asked{};                                                                            \
+        const cudaError_t e = tq_grow_smem(kern, smem, asked);                                                 \
+        if (e != cudaSuccess) TQ_FAIL(-1, "attention_tiled: %zu bytes of shared memory refused: %s", smem, cudaGetErrorString(e)); \
         tq_launch(grid, TILED_WARPS * 32, smem, stream)(kern, (const TA*)q, (const TA*)cache, cu_seqlens, seq_start, \
             page_table, table_stride, page_size, window, scale, (TA*)out, n_seqs, nh, nkv, hd, n_pages);        \
     } while (0)

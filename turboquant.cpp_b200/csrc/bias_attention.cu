@@ -1169,13 +1169,9 @@ TQ_EXPORT int tq_bias_attention_group(const void* q, const void* cache, const fl
     if (!done && dk == DK_ && dv == DV_ && gc == GC_) {                                                               \
         constexpr int kpi = 32 / (DK_ / 8), loads = kpi >= 8 ? 1 : 8 / kpi, nvc = DV_ / 8 > DK_ / 8 ? DV_ / DK_ : 1;   \
         constexpr int ring_bytes = BA_WARPS * BG_STAGES * loads * (1 + nvc) * 32 * 16;                                \
-        static bool configured = false;                                                                               \
-        if (!configured) {                                                                                            \
-            cudaError_t e = cudaFuncSetAttribute(bias_attention_group_kernel<DK_, DV_, GC_>,                           \
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, ring_bytes);            \
-            if (e != cudaSuccess) TQ_FAIL(-1, "bias_attention_group: %d bytes of shared memory refused: %s", ring_bytes, cudaGetErrorString(e)); \
-            configured = true;                                                                                        \
-        }                                                                                                             \
+        static std::atomic<unsigned long long> asked{0};                                                       \
+        const cudaError_t e = tq_reserve_smem(bias_attention_group_kernel<DK_, DV_, GC_>, ring_bytes, asked);  \
+        if (e != cudaSuccess) TQ_FAIL(-1, "bias_attention_group: %d bytes of shared memory refused: %s", ring_bytes, cudaGetErrorString(e)); \
         tq_launch(grid, BA_WARPS * 32, ring_bytes, stream)(bias_attention_group_kernel<DK_, DV_, GC_>, (const __nv_bfloat16*)q,  \
             (const __nv_bfloat16*)cache, bias_t, far, sink, positions, seq_of_token, page_table, table_stride, page_size, \
             window, keep_first, cell, scale, softcap, (__nv_bfloat16*)out, partial, n_splits, nh, nkv, n_seqs, n_pages);             \
@@ -1646,12 +1642,9 @@ int launch_bias_heads(const void* q, const void* cache, const float* bias_t, int
     const int ring = BA_WARPS * BH_STAGES * BH_K * (DK + DV + 8) * (int)sizeof(__nv_bfloat16);
     const int merge = BA_WARPS * 8 * NT * (2 + DV + 4) * (int)sizeof(float);
     const int smem = ring > merge ? ring : merge;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) TQ_FAIL(-1, "bias_attention_heads: %d bytes of shared memory refused: %s", smem, cudaGetErrorString(e));
-        configured = true;
-    }
+    static std::atomic<unsigned long long> asked{0};
+    const cudaError_t e = tq_reserve_smem(kern, smem, asked);
+    if (e != cudaSuccess) TQ_FAIL(-1, "bias_attention_heads: %d bytes of shared memory refused: %s", smem, cudaGetErrorString(e));
     const int chunks = (nh / nkv + 8 * NT - 1) / (8 * NT);
     dim3 grid(T_, nkv * chunks, n_splits);
     tq_launch(grid, BA_WARPS * 32, smem, stream)(kern, (const __nv_bfloat16*)q, (const __nv_bfloat16*)cache, bias_t, far, sink,
@@ -1696,12 +1689,9 @@ int launch_bias_runs(const void* q, const void* cache, const float* bias_t, int 
                      cudaStream_t stream) {
     auto kern = bias_attention_runs_kernel<DK, DV>;
     const int smem = 2 * BR_K * (DK + DV + 8) * (int)sizeof(__nv_bfloat16);
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) TQ_FAIL(-1, "bias_attention_runs: %d bytes of shared memory refused: %s", smem, cudaGetErrorString(e));
-        configured = true;
-    }
+    static std::atomic<unsigned long long> asked{0};
+    const cudaError_t e = tq_reserve_smem(kern, smem, asked);
+    if (e != cudaSuccess) TQ_FAIL(-1, "bias_attention_runs: %d bytes of shared memory refused: %s", smem, cudaGetErrorString(e));
     dim3 grid(nh, n_seqs, (max_run + BR_Q - 1) / BR_Q);
     tq_launch(grid, BR_WARPS * 32, smem, stream)(kern, (const __nv_bfloat16*)q, (const __nv_bfloat16*)cache, bias_t, far,
         sink, cu_seqlens, seq_start, page_table, table_stride, window, keep_first, cell, scale, softcap, (__nv_bfloat16*)out, nh, nkv, n_pages);

@@ -12,6 +12,7 @@
 #include <stdlib.h>
 #include <math.h>
 #include <atomic>
+#include <mutex>
 
 #define TQ_EXPORT extern "C" __attribute__((visibility("default")))
 
@@ -43,6 +44,24 @@ inline cudaError_t tq_reserve_smem(K kernel, int bytes, std::atomic<unsigned lon
     if (asked.load(std::memory_order_relaxed) & bit) return cudaSuccess;
     e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e == cudaSuccess) asked.fetch_or(bit, std::memory_order_relaxed);
+    return e;
+}
+
+// The same for a kernel whose need differs from call to call; `asked` holds the most asked for on each device.  (Below 48 KB too: a kernel
+// gets that much unasked, its static arrays among it.)
+struct TqSmemAsked { std::atomic<int> bytes[64]; };
+template <typename K>
+inline cudaError_t tq_grow_smem(K kernel, size_t bytes, TqSmemAsked& asked) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::atomic<int>* most = dev < 64 ? &asked.bytes[dev] : nullptr;
+    if (most && most->load(std::memory_order_relaxed) >= (int)bytes) return cudaSuccess;
+    static std::mutex one;             // or a smaller need of another thread could take back a larger one's
+    const std::lock_guard<std::mutex> lock(one);
+    if (most && most->load(std::memory_order_relaxed) >= (int)bytes) return cudaSuccess;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess && most) most->store((int)bytes, std::memory_order_relaxed);
     return e;
 }
 

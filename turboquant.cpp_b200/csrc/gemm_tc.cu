@@ -695,12 +695,9 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mxt,
            TqGlu act = TqGlu{INFINITY, 1.0f, 0.0f}, int map = TQ_MAP_COPY) {
     using T = Tile<BN, PAIR>;
     auto kern = gemm_tc_kernel<BN, SWIGLU, TO, PAIR, KSPLIT, SECOND>;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM_BYTES);
-        if (e != cudaSuccess) TQ_FAIL(-1, "gemm_tc: cannot reserve %d bytes of shared memory: %s", T::SMEM_BYTES, cudaGetErrorString(e));
-        configured = true;
-    }
+    static std::atomic<unsigned long long> asked{0};
+    const cudaError_t e = tq_reserve_smem(kern, T::SMEM_BYTES, asked);
+    if (e != cudaSuccess) TQ_FAIL(-1, "gemm_tc: cannot reserve %d bytes of shared memory: %s", T::SMEM_BYTES, cudaGetErrorString(e));
     // persistent CTAs (or pairs): at most what the GPU runs at once; each walks tiles w, w + workers, ...
     static int resident = 0;
     if (resident == 0) {

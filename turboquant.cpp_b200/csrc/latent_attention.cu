@@ -644,12 +644,9 @@ TQ_EXPORT int tq_latent_attention(const void* q_lat, const void* q, int q_dim, i
 #define LATM_LAUNCH(OT_, NW_)                                                                                         \
         do {                                                                                                       \
             auto kern = latent_attention_mma_kernel<OT_, NW_>;                                                         \
-            static size_t allowed = 48 * 1024;                                                                     \
-            if (smem > allowed) {                                                                                  \
-                cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-                if (e != cudaSuccess) TQ_FAIL(-1, "latent_attention: %d bytes of shared memory refused: %s", (int)smem, cudaGetErrorString(e)); \
-                allowed = smem;                                                                                    \
-            }                                                                                                      \
+            static TqSmemAsked asked{};                                                                        \
+            const cudaError_t e = tq_grow_smem(kern, smem, asked);                                             \
+            if (e != cudaSuccess) TQ_FAIL(-1, "latent_attention: %d bytes of shared memory refused: %s", (int)smem, cudaGetErrorString(e)); \
             tq_launch(grid, NW_ * 32, smem, stream)(kern, (const __nv_bfloat16*)q_lat,                             \
                 (const __nv_bfloat16*)q, q_dim, q_off, (const __nv_bfloat16*)cache, sink, positions, seq_of_token, page_table, \
                 table_stride, page_size, window, scale, (__nv_bfloat16*)out, partial, H, R, rot, n_seqs, n_pages); \

@@ -561,10 +561,9 @@ TQ_EXPORT int tq_moe_align(const int* ids, int P, int E, int tile_rows, int chun
     tq_launch(n_chunks, threads, (size_t)E * sizeof(int), stream)(moe_chunk_hist_kernel, ids, P, E, chunk, chunk_hist);
     TQ_CHECK_LAUNCH("moe_chunk_hist");
     const size_t smem = (size_t)(4 * E + 2 + (threads / 32) * E) * sizeof(int);
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(moe_chunk_place_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        TQ_REQUIRE(e == cudaSuccess, "moe_align: %zu bytes of shared memory refused: %s", smem, cudaGetErrorString(e));
-    }
+    static TqSmemAsked asked{};
+    const cudaError_t e = tq_grow_smem(moe_chunk_place_kernel, smem, asked);
+    TQ_REQUIRE(e == cudaSuccess, "moe_align: %zu bytes of shared memory refused: %s", smem, cudaGetErrorString(e));
     tq_launch(n_chunks, threads, smem, stream)(moe_chunk_place_kernel, ids, P, E, tile_rows, chunk, n_chunks, chunk_hist, counts,
                                                sorted_pair, row_of_pair, expert_offset, tile_expert, tile_row0, tile_count,
                                                n_tiles);
@@ -1075,12 +1074,9 @@ router_small_kernel(const TA* __restrict__ x, const TW* __restrict__ wr, const T
 template <typename TA, typename TW, typename... Args>
 static cudaError_t launch_router_cluster(size_t smem, cudaStream_t stream, Args... args) {
     auto kern = router_cluster_kernel<TA, TW>;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMALL_CLUSTER_DYNAMIC_BYTES);
-        if (e != cudaSuccess) return e;
-        configured = true;
-    }
+    static std::atomic<unsigned long long> asked{0};
+    const cudaError_t e = tq_reserve_smem(kern, SMALL_CLUSTER_DYNAMIC_BYTES, asked);
+    if (e != cudaSuccess) return e;
     tq_launch(SMALL_CLUSTER, SMALL_THREADS, smem, stream, SMALL_CLUSTER)(kern, args...);
     return cudaSuccess;
 }
@@ -1396,12 +1392,9 @@ int launch_grouped_gemv(const void* A, const void* W, void* C, const int* te, co
                         int by, int R, int N, int K, int tile_rows, TqGlu act, int map, cudaStream_t stream) {
     auto kern = grouped_gemv_kernel<TA, TW, TO, SWIGLU>;
     const int smem = GV_ROWS * GV_KC * (int)sizeof(float);
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) TQ_FAIL(-1, "grouped_gemm: %d bytes of shared memory refused: %s", smem, cudaGetErrorString(e));
-        configured = true;
-    }
+    static std::atomic<unsigned long long> asked{0};
+    const cudaError_t e = tq_reserve_smem(kern, smem, asked);
+    if (e != cudaSuccess) TQ_FAIL(-1, "grouped_gemm: %d bytes of shared memory refused: %s", smem, cudaGetErrorString(e));
     constexpr int cols = GV_WARPS;
     dim3 grid((N + cols - 1) / cols, by);
     // 16-byte (8-byte) loads of four weights: rows of K values that start on such a boundary

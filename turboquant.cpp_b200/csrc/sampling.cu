@@ -339,12 +339,9 @@ TQ_EXPORT int tq_sample_rows(const float* logits, int R, int V, float temperatur
     const int cluster = row_cluster(V), slice = (V + cluster - 1) / cluster;
     if (slice > SAMPLE_SMEM_FLOATS) p_in_global = 1;
     const size_t smem = p_in_global ? 0 : (size_t)slice * sizeof(float);
-    static size_t smem_set = 0;
-    if (smem > smem_set) {
-        cudaError_t e = cudaFuncSetAttribute(sample_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        TQ_REQUIRE(e == cudaSuccess, "sample_rows: %zu bytes of shared memory refused: %s", smem, cudaGetErrorString(e));
-        smem_set = smem;
-    }
+    static TqSmemAsked asked{};
+    const cudaError_t e = tq_grow_smem(sample_rows_kernel, smem, asked);
+    TQ_REQUIRE(e == cudaSuccess, "sample_rows: %zu bytes of shared memory refused: %s", smem, cudaGetErrorString(e));
     tq_launch(R * cluster, SAMPLE_THREADS, smem, stream, cluster)(sample_rows_kernel, logits, V, slice, temperature,
                                                                   top_p, uniforms, work, p_in_global, out);
     TQ_CHECK_LAUNCH("sample_rows");

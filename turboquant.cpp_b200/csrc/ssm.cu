@@ -1572,11 +1572,9 @@ TQ_EXPORT int tq_delta_scan_runs(const float* xqkv, int C, int q_off, int k_off,
     const bool few_blocks = (long long)grid.x * grid.y * grid.z <= 2LL * n_sms;
 #define DELTA_ROWS_LAUNCH(RP, HD)                                                                                      \
     do {                                                                                                               \
-        static bool roomy = false;             /* asked for once: two chunks' rows can pass the 48 KB a kernel gets unasked */ \
-        if (smem > 48 * 1024 && !roomy) {                                                                              \
-            cudaFuncSetAttribute(delta_scan_rows_kernel<RP, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024); \
-            roomy = true;                                                                                              \
-        }                                                                                                              \
+        static TqSmemAsked asked{};            /* two chunks' rows can pass the 48 KB a kernel gets unasked */ \
+        const cudaError_t e = tq_grow_smem(delta_scan_rows_kernel<RP, HD>, smem, asked);                       \
+        TQ_REQUIRE(e == cudaSuccess, "delta_scan_runs: %zu bytes of shared memory refused: %s", (size_t)smem, cudaGetErrorString(e)); \
         tq_launch(grid, 256, smem, stream, 1, few_blocks ? false : true)(delta_scan_rows_kernel<RP, HD>, (const float*)rows, R, xqkv, C, \
             v_off, state, slot_stride, y, heads, kv_heads, dk, dv, tc, vec, cu_seqlens, slots);                         \
     } while (0)
