@@ -2,7 +2,8 @@
 library of csrc/ssm.cu) and the delta rule with one decay per head (csrc/delta_chunks.cu)."""
 from __future__ import annotations
 
-from ctypes import c_float, c_int, c_longlong, c_void_p
+from ctypes import c_float, c_longlong, c_void_p
+from functools import lru_cache
 from typing import Optional, Sequence
 
 import torch
@@ -66,11 +67,18 @@ def memory_chunks(rows: torch.Tensor, q_off: int, k_off: int, v_off: int, gates:
         c_void_p(at), c_void_p(at + 4 * group * per_chunk), *ints(chunks, group, n_seqs, heads, dk, dv), ptr(cu_seqlens), ptr(slots), stream()), kernels=3 * -(-chunks // group))
 
 
+@lru_cache(maxsize=256)
 def delta_bytes(group: int, heads: int, kv_heads: int, dk: int, dv: int) -> int:
-    """Bytes of scratch that a group of the delta rule's chunks takes (csrc/delta_chunks.cu)."""
+    """Bytes of scratch that a group of the delta rule's chunks takes (csrc/delta_chunks.cu); as many times those of one chunk."""
     lib = load_kernel("delta_chunks")
     lib.tq_delta_chunks_bytes.restype = c_longlong
     return int(lib.tq_delta_chunks_bytes(*ints(group, heads, kv_heads, dk, dv)))
+
+
+@lru_cache(maxsize=256)
+def delta_rows_width(heads: int, kv_heads: int, dk: int) -> int:
+    """Floats of a token's prepared row with one decay per head (csrc/ssm.cu)."""
+    return int(load_kernel(_LIB).tq_delta_rows_width(*ints(heads, kv_heads, dk, 1)))
 
 
 def delta_chunks(xqkv: torch.Tensor, q_off: int, k_off: int, v_off: int, proj: torch.Tensor, b_off: int, a_raw: torch.Tensor, a_off: int,
@@ -88,18 +96,20 @@ def delta_chunks(xqkv: torch.Tensor, q_off: int, k_off: int, v_off: int, proj: t
     if not usable(dk, dv, xqkv, v_off) or tuple(state.shape[1:]) != (heads, dv, dk) or not state[0].is_contiguous() or y.numel() != T * heads * dv \
             or dt_bias.numel() != heads or a_log.numel() != heads or slots.numel() < n_seqs or y.data_ptr() % 16:
         raise KernelError("delta_chunks: sizes of 64 or 128, aligned rows, one decay per head, a state row of [heads, vdim, dim]")
-    lib = load_kernel(_LIB)
-    rows = torch.empty((T, int(lib.tq_delta_rows_width(*ints(heads, kv_heads, dk, 1)))), dtype=torch.float32, device=xqkv.device)
-    check(_LIB, lib.tq_delta_prepare(
-        ptr(xqkv), *ints(xqkv.shape[1], q_off, k_off), ptr(proj), *ints(proj.shape[1], b_off), ptr(a_raw), *ints(a_raw.shape[1], a_off, 1), ptr(dt_bias),
-        ptr(a_log), ptr(rows), *ints(T, heads, kv_heads, dk), c_float(unit_eps), c_float(q_scale), stream()))
     if chunks == 0:
         return y
-    most = max(1, SCRATCH_BYTES // delta_bytes(1, heads, kv_heads, dk, dv))
-    group = -(-chunks // -(-chunks // most))
-    scratch = torch.empty(delta_bytes(group, heads, kv_heads, dk, dv), dtype=torch.uint8, device=xqkv.device)
+    lib, at, st = load_kernel(_LIB), stream(), ptr(xqkv)
+    each = delta_bytes(1, heads, kv_heads, dk, dv)
+    group = -(-chunks // -(-chunks // max(1, SCRATCH_BYTES // each)))
+    # one buffer: the chunks' scratch, then the prepared rows
+    width = delta_rows_width(heads, kv_heads, dk)
+    buf = torch.empty(group * each + 4 * T * width, dtype=torch.uint8, device=xqkv.device)
+    rows = c_void_p(buf.data_ptr() + group * each)
+    check(_LIB, lib.tq_delta_prepare(
+        st, *ints(xqkv.shape[1], q_off, k_off), ptr(proj), *ints(proj.shape[1], b_off), ptr(a_raw), *ints(a_raw.shape[1], a_off, 1), ptr(dt_bias),
+        ptr(a_log), rows, *ints(T, heads, kv_heads, dk), c_float(unit_eps), c_float(q_scale), at))
     check("delta_chunks", load_kernel("delta_chunks").tq_delta_chunks(
-        ptr(rows), c_int(rows.shape[1]), ptr(xqkv), *ints(xqkv.shape[1], v_off), ctypes_ptr(state), c_longlong(state.stride(0)), ptr(y), ptr(scratch),
+        rows, *ints(width), st, *ints(xqkv.shape[1], v_off), ctypes_ptr(state), c_longlong(state.stride(0)), ptr(y), ptr(buf),
         *ints(chunks, group, n_seqs, heads, kv_heads, dk, dv), ptr(cu_seqlens), ptr(slots), ptr(status if status is not None else status_word(xqkv.device)),
-        stream()), kernels=3 * -(-chunks // group))
+        at), kernels=3 * -(-chunks // group))
     return y
