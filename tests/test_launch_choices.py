@@ -112,6 +112,25 @@ def test_when_a_matrix_memory_goes_in_chunks(monkeypatch):
     assert in_chunks([2048] + ones(127), heads=4) and in_chunks([1024] * 8, heads=8, d=64) and not in_chunks([512] + ones(63), heads=8, d=64)
 
 
+def test_when_a_delta_rule_goes_in_chunks():
+    """Steps that were timed in both forms, of heads of 64 and of 128, and a GPU of half the multiprocessors, whose rounds are twice as many."""
+    from types import SimpleNamespace
+
+    from turboquant_cpp_b200.parts import make_mixer
+
+    def in_chunks(lens, heads=16, dk=128, dv=128, sms=148):
+        m = make_mixer("head_delta", prefix="", hidden=64, heads=heads, kv_heads=heads, dim=dk, vdim=dv, taps=4, eps=1e-5)
+        return m._in_chunks(SimpleNamespace(max_q_len=max(lens), n_seqs=len(lens), n_tokens=sum(lens), host_q_lens=lens), sms)
+    ones = lambda n: [1] * n
+    for lens in ([512], [2048], [4096], [1000, 1048], [512] * 8, [2048] + ones(31)):
+        assert in_chunks(lens), lens
+    for lens in ([1], [64], [300], [40] * 16, [512] + ones(31), [2048] + ones(63), [2048] + ones(127)):
+        assert not in_chunks(lens), lens
+    assert in_chunks([700], 4, 64, 64) and in_chunks([700], 16, 64, 64) and in_chunks([2048] + ones(127), 4, 64, 64) and not in_chunks([512], 4, 64, 64)
+    assert in_chunks([2048], 32, 64, 64) and not in_chunks([512] * 8, 32, 64, 64) and in_chunks([2048] * 4, 16, 64, 128) and not in_chunks([256] * 2, 16, 64, 128)
+    assert in_chunks([2048], 8, 128, 128, 74) and not in_chunks([2048], 16, 96, 128)          # sizes that the chunks are not built for
+
+
 def test_expanded_latent_keys_take_a_bounded_scratch():
     """One prompt expands whatever its length (the scores of the other path take more); many prompts with long histories do not
     where their keys and values would take several times what that path takes."""

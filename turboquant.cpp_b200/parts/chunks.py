@@ -16,15 +16,20 @@ ROUNDS = 4
 _sm_counts = {}
 
 
+def sm_count(device) -> int:
+    """Multiprocessors of a device, asked for once."""
+    key = str(device)
+    if key not in _sm_counts:
+        _sm_counts[key] = torch.cuda.get_device_properties(device).multi_processor_count
+    return _sm_counts[key]
+
+
 def cut_size(ctx: StepContext, heads: int, columns: int) -> Optional[int]:
     """The tokens of a chunk if this step's runs are worth cutting (see `cut_runs`), else None."""
     lens = list(ctx.host_q_lens)
     if not lens or len(lens) != ctx.n_seqs or max(lens) < 2 * MIN_CHUNK:
         return None
-    key = str(ctx.device)
-    if key not in _sm_counts:
-        _sm_counts[key] = torch.cuda.get_device_properties(ctx.device).multi_processor_count
-    room, warps = _sm_counts[key] * KS.SCAN_WARPS_PER_SM, KS.scan_warps(len(lens), heads, columns)
+    room, warps = sm_count(ctx.device) * KS.SCAN_WARPS_PER_SM, KS.scan_warps(len(lens), heads, columns)
     if room // warps < 2:
         return None
     cuts = ROUNDS * room // warps

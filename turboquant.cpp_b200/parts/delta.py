@@ -31,6 +31,7 @@ from ..kernels import ssm as KS
 from ..kernels.linear import linear
 from ..weights.loader import WeightSpec, WeightStore
 from .base import LayerCache, Mixer, StateNeed, StepContext, register_mixer
+from .chunks import sm_count
 
 UNIT_EPS = 1e-6          # inside the root of the unit vectors of q and k
 
@@ -136,7 +137,8 @@ register_mixer("channel_delta", ChannelDeltaMixer)
 
 
 class HeadDeltaMixer(Mixer):
-    """The delta rule with one decay per head (see the module's header)."""
+    """The delta rule with one decay per head (see the module's header).  An element of a value that is not finite is lost in its own
+    column of its head, from its token on and in the state, whichever form a step takes; of a key, a beta or a decay the whole head is."""
 
     runs_alone = True
     RUNS_MIN = ChannelDeltaMixer.RUNS_MIN
@@ -152,6 +154,7 @@ class HeadDeltaMixer(Mixer):
         self.channels = 2 * self.qk_size + self.inner                         # what the convolution sees: q | k | v
         self.kept_size = (self.taps - 1) * self.channels
         self.state_size = self.heads * self.vdim * self.dim
+        self.chunk_sizes = KR.takes(self.dim, self.vdim)
         self.b_off = self.channels
         self.a_off, self.g_off = self.b_off + self.heads, self.b_off + 2 * self.heads
         self.w_in = self.w_conv = self.dt_bias = self.a_log = self.w_norm = self.w_o = None
@@ -176,7 +179,7 @@ class HeadDeltaMixer(Mixer):
         self.w_o = store.get(p + "o")
 
     def kernels(self) -> List[str]:
-        return (["ssm"] + (["delta_chunks"] if KR.takes(self.dim, self.vdim) else [])
+        return (["ssm"] + (["delta_chunks"] if self.chunk_sizes else [])
                 + (["gemv"] if getattr(self, "run_dtype", None) == torch.bfloat16 else []) + self.product_kernels(self.hidden, self.inner))
 
     def state_need(self) -> StateNeed:
@@ -195,15 +198,25 @@ class HeadDeltaMixer(Mixer):
         """The fused input projection as part of a wider one."""
         self.w_in = w
 
-    def _in_chunks(self, ctx: StepContext) -> bool:
-        """Whether a step's runs go in chunks of 64 tokens as matrix products, or token by token: by the times of either on B200, us.  A walk is
-        as long as its longest run, or as all its tokens where its blocks (16 columns of a head's state) are more than the SMs; chunks
-        are a chain of a link per chunk, likewise, and work per chunk and head beside it.  Walk / chunks, 16 heads of 128: one run of
-        2,048 337 / 187, 1,000 and 1,048 together 257 / 192, 64 26 / 44; 8 heads: four runs of 300 82 / 81, one of 128 30 / 46; 4 heads: 512
-        88 / 57, 300 and 257 58 / 51."""
-        n, wide = KR.chunks_of(ctx.host_q_lens, ctx.n_tokens, ctx.n_seqs), self.heads * -(-self.vdim // 16) / 148
-        walk = 12 + 0.158 * max(ctx.max_q_len, 0.88 * ctx.n_tokens * wide)
-        return walk > 36 + 2.45 * max(-(-ctx.max_q_len // KR.CHUNK), n * wide) + 0.136 * n * self.heads
+    def _in_chunks(self, ctx: StepContext, sms: int = 0) -> bool:
+        """Whether a step's runs go in chunks of 64 tokens as matrix products, or token by token: by the times of either on B200 (sms:
+        multiprocessors, 0: the current device's).  A walk is as long as its longest run, or as all its tokens where its blocks (16 columns of a
+        head's state) are more than the SMs; chunks are a chain of a link per chunk, likewise, and work per chunk and head beside it.
+        Runs of less than 256 tokens and walks of less than 70 us (470 tokens with keys of 128, 560 of 64) stay walks: the layer is then as
+        long as its launches take, of which chunks have two more (16 heads of 64, 512 tokens, a pass among others 113 us, in chunks 132).  The
+        constants are a fit to 480 measured layers of 4 to 32 heads of 64 and 128.  Layer, walk /
+        chunks, us, 16 heads of 128: one run of 2,048 436 / 284, 512 128 / 111, 300 89 / 96, 1,000 and 1,048 together 356 / 289; of 64: 2,048
+        329 / 202, 700 128 / 90, 400 85 / 73; 4 heads of 64: 512 89 / 63; 8 heads of 128: four runs of 300 125 / 129, 512 beside 31 of one
+        token 179 / 196; 32 heads of 64: eight runs of 512 547 / 597."""
+        if ctx.max_q_len < 256 or not self.chunk_sizes:
+            return False
+        dk, dv, wide = self.dim / 128, self.vdim / 128, self.heads * -(-self.vdim // 16) / (sms or sm_count(torch.cuda.current_device()))
+        walk = (0.101 + 0.048 * dk) * max(ctx.max_q_len, 0.716 * ctx.n_tokens * wide)
+        if walk <= 70:
+            return False
+        n = KR.chunks_of(ctx.host_q_lens, ctx.n_tokens, ctx.n_seqs)
+        links = max(-(-ctx.max_q_len // KR.CHUNK), n * wide)
+        return walk > 20 + (1.37 + 0.98 * dk) * links + (0.072 + (0.037 + 0.043 * dk) * dv) * n * self.heads
 
     def forward(self, xn: torch.Tensor, ctx: StepContext, cache: LayerCache, projected: Optional[torch.Tensor] = None,
                 offset: int = 0) -> torch.Tensor:
@@ -224,7 +237,7 @@ class HeadDeltaMixer(Mixer):
         else:
             KS.conv_silu(proj, offset, self.w_conv, None, kept, qkv, ctx.seq_of_token, ctx.cu_seqlens, ctx.slots)
             y = torch.empty((T, self.inner), dtype=torch.float32, device=dev)
-            if KR.usable(dk, dv, qkv, 2 * self.qk_size) and self._in_chunks(ctx):
+            if self._in_chunks(ctx) and KR.usable(dk, dv, qkv, 2 * self.qk_size):
                 KR.delta_chunks(qkv, 0, self.qk_size, 2 * self.qk_size, proj, b, proj, a, self.dt_bias, self.a_log, S, y,
                                 KR.chunks_of(ctx.host_q_lens, T, ctx.n_seqs), H, G, dk, dv, UNIT_EPS, dk ** -0.5, ctx.cu_seqlens, ctx.slots,
                                 status=ctx.status)
