@@ -27,15 +27,12 @@ from ..kernels import ssm as KS
 from ..kernels.linear import linear
 from ..weights.loader import WeightSpec, WeightStore
 from .base import LayerCache, Mixer, StateNeed, StepContext, register_mixer
-from .chunks import MIN_CHUNK, cut_runs, cut_size
+from .chunks import MIN_CHUNK, cut_runs, cut_size, sm_count
 
 DENOMINATOR_FLOOR = 1e-6
 
 
 class MatrixMemoryMixer(Mixer):
-    # uncut runs take the matrix form from this length of the longest on (see `_in_chunks`)
-    CHUNKS_MIN = 640
-
     def __init__(self, prefix: str, hidden: int, heads: int, dim: int, vdim: int, gate_cap: float, eps: float):
         if heads < 1 or vdim < 1 or not 1 <= dim <= KS.MAX_STATE:
             raise ValueError(f"matrix memory '{prefix}': {heads} heads, keys of {dim} (1..{KS.MAX_STATE}), values of {vdim}")
@@ -83,16 +80,26 @@ class MatrixMemoryMixer(Mixer):
         """The fused input projection as part of a wider one."""
         self.w_in = w
 
-    def _in_chunks(self, ctx: StepContext, cuts: bool) -> bool:
-        """Whether a step's runs go in chunks of 64 tokens as matrix products, or token by token.  A chunk costs the same however
-        few tokens it holds (some 5 us a chunk of 16 heads of 128 x 129 on B200) and a walk as long as its longest run (0.3 us a
-        token of 128-element keys), so a step of one prompt and many sequences of one token is a walk.  Layer of 16 such heads, walk / chunks,
-        us: one run of 512 beside 31 of one token 175 / 259, beside 63 192 / 487; 2,048 beside 31 594 / 389, beside 63 615 / 622,
-        beside 127 651 / 1,071; 4,096 beside 63 1,174 / 776; 1,024 twice 320 / 182; 300 twice 103 / 113, four times 120 / 137
-        (there the launches count); 2,048 four times 675 / 687.  Where a walk would be cut (cuts), chunks were the faster form in every
-        step measured: one run of 130 183 / 115, of 2,048 287 / 185, of 8,192 1,022 / 718."""
-        return cuts or (ctx.max_q_len >= self.CHUNKS_MIN and 88 * ctx.max_q_len >=
-                        KR.chunks_of(ctx.host_q_lens, ctx.n_tokens, ctx.n_seqs) * self.heads * self.vdim)
+    def _in_chunks(self, ctx: StepContext, cuts: bool, sms: int = 0) -> bool:
+        """Whether a step's runs go in chunks of 64 tokens as matrix products, or token by token (sms: multiprocessors, 0: the device's).  A
+        chunk costs the same however few tokens it holds, a walk is as long as its longest run, or as all its tokens where they fill the GPU, so
+        a step of one prompt and many sequences of one token is a walk.  The constants are a fit to 335 measured layers of 4 to 32
+        heads of 64 and 128.  Layer, walk / chunks, us, 16 heads of 128 x 129: 512 eight times 390 / 334; 2,048 four times 739 / 666, beside 31 of
+        one token 617 / 384, beside 63 635 / 607, beside 127 680 / 1,215; 1,024 beside 31 329 / 293; 512 beside 31 187 / 256, beside 63 210 /
+        476; 300 four times 133 / 136, eight times 243 / 230; 64 eight times 70 / 105; 256 sixty-four times 1,413 / 1,581; of 64 x 65:
+        1,024 beside 31 208 / 118, 512 beside 31 112 / 105.  Runs of less than 512 tokens, which gain a tenth at most, and layers of some
+        100 us stay walks: those are as long as their launches take, of which chunks have more (300 four times, 8 heads of 128, 108 us
+        a pass among others walked, 129 in chunks).
+        Where a walk would be cut (cuts), chunks were the shorter form in every step measured but some of a single run of 8 heads or fewer (8
+        heads of 128, 128 tokens 52 / 60): one run of 200 71 / 67, of 2,048 306 / 174, of 4,096 565 / 350."""
+        if cuts or ctx.max_q_len < 512:
+            return cuts
+        dk, dv, wide = self.dim / 128, self.vdim / 128, self.heads * (self.vdim + 1) / (16 * (sms or sm_count(ctx.device)))
+        walk = (0.086 + 0.051 * dk) * max(ctx.max_q_len, 0.286 * ctx.n_tokens * wide)
+        if walk + 0.015 * ctx.n_tokens <= 100:
+            return False
+        n = KR.chunks_of(ctx.host_q_lens, ctx.n_tokens, ctx.n_seqs)
+        return walk > 15 + ((0.008 + 0.021 * (dk + dv) + 0.007 * dk * dv) * n + 0.156 * dk * dv * ctx.n_seqs) * self.heads
 
     def forward(self, xn: torch.Tensor, ctx: StepContext, cache: LayerCache, projected: Optional[torch.Tensor] = None,
                 offset: int = 0) -> torch.Tensor:
@@ -113,7 +120,7 @@ class MatrixMemoryMixer(Mixer):
             gates, m, y, dots = f32(T, H, 2), f32(T, H), f32(T, self.inner), f32(T, H)
             KS.memory_gates(proj, i, f, self.i_bias, self.f_bias, self.cap, tops, gates, m, H, ctx.cu_seqlens, ctx.slots)
             size = cut_size(ctx, H, dv + 1) if ctx.max_q_len >= 2 * MIN_CHUNK else None
-            in_chunks = self._in_chunks(ctx, size is not None) and KR.usable(dk, dv, proj, q, k, v)
+            in_chunks = KR.takes(dk, dv) and self._in_chunks(ctx, size is not None) and KR.usable(dk, dv, proj, q, k, v)
             if in_chunks:
                 KR.memory_chunks(proj, q, k, v, gates, S, y, dots, KR.chunks_of(ctx.host_q_lens, T, ctx.n_seqs), H, dk, dv, ctx.cu_seqlens, ctx.slots)
             scan = lambda st, out, nq, cu, slots: KS.memory_scan(proj, q, k, v, gates, st, out, nq, H, dk, dv, cu, slots)
