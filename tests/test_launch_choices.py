@@ -131,6 +131,22 @@ def test_when_a_delta_rule_goes_in_chunks():
     assert in_chunks([2048], 8, 128, 128, 74) and not in_chunks([2048], 16, 96, 128)          # sizes that the chunks are not built for
 
 
+def test_branches_with_a_walk_stay_on_one_stream(monkeypatch):
+    """A walk wants the GPU to itself, the delta rule in chunks does not."""
+    from types import SimpleNamespace
+
+    from turboquant_cpp_b200.parts import delta, make_mixer
+    monkeypatch.setattr(delta, "sm_count", lambda device: 148)
+    monkeypatch.setattr("torch.cuda.current_device", lambda: 0)
+    step = lambda lens: SimpleNamespace(max_q_len=max(lens), n_seqs=len(lens), n_tokens=sum(lens), host_q_lens=lens)
+    one = dict(prefix="", hidden=64, heads=16, kv_heads=16, taps=4, eps=1e-5)
+    chunked, walked = make_mixer("head_delta", dim=128, vdim=128, **one), make_mixer("head_delta", dim=96, vdim=128, **one)
+    channel = make_mixer("channel_delta", dim=128, vdim=128, **one)
+    memory = make_mixer("matrix_memory", prefix="", hidden=64, heads=16, dim=128, vdim=128, gate_cap=20.0, eps=1e-5)
+    assert not chunked.alone(step([2048])) and chunked.alone(step([300])) and walked.alone(step([2048]))
+    assert channel.alone(step([2048])) and not memory.alone(step([2048]))
+
+
 def test_expanded_latent_keys_take_a_bounded_scratch():
     """One prompt expands whatever its length (the scores of the other path take more); many prompts with long histories do not
     where their keys and values would take several times what that path takes."""

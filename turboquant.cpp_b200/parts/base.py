@@ -212,6 +212,10 @@ class PositionEncoding(Part):
 class Mixer(Part):
     runs_alone = False            # whether runs of many tokens go through a long kernel of few blocks that wants the GPU to itself
 
+    def alone(self, ctx: StepContext) -> bool:
+        """Whether this step's do."""
+        return self.runs_alone
+
     def cache_need(self) -> Optional[KVNeed]:
         return None
 

@@ -198,6 +198,9 @@ class HeadDeltaMixer(Mixer):
         """The fused input projection as part of a wider one."""
         self.w_in = w
 
+    def alone(self, ctx: StepContext) -> bool:
+        return self.runs_alone and not self._in_chunks(ctx)        # a walk is one long kernel of few blocks, chunks are several of many
+
     def _in_chunks(self, ctx: StepContext, sms: int = 0) -> bool:
         """Whether a step's runs go in chunks of 64 tokens as matrix products, or token by token: by the times of either on B200 (sms:
         multiprocessors, 0: the current device's).  A walk is as long as its longest run, or as all its tokens where its blocks (16 columns of a

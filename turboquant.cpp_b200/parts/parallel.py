@@ -25,7 +25,8 @@ class ParallelMixer(Mixer):
     # The branches run on two streams: neither waits for the other.  Prompts stay on one where launches, not the GPU, bound
     # the step (a smaller stream), and where a branch wants the GPU to itself.  Measured on B200, one stream / two: decoding
     # with a delta rule beside attention 0.588 / 0.566 ms (batch 8, width 2,048), with retention 0.692 / 0.674 ms; a prompt
-    # with retention 5.79 / 5.26 ms, with a delta rule 4.33 / 4.49 ms.
+    # with retention 5.79 / 5.26 ms, with a delta rule token by token 4.33 / 4.49 ms; the branches of a layer of width 2,048, delta rule in
+    # chunks beside attention, 1,600 tokens 361 / 305 us, 2,048 429 / 392, 8,192 1,737 / 1,705.
     SIDE_BY_SIDE = side.ENABLED
     SIDE_MIN_ELEMENTS = 3 << 20
 
@@ -85,8 +86,8 @@ class ParallelMixer(Mixer):
         if self.w_in is not None:
             proj = linear(xn, self.w_in, out_dtype=torch.float32, status=ctx.status)
             left_in, right_in = {"projected": proj}, {"projected": proj, "offset": self.left.input_weight().shape[0]}
-        runs_apart = xn.numel() >= self.SIDE_MIN_ELEMENTS and not (self.left.runs_alone or self.right.runs_alone)
-        if self.SIDE_BY_SIDE and (ctx.max_q_len == 1 or runs_apart):
+        if self.SIDE_BY_SIDE and (ctx.max_q_len == 1 or (xn.numel() >= self.SIDE_MIN_ELEMENTS
+                                                         and not (self.left.alone(ctx) or self.right.alone(ctx)))):
             other = side.fork(xn.device)
             with torch.cuda.stream(other):
                 b = self.right.forward(xn, ctx, cache, **right_in)
