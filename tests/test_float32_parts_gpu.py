@@ -18,9 +18,11 @@ def inputs(T, N, K, exact_weights, seed=0):
 
 
 def bound(x, w):
-    """What a result may be off by, of the sum of |x| |w|: products left out 2^-26 (2^-21 if the parts were cut, not rounded); the tensor cores cut bits off (2^-23 each) at 4
-    additions of 16 products and inside each, 8 in all; K / 64 + 1 rounded additions of 2^-24."""
-    return (x.double().abs() @ w.double().abs().t()) * (2.0 ** -21 + 8 * 2.0 ** -23 + (x.shape[1] / 64 + 1) * 2.0 ** -24)
+    """What a result may be off by, of the sum of |x| |w|: products left out 2^-26; the tensor cores cut bits off (2^-23 each) at 4
+    additions of 16 products and inside each, 8 in all, and at every product of the smaller ones (2^-8 of the sum, five a block of 16);
+    K / 64 + 1 rounded additions of 2^-24."""
+    K = x.shape[1]
+    return (x.double().abs() @ w.double().abs().t()) * (2.0 ** -26 + (8 + 5 * K / 16 * 2.0 ** -8) * 2.0 ** -23 + (K / 64 + 1) * 2.0 ** -24)
 
 
 @pytest.mark.parametrize("T,N,K,tokens", [(1, 1, 4, 0), (16, 256, 32, 0), (17, 257, 36, 16), (31, 255, 60, 32), (128, 128, 64, 0), (129, 300, 100, 96),
@@ -80,6 +82,8 @@ CASES = [  # H, G, head size, page, runs, held, window
     (4, 1, 64, 48, [200, 20], [13, 0], 70),              # a tile of keys lies in two pages
     (2, 2, 128, 16, [129, 65], [0, 500], 33),
     (16, 16, 128, 64, [700], [0], 0),
+    (4, 2, 128, 64, [1, 1, 200, 1, 1], [300, 5, 0, 64, 1000], 0),                # a prompt beside sequences that bring one token
+    (8, 2, 64, 64, [1] * 9 + [70], [40 * i + 1 for i in range(9)] + [3], 50),
 ]
 
 
@@ -108,22 +112,42 @@ def test_attention_f32(case, spread):
     out = torch.full((T, H * hd), math.nan, device=DEV)
     run = lambda: KA.attention_tiled(q, cache, i32(cu), i32(held), i32(table), page, window, hd ** -0.5, out, len(runs), H, G, hd)
     run()
-    for i in range(len(runs)):
-        mine = slice(cu[i], cu[i + 1])
-        want, mag = attend(q[mine].double(), rows[i][0].double(), rows[i][1].double(), held[i], hd ** -0.5, window, 0, 0, 0.0, None, None)
-        # a score is off by about its products' 2^-21 and its sums' 2^-20, of the size of |q| |k| / sqrt(hd); so is a weight, relatively
-        size = q[mine].double().norm(dim=2).max() * rows[i][0].double().norm(dim=2).max() * hd ** -0.5
-        assert bool(((out[mine].view(-1, H, hd).double() - want).abs() <= mag * (2.0 ** -20 * size + 2.0 ** -18)).all())
-    # a key of -inf has no weight; a value of inf shows in the rows that see it, a NaN too, and in no others
-    first = int(table[0, 0])
-    cache[first, 0, 0, 0] = 0.0
-    cache[first, 0, 0, 0, 1] = -math.inf
-    q[..., 1] = q[..., 1].abs() + 0.1
+    tf32, torch.backends.cuda.matmul.allow_tf32 = torch.backends.cuda.matmul.allow_tf32, False
+
+    def compare(first_row=0):
+        """The whole step's error beside that of the same formulas in float32: a part of the operands or a product left out is ten times it."""
+        ours = theirs = size = 0.0
+        for i in range(len(runs)):
+            skip = first_row if i == 0 else 0
+            mine = slice(cu[i] + skip, cu[i + 1])
+            args = (held[i] + skip, hd ** -0.5, window, 0, 0, 0.0, None, None)
+            want, _ = attend(q[mine].double(), rows[i][0].double(), rows[i][1].double(), *args)
+            single, _ = attend(q[mine], rows[i][0], rows[i][1], *args)
+            got = out[mine].view(-1, H, hd).double()
+            ours, theirs, size = ours + (got - want).square().sum(), theirs + (single.double() - want).square().sum(), size + want.square().sum()
+        assert float(ours) ** 0.5 <= 2 * float(theirs) ** 0.5 + 2.0 ** -25 * float(size) ** 0.5, (float(ours / size) ** 0.5, float(theirs / size) ** 0.5)
+
+    try:
+        compare()
+        # a key of -inf has no weight (the row that sees no other key has no result)
+        first, alone = int(table[0, 0]), 1 if held[0] == 0 else 0
+        cache[first, 0, 0, 0, 1] = -math.inf
+        rows[0][0][0, 0, 1] = -math.inf
+        q[..., 1] = q[..., 1].abs() + 0.1
+        run()
+        compare(alone)
+        assert bool(out[alone:].isfinite().all())
+    finally:
+        torch.backends.cuda.matmul.allow_tf32 = tf32
+    # a value of inf shows in the rows that see it, and in no others
+    was, key = out.clone(), 1 if len(runs) == 1 else 0           # not the key that has no weight
+    cache[int(table[-1, 0]), 1, 0, key, 0] = math.inf
     run()
-    assert bool(out[cu[0] + 1:cu[1]].isfinite().all()) if held[0] == 0 else True
-    cache[int(table[-1, 0]), 1, 0, 0, 0] = math.inf
-    run()
-    sees = (torch.arange(runs[-1], device=DEV) + held[-1] < window) if window else torch.ones(runs[-1], dtype=torch.bool, device=DEV)
-    got = out[cu[-2]:].view(-1, H, hd)[:, :H // G, 0]
-    if len(runs) > 1:
-        assert bool(((got == math.inf) == sees[:, None]).all()) and bool(out[:cu[1]].isfinite().logical_not().sum() <= H * hd)
+    pos = torch.arange(runs[-1], device=DEV) + held[-1]
+    sees = (pos >= key) & (pos - key < window if window else pos >= 0)
+    met = torch.zeros((T, H, hd), dtype=torch.bool, device=DEV)
+    met[cu[-2]:, :H // G, 0] = sees[:, None]
+    got, rest = out.view(T, H, hd), ~met
+    rest[:alone] = False
+    assert bool((got[met] == math.inf).all())
+    torch.testing.assert_close(got[rest], was.view(T, H, hd)[rest], rtol=1e-5, atol=1e-5)      # rows that met it are summed again, key by key
