@@ -6,7 +6,8 @@
 //   (1 + B) U = diag(beta) (V - diag(A) K S),   B[t][s] = beta_t D[t][s] k_t . k_s for s < t,
 // so with T = (1 + B)^-1
 //   U = T diag(beta) (V - diag(A) K S);   S' = A_last S + K^T diag(D[last]) U;   o = diag(A) Q S + (D o Q K^T) U.
-// A chain of one link per chunk instead of one per token.  Three launches:
+// A chain of one link per chunk instead of one per token.  (The chunkwise form of Yang, Wang, Zhang, Shen and Kim, "Parallelizing
+// linear transformers with the delta rule over sequence length", 2024, with decays.)  Three launches:
 //   delta_solve    T of every chunk, side by side: by blocks of 16, the diagonal ones by forward substitution, the others from them, in
 //                  float32 on the CUDA cores.  Leaves T and K in parts, as the next launches' shared memory holds them
 //   delta_chain    the chunks in order; a CTA has 16 columns of a head's state, in registers.  Three products a link, 64 x 128 x 16,

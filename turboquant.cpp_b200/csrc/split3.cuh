@@ -1,4 +1,5 @@
-// float32 as the exact sum of three bfloat16 values, for float32 products on the tensor cores.
+// float32 as the exact sum of three bfloat16 values, for float32 products on the tensor cores (the scheme of Henry, Tang and Heinecke,
+// "Leveraging the bfloat16 artificial intelligence datatype for higher-precision computations", 2019).
 //
 // x = h + m + l: h is x rounded to bfloat16, m what is left rounded, l the rest, which bfloat16 holds exactly (24 bits are 8 and two
 // times 8 with a sign; below 2^-110 the last bits of l go).  Of the nine products of two such sums the six largest are taken, h h', h m',

@@ -203,7 +203,7 @@ def group_heads(dtype: torch.dtype, dk: int, dv: int, per_kv: int) -> int:
 
 def heads_form(dtype: torch.dtype, dk: int, dv: int, per_kv: int, page_size: int) -> bool:
     """Whether steps of single tokens take the tensor-core token form (up to sixteen heads of a key/value head are the
-    rows of a tile): bfloat16, sizes of 32, 64 or 128, pages that are multiples of 16, and at least HEADS_FORM_MIN
+    columns of a product, its keys the rows): bfloat16, sizes of 32, 64 or 128, pages that are multiples of 16, and at least HEADS_FORM_MIN
     query heads per key/value head (TQ_BIAS_TOKEN_FORM=group|heads forces one)."""
     import os
     if dtype != torch.bfloat16 or dk not in RUN_SIZES or dv not in RUN_SIZES or page_size % 16:

@@ -17,7 +17,7 @@ _LIB = "ssm"
 CHUNK = 64               # csrc/chunks.cuh L
 SIZES = (64, 128)        # key and value sizes the kernels are built for
 # the most bytes of chunks' states a step holds at a time, 126 chunks of 16 heads of 128 x 129; longer steps go in groups of equal size
-# (8,192 tokens of that layer: 718 us in one piece of 135 MB, 746 in groups of 63, 63 and 2)
+# (4,096 tokens of 32 such heads, a matrix memory's layer: 665 us in two groups)
 SCRATCH_BYTES = 128 << 20
 
 

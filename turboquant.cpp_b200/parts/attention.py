@@ -124,8 +124,8 @@ class AttentionMixer(Mixer):
                                  self.window, self.scale, o, ctx.n_seqs, ctx.max_q_len, self.n_heads, self.n_kv_heads,
                                  self.head_dim, status=ctx.status)
         elif ctx.max_q_len >= self.PREFILL_MIN_RUN and self.head_dim % 4 == 0:
-            # long runs where the tensor-core kernel does not apply (float32, other head sizes): exact fp32 on CUDA
-            # cores, 32 queries sharing each tile of keys
+            # long runs where the bfloat16 prompt kernel does not apply: float32 heads of 64 and 128 on the tensor cores in three
+            # bfloat16 parts, 64 queries sharing each tile of keys; other head sizes on the fp32 units, 32 queries
             KA.attention_tiled(q, cache.kv, ctx.cu_seqlens, ctx.seq_start, cache.page_table, cache.page_size,
                                self.window, self.scale, o, ctx.n_seqs, self.n_heads, self.n_kv_heads, self.head_dim)
         elif KA.split_usable(self.n_heads, self.n_kv_heads, self.head_dim, cache.page_size):

@@ -282,8 +282,10 @@ class MoEFeedForward(FeedForward):
         # A2.7B sizes batch 8: 2,214 / 2,287, batch 16: 3,228 / 3,147; 57B-A14B sizes batch 1: 177 / 190, batch 8: 602 / 586.)
         shared_after = small and (T * k >= self.n_experts if self.SHARED_AFTER_ROUTER is None else self.SHARED_AFTER_ROUTER)
         # Long prompts, whose products fill the GPU one CTA an SM on either stream: launched early, a product's waiting CTAs would hold SMs that the
-        # other stream's kernels still need.  (2,048 tokens, 60 experts of 1,408 and a shared one of 5,632: 421 us with early launches, 403
-        # without; with early launches of some of the products only 414 to 422.)
+        # other stream's kernels still need.  (2,048 tokens that had not been run before, 60 experts of 1,408 and a shared one of 5,632: layer
+        # after layer 382 us with early launches, 350 without; a single layer behind an idle GPU 357 and 370.  A prompt of eight layers
+        # of the model 4.81 ms and 4.57, of 4,096 tokens 8.19 and 7.78, of 1,500 and less the same.  Early launches of some of the products
+        # only: no better than all of them.)
         apart = self.ws13 is not None and not dual and tile >= KT.PAIR_MIN_TILE
 
         def select(logits):
