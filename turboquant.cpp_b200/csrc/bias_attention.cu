@@ -1424,11 +1424,10 @@ __device__ __forceinline__ uint32_t bh_turn(uint32_t x) {      // an 8 x 8 tile 
     asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
     return y;
 }
-// What the upper 16 bits of a weight leave, which is not negative; more than zero where the weight is, so that an infinite value
-// times both parts is that infinity and not a NaN (2^-126 of a value is nothing beside a sum of weights of one or more).
+// What the upper 16 bits of a weight leave, which is not negative; 2^-30 of the weight more, so that it is not zero beside a weight either: an
+// infinite value times both parts is that infinity and not a NaN.
 __device__ __forceinline__ float bh_rest(float w) {
-    const float upper = __uint_as_float(__float_as_uint(w) & 0xffff0000u), left = w - upper;
-    return upper > 0.f ? fmaxf(left, 1.17549435e-38f) : left;
+    return fmaf(w, 9.31322575e-10f, w - __uint_as_float(__float_as_uint(w) & 0xffff0000u));
 }
 template <int DK, int DV, int NT>
 __global__ void __launch_bounds__(BA_WARPS * 32, 3)
