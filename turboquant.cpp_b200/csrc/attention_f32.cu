@@ -3,10 +3,10 @@
 //
 // The reference's prompt attention is float32 (src/engine/tq_transformer.c:1909-2191).  On the fp32 units 64 x 64 scores and their part of
 // the outputs are 1 M multiply-adds, 8,192 cycles of an SM before a single operand is read from shared memory (the kernel for
-// other head sizes, csrc/attention.cu, takes 4.6 times that); as six bfloat16 products they are 6,600 of mma.sync (960 multiply-adds a
+// other head sizes, csrc/attention.cu, takes 4.6 times that); as six bfloat16 products they are 6,200 of mma.sync (1,019 multiply-adds a
 // cycle and SM measured), whose operands a warp reads once for 16 rows.
 // 16 heads of 128, one prompt: 82 us for 700 tokens (287 before), 19 for 100 (47), 420 for 2,048 (1,662); errors against 64 bits
-// 1.5e-7 (3.6e-7), queries of spread 5 3.1e-7 (1.05e-6).  What bounds it: the tensor cores are active 49 % of the time, the rest is a warp's
+// 1.5e-7 (3.6e-7), queries of spread 5 3.1e-7 (1.05e-6).  What bounds it: the tensor cores are active 39 % of the time, the rest is a warp's
 // own chain of splitting, products and exponentials, two warps a scheduler (their sums take 255 registers).
 //   A CTA takes 64 consecutive new tokens of one sequence and one query head, a warp of either half of it 16 of them.  Queries, scaled,
 //   lie in shared memory in three parts.  The halves take every other 32 keys each, with sums of their own that are put together

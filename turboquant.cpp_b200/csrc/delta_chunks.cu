@@ -15,7 +15,7 @@
 //   delta_outputs  the outputs of every chunk, side by side
 // 2,048 tokens, 16 heads of 128: 187 us with delta_prepare (12), the solving 40, the chain 80 and the outputs 54; token by token 337.
 // Errors against 64 bits are those of the walk: outputs 1.8e-7 to 2.1e-7, states 1.6e-7 to 1.9e-7 (walk 1.8e-7 to 2.1e-7, 1.6e-7 to 1.9e-7).
-// A link is 2.4 us: products 1.1 (960 multiply-adds a cycle and SM), the rest their way through shared memory and 72 KB of K and T.
+// A link is 2.4 us: products 1.0 (1,019 multiply-adds a cycle and SM), the rest their way through shared memory and 72 KB of K and T.
 // Chains that were longer: W = T diag(beta A) K in the place of K S, a product less but 96 KB, 2.1 us and a third more work beside the chain;
 // the same with keys brought in float32 and split by four more warps 2.9.
 // A long step does this for a group of chunks after the other, the kept state going from group to group.

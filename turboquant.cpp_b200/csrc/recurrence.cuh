@@ -11,9 +11,9 @@
 // a walk does 2 multiply-adds an element of the state and token, a chain of its tokens with a shuffle tree each, and long runs are
 // walked twice to fill the GPU; in chunks it is 2 + 64 (1 / dk + 1 / dv) of them, all in products.
 // Everything is kept and added up in float32; products are six bfloat16 ones whose largest are summed over at most 64 elements.
-// 682 + 1,366 tokens, 16 heads of 128 x 129: 33 us for the chunks' sums, 17 for the starts and 54 for the outputs (as products on the
+// 682 + 1,366 tokens, 16 heads of 128 x 129: 33 us for the chunks' sums, 17 for the starts and 56 for the outputs (as products on the
 // fp32 units 37, 16 and 79, bound by what they read of shared memory; token by token 289).  With one CTA an SM the outputs take 89; what bounds
-// either kernel with two is a warp's own chain of loads, splitting and products, the tensor cores are active 32 to 40 % of the time.
+// either kernel with two is a warp's own chain of loads, splitting and products, the tensor cores are active 41 to 42 % of the time.
 // An element of a value that is not finite takes no part in earlier tokens' outputs; the token's own and all later ones are NaN in its
 // column, and in no other.
 // Part of csrc/ssm.cu's library.

@@ -17,7 +17,7 @@ _LIB = "ssm"
 CHUNK = 64               # csrc/chunks.cuh L
 SIZES = (64, 128)        # key and value sizes the kernels are built for
 # the most bytes of chunks' states a step holds at a time, 126 chunks of 16 heads of 128 x 129; longer steps go in groups of equal size
-# (4,096 tokens of 32 such heads, a matrix memory's layer: 665 us in two groups)
+# (8,192 tokens of that layer: 780 us in one piece, 788 in two groups; of the delta rule, whose chunks take 130 KB a head, 1,102 and 1,163)
 SCRATCH_BYTES = 128 << 20
 
 
