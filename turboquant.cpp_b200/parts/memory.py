@@ -13,7 +13,8 @@ m only keeps the exponentials in range: with S e^m and n e^m the recurrence is l
 is one float32 row: S column by column with n as one more column (the value of which is one), [H, dv + 1, dk], and m [H].
 The fused input projection [q | k | v | z | i | f] leaves the library's product as float32; everything behind it is
 float32 up to the gated norm's output.  Long runs go in chunks of 64 tokens as matrix products (`kernels.recurrence`, keys and values
-of 64 or 128), others token by token, cut into chunks where that fills the GPU (`chunks.cut_runs`).
+of 64 or 128), others token by token, cut into chunks where that fills the GPU (`chunks.cut_runs`).  In every form an element of a
+value that is not finite is lost in its own column of S, from its token on (in chunks as a NaN, whatever it was).
 """
 from __future__ import annotations
 
